@@ -18,6 +18,11 @@ FILES = ["utils/__init__.py", "utils/quant_utils.py", "utils/hadamard_utils.py",
          "dirotq_fused_unrotation_fast.py", "speedup/weight_only_nvfp4.py"]
 
 
+def present(ref_root: str) -> bool:
+    """Whether `ref_root` holds a checkout (an empty folder is none)."""
+    return all(os.path.exists(os.path.join(ref_root, rel)) for rel in FILES if not rel.endswith("__init__.py"))
+
+
 def make(ref_root: str) -> str:
     for rel in FILES:
         src = os.path.join(ref_root, rel)
