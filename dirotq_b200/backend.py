@@ -57,8 +57,9 @@ class SharedActivation:
 
     @staticmethod
     def _key(x: torch.Tensor):
-        stream = torch.cuda.current_stream(x.device).cuda_stream if x.is_cuda else 0
-        return (x.data_ptr(), x._version, tuple(x.shape), tuple(x.stride()), x.dtype, x.device.index, stream)
+        idx = x.device.index
+        stream = torch._C._cuda_getCurrentRawStream(idx) if x.is_cuda else 0
+        return (x.data_ptr(), x._version, x.shape, x.stride(), x.dtype, idx, stream)
 
     def lookup(self, x: torch.Tensor, member_id: int) -> bool:
         """True if the workspace already holds this tensor's codes and `member_id` has not used them yet."""
@@ -225,61 +226,39 @@ def linear_forward(st: LayerState, x2d: torch.Tensor, out: Optional[torch.Tensor
     elif CACHE_WEIGHT_PANEL == "auto" and st.folded is not None and st.folded.panel is None and M > PANEL_CACHE_MAX_ROWS:
         st.panel_declined = True        # over the budget: asked once, not on every call
     ws = st.workspace(M, x2d.device)
-    watch = ops.status_watch(x2d.device) if WATCH_STATUS else None
-    if watch is not None:
+    watch = ops.status_watch(x2d.device)
+    if WATCH_STATUS:
         watch.poll()                    # a wait that ran out in an earlier call surfaces here (no synchronisation)
-    status = C.c_void_p(ops.status_word(x2d.device).data_ptr())
-    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    lib = _lib.lib()
+    lin, yp, wsp, wsn, status, stream = C.byref(st.c_struct()), y.data_ptr(), ws.data_ptr(), ws.numel(), watch.ptr, ops.stream_ptr()
     if st.handed is not None:
         hit = st.handed_key == SharedActivation._key(x2d)
         st.handed, st.handed_key = None, None
         if hit:
             # the producer's epilogue left this tensor's codes, scales and 16-bit channels in the workspace
             st.chain_hits += 1
-            check(_lib.lib().dirotq_linear_gemm_prequantised(C.byref(st.c_struct()), M, C.c_void_p(y.data_ptr()),
-                                                             C.c_void_p(ws.data_ptr()), ws.numel(), status, stream),
-                  "dirotq_linear_gemm_prequantised")
+            check(lib.dirotq_linear_gemm_prequantised(lin, M, yp, wsp, wsn, status, stream), "dirotq_linear_gemm_prequantised")
             if out is not None:
                 ops.mark_written(out)
-            if watch is not None:
-                watch.post()
             return y
     nxt = st.chain_next
     if nxt is not None and st.shared is None and not nxt.hadamard_low_dim:
         nws = nxt.workspace(M, x2d.device)
-        yp = C.c_void_p(y.data_ptr() if st.chain_keep_output else 0)
-        check(_lib.lib().dirotq_linear_forward_chain(C.byref(st.c_struct()), C.c_void_p(x2d.data_ptr()), M, yp,
-                                                     C.c_void_p(ws.data_ptr()), ws.numel(), C.byref(nxt.c_struct()),
-                                                     C.c_void_p(nws.data_ptr()), nws.numel(), status, stream),
+        check(lib.dirotq_linear_forward_chain(lin, x2d.data_ptr(), M, yp if st.chain_keep_output else None, wsp, wsn,
+                                              C.byref(nxt.c_struct()), nws.data_ptr(), nws.numel(), status, stream),
               "dirotq_linear_forward_chain")
         if out is not None:
             ops.mark_written(out)
         nxt.handed, nxt.handed_key = y, SharedActivation._key(y)
-        if watch is not None:
-            watch.post()
         return y
-    if st.shared is not None:
-        if st.shared.lookup(x2d, st.member_id):
-            check(_lib.lib().dirotq_linear_gemm(C.byref(st.c_struct()), M, C.c_void_p(y.data_ptr()),
-                                                C.c_void_p(ws.data_ptr()), ws.numel(),
-                                                C.c_void_p(ops.status_word(x2d.device).data_ptr()),
-                                                C.c_void_p(torch.cuda.current_stream().cuda_stream)),
-                  "dirotq_linear_gemm")
-            if out is not None:
-                ops.mark_written(out)
-            if watch is not None:
-                watch.post()
-            return y
-        st.shared.store(x2d, st.member_id)
-    check(_lib.lib().dirotq_linear_forward(C.byref(st.c_struct()), C.c_void_p(x2d.data_ptr()), M,
-                                           C.c_void_p(y.data_ptr()), C.c_void_p(ws.data_ptr()), ws.numel(),
-                                           C.c_void_p(ops.status_word(x2d.device).data_ptr()),
-                                           C.c_void_p(torch.cuda.current_stream().cuda_stream)),
-          "dirotq_linear_forward")
+    if st.shared is not None and st.shared.lookup(x2d, st.member_id):
+        check(lib.dirotq_linear_gemm(lin, M, yp, wsp, wsn, status, stream), "dirotq_linear_gemm")
+    else:
+        if st.shared is not None:
+            st.shared.store(x2d, st.member_id)
+        check(lib.dirotq_linear_forward(lin, x2d.data_ptr(), M, yp, wsp, wsn, status, stream), "dirotq_linear_forward")
     if out is not None:
         ops.mark_written(out)
-    if watch is not None:
-        watch.post()
     return y
 
 
@@ -600,7 +579,7 @@ def prepare_w4a16(w, device="cuda", explicit: Optional[dict] = None, group: int 
 
 def _fused_forward_b200(self, x):
     """ActQuantWrapper.forward on the B200 kernels (contract: dirotq_fused_unrotation_fast.py:56-141)."""
-    if self.quantizer.bits >= 16:
+    if self._modules["quantizer"].bits >= 16:
         s16 = getattr(self, "_b200_w4a16", None)
         if s16 is None and getattr(self, "_b200_explicit", None) is not None:
             s16 = prepare_w4a16(self, x.device, self._b200_explicit)     # synthetic layer: no dense weight
@@ -609,8 +588,8 @@ def _fused_forward_b200(self, x):
             return self.module(x).to(x.dtype)
         shp = x.shape
         x2d = x.reshape(-1, shp[-1]).to(torch.bfloat16).contiguous()
-        y = w4a16_forward(s16, x2d)
-        return y.reshape(*shp[:-1], s16.w.N).to(x.dtype)
+        y = w4a16_forward(s16, x2d).view(*shp[:-1], s16.w.N)
+        return y if x.dtype is torch.bfloat16 else y.to(x.dtype)
     st = getattr(self, "_b200_state", None)
     if st is None:
         st = prepare_layer(self, x.device, getattr(self, "_b200_explicit", None))
@@ -620,8 +599,8 @@ def _fused_forward_b200(self, x):
     x2d = x.reshape(-1, shp[-1])
     if x2d.dtype != torch.bfloat16:
         x2d = x2d.to(torch.bfloat16)     # the kernels compute in bf16 (fp16 pipelines are converted here)
-    y = linear_forward(st, x2d.contiguous())
-    return y.reshape(*shp[:-1], st.out_features).to(x_dtype)
+    y = linear_forward(st, x2d.contiguous()).view(*shp[:-1], st.out_features)
+    return y if x_dtype is torch.bfloat16 else y.to(x_dtype)
 
 
 # Sibling layers with equal rotation and format (to_q / to_k / to_v) rotate and quantise their common
