@@ -489,6 +489,19 @@ def test_hadamard_front_end_model_sizes(D, low_dim):
     assert torch.equal(y2.view(torch.int16), O.hadamard_low(x, low_dim, None, fp32=False).view(torch.int16))
 
 
+@pytest.mark.parametrize("low_dim", [16, 32, 64, 128, 256, 1024])
+def test_hadamard_front_end_short_transforms(low_dim):
+    """Transforms that share a block with other rows, at row counts that leave the last block partly empty: every pass
+    split of the kernel (one pass, two, three; a last pass of one to three stages), bit-identical to the oracle."""
+    from dirotq_b200 import ops
+    g = torch.Generator().manual_seed(low_dim)
+    flips = (torch.randint(0, 2, (low_dim,), generator=g).float() * 2 - 1).to(torch.bfloat16)
+    for M in (1, 2, 257):
+        x = torch.randn(M, low_dim + 8, generator=g).to(torch.bfloat16)
+        y = ops.hadamard_low(x.cuda(), low_dim, flips.cuda()).cpu()
+        assert torch.equal(y.view(torch.int16), O.hadamard_low(x, low_dim, flips, fp32=False).view(torch.int16)), M
+
+
 @pytest.mark.parametrize("quant", ["int4", "int8", "nvfp4"])
 def test_gelu_fused_into_the_gemm_epilogue(quant):
     """ff.net.0 = GELU(proj(x)): with the activation fused into the up-projection's epilogue the module returns
