@@ -38,15 +38,23 @@
 //                  (tcgen05.st); for a tail stage it copies the bf16 rows from the raw ring instead
 //   UMMA issuer    tcgen05.mma kind::f16 (A from TMEM, B from smem descriptor), 4 x K=16 per chunk, fp32
 //                  128 x BN accumulator in TMEM; the bf16 tail accumulates into the same tile
-//   8 epilogue warps  tcgen05.ld, * rs[m] * cs[n], + bias, bf16 -> 32 x 32 staging patches -> TMA stores; two
-//                  accumulators alternate so the next tile's UMMAs overlap the epilogue
+//   8 epilogue warps  tcgen05.ld, * rs[m] * cs[n], + bias, bf16 in registers, accumulator handed back, then 32 x 32 staging
+//                  patches -> TMA stores.  128-wide tiles have two accumulators, 256-wide tiles one (the columns it leaves
+//                  hold eight stages of activations)
+// PAIR (256-wide tiles of long launches): clusters of two CTAs drive one tcgen05.mma.cta_group::2 on a 256 x 256 tile.  Each
+// CTA converts its own 128 rows into its own tensor memory, fetches half of the weight tile (the tensor core reads the other
+// half from the peer's shared memory) and runs the epilogue of its 128 rows.  One barrier per stage in the leader counts the
+// weight bytes of both CTAs and one arrival per converter warp of both (from the peer without memory ordering: their payload
+// is tensor memory); commits arrive in both CTAs; accumulator-empty in the leader counts the epilogue warps of both.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <atomic>
 #include "layout.cuh"
 #include "launchers.cuh"
 #include "ptx.cuh"
+#include "ptx_pair.cuh"
 #include "tma_host.cuh"
 #include "quant_math.cuh"
 
@@ -69,28 +77,38 @@ constexpr int GF_EPI_WARPS = 8;
 
 // A chunk of a 128-row tile is four conversion units of 32 rows (a thread per row = TMEM lane); a group is
 // the four warps that cover the four lane quarters.
-template <int BN, bool A8 = false> struct GfCfg {
+template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
   static constexpr int GROUP_WARPS = 4;
   static constexpr int GROUPS = GF_GROUPS;
   static constexpr int CONV_WARPS = GROUPS * GROUP_WARPS;
-  static constexpr int THREADS = (GF_EPI_WARPS + 3 + CONV_WARPS) * 32;
-  static constexpr int B_EXP = BN * 128;                   // BN rows x 64 halves
+  // Warpgroups: epilogue (warps 0..7), issuer and the two producers (8..11, the last one idle), converters (12..19).  The
+  // launch gives every thread 96 registers; the producers' and converters' groups hand some back to the epilogue's, which
+  // holds a quarter row of the tile (64 registers of bf16 pairs) besides the piece in work and the one being fetched.
+  static constexpr int THREADS = (GF_EPI_WARPS + 4 + CONV_WARPS) * 32;
+  static constexpr int REGS_LAUNCH = 96, REGS_EPI = 136, REGS_PROD = 48, REGS_CONV = 80;
+  static_assert(GF_EPI_WARPS * REGS_EPI + 4 * REGS_PROD + CONV_WARPS * REGS_CONV <= THREADS / 32 * REGS_LAUNCH,
+                "setmaxnreg draws on the registers of the launch");
+  static constexpr int BN_OWN = PAIR ? BN / 2 : BN;         // weight rows this CTA fetches
+  static constexpr int B_EXP = BN_OWN * 128;               // BN_OWN rows x 64 halves
   static constexpr int EXP_STAGE = B_EXP;                  // only the weight operand is staged in shared memory
   static constexpr int RAW_A = 128 * 32 * GF_CPS * (A8 ? 2 : 1);   // 8-bit activation codes: two 128-byte boxes per row
   static constexpr int OFF_C = RAW_A;                      // [chunk][128] 8-byte records
   static constexpr int RAW_STAGE = OFF_C + GF_CPS * 128 * 8;
-  // Accumulators: two (the next tile's UMMAs overlap the epilogue) up to 192 columns; a 256-wide tile has one, and its
+  // Accumulators: two of 128 columns (the next tile's UMMAs overlap the epilogue); a 256-wide tile has one, and its
   // UMMAs wait until the epilogue has read the previous tile out of tensor memory.
-  static constexpr int NACC = BN > 192 ? 1 : 2;
+  static constexpr int NACC = BN == 256 ? 1 : 2;
   // Operand stages in flight: every tensor-memory column the accumulators leave free holds activations
   // (32 columns per 64-wide chunk), as far as shared memory holds the weight tiles beside them.
   static constexpr int RAW_STAGES = GF_RAW_DEF;
   static constexpr int STG_BYTES = GF_EPI_WARPS * 2048;     // per epilogue warp: 32 rows x 32 bf16 output staging
+  static constexpr int PIECES = BN / 32;                    // 16-column pieces of an epilogue warp
+  static constexpr int TAB_WARP = PIECES * 8 * 8;           // per epilogue warp: {cs pair, bias pair} in bf16 per column pair
+  static constexpr int TAB_BYTES = GF_EPI_WARPS * TAB_WARP;
   static constexpr int EXP_TMEM = (512 - NACC * BN) / 32;
-  static constexpr int EXP_SMEM = (232448 - 1024 - 256 - STG_BYTES - RAW_STAGES * RAW_STAGE) / EXP_STAGE;
+  static constexpr int EXP_SMEM = (232448 - 1024 - 256 - STG_BYTES - TAB_BYTES - RAW_STAGES * RAW_STAGE) / EXP_STAGE;
   static constexpr int EXP_CAP = EXP_TMEM < GF_EXP_MAX ? EXP_TMEM : GF_EXP_MAX;
   static constexpr int EXP_STAGES = EXP_CAP < EXP_SMEM ? EXP_CAP : EXP_SMEM;
-  static constexpr int SMEM_BYTES = EXP_STAGES * EXP_STAGE + RAW_STAGES * RAW_STAGE + STG_BYTES + 1024 + 256;
+  static constexpr int SMEM_BYTES = EXP_STAGES * EXP_STAGE + RAW_STAGES * RAW_STAGE + STG_BYTES + TAB_BYTES + 1024 + 256;
   static constexpr int TMEM_A0 = NACC * BN;                 // first column of the activation operand slots
   static constexpr int TMEM_COLS = 512;                     // accumulators + EXP_STAGES x 32 columns of A
   static_assert(NACC * BN + EXP_STAGES * 32 <= 512 && EXP_STAGES >= 2, "tensor memory");
@@ -110,6 +128,9 @@ template <int N> struct GfRing {
 
 __device__ __forceinline__ void gf_sts128(uint32_t addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void gf_sts64(uint32_t addr, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(addr), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ uint2 gf_lds64(uint32_t addr) {
   uint2 v;
@@ -149,23 +170,43 @@ __device__ __forceinline__ uint32_t hmul2_2m4(uint32_t m) {
   return r;
 }
 
+// bf16 pair of { v0 * rs * cs0 + b0, v1 * rs * cs1 + b1 } from bf16 pairs cs and b; rs and cs are powers of two, so only the
+// sum and the conversion round
+__device__ __forceinline__ uint32_t scale_pair(uint32_t v0, uint32_t v1, float rs, uint32_t cs, uint32_t b) {
+  uint32_t r;
+  asm("{\n\t.reg .b64 v, s, c, b;\n\t.reg .b32 lo, hi, c0, c1, b0, b1;\n\t"
+      "shl.b32 c0, %4, 16;\n\tand.b32 c1, %4, 0xffff0000;\n\t"
+      "shl.b32 b0, %5, 16;\n\tand.b32 b1, %5, 0xffff0000;\n\t"
+      "mov.b64 v, {%1, %2};\n\tmov.b64 s, {%3, %3};\n\tmov.b64 c, {c0, c1};\n\tmov.b64 b, {b0, b1};\n\t"
+      "mul.rn.f32x2 c, c, s;\n\t"
+      "fma.rn.f32x2 v, v, c, b;\n\t"
+      "mov.b64 {lo, hi}, v;\n\t"
+      "cvt.rn.bf16x2.f32 %0, hi, lo;\n\t}"
+      : "=r"(r)
+      : "r"(v0), "r"(v1), "r"(__float_as_uint(rs)), "r"(cs), "r"(b));
+  return r;
+}
+
 // AMODE: 0 = signed 4-bit activation codes, 1 = unsigned 4-bit with zero points, 2 = unsigned 8-bit with zero points
-template <int BN, int AMODE>
-__global__ void __launch_bounds__(GfCfg<BN, AMODE == 2>::THREADS, 1)
+// PAIR: see the head of this file
+template <int BN, int AMODE, bool PAIR>
+__global__ void __launch_bounds__(GfCfg<BN, AMODE == 2, PAIR>::THREADS, 1)
 gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   constexpr bool ASYM = AMODE != 0, A8 = AMODE == 2;
-  using Cfg = GfCfg<BN, A8>;
+  using Cfg = GfCfg<BN, A8, PAIR>;
   constexpr int GF_EXP_STAGES = Cfg::EXP_STAGES, GF_RAW_STAGES = Cfg::RAW_STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* raw_area = smem + GF_EXP_STAGES * Cfg::EXP_STAGE;
   uint8_t* stg_area = raw_area + GF_RAW_STAGES * Cfg::RAW_STAGE;       // 1024-byte aligned
-  uint64_t* bars = reinterpret_cast<uint64_t*>(stg_area + Cfg::STG_BYTES);
+  uint8_t* tab_area = stg_area + Cfg::STG_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(tab_area + Cfg::TAB_BYTES);
   constexpr int NB = 2 * GF_RAW_STAGES + 3 * GF_EXP_STAGES + 4;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NB);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;            // 0 = leader (issues the pair's UMMAs)
   const uint32_t bar0 = smem_u32(bars);
   auto rawf_bar = [&](int s) { return bar0 + 8u * s; };
   auto rawe_bar = [&](int s) { return bar0 + 8u * (GF_RAW_STAGES + s); };
@@ -175,20 +216,29 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   auto accf_bar = [&](int b) { return bar0 + 8u * (2 * GF_RAW_STAGES + 3 * GF_EXP_STAGES + b); };
   auto acce_bar = [&](int b) { return bar0 + 8u * (2 * GF_RAW_STAGES + 3 * GF_EXP_STAGES + 2 + b); };
 
-  constexpr int W_MMA = GF_EPI_WARPS, W_TMA = GF_EPI_WARPS + 1, W_TMB = GF_EPI_WARPS + 2;
+  constexpr int W_MMA = GF_EPI_WARPS, W_TMA = GF_EPI_WARPS + 1, W_TMB = GF_EPI_WARPS + 2, W_CONV = GF_EPI_WARPS + 4;
   if (threadIdx.x == 0) {
     for (int s = 0; s < GF_RAW_STAGES; ++s) { mbar_init(rawf_bar(s), 1); mbar_init(rawe_bar(s), Cfg::CONV_WARPS); }
-    for (int s = 0; s < GF_EXP_STAGES; ++s) { mbar_init(expf_bar(s), Cfg::GROUP_WARPS); mbar_init(expe_bar(s), 1); mbar_init(expw_bar(s), 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), GF_EPI_WARPS); }
+    for (int s = 0; s < GF_EXP_STAGES; ++s) {
+      // pairs: one barrier per stage, in the leader, counts the weight bytes and the converter warps of both CTAs
+      mbar_init(expf_bar(s), PAIR ? 1 + 2 * Cfg::GROUP_WARPS : Cfg::GROUP_WARPS);
+      mbar_init(expe_bar(s), 1);
+      mbar_init(expw_bar(s), 1);
+    }
+    for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), (PAIR ? 2 : 1) * GF_EPI_WARPS); }
     abort_flag[0] = 0;
     abort_flag[1] = a.wait_limit_k;
     fence_mbar_init();
     prefetch_tmap(&tm.xq);
     prefetch_tmap(&tm.wp);
   }
-  if (warp == W_MMA) tmem_alloc(smem_u32(tmem_slot), Cfg::TMEM_COLS);
+  if (warp == W_MMA) {
+    if constexpr (PAIR) tmem_alloc_pair(smem_u32(tmem_slot), Cfg::TMEM_COLS);
+    else tmem_alloc(smem_u32(tmem_slot), Cfg::TMEM_COLS);
+  }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();   // both CTAs' barriers exist before anything arrives on them remotely
   tc_fence_after();
   pdl_launch_dependents();
   pdl_wait();                       // the kernels that produced the codes / records have completed
@@ -201,7 +251,8 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   const int n_main = hc ? (a.n_chunks + 1) >> 1 : a.n_chunks;      // operand stages of codes
   const int n_tail = (a.kt + 63) >> 6;
   const int n_tiles_n = (int)((a.N + BN - 1) / BN);
-  const int n_tiles_m = (int)((a.M + 127) / 128);
+  constexpr int TILE_M = PAIR ? 256 : 128;
+  const int n_tiles_m = (int)((a.M + TILE_M - 1) / TILE_M);
   const int total_tiles = n_tiles_n * n_tiles_m;
   // Tile order: column tiles in groups of `a.raster` (n fastest inside a group, then m, then the next group), so the
   // tiles in flight at one time share a bounded set of weight columns and activation rows in L2.
@@ -213,94 +264,19 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
     tm_ = r / width;
     tn_ = grp * rast + (r - tm_ * width);
   };
-  // Persistent CTA: tiles blockIdx.x, blockIdx.x + gridDim.x, ... with n fastest, so CTAs running at
+  const int first = PAIR ? (int)cluster_id_x() : (int)blockIdx.x, step = PAIR ? (int)cluster_count_x() : (int)gridDim.x;
+  // Persistent CTA (pair): tiles first, first + step, ... with n fastest, so CTAs running at
   // the same time read the same activation rows through L2.  Rings and the accumulator counter run on
   // across tiles.  Operand stage q of the kernel-wide sequence (chunks and tail stages of all tiles)
   // lives in slot q % EXP_STAGES; its barrier phase is (q / EXP_STAGES) & 1.
 
-  if (warp == W_TMA) {
-    // ------------------------------ TMA producer ---------------------------------------------
-    if (lane == 0) {
-      GfRing<GF_RAW_STAGES> r;
-      uint32_t issued = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        int tm_, tn_;
-        tile_mn(t, tm_, tn_);
-        const int m0 = tm_ * 128;
-        for (int c = 0; c < n_raw; c += GF_CPS) {
-          if (!mbar_wait_hot(rawe_bar(r.s), r.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
-          const uint32_t sb = raw_base + r.s * Cfg::RAW_STAGE;
-          const uint32_t bar = rawf_bar(r.s);
-          const int nv = min(GF_CPS, n_raw - c);
-          // 8-bit codes: the second 128-byte box is issued only when it holds a chunk (a box that lies
-          // wholly outside the tensor is never requested; its bytes are not part of the count either)
-          const bool second_box = A8 && nv > 2;
-          mbar_expect_tx(bar, (uint32_t)(Cfg::RAW_A - ((A8 && !second_box) ? 128 * 128 : 0) + nv * 128 * 8));
-          if constexpr (A8) {
-            tma_load_2d(sb, &tm.xq, bar, c * 64, m0);
-            if (second_box) tma_load_2d(sb + 128 * 128, &tm.xq, bar, c * 64 + 128, m0);
-          } else {
-            tma_load_2d(sb, &tm.xq, bar, c * 32, m0);
-          }
-          for (int j = 0; j < nv; ++j)
-            bulk_load(sb + Cfg::OFF_C + j * 128 * 8, a.a_const + ((int64_t)(c + j) * a.ldm + m0), 128 * 8, bar);
-          issued |= 1u << r.s;
-          r.next();
-        }
-        // tail: the activations' bf16 tile travels through the raw ring like a chunk (its rows go on to TMEM)
-        for (int st = 0; st < n_tail && ok; ++st) {
-          if (!mbar_wait_hot(rawe_bar(r.s), r.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
-          const uint32_t bar = rawf_bar(r.s);
-          mbar_expect_tx(bar, 128u * 128u);                    // one 128 x 64 bf16 tile
-          tma_load_2d(raw_base + r.s * Cfg::RAW_STAGE, &tm.xt, bar, st * 64, m0);
-          issued |= 1u << r.s;
-          r.next();
-        }
-      }
-      if (!ok) {
-        const long long t0 = clock64();
-        for (int i = 0; i < GF_RAW_STAGES; ++i) {
-          if (!(issued & (1u << i))) continue;
-          const uint32_t last_ph = (i < r.s) ? r.ph : (r.ph ^ 1);
-          while (!mbar_try(rawf_bar(i), last_ph))
-            if (clock64() - t0 > kWaitLimitCycles / 8) { if (a.status) atomicCAS(a.status, 0, ERR_WAIT_DRAIN); break; }
-        }
-      }
-    }
-  } else if (warp == W_TMB) {
-    // ------------------------------ weight-tile producer ---------------------------------------
-    // Operand stage q's weight tile goes straight into slot q % EXP_STAGES as soon as the slot is free.
-    if (lane == 0) {
-      int q = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        int tm_, tn_;
-        tile_mn(t, tm_, tn_);
-        const int n0 = tn_ * BN;
-        for (int st = 0; st < n_main + n_tail; ++st, ++q) {
-          const int es = q % GF_EXP_STAGES;
-          if (!mbar_wait_hot(expe_bar(es), (uint32_t)(((q / GF_EXP_STAGES) & 1) ^ 1), abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
-          const uint32_t bar = expw_bar(es);
-          mbar_expect_tx(bar, Cfg::B_EXP);                     // the box is counted whole, zero fill included
-          if (st < n_main) tma_load_2d(exp_base + es * Cfg::EXP_STAGE, &tm.wp, bar, st * 64, n0);
-          else tma_load_2d(exp_base + es * Cfg::EXP_STAGE, &tm.wt, bar, (st - n_main) * 64, n0);
-        }
-      }
-      if (!ok) {
-        // the copies of the last EXP_STAGES stages issued may still be in flight
-        const long long t0 = clock64();
-        for (int qq = max(0, q - GF_EXP_STAGES); qq < q; ++qq)
-          while (!mbar_try(expw_bar(qq % GF_EXP_STAGES), (uint32_t)((qq / GF_EXP_STAGES) & 1)))
-            if (clock64() - t0 > kWaitLimitCycles / 8) { if (a.status) atomicCAS(a.status, 0, ERR_WAIT_DRAIN); break; }
-      }
-    }
-  } else if (warp > W_TMB) {
+  if (warp >= W_CONV) {
+    reg_dealloc<Cfg::REGS_CONV>();
     // ------------------------------ converters ------------------------------------------------
     // Two groups take alternate operand stages (stage q goes to group q % GROUPS), so one group's barrier
     // waits, shared-memory latencies and fences overlap the other group's arithmetic.  A warp owns the 32
     // activation rows of its own TMEM lane quarter (warp index mod 4).
-    const int cw = warp - (W_TMB + 1);
+    const int cw = warp - W_CONV;
     constexpr int GW = Cfg::GROUP_WARPS;
     const int grp = cw / GW;
     const int quarter = warp & 3;
@@ -308,9 +284,13 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
     GfRing<GF_RAW_STAGES> r;
     int q = 0;
     bool ok = true;
+    auto exp_ready = [&](int es) {                          // this warp's rows of the stage are in tensor memory
+      if (PAIR && rank != 0) mbar_arrive_cluster_relaxed(map_to_rank(expf_bar(es), 0));
+      else mbar_arrive(expf_bar(es));
+    };
     auto exp_slot = [](int qq) { return qq % Cfg::EXP_STAGES; };
     auto exp_phase = [](int qq) { return (uint32_t)((qq / Cfg::EXP_STAGES) & 1); };
-    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+    for (int t = first; t < total_tiles && ok; t += step) {
       for (int c = 0; c < n_raw && ok; c += GF_CPS) {
         if (!mbar_wait_hot(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         const uint32_t sraw = raw_base + r.s * Cfg::RAW_STAGE;
@@ -407,7 +387,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(expf_bar(es));
+          if (lane == 0) exp_ready(es);
         }
         if (!ok) break;
         __syncwarp();
@@ -433,18 +413,113 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(expf_bar(es));
+          if (lane == 0) exp_ready(es);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(rawe_bar(r.s));
         r.next();
       }
     }
+  } else if (warp >= W_MMA) {
+  reg_dealloc<Cfg::REGS_PROD>();
+  if (warp == W_TMA) {
+    // ------------------------------ TMA producer ---------------------------------------------
+    if (lane == 0) {
+      GfRing<GF_RAW_STAGES> r;
+      uint32_t issued = 0;
+      bool ok = true;
+      for (int t = first; t < total_tiles && ok; t += step) {
+        int tm_, tn_;
+        tile_mn(t, tm_, tn_);
+        const int m0 = tm_ * TILE_M + (int)rank * 128;
+        // the second half of a pair's last tile may lie past the end: codes arrive as zero fill, and the records (bulk
+        // copies know no bounds) are those of the last row block; none of its rows is ever stored
+        const int64_t mrec = PAIR ? min((int64_t)m0, a.ldm - 128) : (int64_t)m0;
+        for (int c = 0; c < n_raw; c += GF_CPS) {
+          if (!mbar_wait_hot(rawe_bar(r.s), r.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+          const uint32_t sb = raw_base + r.s * Cfg::RAW_STAGE;
+          const uint32_t bar = rawf_bar(r.s);
+          const int nv = min(GF_CPS, n_raw - c);
+          // 8-bit codes: the second 128-byte box is issued only when it holds a chunk (a box that lies
+          // wholly outside the tensor is never requested; its bytes are not part of the count either)
+          const bool second_box = A8 && nv > 2;
+          mbar_expect_tx(bar, (uint32_t)(Cfg::RAW_A - ((A8 && !second_box) ? 128 * 128 : 0) + nv * 128 * 8));
+          if constexpr (A8) {
+            tma_load_2d(sb, &tm.xq, bar, c * 64, m0);
+            if (second_box) tma_load_2d(sb + 128 * 128, &tm.xq, bar, c * 64 + 128, m0);
+          } else {
+            tma_load_2d(sb, &tm.xq, bar, c * 32, m0);
+          }
+          for (int j = 0; j < nv; ++j)
+            bulk_load(sb + Cfg::OFF_C + j * 128 * 8, a.a_const + ((int64_t)(c + j) * a.ldm + mrec), 128 * 8, bar);
+          issued |= 1u << r.s;
+          r.next();
+        }
+        // tail: the activations' bf16 tile travels through the raw ring like a chunk (its rows go on to TMEM)
+        for (int st = 0; st < n_tail && ok; ++st) {
+          if (!mbar_wait_hot(rawe_bar(r.s), r.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+          const uint32_t bar = rawf_bar(r.s);
+          mbar_expect_tx(bar, 128u * 128u);                    // one 128 x 64 bf16 tile
+          tma_load_2d(raw_base + r.s * Cfg::RAW_STAGE, &tm.xt, bar, st * 64, m0);
+          issued |= 1u << r.s;
+          r.next();
+        }
+      }
+      if (!ok) {
+        const long long t0 = clock64();
+        for (int i = 0; i < GF_RAW_STAGES; ++i) {
+          if (!(issued & (1u << i))) continue;
+          const uint32_t last_ph = (i < r.s) ? r.ph : (r.ph ^ 1);
+          while (!mbar_try(rawf_bar(i), last_ph))
+            if (clock64() - t0 > kWaitLimitCycles / 8) { if (a.status) atomicCAS(a.status, 0, ERR_WAIT_DRAIN); break; }
+        }
+      }
+    }
+  } else if (warp == W_TMB) {
+    // ------------------------------ weight-tile producer ---------------------------------------
+    // Operand stage q's weight tile goes straight into slot q % EXP_STAGES as soon as the slot is free.
+    if (lane == 0) {
+      int q = 0;
+      bool ok = true;
+      for (int t = first; t < total_tiles && ok; t += step) {
+        int tm_, tn_;
+        tile_mn(t, tm_, tn_);
+        const int n0 = tn_ * BN;
+        for (int st = 0; st < n_main + n_tail; ++st, ++q) {
+          const int es = q % GF_EXP_STAGES;
+          if (!mbar_wait_hot(expe_bar(es), (uint32_t)(((q / GF_EXP_STAGES) & 1) ^ 1), abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+          if constexpr (PAIR) {
+            // this CTA's half of the weight rows; the bytes of both halves are counted in the leader
+            const uint32_t bar = map_to_rank(expf_bar(es), 0);
+            const int row_b = n0 + (int)rank * Cfg::BN_OWN;
+            if (rank == 0) mbar_expect_tx(expf_bar(es), 2 * Cfg::B_EXP);
+            if (st < n_main) tma_load_2d_pair(exp_base + es * Cfg::EXP_STAGE, &tm.wp, bar, st * 64, row_b);
+            else tma_load_2d_pair(exp_base + es * Cfg::EXP_STAGE, &tm.wt, bar, (st - n_main) * 64, row_b);
+            continue;
+          }
+          const uint32_t bar = expw_bar(es);
+          mbar_expect_tx(bar, Cfg::B_EXP);                     // the box is counted whole, zero fill included
+          if (st < n_main) tma_load_2d(exp_base + es * Cfg::EXP_STAGE, &tm.wp, bar, st * 64, n0);
+          else tma_load_2d(exp_base + es * Cfg::EXP_STAGE, &tm.wt, bar, (st - n_main) * 64, n0);
+        }
+      }
+      if (!ok) {
+        // the copies of the last EXP_STAGES stages issued may still be in flight
+        const long long t0 = clock64();
+        if constexpr (PAIR) {
+          // their completion is counted in the leader, where the peer cannot test it: a bounded time to land
+          while (clock64() - t0 < 2000000LL) __nanosleep(1000);
+        } else
+        for (int qq = max(0, q - GF_EXP_STAGES); qq < q; ++qq)
+          while (!mbar_try(expw_bar(qq % GF_EXP_STAGES), (uint32_t)((qq / GF_EXP_STAGES) & 1)))
+            if (clock64() - t0 > kWaitLimitCycles / 8) { if (a.status) atomicCAS(a.status, 0, ERR_WAIT_DRAIN); break; }
+      }
+    }
   } else if (warp == W_MMA) {
     // ------------------------------ UMMA issuer ----------------------------------------------
-    if (lane == 0) {
-      const uint32_t idesc_h = idesc_dense(ACC_F32, FMT_F16, FMT_F16, 128, BN);
-      const uint32_t idesc_bf = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, 128, BN);
+    if (lane == 0 && rank == 0) {
+      const uint32_t idesc_h = idesc_dense(ACC_F32, FMT_F16, FMT_F16, TILE_M, BN);
+      const uint32_t idesc_bf = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, TILE_M, BN);
       int use = 0;
       bool ok = true;
       // loop-invariant pieces of the per-stage operands: barrier addresses are 8 bytes per slot apart, the weight
@@ -458,7 +533,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
       const uint32_t bdesc_lo0 = (uint32_t)bdesc0, bdesc_hi = (uint32_t)(bdesc0 >> 32);
       constexpr uint32_t kDescStep = Cfg::EXP_STAGE >> 4;
       const uint32_t a_tmem0 = tmem_base + Cfg::TMEM_A0;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      for (int t = first; t < total_tiles && ok; t += step) {
         const int buf = Cfg::NACC == 2 ? (use & 1) : 0;
         const uint32_t acc_ph = (uint32_t)(Cfg::NACC == 2 ? (use >> 1) & 1 : use & 1);
         if (!mbar_wait_hot(acce_bar(buf), acc_ph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) { ok = false; break; }
@@ -476,211 +551,215 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           uint32_t ph1 = ph0;
           if (two && ++es1 == GF_EXP_STAGES) { es1 = 0; ph1 ^= 1u; }
           const uint32_t w0 = expw0 + 8u * es0, w1 = expw0 + 8u * es1;       // expf / expe lie at fixed offsets from expw
-          const uint32_t rdy = mbar_test4(w0, ph0, w0 - kFullOff, ph0, w1, ph1, w1 - kFullOff, ph1);
-          if (rdy != 15u) {
-            if (!(rdy & 1u)) ok = mbar_wait_hot(w0, ph0, abort_flag, a.status, ERR_WAIT_FULL);
-            if (ok && !(rdy & 2u)) ok = mbar_wait_hot(w0 - kFullOff, ph0, abort_flag, a.status, ERR_WAIT_FULL);
-            if (ok && !(rdy & 4u)) ok = mbar_wait_hot(w1, ph1, abort_flag, a.status, ERR_WAIT_FULL);
-            if (ok && !(rdy & 8u)) ok = mbar_wait_hot(w1 - kFullOff, ph1, abort_flag, a.status, ERR_WAIT_FULL);
-            if (!ok) break;
-          }
-          tc_fence_after();
-          umma_f16_ts_x4(d, a_tmem0 + 32u * es0, bdesc_lo0 + kDescStep * es0, bdesc_hi, st < n_main ? idesc_h : idesc_bf,
-                         st > 0 ? 1u : 0u);
-          umma_commit(w0 - kEmptyOff);
-          if (two) {
-            umma_f16_ts_x4(d, a_tmem0 + 32u * es1, bdesc_lo0 + kDescStep * es1, bdesc_hi, st + 1 < n_main ? idesc_h : idesc_bf, 1u);
-            umma_commit(w1 - kEmptyOff);
-            st += 2;
+          if constexpr (PAIR) {
+            // one barrier per stage covers both operands in both CTAs
+            const uint32_t f0 = w0 - kFullOff, f1 = w1 - kFullOff;
+            const uint32_t rdy = mbar_test2(f0, ph0, f1, ph1);
+            if (rdy != 3u) {
+              if (!(rdy & 1u)) ok = mbar_wait_hot(f0, ph0, abort_flag, a.status, ERR_WAIT_FULL);
+              if (ok && !(rdy & 2u)) ok = mbar_wait_hot(f1, ph1, abort_flag, a.status, ERR_WAIT_FULL);
+              if (!ok) break;
+            }
+            tc_fence_after();
+            umma_f16_ts_x4_pair(d, a_tmem0 + 32u * es0, bdesc_lo0 + kDescStep * es0, bdesc_hi, st < n_main ? idesc_h : idesc_bf,
+                                st > 0 ? 1u : 0u);
+            umma_commit_pair_both(w0 - kEmptyOff);
+            if (two) {
+              umma_f16_ts_x4_pair(d, a_tmem0 + 32u * es1, bdesc_lo0 + kDescStep * es1, bdesc_hi,
+                                  st + 1 < n_main ? idesc_h : idesc_bf, 1u);
+              umma_commit_pair_both(w1 - kEmptyOff);
+            }
           } else {
-            st += 1;
+            const uint32_t rdy = mbar_test4(w0, ph0, w0 - kFullOff, ph0, w1, ph1, w1 - kFullOff, ph1);
+            if (rdy != 15u) {
+              if (!(rdy & 1u)) ok = mbar_wait_hot(w0, ph0, abort_flag, a.status, ERR_WAIT_FULL);
+              if (ok && !(rdy & 2u)) ok = mbar_wait_hot(w0 - kFullOff, ph0, abort_flag, a.status, ERR_WAIT_FULL);
+              if (ok && !(rdy & 4u)) ok = mbar_wait_hot(w1, ph1, abort_flag, a.status, ERR_WAIT_FULL);
+              if (ok && !(rdy & 8u)) ok = mbar_wait_hot(w1 - kFullOff, ph1, abort_flag, a.status, ERR_WAIT_FULL);
+              if (!ok) break;
+            }
+            tc_fence_after();
+            umma_f16_ts_x4(d, a_tmem0 + 32u * es0, bdesc_lo0 + kDescStep * es0, bdesc_hi, st < n_main ? idesc_h : idesc_bf,
+                           st > 0 ? 1u : 0u);
+            umma_commit(w0 - kEmptyOff);
+            if (two) {
+              umma_f16_ts_x4(d, a_tmem0 + 32u * es1, bdesc_lo0 + kDescStep * es1, bdesc_hi,
+                             st + 1 < n_main ? idesc_h : idesc_bf, 1u);
+              umma_commit(w1 - kEmptyOff);
+            }
           }
+          st += two ? 2 : 1;
           es0 = es1;
           ph0 = ph1;
           if (++es0 == GF_EXP_STAGES) { es0 = 0; ph0 ^= 1u; }
         }
-        if (ok) { umma_commit(accf_bar(buf)); ++use; }
+        if (ok) {
+          if constexpr (PAIR) umma_commit_pair_both(accf_bar(buf));
+          else umma_commit(accf_bar(buf));
+          ++use;
+        }
       }
     }
+  }
   } else {
+    reg_alloc<Cfg::REGS_EPI>();
     // ------------------------------ epilogue: 8 warps -----------------------------------------
-    // warp w: TMEM lane quarter w & 3 (32 rows), column half w >> 2 (BN / 2 columns), 32 columns at a time:
-    // tcgen05.ld -> * rs[m] * cs[n] + bias -> bf16 -> the warp's 32 x 32 staging patch in shared memory
-    // (64-byte rows, 64-byte swizzle: conflict-free) -> one TMA store, which clips the patch at the edges
-    // of y.  A row-per-thread store straight to global memory would put 32 separate 16-byte segments per
-    // instruction through the load/store unit that the converter warps depend on.
+    // warp w: TMEM lane quarter w & 3 (32 rows), half of the columns.  Two steps: the warp's share of the accumulator is
+    // read, scaled by rs[m] * cs[n], offset by the bias and rounded to bf16 pairs in registers, and the accumulator is
+    // handed back; only then come the activation, the quantiser and the stores.  A 256-wide tile has one accumulator, so
+    // everything before the hand-back is time its UMMAs wait: 6200 cycles of a 16900-cycle tile at K = 1152 with the
+    // per-column factors loaded from global memory between the reads and activation and stores inside, 2900 with them
+    // outside and the factors from shared memory, 1700 with each 16-column piece's loads in flight while the piece before it
+    // is worked on (which takes the registers).  The factors come from a table of the warp's own, filled while the UMMAs of
+    // the tile still run, as bf16 pairs: cs is a power of two.
+    // Stores: bf16 -> the warp's 32 x 32 staging patch in shared memory (64-byte rows, 64-byte swizzle: conflict-free)
+    // -> one TMA store, which clips the patch at the edges of y.  A row-per-thread store straight to global memory would
+    // put 32 separate 16-byte segments per instruction through the load/store unit that the converter warps depend on.
     const int q = warp & 3, ch = warp >> 2;
     const int trow = q * 32 + lane;
     constexpr int CW = BN / 2;
     const uint32_t stg = smem_u32(stg_area) + warp * 2048;
     const uint32_t stg_row = stg + lane * 64;
     const int stg_sw = (lane >> 1) & 3;
+    const uint32_t tab = smem_u32(tab_area) + warp * Cfg::TAB_WARP;
+    auto acc_release = [&](int b) {
+      if (PAIR && rank != 0) mbar_arrive_cluster_relaxed(map_to_rank(acce_bar(b), 0));
+      else mbar_arrive(acce_bar(b));
+    };
+    const bool qout = a.q_codes != nullptr;
+    auto put_patch = [&](const uint32_t* w16, int col, int row) {     // 32 columns of the warp's 32 rows -> y
+      if (lane == 0) bulk_wait_read0();              // the previous patch has left the staging buffer
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        gf_sts128(stg_row + (uint32_t)((i ^ stg_sw) << 4), w16[4 * i], w16[4 * i + 1], w16[4 * i + 2], w16[4 * i + 3]);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_2d(&tm.y, stg, col, row);
+        bulk_commit_group();
+      }
+    };
+    auto gelu_pairs = [&](uint32_t* w16) {
+#pragma unroll
+      for (int e = 0; e < 16; ++e) {
+        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w16[e]));
+        const __nv_bfloat162 h = __floats2bfloat162_rn(gelu_tanh_bf16(f.x), gelu_tanh_bf16(f.y));
+        w16[e] = *reinterpret_cast<const uint32_t*>(&h);
+      }
+    };
     int use = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+    for (int t = first; t < total_tiles && ok; t += step) {
       int tm_, tn_;
       tile_mn(t, tm_, tn_);
-      const int m0 = tm_ * 128, n0 = tn_ * BN;
+      const int m0 = tm_ * TILE_M + (int)rank * 128, n0 = tn_ * BN;
       const int64_t row = (int64_t)m0 + trow;
       const float rs = (row < a.M) ? __ldg(a.rs + row) : 0.f;
+      __syncwarp();                                  // every lane has read the previous tile's table
+      for (int i = lane; i < Cfg::PIECES * 8; i += 32) { // one column pair each
+        const int64_t col = (int64_t)n0 + ch * CW + 2 * i;
+        uint32_t cp = 0u, bp = 0u;
+        if (col < a.N) {
+          const float2 c = __ldg(reinterpret_cast<const float2*>(a.cs + col));
+          cp = __byte_perm(__float_as_uint(c.x), __float_as_uint(c.y), 0x7632);      // powers of two: exact in bf16
+          if (a.bias) bp = __ldg(reinterpret_cast<const uint32_t*>(a.bias + col));
+        }
+        gf_sts64(tab + i * 8, cp, bp);
+      }
       const int buf = Cfg::NACC == 2 ? (use & 1) : 0;
-      if (!mbar_wait(accf_bar(buf), (uint32_t)(Cfg::NACC == 2 ? (use >> 1) & 1 : use & 1), abort_flag, a.status, ERR_WAIT_ACC_FULL)) { ok = false; break; }
+      const uint32_t acc_ph = (uint32_t)(Cfg::NACC == 2 ? (use >> 1) & 1 : use & 1);
+      if (!mbar_wait(accf_bar(buf), acc_ph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) { ok = false; break; }
       __syncwarp();
       tc_fence_after();
       ++use;
       const uint32_t tl = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + ch * CW;
-      if (a.q_codes) {
-        // ---- quantise-out: every 64 columns of the tile are one group of the following layer; the two warps of a
-        // lane quarter take them alternately (a 192-wide tile: groups 0 and 2 here, group 1 there) ----
-#pragma unroll 1
-        for (int gi = ch; gi < BN / 64; gi += 2) {
-          uint32_t v[64];
-          const uint32_t tg = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + gi * 64;
-          tmem_ld32(tg, v);
-          tmem_ld32(tg + 32, v + 32);
-          tmem_wait_ld();
-          if (gi + 2 >= BN / 64) {                      // the accumulator is out of TMEM: hand it back
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(acce_bar(buf));
-          }
-          const int64_t col0 = (int64_t)n0 + gi * 64;
-          if (col0 + 64 > a.N) continue;               // padding of the last tile (N is a multiple of 64 here)
-          uint32_t w[32];                               // the activated output, bf16 pairs: what the next quantiser sees
+      uint32_t w[Cfg::PIECES * 8];                    // the output before activation, bf16 pairs
+      uint32_t v[2][16];
+      uint4 f[2][4];
+      auto fetch = [&](int c) {                       // a piece's accumulators and factors
+        tmem_ld16(tl + c * 16, v[c & 1]);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4 c0 = __ldg(reinterpret_cast<const float4*>(a.cs + col0 + 8 * i));
-            const float4 c1 = __ldg(reinterpret_cast<const float4*>(a.cs + col0 + 8 * i + 4));
-            const float cs8[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-            float b[8];
-            if (a.bias) {
-              const uint4 bb = __ldg(reinterpret_cast<const uint4*>(a.bias + col0 + 8 * i));
-              const __nv_bfloat162* bh = reinterpret_cast<const __nv_bfloat162*>(&bb);
+        for (int e = 0; e < 4; ++e) f[c & 1][e] = gf_lds128(tab + (c * 4 + e) * 16);
+      };
+      fetch(0);
 #pragma unroll
-              for (int e2 = 0; e2 < 4; ++e2) { float2 f = __bfloat1622float2(bh[e2]); b[2 * e2] = f.x; b[2 * e2 + 1] = f.y; }
-            } else {
+      for (int c = 0; c < Cfg::PIECES; ++c) {
+        tmem_wait_ld16(v[c & 1]);
+        if (c + 1 < Cfg::PIECES) fetch(c + 1);
 #pragma unroll
-              for (int e2 = 0; e2 < 8; ++e2) b[e2] = 0.f;
-            }
+        for (int e = 0; e < 4; ++e) {
+          const uint4 k = f[c & 1][e];
+          w[8 * c + 2 * e] = scale_pair(v[c & 1][4 * e], v[c & 1][4 * e + 1], rs, k.x, k.y);
+          w[8 * c + 2 * e + 1] = scale_pair(v[c & 1][4 * e + 2], v[c & 1][4 * e + 3], rs, k.z, k.w);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) acc_release(buf);                // the accumulator is out of TMEM
+      if (!qout) {
 #pragma unroll
-            for (int e2 = 0; e2 < 4; ++e2) {
-              float f0 = __fmaf_rn(__uint_as_float(v[8 * i + 2 * e2]), rs * cs8[2 * e2], b[2 * e2]);
-              float f1 = __fmaf_rn(__uint_as_float(v[8 * i + 2 * e2 + 1]), rs * cs8[2 * e2 + 1], b[2 * e2 + 1]);
-              if (a.act == 1) { f0 = gelu_tanh_bf16(f0); f1 = gelu_tanh_bf16(f1); }
-              __nv_bfloat162 h = __floats2bfloat162_rn(f0, f1);
-              w[4 * i + e2] = *reinterpret_cast<uint32_t*>(&h);
-            }
-          }
-          if (a.y) {                                    // the bf16 tensor as well, when the caller wants it
-#pragma unroll
-            for (int g = 0; g < 2; ++g) {
-              if (lane == 0) bulk_wait_read0();
-              __syncwarp();
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                gf_sts128(stg_row + (uint32_t)((i ^ stg_sw) << 4), w[16 * g + 4 * i], w[16 * g + 4 * i + 1], w[16 * g + 4 * i + 2],
-                          w[16 * g + 4 * i + 3]);
-              fence_proxy_async_smem();
-              __syncwarp();
-              if (lane == 0) {
-                tma_store_2d(&tm.y, stg, (int)col0 + 32 * g, m0 + q * 32);
-                bulk_commit_group();
-              }
-            }
-          }
-          if (col0 >= a.q_len) {                        // the following layer's 16-bit channels
-            if (row < a.M) {
-              uint4* t = reinterpret_cast<uint4*>(a.q_tail + row * a.q_tail_pitch + (col0 - a.q_len));
-#pragma unroll
-              for (int i = 0; i < 8; ++i) t[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-            }
-            continue;
-          }
-          if (row < a.M) {
-            const int chunk = (int)(col0 >> 6);
-            uint4* dst = reinterpret_cast<uint4*>(a.q_codes + row * a.q_row_bytes + (int64_t)chunk * 32);
-            GroupParams p;
-            if (a.q_mode == DIROTQ_INT4_SYM) {
-              const float amax = fmaxf(fmaxf(amax_bf16x16(w), amax_bf16x16(w + 8)), fmaxf(amax_bf16x16(w + 16), amax_bf16x16(w + 24)));
-              p = int_sym_params<true>(amax, -amax, a.q_clip, 7.f);
-              const float rcp = __frcp_rn(p.scale);
-              dst[0] = int_sym_planar32_packed(w, rcp, a.q_clip < 1.f);
-              dst[1] = int_sym_planar32_packed(w + 16, rcp, a.q_clip < 1.f);
-            } else {
-              float mx = -INFINITY, mn = INFINITY;
-              minmax_bf16x16(w, mx, mn);
-              minmax_bf16x16(w + 8, mx, mn);
-              minmax_bf16x16(w + 16, mx, mn);
-              minmax_bf16x16(w + 24, mx, mn);
-              p = int_asym_params<true>(mx, mn, a.q_clip, 15.f);
-              const float rcp = __frcp_rn(p.scale);
-              dst[0] = int_asym_planar32_packed(w, rcp, p.zero);
-              dst[1] = int_asym_planar32_packed(w + 16, rcp, p.zero);
-              a.q_zeros[(int64_t)chunk * a.q_ldm + row] = __float2bfloat16_rn(p.zero);
-            }
-            a.q_scales[(int64_t)chunk * a.q_ldm + row] = __float2bfloat16_rn(p.scale);
+        for (int g = 0; g < CW / 32; ++g) {
+          const int64_t col0 = (int64_t)n0 + ch * CW + g * 32;
+          if (col0 < a.N) {                            // warp-uniform: otherwise nothing of this patch lies inside y
+            if (a.act == 1) gelu_pairs(w + 16 * g);
+            put_patch(w + 16 * g, (int)col0, m0 + q * 32);
           }
         }
         continue;
       }
-#pragma unroll 1
-      for (int g = 0; g < CW / 32; ++g) {
-        uint32_t v[32];
-        tmem_ld32(tl + g * 32, v);
-        tmem_wait_ld();
-        if (g == CW / 32 - 1) {                      // the accumulator is out of TMEM: hand it back
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(acce_bar(buf));
+      // ---- quantise-out: every 64 columns of the tile are one group of the following layer ----
+#pragma unroll
+      for (int k = 0; k < Cfg::PIECES / 4; ++k) {
+        const int64_t col0 = (int64_t)n0 + ch * CW + k * 64;
+        if (col0 + 64 > a.N) break;                   // padding of the last tile (N is a multiple of 64 here)
+        uint32_t* wk = w + 32 * k;                    // the activated output: what the next quantiser sees
+        if (a.act == 1) { gelu_pairs(wk); gelu_pairs(wk + 16); }
+        if (a.y) {                                    // the bf16 tensor as well, when the caller wants it
+          put_patch(wk, (int)col0, m0 + q * 32);
+          put_patch(wk + 16, (int)col0 + 32, m0 + q * 32);
         }
-        const int64_t col0 = (int64_t)n0 + ch * CW + g * 32;
-        if (col0 >= a.N) continue;                     // warp-uniform: nothing of this patch lies inside y
-        if (lane == 0) bulk_wait_read0();              // the previous patch has left the staging buffer
-        __syncwarp();
+        if (row >= a.M) continue;
+        if (col0 >= a.q_len) {                        // the following layer's 16-bit channels
+          uint4* t4 = reinterpret_cast<uint4*>(a.q_tail + row * a.q_tail_pitch + (col0 - a.q_len));
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          uint32_t w[4] = {0u, 0u, 0u, 0u};
-          if (col0 + 8 * i + 8 <= a.N) {
-            const float4 c0 = __ldg(reinterpret_cast<const float4*>(a.cs + col0 + 8 * i));
-            const float4 c1 = __ldg(reinterpret_cast<const float4*>(a.cs + col0 + 8 * i + 4));
-            const float cs8[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-            float b[8];
-            if (a.bias) {
-              const uint4 bb = __ldg(reinterpret_cast<const uint4*>(a.bias + col0 + 8 * i));
-              const __nv_bfloat162* bh = reinterpret_cast<const __nv_bfloat162*>(&bb);
-#pragma unroll
-              for (int e2 = 0; e2 < 4; ++e2) { float2 f = __bfloat1622float2(bh[e2]); b[2 * e2] = f.x; b[2 * e2 + 1] = f.y; }
-            } else {
-#pragma unroll
-              for (int e2 = 0; e2 < 8; ++e2) b[e2] = 0.f;
-            }
-#pragma unroll
-            for (int e2 = 0; e2 < 4; ++e2) {
-              float f0 = __fmaf_rn(__uint_as_float(v[8 * i + 2 * e2]), rs * cs8[2 * e2], b[2 * e2]);
-              float f1 = __fmaf_rn(__uint_as_float(v[8 * i + 2 * e2 + 1]), rs * cs8[2 * e2 + 1], b[2 * e2 + 1]);
-              if (a.act == 1) { f0 = gelu_tanh_bf16(f0); f1 = gelu_tanh_bf16(f1); }
-              __nv_bfloat162 h = __floats2bfloat162_rn(f0, f1);
-              w[e2] = *reinterpret_cast<uint32_t*>(&h);
-            }
-          }
-          gf_sts128(stg_row + (uint32_t)((i ^ stg_sw) << 4), w[0], w[1], w[2], w[3]);
+          for (int i = 0; i < 8; ++i) t4[i] = make_uint4(wk[4 * i], wk[4 * i + 1], wk[4 * i + 2], wk[4 * i + 3]);
+          continue;
         }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          tma_store_2d(&tm.y, stg, (int)col0, m0 + q * 32);
-          bulk_commit_group();
+        const int chunk = (int)(col0 >> 6);
+        uint4* dst = reinterpret_cast<uint4*>(a.q_codes + row * a.q_row_bytes + (int64_t)chunk * 32);
+        GroupParams p;
+        if (a.q_mode == DIROTQ_INT4_SYM) {
+          const float amax = fmaxf(fmaxf(amax_bf16x16(wk), amax_bf16x16(wk + 8)), fmaxf(amax_bf16x16(wk + 16), amax_bf16x16(wk + 24)));
+          p = int_sym_params<true>(amax, -amax, a.q_clip, 7.f);
+          const float rcp = __frcp_rn(p.scale);
+          dst[0] = int_sym_planar32_packed(wk, rcp, a.q_clip < 1.f);
+          dst[1] = int_sym_planar32_packed(wk + 16, rcp, a.q_clip < 1.f);
+        } else {
+          float mx = -INFINITY, mn = INFINITY;
+          minmax_bf16x16(wk, mx, mn);
+          minmax_bf16x16(wk + 8, mx, mn);
+          minmax_bf16x16(wk + 16, mx, mn);
+          minmax_bf16x16(wk + 24, mx, mn);
+          p = int_asym_params<true>(mx, mn, a.q_clip, 15.f);
+          const float rcp = __frcp_rn(p.scale);
+          dst[0] = int_asym_planar32_packed(wk, rcp, p.zero);
+          dst[1] = int_asym_planar32_packed(wk + 16, rcp, p.zero);
+          a.q_zeros[(int64_t)chunk * a.q_ldm + row] = __float2bfloat16_rn(p.zero);
         }
+        a.q_scales[(int64_t)chunk * a.q_ldm + row] = __float2bfloat16_rn(p.scale);
       }
     }
     if (lane == 0) bulk_wait_all0();                   // the output is in global memory before the CTA retires
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();   // neither CTA retires while the other may still read its shared memory
   if (warp == W_MMA) {
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
+    else tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
 }
 
@@ -899,39 +978,72 @@ int launch_fold_weight_scales(const float* s, int n_chunks, int64_t N, int64_t l
   return cudaGetLastError() == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
 }
 
-template <int BN, int AMODE>
+template <int BN, int AMODE, bool PAIR>
 static int launch_gf(const GfMaps& tm, const GemmIntF16Args& a, cudaStream_t st) {
-  using Cfg = GfCfg<BN, AMODE == 2>;
-  auto k = gemm_int_f16_kernel<BN, AMODE>;
+  using Cfg = GfCfg<BN, AMODE == 2, PAIR>;
+  auto k = gemm_int_f16_kernel<BN, AMODE, PAIR>;
   static PerDeviceOnce attr_once;
   if (int rc = set_max_dynamic_smem(attr_once, k, Cfg::SMEM_BYTES)) return rc;
+  // the register split is only sound if the kernel was compiled to the launch's share
+  static const bool regs_ok = [&] {
+    cudaFuncAttributes fa;
+    return cudaFuncGetAttributes(&fa, k) == cudaSuccess && fa.numRegs >= Cfg::REGS_LAUNCH;
+  }();
+  if (!regs_ok) return DIROTQ_E_UNSUPPORTED;
+  if constexpr (PAIR) {
+    const int64_t tiles = ((a.N + BN - 1) / BN) * ((a.M + 255) / 256);
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(Cfg::THREADS);
+    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    // persistent grid: as many pairs as can be resident at once, remembered per device
+    static std::atomic<int> resident[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return DIROTQ_E_CUDA;
+    int max_pairs = resident[dev].load(std::memory_order_relaxed);
+    if (max_pairs <= 0) {
+      cfg.gridDim = dim3(2 * (num_sms() / 2));
+      cfg.numAttrs = 1;
+      if (cudaOccupancyMaxActiveClusters(&max_pairs, k, &cfg) != cudaSuccess || max_pairs <= 0) max_pairs = num_sms() / 2;
+      resident[dev].store(max_pairs, std::memory_order_relaxed);
+    }
+    cfg.gridDim = dim3(2 * (unsigned)(tiles < max_pairs ? tiles : max_pairs));
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, k, tm, a) == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
+  }
   const int tiles = (int)((a.N + BN - 1) / BN) * (int)((a.M + 127) / 128);
   const int grid = min(tiles, num_sms());
   return launch_pdl(k, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, st, tm, a) == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
 }
 
-// Column-tile width.  The persistent grid runs ceil(tiles / SMs) rounds; a round costs, per 64-wide K stage, a part
-// proportional to the tile width (the UMMAs) and a part that is the same for every width (the issuer's per-stage barrier
-// protocol): 6.84 us for 128 columns and 7.81 us for 192 at K = 1152, i.e. the fixed part is worth about 320 columns.  A
-// 256-wide tile has a single accumulator (tensor memory: 256 + 8 x 32 activation columns), so the part of its epilogue
-// that reads the accumulator is not hidden behind the next tile's UMMAs: about 2300 column-stages per round more.  The
-// choice minimises rounds x ((width + 320) x stages [+ 2300]) -- padded columns and a nearly empty last round both count:
-// 256 for long K and widths that divide (3072 -> 12288 at 18432 rows: 1050 us against 1151 with 192; 12288 -> 3072: 968
-// against 1112; 2240 x 2240: 143 against 152), 192 for K = 1152 (1152 x 1152 at 16384 rows: 48 us against 59 with 128 or
-// 256), 128 where 192 would leave the last of two rounds a third full (1152 x 1152 at 4096 rows: 19.7 us against 21.6).
-// DIROTQ_GF_BN overrides.
-static int pick_bn_f16(int64_t M, int64_t N, int64_t stages) {
-  if (const char* e = getenv("DIROTQ_GF_BN")) return atoi(e);
-  const int cand[3] = {256, 192, 128};
+// Column-tile width.  The persistent grid runs ceil(tiles / SMs) rounds, and a round of 256-wide tiles takes 9/7 of a round
+// of 128-wide ones whatever K is: 8.5 us against 6.6 at K = 1152, 16.6 / 12.9 at 2240, 21.1 / 16.7 at 3072 (the issuer's
+// per-stage barrier protocol does not depend on the width, and the wide tile's single accumulator is handed back before
+// anything else is done with it).  So 256 wherever it saves a quarter of the rounds (1152 -> 3456 at 32768 rows: 213 us
+// against 311; 1152 -> 4608 at 4096: 44 / 62), 128 where both need the same few (1152 x 1152 at 4096 rows: 23.0 / 25.3;
+// 2240 x 2240 at 1024: 28.7 / 30.5).  A 192-wide tile lay between the two everywhere and is gone.  DIROTQ_GF_BN overrides.
+static int pick_bn_f16(int64_t M, int64_t N) {
+  if (const char* e = getenv("DIROTQ_GF_BN")) return atoi(e) > 128 ? 256 : 128;
   const int64_t m_tiles = (M + 127) / 128, sms = num_sms();
-  int best = 128;
-  int64_t best_cost = -1;
-  for (int i = 0; i < 3; ++i) {
-    const int64_t tiles = m_tiles * ((N + cand[i] - 1) / cand[i]);
-    const int64_t cost = ((tiles + sms - 1) / sms) * ((cand[i] + 320) * stages + (cand[i] > 192 ? 2300 : 0));
-    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = cand[i]; }
-  }
-  return best;
+  const int64_t r256 = (m_tiles * ((N + 255) / 256) + sms - 1) / sms, r128 = (m_tiles * ((N + 127) / 128) + sms - 1) / sms;
+  return 9 * r256 < 7 * r128 ? 256 : 128;
+}
+
+// CTA pairs halve the weight traffic of a 256-wide tile and issue one UMMA for two SMs: 204 us against 213 for 1152 -> 3456 at
+// 32768 rows, 185 / 190 for 3072 -> 9216 at 4608.  Their tiles are twice as tall, so the last round is coarser, and a stage's
+// hand-off crosses the pair: 26.1 us against 25.3 for 1152 x 1152 at 4096 rows (two rounds), 44.7 / 44.4 for 1152 -> 4608 (four),
+// level at 32768 x 1152 (nine).  Hence only from five rounds on.  DIROTQ_GF_PAIR overrides (0 or 1).
+static bool pick_pair_f16(int64_t M, int64_t N) {
+  if (const char* e = getenv("DIROTQ_GF_PAIR")) return atoi(e) != 0;
+  return ((M + 127) / 128) * ((N + 255) / 256) > 4 * (int64_t)num_sms();
 }
 
 // Column tiles per rasterisation group.  With n fastest over the whole width, the CTAs of one round read every weight
@@ -954,8 +1066,8 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
   if ((reinterpret_cast<uintptr_t>(a.bias) & 15) || (reinterpret_cast<uintptr_t>(a.cs) & 15) || (a.N & 7) ||
       (reinterpret_cast<uintptr_t>(a.a_const) & 15) || (reinterpret_cast<uintptr_t>(a.w_panel) & 15) || !a.w_panel)
     return DIROTQ_E_ALIGN;
-  const int64_t k_stages = (a.half_chunks ? (a.n_chunks + 1) / 2 : a.n_chunks) + (a.kt + 63) / 64;
-  int BN = a.force_bn ? a.force_bn : pick_bn_f16(a.M, a.N, k_stages);
+  const int BN = a.force_bn ? a.force_bn : pick_bn_f16(a.M, a.N);
+  const bool pair = BN == 256 && pick_pair_f16(a.M, a.N);
   if (a.q_codes) {
     if (a.N % 64 || a.q_len % 64 || a.q_len <= 0 || a.q_len > a.N || a.q_row_bytes < a.q_len / 2 || (a.q_row_bytes & 15) ||
         (a.q_len < a.N && (!a.q_tail || a.q_tail_pitch < a.N - a.q_len || (a.q_tail_pitch & 7) ||
@@ -966,16 +1078,13 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
   } else if (!a.y) {
     return DIROTQ_E_ARG;
   }
-#ifdef GF_FORCE_BN
-  BN = GF_FORCE_BN;
-#endif
   GfMaps tm;
   int rc = make_tmap_2d_sw(&tm.xq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.xq, (uint64_t)a.x_row_bytes, (uint64_t)a.M,
                            (uint64_t)a.x_row_bytes, 32 * GF_CPS, 128, 32 * GF_CPS);
   if (rc) return rc;
   const uint64_t n_stage = a.half_chunks ? (uint64_t)((a.n_chunks + 1) / 2) : (uint64_t)a.n_chunks;
   if (a.raster == 0) a.raster = pick_raster_f16(BN, a.N, (int64_t)n_stage * 64 + ((a.kt + 63) / 64) * 64);
-  rc = make_tmap_2d(&tm.wp, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.w_panel, n_stage * 64, (uint64_t)a.N, n_stage * 128, BN);
+  rc = make_tmap_2d(&tm.wp, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.w_panel, n_stage * 64, (uint64_t)a.N, n_stage * 128, pair ? BN / 2 : BN);
   if (rc) return rc;
   // without an output tensor (quantise-out only) the map is never used: any valid address will do
   rc = make_tmap_2d_sw(&tm.y, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.y ? (const void*)a.y : a.w_panel, (uint64_t)a.N, (uint64_t)a.M, (uint64_t)a.N * 2,
@@ -984,23 +1093,27 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
   if (a.kt > 0) {
     rc = make_tmap_2d(&tm.xt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.xt, (uint64_t)a.kt, (uint64_t)a.M, (uint64_t)a.kt_pitch * 2, 128);
     if (rc) return rc;
-    rc = make_tmap_2d(&tm.wt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.wt, (uint64_t)a.kt, (uint64_t)a.N, (uint64_t)a.kt_pitch * 2, BN);
+    rc = make_tmap_2d(&tm.wt, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.wt, (uint64_t)a.kt, (uint64_t)a.N, (uint64_t)a.kt_pitch * 2, pair ? BN / 2 : BN);
     if (rc) return rc;
   } else {
     tm.xt = tm.xq;
     tm.wt = tm.wp;
   }
   const int amode = a.a_mode == DIROTQ_INT4_SYM ? 0 : a.a_mode == DIROTQ_INT4_ASYM ? 1 : 2;
+  if (BN == 256 && pair) {
+    switch (amode) {
+      case 0: return launch_gf<256, 0, true>(tm, a, st);
+      case 1: return launch_gf<256, 1, true>(tm, a, st);
+      case 2: return launch_gf<256, 2, true>(tm, a, st);
+    }
+  }
   switch (BN * 4 + amode) {
-    case 256 * 4 + 0: return launch_gf<256, 0>(tm, a, st);
-    case 256 * 4 + 1: return launch_gf<256, 1>(tm, a, st);
-    case 256 * 4 + 2: return launch_gf<256, 2>(tm, a, st);
-    case 192 * 4 + 0: return launch_gf<192, 0>(tm, a, st);
-    case 192 * 4 + 1: return launch_gf<192, 1>(tm, a, st);
-    case 192 * 4 + 2: return launch_gf<192, 2>(tm, a, st);
-    case 128 * 4 + 0: return launch_gf<128, 0>(tm, a, st);
-    case 128 * 4 + 1: return launch_gf<128, 1>(tm, a, st);
-    case 128 * 4 + 2: return launch_gf<128, 2>(tm, a, st);
+    case 256 * 4 + 0: return launch_gf<256, 0, false>(tm, a, st);
+    case 256 * 4 + 1: return launch_gf<256, 1, false>(tm, a, st);
+    case 256 * 4 + 2: return launch_gf<256, 2, false>(tm, a, st);
+    case 128 * 4 + 0: return launch_gf<128, 0, false>(tm, a, st);
+    case 128 * 4 + 1: return launch_gf<128, 1, false>(tm, a, st);
+    case 128 * 4 + 2: return launch_gf<128, 2, false>(tm, a, st);
   }
   return DIROTQ_E_ARG;
 }

@@ -57,6 +57,21 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity, uint32_t
       : "memory");
   return ok != 0;
 }
+// Two phase tests issued back to back (see mbar_test4).
+__device__ __forceinline__ uint32_t mbar_test2(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1) {
+  uint32_t m;
+  asm volatile(
+      "{\n\t.reg .pred q0, q1;\n\t.reg .u32 t0, t1;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 q0, [%1], %2;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 q1, [%3], %4;\n\t"
+      "selp.u32 t0, 1, 0, q0;\n\t"
+      "selp.u32 t1, 2, 0, q1;\n\t"
+      "or.b32 %0, t0, t1;\n\t}"
+      : "=r"(m)
+      : "r"(b0), "r"(p0), "r"(b1), "r"(p1)
+      : "memory");
+  return m;
+}
 // Four phase tests issued back to back, so that their latencies overlap (a test costs about a hundred
 // cycles even when the phase has long completed).  Bit i of the result: barrier i's phase is complete.
 __device__ __forceinline__ uint32_t mbar_test4(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2,
@@ -353,6 +368,17 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
+// waits for this thread's TMEM loads and names the registers they fill, so that no use of these moves before the wait
+__device__ __forceinline__ void tmem_wait_ld16(uint32_t* r) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]),
+                 "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+               :: "memory");
+}
+// Register split between the warpgroups of a block (all four warps of a group execute the same one).  The sum over the
+// groups must not exceed what the block was launched with.
+template <int N> __device__ __forceinline__ void reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 // registers -> TMEM: 32 consecutive 32-bit columns of this thread's lane
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
   asm volatile(

@@ -66,6 +66,11 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// the same, one arrival on the barrier at this shared-memory offset in BOTH CTAs of the pair
+__device__ __forceinline__ void umma_commit_pair_both(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
 // 32 rows x 16 bytes of EACH CTA's shared memory -> that CTA's TMEM lanes 0..31 (4 columns), replicated to all four
 // lane quarters; issued once by the leader
 __device__ __forceinline__ void tmem_cp_32x128b_x4_pair(uint32_t taddr, uint64_t sdesc) {
@@ -107,6 +112,24 @@ __device__ __forceinline__ void umma_f16_ss_x4_pair(uint32_t d_tmem, uint32_t a_
       "add.u32 x, %1, 6;\n\tadd.u32 y, %2, 6;\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t"
       "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, t;\n\t}"
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accum0)
+      : "memory");
+}
+// The four K = 16 pair UMMAs of one 64-wide operand stage, A from the tensor memory of both CTAs (each holds its own 128
+// rows at the same columns, 8 per step), B through a shared-memory descriptor (each CTA holds N/2 rows at the same offset).
+__device__ __forceinline__ void umma_f16_ts_x4_pair(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc_lo, uint32_t bdesc_hi,
+                                                    uint32_t idesc, uint32_t accum0) {
+  asm volatile(
+      "{\n\t.reg .pred p, t;\n\t.reg .b64 d0, d1, d2, d3;\n\t.reg .b32 l1, l2, l3, a1, a2, a3;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "add.u32 l1, %2, 2;\n\tadd.u32 l2, %2, 4;\n\tadd.u32 l3, %2, 6;\n\t"
+      "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
+      "mov.b64 d0, {%2, %3};\n\tmov.b64 d1, {l1, %3};\n\tmov.b64 d2, {l2, %3};\n\tmov.b64 d3, {l3, %3};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], d0, %4, p;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], d1, %4, t;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a2], d2, %4, t;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a3], d3, %4, t;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(bdesc_lo), "r"(bdesc_hi), "r"(idesc), "r"(accum0)
       : "memory");
 }
 

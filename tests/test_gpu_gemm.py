@@ -239,6 +239,28 @@ def test_int_f16_gemm_edge_shapes(mode, M, N, D, tail):
     assert rel_l2(y.float().cpu(), y_ref) < 4e-3
 
 
+@pytest.mark.parametrize("mode,M,N,D,tail", [("sym", 2401, 2056, 64, 0), ("int8", 2401, 2056, 192, 8),
+                                             ("sym", 15204, 1032, 128, 8), ("asym", 15240, 1032, 64, 0),
+                                             ("int8", 15233, 1032, 192, 72), ("sym", 15359, 1280, 576, 64)])
+def test_int_f16_gemm_wide_tiles(mode, M, N, D, tail):
+    """256-wide tiles on one CTA (2401 rows) and on CTA pairs (over four rounds of tiles): a last pair whose second half lies
+    past the end (15204 = 118 * 128 + 100), holds one row (15233) or all but one; a last column tile of 8 columns; K from one
+    stage to more stages than the operand ring holds."""
+    from dirotq_b200 import ops
+    m = {"sym": ops.INT4_SYM, "asym": ops.INT4_ASYM, "int8": ops.INT8_ASYM}[mode]
+    fmt = ops.ActFormat(m, D, tail_len=tail)
+    x, act, dec, qw, sw, pk, w_tail, bias = _setup_int(ops, M, N, fmt, 37)
+    lay = act.layout
+    wt = ops.pad_tail_weight(w_tail, lay.tail_pitch, N, "cuda")
+    folded = ops.fold_weight_scales_f16(pk, wt, lay.tail_total)
+    y = ops.gemm_w4a4_int_f16(act, pk, folded, bias.cuda()).float().cpu()
+    ops.check_status()
+    y_ref, _ = _oracle_int(dec, lay, qw, sw, w_tail, bias, mode != "sym")
+    assert rel_l2(y, y_ref) < 4e-3
+    # the ragged edges by themselves (a global norm would hide a few rows or columns)
+    assert rel_l2(y[-(M % 128 or 128):], y_ref[-(M % 128 or 128):]) < 4e-3 and rel_l2(y[:, -8:], y_ref[:, -8:]) < 4e-3
+
+
 def test_int_f16_gemm_empty_batch():
     from dirotq_b200 import ops
     fmt = ops.ActFormat(ops.INT4_SYM, 128, tail_len=64)
