@@ -777,16 +777,19 @@ __device__ __forceinline__ uint32_t half_twice(float v) {
   return h | (h << 16);
 }
 
-// Block = 64 rows x 4 chunk phases (thread tid: row tid & 63, chunks c = tid >> 6 (mod 4)).
-template <typename ST>
+// Block = ROWS rows x 256 / ROWS chunk phases (thread tid: row tid % ROWS, chunks c = tid / ROWS (mod 256 / ROWS)).
+// What this kernel takes is latency: two dependent passes over a few hundred bytes per thread.  So a thread's scales and zero
+// points are loaded at once, ahead of the maximum, and kept; and short calls get 16-row blocks (see fold_small_blocks).
+template <typename ST, int ROWS>
 __device__ __forceinline__ void fold_scales_block(int block, const ST* __restrict__ s, const __nv_bfloat16* __restrict__ z,
                                                   int n_chunks, int64_t rows, int64_t ld_in, uint2* __restrict__ rec,
                                                   int64_t ld_rec, float* __restrict__ rs, const __nv_bfloat16* __restrict__ tail,
                                                   __nv_bfloat16* __restrict__ tail_out, int kt_pitch) {
-  __shared__ float part_max[4][64];
-  __shared__ float inv_s[64];
-  const int lr = threadIdx.x & 63, part = threadIdx.x >> 6;
-  const int64_t r0 = (int64_t)block * 64;
+  constexpr int P = 256 / ROWS;
+  __shared__ float part_max[P][ROWS];
+  __shared__ float inv_s[ROWS];
+  const int lr = threadIdx.x % ROWS, part = threadIdx.x / ROWS;
+  const int64_t r0 = (int64_t)block * ROWS;
   const int64_t r = r0 + lr;
   // the tail tile's loads go out first: they do not depend on the scales
   const int units = tail ? kt_pitch / 8 : 0;             // 16-byte units per row
@@ -798,18 +801,30 @@ __device__ __forceinline__ void fold_scales_block(int block, const ST* __restric
     for (int it = 0; it < TAIL_IT; ++it) {
       const int i = threadIdx.x + it * 256;
       const int rr = i / units;
-      if (i < 64 * units && r0 + rr < rows) {
+      if (i < ROWS * units && r0 + rr < rows) {
         tv[it] = __ldg(reinterpret_cast<const uint4*>(tail + (r0 + rr) * kt_pitch) + (i % units));
         n_it = it + 1;
       }
     }
   }
+  constexpr int KEEP = 5;
+  float sv[KEEP], zv[KEEP];
+#pragma unroll
+  for (int k = 0; k < KEEP; ++k) {
+    const int c = part + k * P;
+    const bool in = r < rows && c < n_chunks;
+    sv[k] = in ? scale_to_float<ST>(s[(int64_t)c * ld_in + r]) : 0.f;
+    zv[k] = in && z ? __bfloat162float(z[(int64_t)c * ld_in + r]) : 8.f;
+  }
   float smax = 0.f;
+#pragma unroll
+  for (int k = 0; k < KEEP; ++k) smax = fmaxf(smax, fabsf(sv[k]));
   if (r < rows)
-    for (int c = part; c < n_chunks; c += 4) smax = fmaxf(smax, fabsf(scale_to_float<ST>(s[(int64_t)c * ld_in + r])));
+    for (int c = part + KEEP * P; c < n_chunks; c += P) smax = fmaxf(smax, fabsf(scale_to_float<ST>(s[(int64_t)c * ld_in + r])));
   part_max[part][lr] = smax;
   __syncthreads();
-  smax = fmaxf(fmaxf(part_max[0][lr], part_max[1][lr]), fmaxf(part_max[2][lr], part_max[3][lr]));
+#pragma unroll
+  for (int k = 0; k < P; ++k) smax = fmaxf(smax, part_max[k][lr]);
   int E = (int)((__float_as_uint(smax) >> 23) & 0xFF) - 127;          // smax = 1.f * 2^E
   E = max(-100, min(100, E));
   const float inv = __uint_as_float((uint32_t)(127 - 10 - E) << 23);  // 2^(-10 - E): smax * inv in [2^-10, 2^-9)
@@ -818,14 +833,17 @@ __device__ __forceinline__ void fold_scales_block(int block, const ST* __restric
     if (r < rows) rs[r] = __uint_as_float((uint32_t)(127 + 10 + E) << 23);
   }
   const float up = inv * 16777216.f;                                    // * 2^24 (E >= -100 keeps this finite)
+  auto record = [&](int c, float sc, float zp) {
+    rec[(int64_t)c * ld_rec + r] = make_uint2(half_twice(sc * up), half_twice(-zp * sc * inv));
+  };
   if (r < rows) {
-    for (int c = part; c < n_chunks; c += 4) {
-      const float sc = scale_to_float<ST>(s[(int64_t)c * ld_in + r]);
-      const float zp = z ? __bfloat162float(z[(int64_t)c * ld_in + r]) : 8.f;
-      rec[(int64_t)c * ld_rec + r] = make_uint2(half_twice(sc * up), half_twice(-zp * sc * inv));
-    }
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k)
+      if (part + k * P < n_chunks) record(part + k * P, sv[k], zv[k]);
+    for (int c = part + KEEP * P; c < n_chunks; c += P)
+      record(c, scale_to_float<ST>(s[(int64_t)c * ld_in + r]), z ? __bfloat162float(z[(int64_t)c * ld_in + r]) : 8.f);
   } else if (r < ld_rec) {
-    for (int c = part; c < n_chunks; c += 4) rec[(int64_t)c * ld_rec + r] = make_uint2(0u, 0u);
+    for (int c = part; c < n_chunks; c += P) rec[(int64_t)c * ld_rec + r] = make_uint2(0u, 0u);
   }
   if (tail == nullptr) return;
   __syncthreads();
@@ -843,22 +861,22 @@ __device__ __forceinline__ void fold_scales_block(int block, const ST* __restric
 #pragma unroll
   for (int it = 0; it < TAIL_IT; ++it)
     if (it < n_it) scale_store(threadIdx.x + it * 256, tv[it]);
-  // wide tails (more than 4 x 256 units per 64 rows): the rest, load and store in turn
-  for (int i = threadIdx.x + TAIL_IT * 256; i < 64 * units; i += 256) {
+  // wide tails (more than 4 x 256 units per block): the rest, load and store in turn
+  for (int i = threadIdx.x + TAIL_IT * 256; i < ROWS * units; i += 256) {
     const int rr = i / units;
     if (r0 + rr >= rows) break;
     scale_store(i, __ldg(reinterpret_cast<const uint4*>(tail + (r0 + rr) * kt_pitch) + (i % units)));
   }
 }
 
-template <typename ST>
+template <typename ST, int ROWS>
 __global__ void __launch_bounds__(256)
 fold_scales_kernel(const ST* __restrict__ s, const __nv_bfloat16* __restrict__ z, int n_chunks, int64_t rows, int64_t ld_in,
                    uint2* __restrict__ rec, int64_t ld_rec, float* __restrict__ rs,
                    const __nv_bfloat16* __restrict__ tail, __nv_bfloat16* __restrict__ tail_out, int kt_pitch) {
   pdl_launch_dependents();
   pdl_wait();
-  fold_scales_block<ST>((int)blockIdx.x, s, z, n_chunks, rows, ld_in, rec, ld_rec, rs, tail, tail_out, kt_pitch);
+  fold_scales_block<ST, ROWS>((int)blockIdx.x, s, z, n_chunks, rows, ld_in, rec, ld_rec, rs, tail, tail_out, kt_pitch);
 }
 
 // Weight pre-pass: codes + records -> the fp16 panel [N, n_chunks * 64] the GEMM's weight-tile TMA reads.
@@ -919,11 +937,12 @@ struct FoldExpandArgs {
   int fold_blocks;
   int hc;
 };
+template <int ROWS>
 __global__ void __launch_bounds__(256) fold_expand_kernel(const FoldExpandArgs a) {
   pdl_launch_dependents();
   pdl_wait();
   if ((int)blockIdx.x < a.fold_blocks)
-    fold_scales_block<__nv_bfloat16>((int)blockIdx.x, a.s, a.z, a.n_chunks, a.rows, a.ld_in, a.rec, a.ld_rec, a.rs, a.tail,
+    fold_scales_block<__nv_bfloat16, ROWS>((int)blockIdx.x, a.s, a.z, a.n_chunks, a.rows, a.ld_in, a.rec, a.ld_rec, a.rs, a.tail,
                                      a.tail_out, a.kt_pitch);
   else
     expand_weight_panel_block((int)blockIdx.x - a.fold_blocks, a.wq, a.w_row_bytes, a.w_rec, a.ld_wrec, a.N, a.n_chunks, a.panel,
@@ -944,12 +963,20 @@ int launch_expand_weight_panel(const uint8_t* wq, int n_chunks, int64_t N, const
 int64_t f16_ld_act(int64_t M) { return round_up64(M, 128); }
 int64_t f16_ld_weight(int64_t N) { return round_up64(N, 768); }
 
+// Rows per block of the folding kernels: 64 keeps whole sectors of scales in a warp; with fewer than two such blocks per SM
+// the chip is mostly idle, and 16 rows (a 32-byte sector of scales) spread the work over four times as many: the four linears
+// of a 2240-wide block at 1024 rows (320 16-bit channels, 16 blocks of 64 rows) 186 -> 165 us, of a 1152-wide block at 4096
+// rows 287 -> 281, 3072-wide blocks at 4608 rows 4285 -> 4225; at 32768 rows 64 rows are 0.5 % ahead.
+static bool fold_small_blocks(int64_t ld_rec) { return ld_rec / 64 < 2 * (int64_t)num_sms(); }
+
 int launch_fold_act_scales(const __nv_bfloat16* s, const __nv_bfloat16* z, int n_chunks, int64_t M, int64_t ldm,
                            void* rec, float* rs, const __nv_bfloat16* tail, __nv_bfloat16* tail_out,
                            int kt_pitch, cudaStream_t st) {
   if (M <= 0) return DIROTQ_OK;
   const int64_t ld_rec = f16_ld_act(M);
-  return launch_pdl(fold_scales_kernel<__nv_bfloat16>, dim3((unsigned)(ld_rec / 64)), dim3(256), 0, st, s, z, n_chunks, M,
+  const bool small = fold_small_blocks(ld_rec);
+  return launch_pdl(small ? fold_scales_kernel<__nv_bfloat16, 16> : fold_scales_kernel<__nv_bfloat16, 64>,
+                    dim3((unsigned)(ld_rec / (small ? 16 : 64))), dim3(256), 0, st, s, z, n_chunks, M,
                     ldm, reinterpret_cast<uint2*>(rec), ld_rec, rs, tail, tail_out, kt_pitch) == cudaSuccess
              ? DIROTQ_OK : DIROTQ_E_CUDA;
 }
@@ -964,16 +991,17 @@ int launch_fold_act_and_expand(const __nv_bfloat16* s, const __nv_bfloat16* z, i
   a.ld_rec = f16_ld_act(M); a.rs = rs; a.tail = tail; a.tail_out = tail_out; a.kt_pitch = kt_pitch;
   a.wq = wq; a.w_row_bytes = (int64_t)n_chunks * 32; a.w_rec = reinterpret_cast<const uint2*>(w_rec);
   a.ld_wrec = f16_ld_weight(N); a.N = N; a.panel = reinterpret_cast<uint4*>(panel);
-  a.fold_blocks = (int)(a.ld_rec / 64);
+  const bool small = fold_small_blocks(a.ld_rec);
+  a.fold_blocks = (int)(a.ld_rec / (small ? 16 : 64));
   const unsigned blocks = (unsigned)a.fold_blocks + (unsigned)((N * n_chunks + 255) / 256);
-  return launch_pdl(fold_expand_kernel, dim3(blocks), dim3(256), 0, st, a) == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
+  return launch_pdl(small ? fold_expand_kernel<16> : fold_expand_kernel<64>, dim3(blocks), dim3(256), 0, st, a) == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
 }
 
 int launch_fold_weight_scales(const float* s, int n_chunks, int64_t N, int64_t ldn, void* rec, float* cs,
                               const __nv_bfloat16* tail, __nv_bfloat16* tail_out, int kt_pitch, cudaStream_t st) {
   if (N <= 0) return DIROTQ_OK;
   const int64_t ld_rec = f16_ld_weight(N);
-  fold_scales_kernel<float><<<(unsigned)(ld_rec / 64), 256, 0, st>>>(
+  fold_scales_kernel<float, 64><<<(unsigned)(ld_rec / 64), 256, 0, st>>>(
       s, nullptr, n_chunks, N, ldn, reinterpret_cast<uint2*>(rec), ld_rec, cs, tail, tail_out, kt_pitch);
   return cudaGetLastError() == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
 }
