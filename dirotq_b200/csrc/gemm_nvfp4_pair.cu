@@ -186,6 +186,8 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
     if (lane == 0 && rank == 0) {
       const uint32_t idesc_f4 = idesc_nvf4(256, BN);
       const uint32_t idesc_bf = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, 256, BN);
+      const uint64_t op_d0 = smem_desc_sw128(smem_base);
+      const uint32_t op_lo0 = (uint32_t)op_d0, op_hi = (uint32_t)(op_d0 >> 32);
       GfRingT<STAGES> r;
       int buf = 0;
       uint32_t aph = 0;
@@ -198,26 +200,29 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
           // one wait covers the operand bytes of both CTAs and the scale factors in both CTAs' tensor memory
           if (!mbar_wait(full_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t sA = smem_base + r.s * Cfg::STAGE_BYTES;
-          const uint64_t adesc = smem_desc_sw128(sA), bdesc = smem_desc_sw128(sA + Cfg::A_BYTES);
+          // descriptors from loop-invariant words, a whole stage's UMMAs in one block: what this thread does between UMMAs
+          // is time the tensor pipe idles (an FP4 UMMA of a 128-wide tile keeps it busy for 64 cycles)
+          const uint32_t a_lo = op_lo0 + (uint32_t)r.s * (Cfg::STAGE_BYTES >> 4), b_lo = a_lo + (Cfg::A_BYTES >> 4);
           if (st < n_main) {
             const uint32_t sfa_t = tmem_base + Cfg::SF_COL + r.s * Cfg::SF_SLOT, sfb_t = sfa_t + 16;
             const int nkb = min(4, a.n_chunks - st * 4);
-            for (int kb = 0; kb < nkb; ++kb)
-              umma_nvf4_pair(d, adesc + 2 * kb, bdesc + 2 * kb, idesc_f4, (st > 0 || kb > 0) ? 1u : 0u, sfa_t + kb * 4,
-                             sfb_t + kb * (BN / 32));
+            if (nkb == 4) {
+              umma_nvf4_x4_pair<BN / 32>(d, a_lo, b_lo, op_hi, idesc_f4, st > 0 ? 1u : 0u, sfa_t, sfb_t);
+            } else {
+              const uint64_t hi = (uint64_t)op_hi << 32;
+              for (int kb = 0; kb < nkb; ++kb)
+                umma_nvf4_pair(d, hi | (a_lo + 2 * kb), hi | (b_lo + 2 * kb), idesc_f4, (st > 0 || kb > 0) ? 1u : 0u,
+                               sfa_t + kb * 4, sfb_t + kb * (BN / 32));
+            }
           } else {
-#pragma unroll
-            for (int kb = 0; kb < 4; ++kb) umma_f16_pair(d, adesc + 2 * kb, bdesc + 2 * kb, idesc_bf, 1u);
+            umma_f16_ss_x4_pair(d, a_lo, b_lo, op_hi, idesc_bf, st > 0 ? 1u : 0u);
           }
           // the stage is free in BOTH CTAs once these UMMAs have read it
-          umma_commit_pair(empty_bar(r.s));
-          umma_commit_pair(map_to_rank(empty_bar(r.s), 1));
+          umma_commit_pair_both(empty_bar(r.s));
           r.next();
         }
         if (!ok) break;
-        umma_commit_pair(accf_bar(buf));
-        umma_commit_pair(map_to_rank(accf_bar(buf), 1));
+        umma_commit_pair_both(accf_bar(buf));
         if (NACC == 2) {
           buf ^= 1;
           if (buf == 0) aph ^= 1;

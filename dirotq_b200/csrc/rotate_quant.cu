@@ -713,8 +713,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
           const uint32_t a_lo = op_lo0 + (uint32_t)s * (RQ_STAGE_BYTES >> 4);
           if constexpr (PAIR) {
             umma_f16_ss_x4_pair(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u);
-            umma_commit_pair(empty_bar(s));
-            umma_commit_pair(map_to_rank(empty_bar(s), 1));
+            umma_commit_pair_both(empty_bar(s));
           } else {
             umma_f16_ss_x4(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u);
             umma_commit(empty_bar(s));
@@ -723,8 +722,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
         }
         if (!ok) break;
         if constexpr (PAIR) {
-          umma_commit_pair(accf_bar(buf));
-          umma_commit_pair(map_to_rank(accf_bar(buf), 1));
+          umma_commit_pair_both(accf_bar(buf));
         } else {
           umma_commit(accf_bar(buf));
         }
