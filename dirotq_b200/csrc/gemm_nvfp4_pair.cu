@@ -10,7 +10,7 @@
 // what it keeps.
 //
 // Roles per CTA: warp 0 = TMA producer (codes and the 512-byte scale-factor tiles by tiled TMA), warp 1 = UMMA issuer
-// (leader only; allocates TMEM in both), warps 2..5 = scale-factor movers, warps 6..13 = epilogue.
+// (leader only; allocates TMEM in both), warps 4..7 = scale-factor movers, warps 8..15 = epilogue.
 // Scale factors reach tensor memory through REGISTERS: each mover warp reads the stage's tiles from shared memory
 // (16 bytes per lane and k-block) and writes them into its own TMEM lane quarter with tcgen05.st -- the layout
 // tcgen05.cp.32x128b.warpx4 would produce, four identical copies.  Measured on this kernel, the twelve tcgen05.cp per
@@ -53,8 +53,14 @@ struct GpCfg {
   static constexpr int NACC = BN == 256 ? 1 : 2;
   static constexpr int EPI_WARPS = 8;                       // two per TMEM lane quarter, BN/2 output columns each
   static constexpr int SF_WARPS = 4;                        // one per TMEM lane quarter
-  static constexpr int EPI_WARP0 = 2 + SF_WARPS;
-  static constexpr int THREADS = (2 + SF_WARPS + EPI_WARPS) * 32;
+  // Warpgroups: producer and issuer (warps 0, 1; 2 and 3 idle), movers (4..7), epilogue (8..15).  The launch gives every
+  // thread 128 registers; the first two groups hand some back to the epilogue's, which holds a quarter row of the tile
+  // (128 accumulators of a 256-wide one; with 128 registers it spilled 350 bytes a thread).
+  static constexpr int SF_WARP0 = 4, EPI_WARP0 = SF_WARP0 + SF_WARPS;
+  static constexpr int THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
+  static constexpr int REGS_LAUNCH = 128, REGS_EPI = 184, REGS_PROD = 56, REGS_SF = 72;
+  static_assert(EPI_WARPS * REGS_EPI + SF_WARP0 * REGS_PROD + SF_WARPS * REGS_SF <= THREADS / 32 * REGS_LAUNCH,
+                "setmaxnreg draws on the registers of the launch");
   static constexpr int STG_BYTES = EPI_WARPS * 2 * 2048;    // per epilogue warp: two 32 rows x 32 bf16 staging patches
   static constexpr int TAB_BYTES = BN * 8;                  // per output column of the tile: {scale, bias} as floats
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STG_BYTES + TAB_BYTES + 1024 + 256;
@@ -142,6 +148,8 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
   const int nkb_pad = n_main * 4;                // 64-element k-blocks per row tile in the scale-factor arrays
   const int first = (int)cluster_id_x(), step = (int)cluster_count_x();
 
+  if (warp < Cfg::SF_WARP0) {
+  reg_dealloc<Cfg::REGS_PROD>();
   if (warp == 0) {
     if (lane == 0) {
       GfRingT<STAGES> r;
@@ -231,7 +239,9 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
         }
       }
     }
+  }
   } else if (warp < Cfg::EPI_WARP0) {
+    reg_dealloc<Cfg::REGS_SF>();
     // ---- scale-factor movers: shared memory -> registers -> this warp's TMEM lane quarter ----
     const uint32_t q = warp & 3;
     const uint32_t ready_leader = map_to_rank(full_bar(0), 0);
@@ -278,6 +288,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
       }
     }
   } else {
+    reg_alloc<Cfg::REGS_EPI>();
     constexpr int WCOLS = BN / 2;                       // output columns per epilogue warp
     const int ew = warp - Cfg::EPI_WARP0;
     const int q = warp & 3, half = ew >> 2;
@@ -286,6 +297,28 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
     float2* tab = col_tab + half * WCOLS;               // this half's {scale, bias} per column, shared by its four warps
     constexpr int CPW = WCOLS / 4;                      // table columns filled by each of the half's four warps
     const int tcol = (ew & 3) * CPW + lane;             // this thread's column of the table (lanes below CPW)
+    // Factors of eight columns, read by all lanes from the same address: such a read takes a cycle of the shared-memory pipe
+    // per 4 bytes, and that pipe also feeds the UMMAs.  Without per-column scales only the bias is kept, in bf16: 16 bytes
+    // for eight columns instead of 64.
+    const bool one_scale = a.col_scale == nullptr;
+    auto factors = [&](int i, float (&s8)[8], float (&b8)[8]) {
+      if (one_scale) {
+        const uint4 bb = *(reinterpret_cast<const uint4*>(tab) + i);
+        const uint32_t w4[4] = {bb.x, bb.y, bb.z, bb.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          s8[2 * e] = s8[2 * e + 1] = a.out_scale;
+          b8[2 * e] = __uint_as_float(w4[e] << 16);
+          b8[2 * e + 1] = __uint_as_float(w4[e] & 0xffff0000u);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float4 sb = *reinterpret_cast<const float4*>(tab + 8 * i + 2 * e);      // {s0, b0, s1, b1}
+          s8[2 * e] = sb.x; b8[2 * e] = sb.y; s8[2 * e + 1] = sb.z; b8[2 * e + 1] = sb.w;
+        }
+      }
+    };
     int buf = 0;
     uint32_t aph = 0, patch = 0, tph = 0;
     for (int t = first; t < total_tiles; t += step) {
@@ -299,12 +332,9 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
       if (!mbar_wait(tab_bar(half, 0), tph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) break;   // all four are done with the last table
       if (lane < CPW) {
         const int64_t col = n0 + tcol;
-        float2 e = make_float2(0.f, 0.f);
-        if (col < a.N) {
-          e.x = a.col_scale ? __ldg(a.col_scale + col) * a.out_scale : a.out_scale;
-          e.y = a.bias ? __bfloat162float(a.bias[col]) : 0.f;
-        }
-        tab[tcol] = e;
+        const __nv_bfloat16 b = col < a.N && a.bias ? a.bias[col] : __float2bfloat16_rn(0.f);
+        if (one_scale) reinterpret_cast<__nv_bfloat16*>(tab)[tcol] = b;
+        else tab[tcol] = make_float2(col < a.N ? __ldg(a.col_scale + col) * a.out_scale : 0.f, __bfloat162float(b));
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(tab_bar(half, 1));
@@ -337,13 +367,17 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
           if (col0 + 64 > a.N || row0 >= a.M) continue;  // warp-uniform
           uint32_t w[32];                                // the activated output as bf16 pairs: what that layer's quantiser reads
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float4 sb = *reinterpret_cast<const float4*>(tab + 64 * c + 2 * i);
-            float f0 = __fmaf_rn(__uint_as_float(v[64 * c + 2 * i]), sb.x, sb.y);
-            float f1 = __fmaf_rn(__uint_as_float(v[64 * c + 2 * i + 1]), sb.z, sb.w);
-            if (a.act == 1) { f0 = gelu_tanh_bf16(f0); f1 = gelu_tanh_bf16(f1); }
-            __nv_bfloat162 h2 = __floats2bfloat162_rn(f0, f1);
-            w[i] = *reinterpret_cast<uint32_t*>(&h2);
+          for (int i = 0; i < 8; ++i) {
+            float s8[8], b8[8];
+            factors(8 * c + i, s8, b8);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              float f0 = __fmaf_rn(__uint_as_float(v[64 * c + 8 * i + 2 * e]), s8[2 * e], b8[2 * e]);
+              float f1 = __fmaf_rn(__uint_as_float(v[64 * c + 8 * i + 2 * e + 1]), s8[2 * e + 1], b8[2 * e + 1]);
+              if (a.act == 1) { f0 = gelu_tanh_bf16(f0); f1 = gelu_tanh_bf16(f1); }
+              __nv_bfloat162 h2 = __floats2bfloat162_rn(f0, f1);
+              w[4 * i + e] = *reinterpret_cast<uint32_t*>(&h2);
+            }
           }
           if (a.y != nullptr) {                          // the bf16 tensor as well, when the caller wants it
 #pragma unroll
@@ -405,11 +439,12 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
         for (int i4 = 0; i4 < 4; ++i4) {
           const int i = 4 * p + i4;
           uint32_t w[4];
+          float s8[8], b8[8];
+          factors(i, s8, b8);
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
-            const float4 sb = *reinterpret_cast<const float4*>(tab + 8 * i + 2 * e);    // {s0, b0, s1, b1}, same address in all lanes
-            float f0 = __fmaf_rn(__uint_as_float(v[8 * i + 2 * e]), sb.x, sb.y);
-            float f1 = __fmaf_rn(__uint_as_float(v[8 * i + 2 * e + 1]), sb.z, sb.w);
+            float f0 = __fmaf_rn(__uint_as_float(v[8 * i + 2 * e]), s8[2 * e], b8[2 * e]);
+            float f1 = __fmaf_rn(__uint_as_float(v[8 * i + 2 * e + 1]), s8[2 * e + 1], b8[2 * e + 1]);
             if (a.act == 1) { f0 = gelu_tanh_bf16(f0); f1 = gelu_tanh_bf16(f1); }
             __nv_bfloat162 h2 = __floats2bfloat162_rn(f0, f1);
             w[e] = *reinterpret_cast<uint32_t*>(&h2);
@@ -482,6 +517,12 @@ static int launch_pair(const GemmFp4Args& a, cudaStream_t st) {
   auto k = gemm_nvfp4_pair_kernel<BN, QOUT>;
   static PerDeviceOnce attr_once;
   if (int rc2 = set_max_dynamic_smem(attr_once, k, Cfg::SMEM_BYTES)) return rc2;
+  // the register split is only sound if the kernel was compiled to the launch's share
+  static const bool regs_ok = [&] {
+    cudaFuncAttributes fa;
+    return cudaFuncGetAttributes(&fa, k) == cudaSuccess && fa.numRegs >= Cfg::REGS_LAUNCH;
+  }();
+  if (!regs_ok) return DIROTQ_E_UNSUPPORTED;
   const int tiles = (int)((a.M + 255) / 256) * (int)((a.N + BN - 1) / BN);
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(Cfg::THREADS);

@@ -274,6 +274,16 @@ def test_int_f16_gemm_empty_batch():
     ops.check_status()
 
 
+@pytest.mark.parametrize("tile", ["pair128", "pair256"])
+@pytest.mark.parametrize("M,N,D,tail", [(129, 8, 64, 0), (257, 264, 256, 16), (515, 520, 1152, 80)])
+def test_nvfp4_gemm_pair_tiles(monkeypatch, tile, M, N, D, tail):
+    """Both pair-tile widths at their edges: one k-block, partial and whole stages, a last pair whose second half is empty or
+    holds few rows, a last column tile of 8 columns; the bias table with and without per-channel scales."""
+    monkeypatch.setenv("DIROTQ_NVFP4_TILE", tile)
+    test_nvfp4_gemm(M, N, D, tail)
+    test_nvfp4_gemm_per_channel_weight_scale(M, N, D, tail)
+
+
 # K order of a 64-slot chunk in the expanded operands: per planar-32 block (byte j = code j | code 16+j << 4),
 # per 32-bit word wi of the block: low nibbles of bytes 0 and 2, high nibbles of bytes 0 and 2, then bytes 1 and 3
 def _panel_k_order():
