@@ -58,7 +58,8 @@ def _regions(st, M):
 
 @pytest.mark.parametrize("quant,a_sym", [("int4", True), ("int4", False), ("nvfp4", True)])
 @pytest.mark.parametrize("M,inner,tail_down", [(520, 1536, 0), (300, 1536, 128), (129, 1472, 64),
-                                                (4700, 1536, 128)])     # the last one takes 192-wide column tiles
+                                                (4700, 1536, 128),      # 256-wide column tiles (INT)
+                                                (12929, 1536, 128)])    # 256-wide on CTA pairs, one row in the last half
 def test_epilogue_quantises_for_the_down_projection(quant, a_sym, M, inner, tail_down):
     from dirotq_b200 import backend, ops
     from dirotq_b200.synth import synth_activations
