@@ -38,6 +38,7 @@ _FMT, _LAY = C.POINTER(ActFormatC), C.POINTER(ActLayoutC)
 SIGNATURES = {
     "dirotq_abi_version": (C.c_int, []),
     "dirotq_set_wait_limit_cycles": (C.c_int, [_I64]),
+    "dirotq_stream_capture_id": (_I64, [_P]),
     "dirotq_error_string": (C.c_char_p, [C.c_int]),
     "dirotq_status_string": (C.c_char_p, [C.c_int]),
     "dirotq_act_layout_of": (C.c_int, [_FMT, _LAY]),

@@ -14,7 +14,9 @@ call (dirotq_linear_forward); the quantised weight is packed once, when the laye
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 import sys
+import threading
 import warnings
 import weakref
 import dataclasses
@@ -30,13 +32,102 @@ from .wrapper import ActQuantWrapper
 _HW_NVFP4_ACT_SCALE = 1.0   # static fp32 tensor scale of NVFP4 activations (UE4M3 then covers amax up to 2688)
 
 
+# ---------------------------------------------------------------------------------------------------------------------
+# Scratch.  The kernels get a layer's workspace as a raw pointer, so a buffer serves one place only -- the calls that one
+# stream issues outside a capture, or one captured graph -- and is never replaced while such a pointer can still be followed:
+#   * outside a capture every layer keeps one buffer per stream, for the row count it last saw there (a buffer is allocated
+#     and replaced on its own stream, whose order covers the kernels that still use the old one);
+#   * inside a WorkspaceScope (dit.GraphedCall) the buffers belong to the scope, which whoever replays the graph keeps;
+#   * in a capture without a scope every call gets memory of the graph's own pool, cleared by the graph.
+# ---------------------------------------------------------------------------------------------------------------------
+_LOCAL = threading.local()
+_SCOPE_SERIAL = itertools.count(1)
+
+
+def _place(device) -> tuple:
+    """Where a call runs, as far as scratch and the results held in it go: (device, stream, scope, capture)."""
+    if device.type != "cuda":
+        return (None, 0, 0, 0)
+    idx = device.index if device.index is not None else torch.cuda.current_device()
+    stream = torch._C._cuda_getCurrentRawStream(idx)
+    scope = getattr(_LOCAL, "scope", None)
+    capture = _lib.lib().dirotq_stream_capture_id(stream) if torch._C._cuda_isCurrentStreamCapturing() else 0
+    return (idx, stream, 0 if scope is None else scope.serial, capture)
+
+
+class WorkspaceScope:
+    """The workspaces of one captured step: layers called inside `with scope:` use buffers of the scope's own, made by the
+    eager call that precedes the capture.  They live as long as the scope, so that calls of other sizes or on other streams
+    neither replace nor overwrite what the graph's nodes point at.  Graphs captured under one scope share its buffers and
+    are replayed one after the other.  The buffers are memory of the stream that made the scope, where the replays run: a
+    scope may be dropped while a replay is in flight there."""
+
+    def __init__(self):
+        self.serial = next(_SCOPE_SERIAL)
+        self._home = torch.cuda.current_stream() if torch.cuda.is_available() else None
+        self._ws: Dict[tuple, tuple] = {}              # (id of the owner, rows) -> (owner, buffer)
+        self._outer: list = []
+
+    def __enter__(self):
+        self._outer.append(getattr(_LOCAL, "scope", None))
+        _LOCAL.scope = self
+        return self
+
+    def __exit__(self, *exc):
+        _LOCAL.scope = self._outer.pop()
+        for owner, _ in self._ws.values():             # what was held for calls inside the scope is of no use outside
+            owner.forget(lambda place: place[2] == self.serial)
+
+    def buffer(self, owner, M: int, make) -> torch.Tensor:
+        e = self._ws.get((id(owner), M))
+        if e is None:
+            if self._home is None:
+                e = (owner, make())
+            else:
+                with torch.cuda.stream(self._home):
+                    e = (owner, make())
+                torch.cuda.current_stream(e[1].device).wait_stream(self._home)
+            self._ws[(id(owner), M)] = e
+        return e[1]
+
+
+def _buffer(owner, live: dict, M: int, place: tuple, make) -> torch.Tensor:
+    """The scratch buffer of `owner` (a layer or a sibling group) for a call of M rows at `place`."""
+    scope = getattr(_LOCAL, "scope", None)
+    if scope is not None and (place[3] == 0 or (id(owner), M) in scope._ws):
+        return scope.buffer(owner, M, make)
+    if place[3]:
+        return make()
+    e = live.get(place[:2])
+    if e is None or e[0] != M:
+        e = live[place[:2]] = (M, make())              # keep one size; diffusion steps reuse the same M
+    return e[1]
+
+
+def _drop_places(held: dict, gone):
+    for p in [p for p in held if gone(p)]:
+        held.pop(p, None)
+
+
+class _Held:
+    """A quantised tensor in a workspace: the tensor, what identifies it, and who has used it."""
+    __slots__ = ("x", "key", "seen", "ws", "y_all")
+
+    def __init__(self, x, key, seen, ws=None, y_all=None):
+        self.x, self.key, self.seen, self.ws, self.y_all = x, key, seen, ws, y_all
+
+
+def _tensor_key(x: torch.Tensor) -> tuple:
+    return (x.data_ptr(), x._version, x.shape, x.stride(), x.dtype)
+
+
 class SharedActivation:
     """Quantised activations shared by sibling layers that see the same input through the same rotation
     and format (attn.to_q / to_k / to_v: the reference gives all three `evec @ R1` of one basis,
     models/pixart-sigma/model_utils.py:84-92, and diffusers calls them on one hidden_states tensor).
     The first member called on a tensor rotates and quantises it into the group's workspace; members
-    called next on the SAME tensor run only their GEMM.  "Same" = same storage address, shape and
-    in-place version counter, with a reference held so that the storage cannot be recycled in between;
+    called next on the SAME tensor at the same place (stream, captured graph) run only their GEMM.  "Same" = same storage
+    address, shape and in-place version counter, with a reference held so that the storage cannot be recycled in between;
     the reference is dropped once every member has used it (or by release()).  Buffers that this library
     itself fills through raw pointers (`out=` arguments) have their version counter advanced explicitly
     (ops.mark_written), so a reused output buffer is never mistaken for the tensor quantised before."""
@@ -44,43 +135,53 @@ class SharedActivation:
     def __init__(self, n_members: int):
         self.n_members = n_members
         self.members: list = []          # the LayerStates: the workspace is sized for the largest of them
-        self.ws: Dict[int, torch.Tensor] = {}
-        self.x_ref: Optional[torch.Tensor] = None
-        self.key = None
-        self.seen = set()
+        self.ws: Dict[tuple, tuple] = {}               # see _buffer
+        self.held: Dict[tuple, _Held] = {}             # place -> the tensor whose codes a workspace holds there
         self.hits = 0
         self.misses = 0
         self.fused: Optional["LayerState"] = None     # one layer over the members' weights, concatenated along N
         self.offsets: list = []                        # first output column of each member in the fused layer
-        self.y_all: Optional[torch.Tensor] = None      # [M, sum N]: output of the fused GEMM for the held tensor
         self.incomplete = 0                            # fused passes whose result some member never picked up
 
-    @staticmethod
-    def _key(x: torch.Tensor):
-        idx = x.device.index
-        stream = torch._C._cuda_getCurrentRawStream(idx) if x.is_cuda else 0
-        return (x.data_ptr(), x._version, x.shape, x.stride(), x.dtype, idx, stream)
+    @property
+    def x_ref(self) -> Optional[torch.Tensor]:
+        """A held tensor, if any."""
+        return next((h.x for h in list(self.held.values())), None)
 
-    def lookup(self, x: torch.Tensor, member_id: int) -> bool:
-        """True if the workspace already holds this tensor's codes and `member_id` has not used them yet."""
-        hit = self.x_ref is not None and self.key == self._key(x) and member_id not in self.seen
-        if hit:
-            self.hits += 1
-            self.seen.add(member_id)
-            if len(self.seen) == self.n_members:
-                self.x_ref, self.key = None, None
-        return hit
+    @property
+    def y_all(self) -> Optional[torch.Tensor]:
+        """[M, sum N] output of the fused GEMM for a held tensor, if any."""
+        return next((h.y_all for h in list(self.held.values()) if h.y_all is not None), None)
 
-    def store(self, x: torch.Tensor, member_id: int):
+    def lookup(self, x: torch.Tensor, member_id: int, place: Optional[tuple] = None) -> Optional[_Held]:
+        """The record of this tensor's codes, if a workspace holds them here and `member_id` has not used them yet."""
+        place = _place(x.device) if place is None else place
+        h = self.held.get(place)
+        if h is None or h.key != _tensor_key(x) or member_id in h.seen:
+            return None
+        self.hits += 1
+        h.seen.add(member_id)
+        if len(h.seen) == self.n_members:
+            self.held.pop(place, None)
+        return h
+
+    def store(self, x: torch.Tensor, member_id: int, place: Optional[tuple] = None, ws=None, y_all=None) -> _Held:
+        place = _place(x.device) if place is None else place
         self.misses += 1
-        if self.x_ref is not None and len(self.seen) < self.n_members:
+        if place in self.held:
             self.incomplete += 1
-        self.x_ref, self.key, self.seen = x, self._key(x), {member_id}
+        if place[3]:
+            self.forget(lambda p: p[3] not in (0, place[3]))       # captures that are over
+        h = self.held[place] = _Held(x, _tensor_key(x), {member_id}, ws, y_all)
+        return h
+
+    def forget(self, gone):
+        _drop_places(self.held, gone)
 
     def release(self):
-        """Forget the held activation tensor (it stays referenced until every member has used it, which never
+        """Forget the held activation tensors (they stay referenced until every member has used them, which never
         happens when the members of a group do not all see the same input, e.g. a cross-attention)."""
-        self.x_ref, self.key, self.seen, self.y_all = None, None, set(), None
+        self.held.clear()
 
 
 @dataclass
@@ -107,13 +208,21 @@ class LayerState:
     w_rowscale: Optional[torch.Tensor] = None        # NVFP4: fp32 per-channel weight scale (reference recipe)
     chain_next: Optional["LayerState"] = None        # this layer's GEMM epilogue quantises its output for that layer
     chain_keep_output: bool = True                   # False: the bf16 output itself is never written (nobody else reads it)
-    handed: Optional[torch.Tensor] = None            # consumer side: the producer's output whose codes the workspace holds
-    handed_key: Optional[tuple] = None
+    handed_at: Dict[tuple, _Held] = field(default_factory=dict)    # consumer side: per place, the producer's output whose
+                                                     # codes a workspace of this layer holds
     chain_hits: int = 0
     chain_fed: bool = False                          # a producer's epilogue quantises for this layer
     panel_declined: bool = False                     # a large-batch call found the resident-panel budget spent
     _c: Optional[LinearC] = None
-    _ws: Dict[int, torch.Tensor] = field(default_factory=dict)
+    _ws: Dict[tuple, tuple] = field(default_factory=dict)          # see _buffer
+
+    @property
+    def handed(self) -> Optional[torch.Tensor]:
+        """A producer's output that waits for this layer, if any."""
+        return next((h.x for h in list(self.handed_at.values())), None)
+
+    def forget(self, gone):
+        _drop_places(self.handed_at, gone)
 
     def c_struct(self) -> LinearC:
         if self._c is None:
@@ -125,23 +234,14 @@ class LayerState:
                               int(self.epilogue_act), p(f.panel if f else None))
         return self._c
 
-    def workspace(self, M: int, device) -> torch.Tensor:
-        if self.shared is not None:
-            ws = self.shared.ws.get(M)
-            if ws is None:
-                n = max(int(_lib.lib().dirotq_linear_workspace_bytes(C.byref(m.c_struct()), M))
-                        for m in (self.shared.members or [self]))
-                ws = torch.zeros(max(n, 256), dtype=torch.uint8, device=device)
-                self.shared.ws = {M: ws}
-                self.shared.x_ref, self.shared.key = None, None
-            return ws
-        ws = self._ws.get(M)
-        if ws is None:
-            n = int(_lib.lib().dirotq_linear_workspace_bytes(C.byref(self.c_struct()), M))
-            # zero once: padding entries of the scale-factor tiles are never written afterwards
-            ws = torch.zeros(max(n, 256), dtype=torch.uint8, device=device)
-            self._ws = {M: ws}          # keep one size; diffusion steps reuse the same M
-        return ws
+    def workspace(self, M: int, device, place: Optional[tuple] = None) -> torch.Tensor:
+        place = _place(torch.device(device)) if place is None else place
+        grp = self.shared
+        # zero once: padding entries of the scale-factor tiles are never written afterwards
+        make = lambda: torch.zeros(max([256] + [int(_lib.lib().dirotq_linear_workspace_bytes(C.byref(m.c_struct()), M))
+                                                for m in (grp.members if grp is not None and grp.members else [self])]),
+                                   dtype=torch.uint8, device=device)
+        return _buffer(self, self._ws, M, place, make) if grp is None else _buffer(grp, grp.ws, M, place, make)
 
 
 def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
@@ -194,19 +294,19 @@ def linear_forward(st: LayerState, x2d: torch.Tensor, out: Optional[torch.Tensor
     M = x2d.shape[0]
     if M == 0:
         return out if out is not None else torch.empty(0, st.out_features, dtype=torch.bfloat16, device=x2d.device)
+    place = _place(x2d.device)
     grp = st.shared
     if grp is not None and grp.fused is not None:
         # siblings fused into one layer: the first member called on a tensor runs it, the others take their columns
         if grp.incomplete > 2:
-            grp.fused, grp.y_all = None, None            # the members do not see the same tensor after all: separate GEMMs
+            grp.fused = None                             # the members do not see the same tensor after all: separate GEMMs
+            grp.held.clear()
         else:
-            if not grp.lookup(x2d, st.member_id):
-                grp.store(x2d, st.member_id)
-                grp.y_all = linear_forward(grp.fused, x2d)
+            h = grp.lookup(x2d, st.member_id, place)
+            if h is None:
+                h = grp.store(x2d, st.member_id, place, y_all=linear_forward(grp.fused, x2d))
             off = grp.offsets[st.member_id]
-            part = grp.y_all[:, off:off + st.out_features]
-            if grp.x_ref is None:
-                grp.y_all = None                         # every member has its view
+            part = h.y_all[:, off:off + st.out_features]
             if out is not None:
                 out.copy_(part)
                 return out
@@ -221,42 +321,45 @@ def linear_forward(st: LayerState, x2d: torch.Tensor, out: Optional[torch.Tensor
         half = bool(_lib.lib().dirotq_linear_uses_half_chunks(C.byref(st.c_struct())))
         st.folded.panel = ops.expand_weight_panel_f16(pk, st.folded, half)
         st._c = None
-        if st.shared is None and st.handed is None:
+        if st.shared is None:
             st._ws = {}                 # the workspace no longer needs room for a per-call panel
     elif CACHE_WEIGHT_PANEL == "auto" and st.folded is not None and st.folded.panel is None and M > PANEL_CACHE_MAX_ROWS:
         st.panel_declined = True        # over the budget: asked once, not on every call
-    ws = st.workspace(M, x2d.device)
     watch = ops.status_watch(x2d.device)
     if WATCH_STATUS:
         watch.poll()                    # a wait that ran out in an earlier call surfaces here (no synchronisation)
     lib = _lib.lib()
-    lin, yp, wsp, wsn, status, stream = C.byref(st.c_struct()), y.data_ptr(), ws.data_ptr(), ws.numel(), watch.ptr, ops.stream_ptr()
-    if st.handed is not None:
-        hit = st.handed_key == SharedActivation._key(x2d)
-        st.handed, st.handed_key = None, None
-        if hit:
-            # the producer's epilogue left this tensor's codes, scales and 16-bit channels in the workspace
-            st.chain_hits += 1
-            check(lib.dirotq_linear_gemm_prequantised(lin, M, yp, wsp, wsn, status, stream), "dirotq_linear_gemm_prequantised")
-            if out is not None:
-                ops.mark_written(out)
-            return y
+    lin, yp, status, stream = C.byref(st.c_struct()), y.data_ptr(), watch.ptr, ops.stream_ptr()
+    h = st.handed_at.pop(place, None) if st.handed_at else None
+    if h is not None and h.key == _tensor_key(x2d):
+        # the producer's epilogue left this tensor's codes, scales and 16-bit channels in the workspace
+        st.chain_hits += 1
+        check(lib.dirotq_linear_gemm_prequantised(lin, M, yp, h.ws.data_ptr(), h.ws.numel(), status, stream),
+              "dirotq_linear_gemm_prequantised")
+        if out is not None:
+            ops.mark_written(out)
+        return y
+    h = grp.lookup(x2d, st.member_id, place) if grp is not None else None
+    ws = h.ws if h is not None else st.workspace(M, x2d.device, place)
+    wsp, wsn = ws.data_ptr(), ws.numel()
     nxt = st.chain_next
-    if nxt is not None and st.shared is None and not nxt.hadamard_low_dim:
-        nws = nxt.workspace(M, x2d.device)
+    if nxt is not None and grp is None and not nxt.hadamard_low_dim:
+        nws = nxt.workspace(M, x2d.device, place)
         check(lib.dirotq_linear_forward_chain(lin, x2d.data_ptr(), M, yp if st.chain_keep_output else None, wsp, wsn,
                                               C.byref(nxt.c_struct()), nws.data_ptr(), nws.numel(), status, stream),
               "dirotq_linear_forward_chain")
         if out is not None:
             ops.mark_written(out)
-        nxt.handed, nxt.handed_key = y, SharedActivation._key(y)
+        if place[3]:
+            nxt.forget(lambda p: p[3] not in (0, place[3]))        # captures that are over
+        nxt.handed_at[place] = _Held(y, _tensor_key(y), (), nws)
         return y
-    if st.shared is not None and st.shared.lookup(x2d, st.member_id):
+    if h is not None:
         check(lib.dirotq_linear_gemm(lin, M, yp, wsp, wsn, status, stream), "dirotq_linear_gemm")
     else:
-        if st.shared is not None:
-            st.shared.store(x2d, st.member_id)
         check(lib.dirotq_linear_forward(lin, x2d.data_ptr(), M, yp, wsp, wsn, status, stream), "dirotq_linear_forward")
+        if grp is not None:
+            grp.store(x2d, st.member_id, place, ws)
     if out is not None:
         ops.mark_written(out)
     return y
@@ -515,6 +618,8 @@ _W4A16_SCRATCH: Dict[tuple, torch.Tensor] = {}
 
 
 def _w4a16_scratch(nbytes: int, device) -> torch.Tensor:
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)       # the graph's own: the one below may be outgrown
     key = (torch.device(device).index, torch.cuda.current_stream(device).cuda_stream)
     buf = _W4A16_SCRATCH.get(key)
     if buf is None or buf.numel() < nbytes:

@@ -24,6 +24,13 @@ int dirotq_set_wait_limit_cycles(int64_t cycles) {
   return DIROTQ_OK;
 }
 
+int64_t dirotq_stream_capture_id(void* stream) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &s, &id) != cudaSuccess) return -1;
+  return s == cudaStreamCaptureStatusNone ? 0 : (int64_t)id;
+}
+
 const char* dirotq_error_string(int code) {
   switch (code) {
     case DIROTQ_OK: return "ok";

@@ -249,29 +249,27 @@ class LinearPathStep(nn.Module):
 class GraphedCall:
     """fn() captured once into a CUDA graph and replayed: for steps whose kernels are short enough that launching them
     from Python bounds the step (a batch shard of one sample per GPU: the model-shaped PixArt step is 30 % faster replayed
-    than launched).  fn must be a pure function of device tensors that stay where they are (inputs, weights, the layers'
-    workspaces, all allocated by an earlier call); it is called once on a side stream first, so that lazily built state
-    (resident weight panels, workspaces) exists before the capture.  The status watch of the forward is off during the
-    capture (an event query cannot be captured); call ops.check_status() after replays instead."""
+    than launched).  fn must be a pure function of device tensors that stay where they are (inputs, weights); it is called
+    once on a side stream first, so that lazily built state (resident weight panels, workspaces) exists before the capture.
+    The layers' workspaces inside the graph belong to `scope`, kept here: calls of the same layers outside, of any size and
+    on any stream, leave a replay's scratch alone.  Calls given one scope share it and must be replayed one after the other.
+    A replay does not look at the status word: call ops.check_status()."""
 
-    def __init__(self, fn):
+    def __init__(self, fn, scope=None):
         from . import backend
         self.fn, self.graph, self.out = fn, None, None
-        saved = backend.WATCH_STATUS
-        backend.WATCH_STATUS = False
-        try:
-            cur = torch.cuda.current_stream()
-            side = torch.cuda.Stream()
-            side.wait_stream(cur)
-            with torch.cuda.stream(side), torch.no_grad():
+        self.scope = backend.WorkspaceScope() if scope is None else scope
+        cur = torch.cuda.current_stream()
+        side = torch.cuda.Stream()
+        side.wait_stream(cur)
+        with self.scope, torch.no_grad():
+            with torch.cuda.stream(side):
                 fn()
             cur.wait_stream(side)
             graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph), torch.no_grad():
+            with torch.cuda.graph(graph):
                 self.out = fn()
-            self.graph = graph
-        finally:
-            backend.WATCH_STATUS = saved
+        self.graph = graph
 
     def __call__(self):
         self.graph.replay()
@@ -304,7 +302,9 @@ class HostStreamedStep:
         """Replay the step from a CUDA graph, one per input buffer (small batches: Python's launch cost shows).  The
         result of a replay lives in the graph's own memory; it is overwritten two calls later, after its copy to the
         host has completed."""
-        self.replay = [GraphedCall(lambda b=b: self.step(self.x_dev[b])) for b in range(2)]
+        from . import backend
+        scope = backend.WorkspaceScope()                      # replayed in turn on one stream: one set of workspaces
+        self.replay = [GraphedCall(lambda b=b: self.step(self.x_dev[b]), scope) for b in range(2)]
 
     def __call__(self):
         b = self.i & 1

@@ -400,6 +400,9 @@ int dirotq_abi_version(void);
  * context stays usable and the outputs of that launch are undefined.  The setting is process-wide and applies to
  * launches made after the call.  No counterpart in the reference (its eager kernels have no waits of their own). */
 int dirotq_set_wait_limit_cycles(int64_t cycles);
+/* Identity of the capture `stream` is in: unique in the process, 0 outside a capture, -1 if the stream cannot be asked.
+ * What a captured launch left in a workspace holds for launches of the same capture only. */
+int64_t dirotq_stream_capture_id(void* stream);
 const char* dirotq_error_string(int code);
 /* Text for a positive device status code (which wait ran out). */
 const char* dirotq_status_string(int status);

@@ -359,3 +359,70 @@ def test_fused_layers_over_changing_row_counts():
             want = run(ws_f, ff_f, x)
             ops.check_status()
             assert all(torch.equal(a, b) for a, b in zip(got, want)), (case, quant, a_sym, dim, M)
+
+
+@pytest.mark.parametrize("quant", ["int4", "nvfp4"])
+def test_captured_step_keeps_its_scratch(quant):
+    """A step captured at one size, the same layers then called at others and the memory they let go of overwritten:
+    the replay returns what it returned before."""
+    from dirotq_b200 import backend, dit, ops
+    from dirotq_b200.synth import synth_activations
+    step = dit.LinearPathStep(dit.flux_double_block(k_down=0), 1, quant, device="cuda", seed=4400)
+    backend.preconvert_rotations_to_device(step, "cuda")
+    backend.fuse_gelu_modules(step)
+    backend.fuse_ffn_quantise(step, keep_hidden=False)
+    backend.fuse_sibling_gemms(step)
+    x = {M: synth_activations(M, 3072, torch.Generator().manual_seed(M)).reshape(1, M, 3072).cuda() for M in (300, 640, 1100)}
+    with torch.no_grad():
+        want = {M: step(v).clone() for M, v in x.items()}
+        replay = dit.GraphedCall(lambda: step(x[640]))
+        assert torch.equal(replay(), want[640])
+        for M in (1100, 300, 1100):
+            assert torch.equal(step(x[M]), want[M])
+            junk = [torch.full((n,), 0x7F, dtype=torch.uint8, device="cuda") for n in (1 << 20, 1 << 22, 1 << 24)]
+            assert torch.equal(replay(), want[640])
+        # a graph captured by hand has its scratch in its own pool
+        graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            y = step(x[300])
+        for _ in range(2):
+            graph.replay()
+            assert torch.equal(y, want[300]) and torch.equal(step(x[1100]), want[1100])
+    del junk
+    ops.check_status()
+
+
+@pytest.mark.parametrize("quant", ["int4", "nvfp4"])
+def test_same_layers_called_from_two_streams(quant):
+    """Siblings that share a pass and a feed-forward pair that hands its codes over, called in turns from two streams with
+    different tensors of one size, return what they return alone."""
+    from dirotq_b200 import backend, dit, ops
+    from dirotq_b200.synth import synth_activations
+    M, rounds = 2048, 6
+    root, ff, up, down = _pair(1536, 128, True, 87)
+    assert backend.fuse_ffn_quantise(root, keep_hidden=False) == 1
+    step = dit.LinearPathStep(dit.flux_double_block(k_down=0), 1, quant, device="cuda", seed=4500)
+    backend.preconvert_rotations_to_device(step, "cuda")
+    q, k = step.layers[0], step.layers[1]
+    assert q._b200_state.shared is k._b200_state.shared is not None
+    gen = lambda d, s: synth_activations(M, d, torch.Generator().manual_seed(s)).reshape(1, M, d).cuda()
+    xs = [[gen(384, 10 * s + i) for i in range(rounds)] for s in range(2)]
+    zs = [[gen(3072, 500 + 10 * s + i) for i in range(rounds)] for s in range(2)]
+    with torch.no_grad():
+        want = [[(ff.net[2](ff.net[0](x)), q(z), k(z)) for x, z in zip(xs[s], zs[s])] for s in range(2)]
+        torch.cuda.synchronize()
+        streams, got = [torch.cuda.Stream() for _ in range(2)], [[], []]
+        for i in range(rounds):
+            part = [[], []]
+            for call in (lambda s: q(zs[s][i]), lambda s: ff.net[0](xs[s][i]), lambda s: k(zs[s][i]), lambda s: ff.net[2](part[s][1])):
+                for s in range(2):
+                    with torch.cuda.stream(streams[s]):
+                        part[s].append(call(s))
+            for s in range(2):
+                got[s].append((part[s][3], part[s][0], part[s][2]))
+        torch.cuda.synchronize()
+    for s in range(2):
+        for g, w in zip(got[s], want[s]):
+            assert all(torch.equal(a, b) for a, b in zip(g, w))
+    ops.check_status()

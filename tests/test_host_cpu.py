@@ -278,3 +278,70 @@ def test_modulation_vectors_are_taken_through_their_views():
     v, pitch = ops._mod_vec(torch.zeros(1, D, dtype=torch.bfloat16), B, D)   # one vector shared by all samples
     assert pitch == 0
     assert ops._mod_vec(None, B, D) == (None, 0)
+
+
+def test_workspaces_belong_to_one_stream_or_one_captured_step(monkeypatch):
+    """A layer's scratch is reached by the kernels as a raw pointer: calls at another place (stream, captured graph) get
+    another buffer, a call of another size does not replace what a captured step points at, and codes held at one place
+    are not taken for those of another."""
+    from dirotq_b200 import backend, ops
+    fmt = ops.ActFormat(ops.INT4_SYM, 1152, 64)
+    lay = ops.act_layout(fmt)
+    cpu = torch.device("cpu")
+    here = [(0, 11, 0, 0)]
+    monkeypatch.setattr(backend, "_place", lambda device: here[0])
+    layer = lambda: backend.LayerState(fmt, lay, 1152, None, None, torch.zeros(1), torch.zeros(1), None, None, None)
+    st, a, b = layer(), layer(), layer()
+    grp = backend.SharedActivation(2)
+    grp.members = [a, b]
+    a.shared, b.shared, b.member_id = grp, grp, 1
+    for owner in (st, a):
+        here[0] = (0, 11, 0, 0)
+        w_a = owner.workspace(256, cpu)
+        assert owner.workspace(256, cpu) is w_a
+        here[0] = (0, 12, 0, 0)
+        w_b = owner.workspace(256, cpu)
+        assert w_b.data_ptr() != w_a.data_ptr()
+        here[0] = (0, 11, 0, 0)
+        assert owner.workspace(512, cpu).data_ptr() != w_a.data_ptr()          # one size per stream ...
+        here[0] = (0, 12, 0, 0)
+        assert owner.workspace(256, cpu) is w_b                                # ... and the other stream keeps its own
+    # a captured step: its buffers outlive calls of other sizes, and calls outside get others
+    scope = backend.WorkspaceScope()
+    with scope:
+        here[0] = (0, 13, scope.serial, 0)
+        w_warm = st.workspace(256, cpu)
+        here[0] = (0, 14, scope.serial, 901)
+        assert st.workspace(256, cpu) is w_warm
+        fresh = st.workspace(128, cpu)                                         # not seen by the eager call: the graph's memory
+        assert st.workspace(128, cpu) is not fresh
+    here[0] = (0, 13, 0, 0)
+    assert st.workspace(256, cpu).data_ptr() != w_warm.data_ptr()
+    st.workspace(512, cpu)
+    with scope:
+        here[0] = (0, 13, scope.serial, 0)
+        assert st.workspace(256, cpu) is w_warm
+    # a capture without a scope keeps nothing: the memory is the graph's
+    here[0] = (0, 14, 0, 902)
+    w = st.workspace(256, cpu)
+    assert st.workspace(256, cpu) is not w
+    # codes held at one place are found there only, and end with the scope or capture they belong to
+    x = torch.zeros(4, 8)
+    here[0] = (0, 11, 0, 0)
+    held = grp.store(x, 0, ws=w)
+    for other in ((0, 12, 0, 0), (0, 11, 7, 0), (0, 11, 0, 903)):
+        here[0] = other
+        assert not grp.lookup(x, 1)
+    here[0] = (0, 14, 0, 904)
+    grp.store(x, 0, ws=w)
+    here[0] = (0, 14, 0, 905)
+    assert not grp.lookup(x, 1)
+    grp.store(x, 0, ws=w)
+    assert sorted(grp.held) == [(0, 11, 0, 0), (0, 14, 0, 905)]
+    with scope:
+        here[0] = (0, 13, scope.serial, 0)
+        a.workspace(256, cpu)
+        grp.store(x, 0)
+    assert sorted(grp.held) == [(0, 11, 0, 0), (0, 14, 0, 905)]
+    here[0] = (0, 11, 0, 0)
+    assert grp.lookup(x, 1) is held and (0, 11, 0, 0) not in grp.held
