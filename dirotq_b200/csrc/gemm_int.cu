@@ -79,7 +79,8 @@ gemm_int_kernel(const __grid_constant__ GiMaps tm, const GemmIntArgs a) {
   uint8_t* raw_area = smem + GI_EXP_STAGES * GI_EXP_STAGE_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(raw_area + GI_RAW_STAGES * Cfg::RAW_STAGE_BYTES);
   // barriers: raw_full[R], raw_empty[R], exp_full[E], exp_empty[E], acc_full[NACC], acc_empty[NACC]
-  constexpr int NB = 2 * GI_RAW_STAGES + 2 * GI_EXP_STAGES + 2 * GI_NACC;
+  constexpr int NB = 2 * GI_RAW_STAGES + 2 * GI_EXP_STAGES + 2 * GI_NACC + 1;
+  static_assert(NB * 8 + 4 + AB_WORDS * 4 <= 256, "barrier area");
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NB);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -92,13 +93,15 @@ gemm_int_kernel(const __grid_constant__ GiMaps tm, const GemmIntArgs a) {
   auto accf_bar = [&](int b) { return bar0 + 8u * (2 * GI_RAW_STAGES + 2 * GI_EXP_STAGES + b); };
   auto acce_bar = [&](int b) { return bar0 + 8u * (2 * GI_RAW_STAGES + 2 * GI_EXP_STAGES + GI_NACC + b); };
 
+  const uint32_t drain_bar = bar0 + 8u * (NB - 1);
+
   constexpr int W_MMA = GI_EPI_WARPS, W_TMA = GI_EPI_WARPS + 1;
   if (threadIdx.x == 0) {
     for (int s = 0; s < GI_RAW_STAGES; ++s) { mbar_init(rawf_bar(s), 1); mbar_init(rawe_bar(s), GI_CONV_WARPS); }
     for (int s = 0; s < GI_EXP_STAGES; ++s) { mbar_init(expf_bar(s), GI_CONV_WARPS); mbar_init(expe_bar(s), 1 + GI_EPI_WARPS); }
     for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), GI_EPI_WARPS); }
-    abort_flag[0] = 0;
-    abort_flag[1] = a.wait_limit_k;
+    mbar_init(drain_bar, 1);
+    abort_init(abort_flag, a.wait_limit_k);
     fence_mbar_init();
     prefetch_tmap(&tm.xq);
     prefetch_tmap(&tm.wq);
@@ -131,7 +134,7 @@ gemm_int_kernel(const __grid_constant__ GiMaps tm, const GemmIntArgs a) {
     // ------------------------------ TMA producer ---------------------------------------------
     if (lane == 0) {
       RingN<GI_RAW_STAGES> r;
-      uint32_t issued = 0;
+      int issued = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         const int m0 = (t / n_tiles_n) * 128, n0 = (t % n_tiles_n) * 128;
@@ -148,32 +151,25 @@ gemm_int_kernel(const __grid_constant__ GiMaps tm, const GemmIntArgs a) {
             tma_load_2d(sb + OFF_WSUM, &tm.wsum, bar, n0, st * 2);
             tma_load_2d(sb + OFF_XZ, &tm.xz, bar, m0, st * 2);
           }
-          issued |= 1u << r.s;
+          ++issued;
           r.next();
         }
       }
-      if (!ok) {
-        const long long t0 = clock64();
-        for (int i = 0; i < GI_RAW_STAGES; ++i) {
-          if (!(issued & (1u << i))) continue;
-          const uint32_t last_ph = (i < r.s) ? r.ph : (r.ph ^ 1);
-          while (!mbar_try(rawf_bar(i), last_ph))
-            if (clock64() - t0 > kWaitLimitCycles / 8) { if (a.status) atomicCAS(a.status, 0, ERR_WAIT_DRAIN); break; }
-        }
-      }
+      abort_flag[AB_ISSUED] = issued;
     }
   } else if (warp > W_TMA) {
     // ------------------------------ converters: raw ring -> expanded ring --------------------
     const int ct = threadIdx.x - (W_TMA + 1) * 32;        // 0..63
     RingN<GI_RAW_STAGES> r;
     RingN<GI_EXP_STAGES> e;
-    uint32_t issued_e = 0;
+    uint32_t tail_slots = 0;                              // slots whose last stage is a 16-bit one, filled by TMA from here
     bool ok = true;
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
       const int m0 = (t / n_tiles_n) * 128, n0 = (t % n_tiles_n) * 128;
       for (int st = 0; st < n_main; ++st) {
-        if (!mbar_wait(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
-        if (!mbar_wait(expe_bar(e.s), e.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+        if (!mbar_wait_warp(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp(expe_bar(e.s), e.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+        tail_slots &= ~(1u << e.s);
         const uint32_t sraw = raw_base + r.s * Cfg::RAW_STAGE_BYTES;
         const uint32_t sA = exp_base + e.s * GI_EXP_STAGE_BYTES;
         const uint32_t sB = sA + GI_TILE_BYTES;
@@ -257,7 +253,7 @@ gemm_int_kernel(const __grid_constant__ GiMaps tm, const GemmIntArgs a) {
       // converter warps poll every slot so that no waiter is ever more than one phase away from
       // the barrier it polls.
       for (int st = 0; st < n_tail && ok; ++st) {
-        if (!mbar_wait(expe_bar(e.s), e.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+        if (!mbar_wait_warp(expe_bar(e.s), e.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
         if (ct == 0) {
           const uint32_t sA = exp_base + e.s * GI_EXP_STAGE_BYTES;
           const uint32_t bar = expf_bar(e.s);
@@ -265,19 +261,16 @@ gemm_int_kernel(const __grid_constant__ GiMaps tm, const GemmIntArgs a) {
           mbar_arrive(bar);                                  // second (the other converter warp's slot)
           tma_load_2d(sA, &tm.xt, bar, st * 64, m0);
           tma_load_2d(sA + GI_TILE_BYTES, &tm.wt, bar, st * 64, n0);
-          issued_e |= 1u << e.s;
+          tail_slots |= 1u << e.s;
         }
         e.next();
       }
     }
-    if (!ok && ct == 0) {
-      const long long t0 = clock64();
-      for (int i = 0; i < GI_EXP_STAGES; ++i) {
-        if (!(issued_e & (1u << i))) continue;
-        const uint32_t last_ph = (i < e.s) ? e.ph : (e.ph ^ 1);
-        while (!mbar_try(expf_bar(i), last_ph))
-          if (clock64() - t0 > kWaitLimitCycles / 8) { if (a.status) atomicCAS(a.status, 0, ERR_WAIT_DRAIN); break; }
-      }
+    if (ct == 0) {
+      // for the teardown: one bit per slot to wait for, and above these the parity of its last phase
+      uint32_t parity = 0;
+      for (int i = 0; i < GI_EXP_STAGES; ++i) parity |= (i < e.s ? e.ph : (e.ph ^ 1)) << i;
+      abort_flag[AB_ISSUED2] = (int)(tail_slots | parity << 16);
     }
   } else if (warp == W_MMA) {
     // ------------------------------ UMMA issuer ----------------------------------------------
@@ -346,11 +339,10 @@ gemm_int_kernel(const __grid_constant__ GiMaps tm, const GemmIntArgs a) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) acc[j] = make_float2(0.f, 0.f);
       for (int st = 0; st < n_main && ok; ++st) {
-        if (!mbar_wait(expf_bar(e.s), e.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+        if (!mbar_wait_warp(expf_bar(e.s), e.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         const float* aux = reinterpret_cast<const float*>(smem + e.s * GI_EXP_STAGE_BYTES + 2 * GI_TILE_BYTES);
         const int pair = use & 1;
-        if (!mbar_wait(accf_bar(pair), (use >> 1) & 1, abort_flag, a.status, ERR_WAIT_ACC_FULL)) { ok = false; break; }
-        __syncwarp();
+        if (!mbar_wait_warp(accf_bar(pair), (use >> 1) & 1, abort_flag, a.status, ERR_WAIT_ACC_FULL)) { ok = false; break; }
         tc_fence_after();
         ++use;
         const int nc = min(2, a.n_chunks - st * 2);
@@ -404,14 +396,12 @@ gemm_int_kernel(const __grid_constant__ GiMaps tm, const GemmIntArgs a) {
       }
       if (ok && n_tail > 0) {
         for (int st = 0; st < n_tail; ++st) {
-          if (!mbar_wait(expf_bar(e.s), e.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
-          __syncwarp();
+          if (!mbar_wait_warp(expf_bar(e.s), e.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
           if (lane == 0) mbar_arrive(expe_bar(e.s));
           e.next();
         }
         const int pair = use & 1;
-        if (ok && mbar_wait(accf_bar(pair), (use >> 1) & 1, abort_flag, a.status, ERR_WAIT_ACC_FULL)) {
-          __syncwarp();
+        if (ok && mbar_wait_warp(accf_bar(pair), (use >> 1) & 1, abort_flag, a.status, ERR_WAIT_ACC_FULL)) {
           tc_fence_after();
           uint32_t v[32];
           tmem_ld32(tlane + (2 * pair) * 128, v);
@@ -456,6 +446,20 @@ gemm_int_kernel(const __grid_constant__ GiMaps tm, const GemmIntArgs a) {
   }
   tc_fence_before();
   __syncthreads();
+  if (abort_flag[AB_FLAG]) {        // a wait ran out: nothing may be in flight when shared and tensor memory are given back
+    if (warp == W_TMA && lane == 0) drain_ring(rawf_bar, GI_RAW_STAGES, abort_flag[AB_ISSUED], a.status);
+    if (threadIdx.x == (W_TMA + 1) * 32) {
+      const uint32_t w = (uint32_t)abort_flag[AB_ISSUED2];
+      for (int i = 0; i < GI_EXP_STAGES; ++i)
+        if (w >> i & 1) drain_wait(expf_bar(i), w >> (16 + i) & 1, a.status);
+    }
+    if (warp == W_MMA && lane == 0) {
+      umma_commit(drain_bar);
+      drain_wait(drain_bar, 0, a.status);
+    }
+    __syncwarp();
+    __syncthreads();
+  }
   if (warp == W_MMA) {
     __syncwarp();
     tc_fence_after();

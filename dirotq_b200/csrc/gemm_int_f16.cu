@@ -84,8 +84,9 @@ template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
   // Warpgroups: epilogue (warps 0..7), issuer and the two producers (8..11, the last one idle), converters (12..19).  The
   // launch gives every thread 96 registers; the producers' and converters' groups hand some back to the epilogue's, which
   // holds a quarter row of the tile (64 registers of bf16 pairs) besides the piece in work and the one being fetched.
+  // (128 / 48 / 88 spills nowhere; with 136 / 48 / 80 the converters' votes cost 52 bytes a thread and 2 % of a long call.)
   static constexpr int THREADS = (GF_EPI_WARPS + 4 + CONV_WARPS) * 32;
-  static constexpr int REGS_LAUNCH = 96, REGS_EPI = 136, REGS_PROD = 48, REGS_CONV = 80;
+  static constexpr int REGS_LAUNCH = 96, REGS_EPI = 128, REGS_PROD = 48, REGS_CONV = 88;
   static_assert(GF_EPI_WARPS * REGS_EPI + 4 * REGS_PROD + CONV_WARPS * REGS_CONV <= THREADS / 32 * REGS_LAUNCH,
                 "setmaxnreg draws on the registers of the launch");
   static constexpr int BN_OWN = PAIR ? BN / 2 : BN;         // weight rows this CTA fetches
@@ -105,10 +106,13 @@ template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
   static constexpr int TAB_WARP = PIECES * 8 * 8;           // per epilogue warp: {cs pair, bias pair} in bf16 per column pair
   static constexpr int TAB_BYTES = GF_EPI_WARPS * TAB_WARP;
   static constexpr int EXP_TMEM = (512 - NACC * BN) / 32;
-  static constexpr int EXP_SMEM = (232448 - 1024 - 256 - STG_BYTES - TAB_BYTES - RAW_STAGES * RAW_STAGE) / EXP_STAGE;
+  static constexpr int BAR_BYTES = 384;                     // barriers, tensor-memory address, failure words
+  static constexpr int EXP_SMEM = (232448 - 1024 - BAR_BYTES - STG_BYTES - TAB_BYTES - RAW_STAGES * RAW_STAGE) / EXP_STAGE;
   static constexpr int EXP_CAP = EXP_TMEM < GF_EXP_MAX ? EXP_TMEM : GF_EXP_MAX;
   static constexpr int EXP_STAGES = EXP_CAP < EXP_SMEM ? EXP_CAP : EXP_SMEM;
-  static constexpr int SMEM_BYTES = EXP_STAGES * EXP_STAGE + RAW_STAGES * RAW_STAGE + STG_BYTES + TAB_BYTES + 1024 + 256;
+  static constexpr int SMEM_BYTES = EXP_STAGES * EXP_STAGE + RAW_STAGES * RAW_STAGE + STG_BYTES + TAB_BYTES + 1024 + BAR_BYTES;
+  static constexpr int NBARS = 2 * RAW_STAGES + 3 * EXP_STAGES + 4;
+  static_assert(NBARS * 8 + 4 + AB_WORDS * 4 <= BAR_BYTES && CONV_WARPS <= AB_WORDS - AB_WARP, "barrier area");
   static constexpr int TMEM_A0 = NACC * BN;                 // first column of the activation operand slots
   static constexpr int TMEM_COLS = 512;                     // accumulators + EXP_STAGES x 32 columns of A
   static_assert(NACC * BN + EXP_STAGES * 32 <= 512 && EXP_STAGES >= 2, "tensor memory");
@@ -187,6 +191,61 @@ __device__ __forceinline__ uint32_t scale_pair(uint32_t v0, uint32_t v1, float r
   return r;
 }
 
+// After a wait ran out, by all threads (of both CTAs of a pair) once the roles have stopped: await what is in flight.
+template <int BN, bool A8, bool PAIR>
+__device__ __forceinline__ void gf_teardown(uint8_t* bars, int* status) {
+  using Cfg = GfCfg<BN, A8, PAIR>;
+  constexpr int GF_EXP_STAGES = Cfg::EXP_STAGES, GF_RAW_STAGES = Cfg::RAW_STAGES;
+  constexpr int W_MMA = GF_EPI_WARPS, W_TMA = GF_EPI_WARPS + 1, W_TMB = GF_EPI_WARPS + 2, W_CONV = GF_EPI_WARPS + 4;
+  volatile int* const ab = reinterpret_cast<volatile int*>(bars + 8 * Cfg::NBARS) + 1;
+  const int warp = threadIdx.x >> 5;
+  const uint32_t b0 = smem_u32(bars);
+  auto ring = [&](int first_bar) { return [=](int s) { return b0 + 8u * (first_bar + s); }; };
+  const auto rawf = ring(0), expf = ring(2 * GF_RAW_STAGES), expe = ring(2 * GF_RAW_STAGES + GF_EXP_STAGES),
+             expw = ring(2 * GF_RAW_STAGES + 2 * GF_EXP_STAGES), accf = ring(2 * GF_RAW_STAGES + 3 * GF_EXP_STAGES);
+  const uint32_t ab0 = b0 + 8u * Cfg::NBARS + 4u;
+  const bool one = (threadIdx.x & 31) == 0;                 // one lane per warp
+  const int own = ab[AB_ISSUED2];
+  if (warp == W_TMA && one) drain_ring(rawf, GF_RAW_STAGES, ab[AB_ISSUED], status);
+  if constexpr (PAIR) {
+    // see drain_pair_ring; converters run ahead of the weight tiles, so the furthest role is looked for among all
+    const uint32_t cta = cluster_ctarank();
+    if (threadIdx.x == 0) {
+      int m = own;
+      for (int i = 0; i < Cfg::CONV_WARPS; ++i) m = max(m, ab[AB_WARP + i]);
+      ab[AB_MAX] = m;
+    }
+    __syncwarp();
+    __syncthreads();
+    cluster_sync_all();
+    const uint32_t other = map_to_rank(ab0, cta ^ 1);
+    const int peer = ld_cluster_s32(other + 4u * AB_ISSUED2);
+    const int upto = max((int)ab[AB_MAX], ld_cluster_s32(other + 4u * AB_MAX));
+    if (warp >= W_CONV && one) {
+      const int cw = warp - W_CONV, grp = cw / Cfg::GROUP_WARPS;
+      const uint32_t fb = map_to_rank(expf(0), 0);
+      for (int n = ab[AB_WARP + cw]; n < upto; ++n)
+        if (n % Cfg::GROUPS == grp) mbar_arrive_cluster_relaxed(fb + 8u * (n % GF_EXP_STAGES));
+    }
+    if (warp == W_TMB && one && cta == 0) drain_pair_ring(expf, GF_EXP_STAGES, own, peer, upto, Cfg::B_EXP, status);
+  } else if (warp == W_TMB && one) {
+    drain_ring(expw, GF_EXP_STAGES, own, status);
+  }
+  if (warp == W_MMA && one) {                          // in both CTAs of a pair, where the leader's commits arrive
+    int stages = ab[AB_UMMA], accs = ab[AB_ACC];
+    if constexpr (PAIR) {
+      const uint32_t lead = map_to_rank(ab0, 0);
+      stages = ld_cluster_s32(lead + 4u * AB_UMMA);
+      accs = ld_cluster_s32(lead + 4u * AB_ACC);
+    }
+    drain_ring(expe, GF_EXP_STAGES, stages, status);
+    drain_ring(accf, Cfg::NACC, accs, status);
+  }
+  __syncwarp();
+  __syncthreads();
+  if constexpr (PAIR) cluster_sync_all();
+}
+
 // AMODE: 0 = signed 4-bit activation codes, 1 = unsigned 4-bit with zero points, 2 = unsigned 8-bit with zero points
 // PAIR: see the head of this file
 template <int BN, int AMODE, bool PAIR>
@@ -201,8 +260,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   uint8_t* stg_area = raw_area + GF_RAW_STAGES * Cfg::RAW_STAGE;       // 1024-byte aligned
   uint8_t* tab_area = stg_area + Cfg::STG_BYTES;
   uint64_t* bars = reinterpret_cast<uint64_t*>(tab_area + Cfg::TAB_BYTES);
-  constexpr int NB = 2 * GF_RAW_STAGES + 3 * GF_EXP_STAGES + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NB);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -226,8 +284,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
       mbar_init(expw_bar(s), 1);
     }
     for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), (PAIR ? 2 : 1) * GF_EPI_WARPS); }
-    abort_flag[0] = 0;
-    abort_flag[1] = a.wait_limit_k;
+    abort_init(abort_flag, a.wait_limit_k, PAIR ? map_to_rank(bar0 + 8u * Cfg::NBARS + 4u, rank ^ 1) : 0u);
     fence_mbar_init();
     prefetch_tmap(&tm.xq);
     prefetch_tmap(&tm.wp);
@@ -292,7 +349,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
     auto exp_phase = [](int qq) { return (uint32_t)((qq / Cfg::EXP_STAGES) & 1); };
     for (int t = first; t < total_tiles && ok; t += step) {
       for (int c = 0; c < n_raw && ok; c += GF_CPS) {
-        if (!mbar_wait_hot(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+        if (!mbar_wait_hot_warp(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         const uint32_t sraw = raw_base + r.s * Cfg::RAW_STAGE;
         const int nv = min(GF_CPS, n_raw - c);
         const int njc = hc ? (nv + 1) >> 1 : nv;               // operand stages this raw stage feeds
@@ -381,7 +438,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           }
           }
           const int es = exp_slot(q);
-          if (!mbar_wait_hot(expe_bar(es), exp_phase(q) ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+          if (!mbar_wait_hot_warp(expe_bar(es), exp_phase(q) ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
           tc_fence_after();
           tmem_st32(tmem_base + ((uint32_t)(quarter * 32) << 16) + Cfg::TMEM_A0 + es * 32, y1);
           tmem_wait_st();
@@ -397,7 +454,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
       // tail: the activations' bf16 tile (already divided by rs) arrives in the raw ring and its rows are
       // copied to TMEM like an expanded chunk
       for (int st = 0; st < n_tail && ok; ++st, ++q) {
-        if (!mbar_wait_hot(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+        if (!mbar_wait_hot_warp(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         if (q % Cfg::GROUPS == grp) {
           const int es = exp_slot(q);
           const uint32_t rb = raw_base + r.s * Cfg::RAW_STAGE + rowA * 128;
@@ -407,7 +464,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
             const uint4 v = gf_lds128(rb + (uint32_t)((i ^ (rowA & 7)) << 4));
             y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
           }
-          if (!mbar_wait_hot(expe_bar(es), exp_phase(q) ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+          if (!mbar_wait_hot_warp(expe_bar(es), exp_phase(q) ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
           tc_fence_after();
           tmem_st32(tmem_base + ((uint32_t)(quarter * 32) << 16) + Cfg::TMEM_A0 + es * 32, y);
           tmem_wait_st();
@@ -420,13 +477,20 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         r.next();
       }
     }
+    if (PAIR && lane == 0) {
+      // for the teardown: one past the last stage this warp has arrived for.  Not q: a group walks past the other group's
+      // stages without waiting for their slots, and a stage counted before its slot is free would share its barrier's phase
+      // with the slot's last one.
+      while (q > 0 && (q - 1) % Cfg::GROUPS != grp) --q;
+      abort_flag[AB_WARP + cw] = q;
+    }
   } else if (warp >= W_MMA) {
   reg_dealloc<Cfg::REGS_PROD>();
   if (warp == W_TMA) {
     // ------------------------------ TMA producer ---------------------------------------------
     if (lane == 0) {
       GfRing<GF_RAW_STAGES> r;
-      uint32_t issued = 0;
+      int issued = 0;
       bool ok = true;
       for (int t = first; t < total_tiles && ok; t += step) {
         int tm_, tn_;
@@ -452,7 +516,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           }
           for (int j = 0; j < nv; ++j)
             bulk_load(sb + Cfg::OFF_C + j * 128 * 8, a.a_const + ((int64_t)(c + j) * a.ldm + mrec), 128 * 8, bar);
-          issued |= 1u << r.s;
+          ++issued;
           r.next();
         }
         // tail: the activations' bf16 tile travels through the raw ring like a chunk (its rows go on to TMEM)
@@ -461,19 +525,11 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           const uint32_t bar = rawf_bar(r.s);
           mbar_expect_tx(bar, 128u * 128u);                    // one 128 x 64 bf16 tile
           tma_load_2d(raw_base + r.s * Cfg::RAW_STAGE, &tm.xt, bar, st * 64, m0);
-          issued |= 1u << r.s;
+          ++issued;
           r.next();
         }
       }
-      if (!ok) {
-        const long long t0 = clock64();
-        for (int i = 0; i < GF_RAW_STAGES; ++i) {
-          if (!(issued & (1u << i))) continue;
-          const uint32_t last_ph = (i < r.s) ? r.ph : (r.ph ^ 1);
-          while (!mbar_try(rawf_bar(i), last_ph))
-            if (clock64() - t0 > kWaitLimitCycles / 8) { if (a.status) atomicCAS(a.status, 0, ERR_WAIT_DRAIN); break; }
-        }
-      }
+      abort_flag[AB_ISSUED] = issued;
     }
   } else if (warp == W_TMB) {
     // ------------------------------ weight-tile producer ---------------------------------------
@@ -503,24 +559,14 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           else tma_load_2d(exp_base + es * Cfg::EXP_STAGE, &tm.wt, bar, (st - n_main) * 64, n0);
         }
       }
-      if (!ok) {
-        // the copies of the last EXP_STAGES stages issued may still be in flight
-        const long long t0 = clock64();
-        if constexpr (PAIR) {
-          // their completion is counted in the leader, where the peer cannot test it: a bounded time to land
-          while (clock64() - t0 < 2000000LL) __nanosleep(1000);
-        } else
-        for (int qq = max(0, q - GF_EXP_STAGES); qq < q; ++qq)
-          while (!mbar_try(expw_bar(qq % GF_EXP_STAGES), (uint32_t)((qq / GF_EXP_STAGES) & 1)))
-            if (clock64() - t0 > kWaitLimitCycles / 8) { if (a.status) atomicCAS(a.status, 0, ERR_WAIT_DRAIN); break; }
-      }
+      abort_flag[AB_ISSUED2] = q;
     }
   } else if (warp == W_MMA) {
     // ------------------------------ UMMA issuer ----------------------------------------------
     if (lane == 0 && rank == 0) {
       const uint32_t idesc_h = idesc_dense(ACC_F32, FMT_F16, FMT_F16, TILE_M, BN);
       const uint32_t idesc_bf = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, TILE_M, BN);
-      int use = 0;
+      int use = 0, stages = 0;
       bool ok = true;
       // loop-invariant pieces of the per-stage operands: barrier addresses are 8 bytes per slot apart, the weight
       // descriptor's low word holds the slot address >> 4, the activation slots are 32 tensor-memory columns apart
@@ -589,6 +635,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
             }
           }
           st += two ? 2 : 1;
+          stages += two ? 2 : 1;
           es0 = es1;
           ph0 = ph1;
           if (++es0 == GF_EXP_STAGES) { es0 = 0; ph0 ^= 1u; }
@@ -599,6 +646,8 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           ++use;
         }
       }
+      abort_flag[AB_UMMA] = stages;
+      abort_flag[AB_ACC] = use;
     }
   }
   } else {
@@ -669,8 +718,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
       }
       const int buf = Cfg::NACC == 2 ? (use & 1) : 0;
       const uint32_t acc_ph = (uint32_t)(Cfg::NACC == 2 ? (use >> 1) & 1 : use & 1);
-      if (!mbar_wait(accf_bar(buf), acc_ph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) { ok = false; break; }
-      __syncwarp();
+      if (!mbar_wait_warp(accf_bar(buf), acc_ph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) { ok = false; break; }
       tc_fence_after();
       ++use;
       const uint32_t tl = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + ch * CW;
@@ -755,11 +803,20 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   tc_fence_before();
   __syncthreads();
   if constexpr (PAIR) cluster_sync_all();   // neither CTA retires while the other may still read its shared memory
-  if (warp == W_MMA) {
+  const int end_warp = (int)(tid_anew() >> 5);
+  uint8_t* const end_bars = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(anew(smem_raw)) + 1023) & ~uintptr_t(1023)) +
+                            GF_EXP_STAGES * Cfg::EXP_STAGE + GF_RAW_STAGES * Cfg::RAW_STAGE + Cfg::STG_BYTES + Cfg::TAB_BYTES;
+  volatile int* const ab = reinterpret_cast<volatile int*>(end_bars + 8 * Cfg::NBARS) + 1;
+  if (ab[AB_FLAG]) {                // a wait ran out (in both CTAs of a pair the flag is up)
+    regs_even<Cfg::REGS_LAUNCH>(end_warp < GF_EPI_WARPS);
+    gf_teardown<BN, A8, PAIR>(end_bars, a.status);
+  }
+  if (end_warp == W_MMA) {
     __syncwarp();
     tc_fence_after();
-    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
-    else tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+    const uint32_t tmem = *(reinterpret_cast<volatile uint32_t*>(end_bars + 8 * Cfg::NBARS));
+    if constexpr (PAIR) tmem_dealloc_pair(tmem, Cfg::TMEM_COLS);
+    else tmem_dealloc(tmem, Cfg::TMEM_COLS);
   }
 }
 

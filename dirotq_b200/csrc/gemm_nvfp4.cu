@@ -32,6 +32,7 @@ constexpr int GF_EPI_WARPS = 8;              // two per TMEM lane quarter, 64 ou
 constexpr int GF_THREADS = (2 + GF_EPI_WARPS) * 32;
 constexpr int GF_STG_BYTES = GF_EPI_WARPS * 2048;   // per epilogue warp: 32 rows x 32 bf16 output staging patch
 constexpr int GF_SMEM_BYTES = GF_STAGES * GF_STAGE_BYTES + GF_STG_BYTES + 1024 + 256;
+static_assert((2 * GF_STAGES + 4) * 8 + 4 + AB_WORDS * 4 <= 256, "barrier area");
 constexpr uint32_t GF_TMEM_COLS = 512;
 constexpr uint32_t GF_SFA_COL = 256;         // two alternating slots of 16 columns each
 constexpr uint32_t GF_SFB_COL = 320;
@@ -63,8 +64,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < GF_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), GF_EPI_WARPS); }
-    abort_flag[0] = 0;
-    abort_flag[1] = a.wait_limit_k;
+    abort_init(abort_flag, a.wait_limit_k);
     fence_mbar_init();
     prefetch_tmap(&tm_xq);
     prefetch_tmap(&tm_wq);
@@ -88,7 +88,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
   if (warp == 0) {
     if (lane == 0) {
       GfRing r;
-      uint32_t issued = 0;
+      int issued = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         const int mb = t / n_tiles, nb = t - mb * n_tiles;
@@ -108,20 +108,11 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
             tma_load_2d(sA, &tm_xt, full_bar(r.s), (st - n_main) * 64, mb * 128);
             tma_load_2d(sB, &tm_wt, full_bar(r.s), (st - n_main) * 64, nb * 128);
           }
-          issued |= 1u << r.s;
+          ++issued;
           r.next();
         }
       }
-      if (!ok) {
-        const long long t0 = clock64();
-        for (int i = 0; i < GF_STAGES; ++i) {
-          if (!(issued & (1u << i))) continue;
-          const uint32_t last_ph = (i < r.s) ? r.ph : (r.ph ^ 1);
-          while (!mbar_try(full_bar(i), last_ph)) {
-            if (clock64() - t0 > kWaitLimitCycles / 8) { if (a.status) atomicCAS(a.status, 0, ERR_WAIT_DRAIN); break; }
-          }
-        }
-      }
+      abort_flag[AB_ISSUED] = issued;
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -131,6 +122,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
       int buf = 0;
       uint32_t aph = 0;
       uint32_t sf_slot = 0;
+      int stages = 0, accs = 0;
       const uint64_t op_d0 = smem_desc_sw128(smem_base), sf_d0 = smem_desc_rows16(smem_base);
       const uint32_t op_lo0 = (uint32_t)op_d0, op_hi = (uint32_t)(op_d0 >> 32);
       const uint32_t sf_lo0 = (uint32_t)sf_d0, sf_hi = (uint32_t)(sf_d0 >> 32);
@@ -169,13 +161,17 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
             umma_f16_ss_x4(d, a_lo, a_lo + (GF_TILE_BYTES >> 4), op_hi, idesc_bf, 1u);
           }
           umma_commit(empty_bar(r.s));
+          ++stages;
           r.next();
         }
         if (!ok) break;
         umma_commit(accf_bar(buf));
+        ++accs;
         buf ^= 1;
         if (buf == 0) aph ^= 1;
       }
+      abort_flag[AB_UMMA] = stages;
+      abort_flag[AB_ACC] = accs;
     }
   } else {
     const int q = warp & 3, half = (warp - 2) >> 2;
@@ -184,8 +180,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
     uint32_t aph = 0;
     for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
       const int mb = t / n_tiles, nb = t - mb * n_tiles;
-      if (!mbar_wait(accf_bar(buf), aph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) break;
-      __syncwarp();
+      if (!mbar_wait_warp(accf_bar(buf), aph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 128 + half * 64;
       const int64_t row = (int64_t)mb * 128 + q * 32 + lane;
@@ -260,6 +255,14 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
   }
   tc_fence_before();
   __syncthreads();
+  if (abort_flag[AB_FLAG]) {        // a wait ran out: nothing may be in flight when shared and tensor memory are given back
+    if (warp == 0 && lane == 0) drain_ring(full_bar, GF_STAGES, abort_flag[AB_ISSUED], a.status);
+    if (warp == 1 && lane == 0) {
+      drain_ring(empty_bar, GF_STAGES, abort_flag[AB_UMMA], a.status);
+      drain_ring(accf_bar, 2, abort_flag[AB_ACC], a.status);
+    }
+    __syncthreads();
+  }
   if (warp == 1) {
     __syncwarp();
     tc_fence_after();

@@ -63,13 +63,15 @@ struct GpCfg {
                 "setmaxnreg draws on the registers of the launch");
   static constexpr int STG_BYTES = EPI_WARPS * 2 * 2048;    // per epilogue warp: two 32 rows x 32 bf16 staging patches
   static constexpr int TAB_BYTES = BN * 8;                  // per output column of the tile: {scale, bias} as floats
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STG_BYTES + TAB_BYTES + 1024 + 256;
+  static constexpr int BAR_BYTES = 320;                     // barriers, tensor-memory address, failure words
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + STG_BYTES + TAB_BYTES + 1024 + BAR_BYTES;
   static constexpr uint32_t TMEM_COLS = 512;
   static constexpr uint32_t SF_COL = 256;                   // one slot per shared-memory stage:
   static constexpr uint32_t SF_SLOT = 16 + 16 * (BN / 128); //   16 columns for the activations' factors + 16 per 128 weight rows
   static constexpr uint32_t OP_TX = 2u * (A_BYTES + B_BYTES);   // operand bytes of both CTAs, counted in the leader
   static constexpr uint32_t SF_TX = SFA_BYTES + SFB_BYTES;      // scale-factor bytes, counted in each CTA
   static constexpr int NBARS = 3 * STAGES + 8;
+  static_assert(NBARS * 8 + 4 + AB_WORDS * 4 <= BAR_BYTES && SF_WARPS <= AB_WORDS - AB_WARP, "barrier area");
   static_assert(SF_COL + STAGES * SF_SLOT <= TMEM_COLS, "tensor memory");
   static_assert(STAGE_BYTES % 1024 == 0, "operand tiles need 1024-byte alignment");
   static_assert(SMEM_BYTES <= 232448, "shared memory");
@@ -81,6 +83,38 @@ struct GfRingT {
   uint32_t ph = 0;
   __device__ __forceinline__ void next() { if (++s == STAGES) { s = 0; ph ^= 1; } }
 };
+
+// After a wait ran out, by all threads of both CTAs once their roles have stopped: await what is in flight (see
+// drain_pair_ring).
+template <int BN>
+__device__ __forceinline__ void gp_teardown(uint8_t* bars, int* status) {
+  using Cfg = GpCfg<BN>;
+  constexpr int STAGES = Cfg::STAGES, NACC = Cfg::NACC;
+  volatile int* const ab = reinterpret_cast<volatile int*>(bars + 8 * Cfg::NBARS) + 1;
+  const int warp = threadIdx.x >> 5;
+  const uint32_t b0 = smem_u32(bars), ab0 = b0 + 8u * Cfg::NBARS + 4u, cta = cluster_ctarank();
+  auto ring = [&](int first_bar) { return [=](int s) { return b0 + 8u * (first_bar + s); }; };
+  const auto full = ring(0), empty = ring(STAGES), sffull = ring(2 * STAGES), accf = ring(3 * STAGES);
+  const bool one = (threadIdx.x & 31) == 0;                 // one lane per warp
+  const int own = ab[AB_ISSUED], peer = ld_cluster_s32(map_to_rank(ab0 + 4u * AB_ISSUED, cta ^ 1));
+  const int upto = max(own, peer);                         // movers follow their CTA's producer
+  if (warp >= Cfg::SF_WARP0 && warp < Cfg::EPI_WARP0 && one) {
+    const uint32_t fb = map_to_rank(full(0), 0);
+    for (int n = ab[AB_WARP + (warp & 3)]; n < upto; ++n) mbar_arrive_cluster_relaxed(fb + 8u * (n % STAGES));
+  }
+  if (warp == 0 && one) {
+    if (cta == 0) drain_pair_ring(full, STAGES, own, peer, upto, Cfg::OP_TX / 2, status);
+    drain_ring(sffull, STAGES, own, status);
+  }
+  if (warp == 1 && one) {                              // in both CTAs, where the leader's commits arrive
+    const uint32_t lead = map_to_rank(ab0, 0);
+    drain_ring(empty, STAGES, ld_cluster_s32(lead + 4u * AB_UMMA), status);
+    drain_ring(accf, NACC, ld_cluster_s32(lead + 4u * AB_ACC), status);
+  }
+  __syncwarp();
+  __syncthreads();
+  cluster_sync_all();
+}
 
 // QOUT: the epilogue also quantises its output for a following NVFP4 layer (GemmFp4Args::q_codes).  A separate
 // instantiation, so that the registers this costs do not weigh on the plain kernel.
@@ -122,8 +156,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
       mbar_init(tab_bar(b, 0), 4);
       mbar_init(tab_bar(b, 1), 4);
     }
-    abort_flag[0] = 0;
-    abort_flag[1] = a.wait_limit_k;
+    abort_init(abort_flag, a.wait_limit_k, map_to_rank(bar0 + 8u * Cfg::NBARS + 4u, rank ^ 1));
     fence_mbar_init();
     prefetch_tmap(&tm_xq);
     prefetch_tmap(&tm_wq);
@@ -153,6 +186,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
   if (warp == 0) {
     if (lane == 0) {
       GfRingT<STAGES> r;
+      int issued = 0;
       bool ok = true;
       for (int t = first; t < total_tiles && ok; t += step) {
         const int mp = t / n_tiles, nb = t - mp * n_tiles;
@@ -180,15 +214,11 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
             tma_load_2d_pair(sA, &tm_xt, fb, (st - n_main) * 64, row_a);
             tma_load_2d_pair(sB, &tm_wt, fb, (st - n_main) * 64, row_b);
           }
+          ++issued;
           r.next();
         }
       }
-      if (!ok) {
-        // copies of this CTA may still be in flight towards its shared memory; their completion is counted in the
-        // leader, so the peer cannot test it: give them a bounded time before the CTA may retire
-        const long long t0 = clock64();
-        while (clock64() - t0 < 2000000LL) __nanosleep(1000);
-      }
+      abort_flag[AB_ISSUED] = issued;
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
@@ -197,7 +227,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
       const uint64_t op_d0 = smem_desc_sw128(smem_base);
       const uint32_t op_lo0 = (uint32_t)op_d0, op_hi = (uint32_t)(op_d0 >> 32);
       GfRingT<STAGES> r;
-      int buf = 0;
+      int buf = 0, stages = 0, accs = 0;
       uint32_t aph = 0;
       bool ok = true;
       for (int t = first; t < total_tiles && ok; t += step) {
@@ -227,10 +257,12 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
           }
           // the stage is free in BOTH CTAs once these UMMAs have read it
           umma_commit_pair_both(empty_bar(r.s));
+          ++stages;
           r.next();
         }
         if (!ok) break;
         umma_commit_pair_both(accf_bar(buf));
+        ++accs;
         if (NACC == 2) {
           buf ^= 1;
           if (buf == 0) aph ^= 1;
@@ -238,6 +270,8 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
           aph ^= 1;
         }
       }
+      abort_flag[AB_UMMA] = stages;
+      abort_flag[AB_ACC] = accs;
     }
   }
   } else if (warp < Cfg::EPI_WARP0) {
@@ -246,6 +280,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
     const uint32_t q = warp & 3;
     const uint32_t ready_leader = map_to_rank(full_bar(0), 0);
     GfRingT<STAGES> r;
+    int moved = 0;
     bool ok = true;
     for (int t = first; t < total_tiles && ok; t += step) {
       for (int st = 0; st < n_main + n_tail; ++st) {
@@ -284,9 +319,11 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
           if (rank == 0) mbar_arrive(full_bar(r.s));
           else mbar_arrive_cluster_relaxed(ready_leader + 8u * r.s);
         }
+        ++moved;
         r.next();
       }
     }
+    if (lane == 0) abort_flag[AB_WARP + q] = moved;
   } else {
     reg_alloc<Cfg::REGS_EPI>();
     constexpr int WCOLS = BN / 2;                       // output columns per epilogue warp
@@ -329,7 +366,7 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
       // (hand-offs between the half's four warps go through mbarriers: their waits are bounded like all others)
       __syncwarp();
       if (lane == 0) mbar_arrive(tab_bar(half, 0));
-      if (!mbar_wait(tab_bar(half, 0), tph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) break;   // all four are done with the last table
+      if (!mbar_wait_warp(tab_bar(half, 0), tph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) break;   // all four are done with the last table
       if (lane < CPW) {
         const int64_t col = n0 + tcol;
         const __nv_bfloat16 b = col < a.N && a.bias ? a.bias[col] : __float2bfloat16_rn(0.f);
@@ -338,11 +375,11 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(tab_bar(half, 1));
-      if (!mbar_wait(tab_bar(half, 1), tph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) break;   // table complete
+      if (!mbar_wait_warp(tab_bar(half, 1), tph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) break;   // table complete
       tph ^= 1;
       // a single accumulator keeps the UMMA issuer waiting for this pull: poll instead of sleeping
-      if (!(NACC == 1 ? mbar_wait_hot(accf_bar(buf), aph, abort_flag, a.status, ERR_WAIT_ACC_FULL)
-                      : mbar_wait(accf_bar(buf), aph, abort_flag, a.status, ERR_WAIT_ACC_FULL))) break;
+      if (!(NACC == 1 ? mbar_wait_hot_warp(accf_bar(buf), aph, abort_flag, a.status, ERR_WAIT_ACC_FULL)
+                      : mbar_wait_warp(accf_bar(buf), aph, abort_flag, a.status, ERR_WAIT_ACC_FULL))) break;
       __syncwarp();
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + half * WCOLS;
@@ -473,10 +510,18 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();     // neither CTA retires (or frees TMEM) while the other may still read its shared memory
-  if (warp == 1) {
+  const int end_warp = (int)(tid_anew() >> 5);
+  uint8_t* const end_bars = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(anew(smem_raw)) + 1023) & ~uintptr_t(1023)) +
+                            STAGES * Cfg::STAGE_BYTES + Cfg::STG_BYTES + Cfg::TAB_BYTES;
+  volatile int* const ab = reinterpret_cast<volatile int*>(end_bars + 8 * Cfg::NBARS) + 1;
+  if (ab[AB_FLAG]) {                // a wait ran out (in both CTAs the flag is up)
+    regs_even<Cfg::REGS_LAUNCH>(end_warp >= Cfg::EPI_WARP0);
+    gp_teardown<BN>(end_bars, a.status);
+  }
+  if (end_warp == 1) {
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc_pair(tmem_base, Cfg::TMEM_COLS);
+    tmem_dealloc_pair(*reinterpret_cast<volatile uint32_t*>(end_bars + 8 * Cfg::NBARS), Cfg::TMEM_COLS);
   }
 }
 

@@ -1,7 +1,7 @@
 // Thin inline-PTX layer for sm_100a: mbarrier, TMA (no cluster broadcast forms), tcgen05
 // (TMEM allocation, UMMA issue/commit, TMEM loads, smem->TMEM copies) and descriptor builders.
 // Every wait in this file is bounded: a wait that runs out records a code and returns false so
-// the kernel can unwind (drain its copies, free TMEM) instead of spinning forever.
+// the kernel can unwind (await what it has in flight, free TMEM) instead of spinning forever.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -96,23 +96,67 @@ __device__ __forceinline__ uint32_t mbar_test4(uint32_t b0, uint32_t p0, uint32_
   return m;
 }
 
-// Bounded wait.  Waiters sleep in hardware (20 us per poll) instead of spinning, so they do not
+// Shared words of a CTA's failure handling, behind its barriers.  Once any role gave up, all later waits of the CTA -- of
+// both CTAs of a pair, whose flags are raised together -- return at once; every role stops, and the CTA tears down what the
+// roles left in flight (see drain_ring).
+enum : int {
+  AB_FLAG = 0,      // a role gave up
+  AB_LIMIT = 1,     // the launch's wait limit in units of 1024 cycles
+  AB_POLL = 2,      // how long one poll may sleep (ns): 20 us, less under a short limit
+  AB_PEER = 3,      // shared::cluster address of the peer's AB_FLAG (0 = no peer)
+  AB_ISSUED = 4,    // stages the producer has issued copies for, written when it stops
+  AB_ISSUED2 = 5,   // the same of a second producer
+  AB_UMMA = 6,      // stages and accumulators the issuer has committed UMMAs for
+  AB_ACC = 7,
+  AB_MAX = 8,       // pairs: stages any role of the CTA has got to
+  AB_WARP = 9,      // per warp of a role that arrives on a pair's barriers: stages it has arrived for
+  AB_WORDS = 17,
+};
+__device__ __forceinline__ void abort_init(volatile int* w, int limit_k, uint32_t peer_flag = 0) {
+  w[AB_FLAG] = 0;
+  w[AB_LIMIT] = limit_k > 0 ? limit_k : (int)(kWaitLimitCycles >> 10);
+  w[AB_POLL] = limit_k > 0 && limit_k < 80 ? 250 * limit_k : 20000;
+  w[AB_PEER] = (int)peer_flag;
+  w[AB_ISSUED] = w[AB_ISSUED2] = w[AB_UMMA] = w[AB_ACC] = w[AB_MAX] = 0;
+}
+__device__ __forceinline__ void report_status(int* status, int code) {
+  if (status) atomicCAS(status, 0, code);
+}
+__device__ __forceinline__ void abort_raise(volatile int* abort_flag, int* status, int code) {
+  abort_flag[AB_FLAG] = 1;
+  if (const uint32_t peer = (uint32_t)abort_flag[AB_PEER])
+    asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(peer), "r"(1u) : "memory");
+  report_status(status, code);
+}
+__device__ __forceinline__ bool abort_late(volatile int* abort_flag, long long t0) {
+  return clock64() - t0 > (long long)abort_flag[AB_LIMIT] << 10;
+}
+// The code after the roles starts from scratch: values it shared with what comes before would have to be kept through the
+// roles (in the epilogue of a 256-wide tile, as spills).
+template <typename T> __device__ __forceinline__ T anew(T v) {
+  if constexpr (sizeof(T) == 8) asm volatile("" : "+l"(v));
+  else asm volatile("" : "+r"(v));
+  return v;
+}
+__device__ __forceinline__ uint32_t tid_anew() {
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
+}
+
+// Bounded wait.  Waiters sleep in hardware (up to 20 us per poll) instead of spinning, so they do not
 // compete with the working warps for issue slots; between polls the shared abort flag and the clock
-// are checked.  `abort_flag` lives in shared memory: once any role gave up, all later waits of the
-// CTA return at once.
+// are checked.  For one thread of a warp; a warp whose lanes all wait uses the forms below.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code) {
   if (mbar_try(bar, parity)) return true;
   const long long t0 = clock64();
   while (true) {
-    if (mbar_try(bar, parity, 20000u)) return true;
+    if (mbar_try(bar, parity, abort_flag[AB_POLL])) return true;
     __nanosleep(128);            // keep pollers off the issue ports of the working warps
-    if (*abort_flag) return false;
-    // abort_flag[1]: the launch's wait limit in units of 1024 cycles (0 = the default above)
-    const long long limit = abort_flag[1] > 0 ? ((long long)abort_flag[1] << 10) : kWaitLimitCycles;
-    if (clock64() - t0 > limit) {
-      *abort_flag = 1;
-      if (status) atomicCAS(status, 0, code);
+    if (abort_flag[AB_FLAG]) return false;
+    if (abort_late(abort_flag, t0)) {
+      abort_raise(abort_flag, status, code);
       return false;
     }
   }
@@ -127,6 +171,45 @@ __device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity, vol
   for (int i = 0; i < 4096; ++i)
     if (mbar_try(bar, parity)) return true;
   return mbar_wait(bar, parity, abort_flag, status, code);
+}
+
+// The same for whole warps: one verdict for all lanes, by vote.  Lanes that poll for themselves could see a phase complete
+// and the flag raised, part each, and the warp would come apart in front of its next aligned instruction.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  const long long t0 = clock64();
+  while (true) {
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity, abort_flag[AB_POLL]))) return true;
+    __nanosleep(128);
+    const bool raised = abort_flag[AB_FLAG] != 0, late = abort_late(abort_flag, t0);
+    if (__any_sync(0xffffffffu, raised || late)) {
+      if (late && !raised) abort_raise(abort_flag, status, code);
+      return false;
+    }
+  }
+}
+__device__ __forceinline__ bool mbar_wait_hot_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+#pragma unroll 1
+  for (int i = 0; i < 4096; ++i)
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  return mbar_wait_warp(bar, parity, abort_flag, status, code);
+}
+
+// Teardown after a wait ran out, once every role has stopped: wait (bounded) for one phase, and for those of the last `issued`
+// uses of a ring -- the copies a producer issued, the UMMAs an issuer committed.  `bar_of` gives a slot's barrier.  A commit
+// that arrives in both CTAs of a pair is awaited in both: nothing else holds a CTA until the arrival, which is on its way
+// asynchronously, has reached it.
+__device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity, int* status) {
+  const long long t0 = clock64();
+  while (!mbar_try(bar, parity, 20000u))
+    if (clock64() - t0 > kWaitLimitCycles / 8) {
+      report_status(status, ERR_WAIT_DRAIN);
+      return;
+    }
+}
+template <typename F>
+__device__ __forceinline__ void drain_ring(F bar_of, int slots, int issued, int* status) {
+  for (int q = max(0, issued - slots); q < issued; ++q) drain_wait(bar_of(q % slots), (uint32_t)((q / slots) & 1), status);
 }
 
 // GELU, tanh form (torch.nn.functional.gelu(approximate="tanh")), applied to a value that was first rounded
@@ -376,9 +459,15 @@ __device__ __forceinline__ void tmem_wait_ld16(uint32_t* r) {
                :: "memory");
 }
 // Register split between the warpgroups of a block (all four warps of a group execute the same one).  The sum over the
-// groups must not exceed what the block was launched with.
+// groups must not exceed what the block was launched with.  regs_even gives every group the launch's share back, for code that
+// all run; only behind a barrier that all have passed: a group that took registers back while another still waited for its own
+// would leave both waiting for good.
 template <int N> __device__ __forceinline__ void reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int LAUNCH> __device__ __forceinline__ void regs_even(bool grew) {
+  if (grew) reg_dealloc<LAUNCH>();
+  else reg_alloc<LAUNCH>();
+}
 // registers -> TMEM: 32 consecutive 32-bit columns of this thread's lane
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
   asm volatile(

@@ -44,6 +44,31 @@ __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_add
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
+// A word of either CTA's shared memory (shared::cluster address)
+__device__ __forceinline__ int ld_cluster_s32(uint32_t cluster_addr) {
+  int v;
+  asm volatile("ld.relaxed.cluster.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
+  return v;
+}
+// Takes `bytes` off a barrier's pending count, as a copy of that size would when it lands
+__device__ __forceinline__ void mbar_complete_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// Teardown of a pair's ring after a wait ran out, by the leader's producer thread once both CTAs have stopped.  A stage's
+// barrier (in the leader) expects one arrival with the bytes of both halves, `half` from each CTA; of the stages below
+// `upto` -- as far as any role of either CTA got -- the leader has armed `own` and the peer issued copies for `peer`.
+// What one CTA did and the other did not is made up for, so that every such phase completes exactly when the copies that
+// were issued have landed (the warps that also arrive on these barriers make up for theirs); then the last ring of them
+// is awaited.  No role is more than a ring behind another: a slot is reused only after all arrived for its last stage.
+// (`upto` must not count a stage that a role merely walked past: two stages on one barrier would arrive more often than the
+// phase at hand expects while bytes are missing, which is a fault.)
+template <typename F>
+__device__ __forceinline__ void drain_pair_ring(F bar_of, int slots, int own, int peer, int upto, uint32_t half, int* status) {
+  for (int q = own; q < upto; ++q) mbar_expect_tx(bar_of(q % slots), q < peer ? half : 0u);
+  for (int q = peer; q < own; ++q) mbar_complete_tx(bar_of(q % slots), half);
+  drain_ring(bar_of, slots, upto, status);
+}
+
 // 2-D tiled load into THIS CTA's shared memory; the bytes are counted on `bar`, a shared::cluster address that may
 // name the leader CTA's mbarrier (the cta_group::2 form is what allows the barrier to sit in the peer).
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap, uint32_t bar, int x, int y) {

@@ -607,6 +607,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* stg_area = smem + RQ_STAGES * RQ_STAGE_BYTES;                  // 1024-byte aligned
   uint64_t* bars = reinterpret_cast<uint64_t*>(stg_area + RqCfg<EPI>::STG_BYTES);
+  static_assert((2 * RQ_STAGES + 4) * 8 + 4 + AB_WORDS * 4 <= 256, "barrier area");
   // bars[0..S) full, [S..2S) empty, [2S..2S+2) acc_full, [2S+2..2S+4) acc_empty
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * RQ_STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -618,12 +619,12 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   auto empty_bar = [&](int s) { return bar0 + 8u * (RQ_STAGES + s); };
   auto accf_bar = [&](int b) { return bar0 + 8u * (2 * RQ_STAGES + b); };
   auto acce_bar = [&](int b) { return bar0 + 8u * (2 * RQ_STAGES + 2 + b); };
+  const uint32_t abort_addr = bar0 + 8u * (2 * RQ_STAGES + 4) + 4u;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < RQ_STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), (PAIR ? 2 : 1) * RqCfg<EPI>::EPI_WARPS); }
-    abort_flag[0] = 0;
-    abort_flag[1] = a.wait_limit_k;
+    abort_init(abort_flag, a.wait_limit_k, PAIR ? map_to_rank(abort_addr, rank ^ 1) : 0u);
     fence_mbar_init();
     prefetch_tmap(&tm_x);
     prefetch_tmap(&tm_u);
@@ -649,7 +650,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 0;
-      uint32_t issued = 0;   // bit s set: a load into stage s has been issued at least once
+      int issued = 0;
       bool ok = true;
       for (int t = first; t < total_tiles && ok; t += step) {
         const int mt = t / a.n_tiles, nb = t - mt * a.n_tiles;
@@ -669,31 +670,16 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
             tma_load_2d(sa, &tm_x, full_bar(s), kc * 64, mb * 128);
             tma_load_2d(sa + RQ_A_BYTES, &tm_u, full_bar(s), kc * 64, nb * a.BN);
           }
-          issued |= 1u << s;
+          ++issued;
           if (++s == RQ_STAGES) { s = 0; ph ^= 1; }
         }
       }
-      if (PAIR && !ok) {
-        // the completions of this CTA's copies are counted in the leader, where the peer cannot test them: give
-        // copies in flight a bounded time to land before the CTA may retire
-        const long long t0 = clock64();
-        while (clock64() - t0 < 2000000LL) __nanosleep(1000);
-      } else if (!ok) {
-        // unwind: let copies already in flight land before the CTA exits (bounded)
-        const long long t0 = clock64();
-        for (int i = 0; i < RQ_STAGES; ++i) {
-          if (!(issued & (1u << i))) continue;
-          const uint32_t last_ph = (i < s) ? ph : (ph ^ 1);
-          while (!mbar_try(full_bar(i), last_ph)) {
-            if (clock64() - t0 > kWaitLimitCycles / 8) { if (a.status) atomicCAS(a.status, 0, ERR_WAIT_DRAIN); break; }
-          }
-        }
-      }
+      abort_flag[AB_ISSUED] = issued;
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
       const uint32_t idesc = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, PAIR ? 256 : 128, (uint32_t)a.BN);
-      int s = 0, buf = 0;
+      int s = 0, buf = 0, stages = 0, accs = 0;
       uint32_t ph = 0, aph = 0;
       bool ok = true;
       const uint64_t op_d0 = smem_desc_sw128(smem_base);
@@ -718,6 +704,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
             umma_f16_ss_x4(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u);
             umma_commit(empty_bar(s));
           }
+          ++stages;
           if (++s == RQ_STAGES) { s = 0; ph ^= 1; }
         }
         if (!ok) break;
@@ -726,9 +713,12 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
         } else {
           umma_commit(accf_bar(buf));
         }
+        ++accs;
         buf ^= 1;
         if (buf == 0) aph ^= 1;
       }
+      abort_flag[AB_UMMA] = stages;
+      abort_flag[AB_ACC] = accs;
     }
   } else {
     const int q = warp & 3, half = (warp - 2) >> 2;
@@ -738,8 +728,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     for (int t = first; t < total_tiles; t += step) {
       const int mt = t / a.n_tiles, nb = t - mt * a.n_tiles;
       const int mb = PAIR ? 2 * mt + (int)rank : mt;
-      if (!mbar_wait(accf_bar(buf), aph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) break;
-      __syncwarp();
+      if (!mbar_wait_warp(accf_bar(buf), aph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256;
       const int64_t row = (int64_t)mb * 128 + q * 32 + lane;
@@ -765,6 +754,30 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   tc_fence_before();
   __syncthreads();
   if constexpr (PAIR) cluster_sync_all();   // neither CTA retires while the other may still read its shared memory
+  if (abort_flag[AB_FLAG]) {        // a wait ran out (in both CTAs of a pair the flag is up): await what is in flight
+    if (warp == 0 && lane == 0) {
+      const int own = abort_flag[AB_ISSUED];
+      if constexpr (PAIR) {
+        const int peer = ld_cluster_s32(map_to_rank(abort_addr + 4u * AB_ISSUED, rank ^ 1));
+        if (rank == 0) drain_pair_ring(full_bar, RQ_STAGES, own, peer, max(own, peer), RQ_A_BYTES + bn_own * 128, a.status);
+      } else {
+        drain_ring(full_bar, RQ_STAGES, own, a.status);
+      }
+    }
+    if (warp == 1 && lane == 0) {                       // in both CTAs of a pair, where the leader's commits arrive
+      int stages = abort_flag[AB_UMMA], accs = abort_flag[AB_ACC];
+      if constexpr (PAIR) {
+        const uint32_t lead = map_to_rank(abort_addr, 0);
+        stages = ld_cluster_s32(lead + 4u * AB_UMMA);
+        accs = ld_cluster_s32(lead + 4u * AB_ACC);
+      }
+      drain_ring(empty_bar, RQ_STAGES, stages, a.status);
+      drain_ring(accf_bar, 2, accs, a.status);
+    }
+    __syncwarp();
+    __syncthreads();
+    if constexpr (PAIR) cluster_sync_all();
+  }
   if (warp == 1) {
     __syncwarp();
     tc_fence_after();

@@ -396,7 +396,7 @@ int dirotq_linear_forward_static(const dirotq_linear* lin, const void* x, int64_
 int dirotq_abi_version(void);
 /* Every device-side wait (on a shared-memory stage, an accumulator, scale factors) is bounded: after `cycles` SM clock
  * cycles (0 = the default of 3e9, about 1.5 s) the waiting role writes its code into the caller's status word, raises
- * the CTA's abort flag, the kernel awaits its copies in flight (bounded), frees its tensor memory and returns; the
+ * the CTA's abort flag, the kernel awaits what it has in flight (bounded), frees its tensor memory and returns; the
  * context stays usable and the outputs of that launch are undefined.  The setting is process-wide and applies to
  * launches made after the call.  No counterpart in the reference (its eager kernels have no waits of their own). */
 int dirotq_set_wait_limit_cycles(int64_t cycles);
