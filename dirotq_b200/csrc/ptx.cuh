@@ -119,8 +119,9 @@ __device__ __forceinline__ void abort_init(volatile int* w, int limit_k, uint32_
   w[AB_PEER] = (int)peer_flag;
   w[AB_ISSUED] = w[AB_ISSUED2] = w[AB_UMMA] = w[AB_ACC] = w[AB_MAX] = 0;
 }
+// System scope: the word may be host memory, which the host clears while kernels of other streams still run.
 __device__ __forceinline__ void report_status(int* status, int code) {
-  if (status) atomicCAS(status, 0, code);
+  if (status) atomicCAS_system(status, 0, code);
 }
 __device__ __forceinline__ void abort_raise(volatile int* abort_flag, int* status, int code) {
   abort_flag[AB_FLAG] = 1;

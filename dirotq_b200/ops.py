@@ -85,8 +85,12 @@ def status_word(device) -> torch.Tensor:
     key = dev.index if dev.index is not None else torch.cuda.current_device()
     word = _status.get(key)
     if word is None:
-        word = _status[key] = torch.zeros(8, dtype=torch.int32).pin_memory()
+        word = _status.setdefault(key, _new_status_word())          # one word per device, whichever thread asked first
     return word
+
+
+def _new_status_word() -> torch.Tensor:
+    return torch.zeros(8, dtype=torch.int32).pin_memory()
 
 
 class StatusWatch:
@@ -117,7 +121,7 @@ def status_watch(device) -> StatusWatch:
     key = dev.index if dev.index is not None else torch.cuda.current_device()
     watch = _watch.get(key)
     if watch is None:
-        watch = _watch[key] = StatusWatch(torch.device("cuda", key))
+        watch = _watch.setdefault(key, StatusWatch(torch.device("cuda", key)))
     return watch
 
 
@@ -127,9 +131,10 @@ def set_wait_limit_cycles(cycles: int):
 
 
 def check_status(device=None):
-    """Synchronising read of the status word; raises if a bounded device-side wait ran out."""
+    """Read of the status word once the device's current stream has finished; raises if a bounded device-side wait ran
+    out.  Other streams are not waited for: what they have reported so far counts, and one of them may be capturing."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    torch.cuda.synchronize(dev)
+    torch.cuda.current_stream(dev).synchronize()
     s = int(status_word(dev)[0].item())
     if s != 0:
         status_word(dev).zero_()

@@ -7,7 +7,8 @@
  *
  * Return value: 0 = launched, < 0 = argument rejected on the host before any launch (see
  * dirotq_error_string).  Device-side bounded waits that run out write a positive code into the
- * caller's `status` word (int32, device memory, must be zero before the call); the kernel then
+ * caller's `status` word (int32, must be zero before the call; device memory, or host memory that the device can write,
+ * such as pinned memory: kernels only ever compare-and-swap it, at system scope); the kernel then
  * unwinds and returns normally, so the context stays usable.
  */
 #ifndef DIROTQ_B200_H
@@ -125,7 +126,7 @@ int dirotq_quantize_act(const dirotq_act_format* fmt, const void* x, int64_t x_p
  *           formats the block-diagonal matrix of the H transposed d x d blocks
  *   x_rot : optional bf16 [M, width] output of the rotated tensor (may be NULL)
  *   codes/scales/zeros/tail: as above; all four NULL = rotation only (x_rot required)
- *   status: int32 device word (zero on entry)
+ *   status: int32 word the device can write (zero on entry)
  */
 int dirotq_rotate_quantize(const dirotq_act_format* fmt, const void* x, const void* rot_t, int64_t M, void* x_rot,
                            void* codes, void* scales, void* zeros, void* tail, int32_t* status, void* stream);

@@ -345,3 +345,37 @@ def test_workspaces_belong_to_one_stream_or_one_captured_step(monkeypatch):
     assert sorted(grp.held) == [(0, 11, 0, 0), (0, 14, 0, 905)]
     here[0] = (0, 11, 0, 0)
     assert grp.lookup(x, 1) is held and (0, 11, 0, 0) not in grp.held
+
+
+def test_status_word_is_one_per_device_and_its_check_waits_for_one_stream(monkeypatch):
+    """Two threads that ask for a device's status word first get the same one (kernels write it, the watch reads it), and
+    check_status waits for the current stream, not for the device (another stream may be in a capture)."""
+    from dirotq_b200 import ops
+    monkeypatch.setattr(ops, "_status", {})
+    asked = []
+
+    def new_word():                                   # while one thread makes the word, another one asks for it
+        if not asked:
+            asked.append(None)
+            asked[0] = ops.status_word("cuda:3")
+        return torch.zeros(8, dtype=torch.int32)
+
+    monkeypatch.setattr(ops, "_new_status_word", new_word)
+    word = ops.status_word("cuda:3")
+    assert word is asked[0] and ops.status_word("cuda:3") is word
+    waited = []
+
+    class Stream:
+        def synchronize(self):
+            waited.append(1)
+
+    def whole_device(*a):
+        raise AssertionError("the whole device was waited for")
+
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: Stream())
+    monkeypatch.setattr(torch.cuda, "synchronize", whole_device)
+    ops.check_status("cuda:3")
+    word[0] = 3
+    with pytest.raises(RuntimeError, match="timeout"):
+        ops.check_status("cuda:3")
+    assert len(waited) == 2 and int(word[0]) == 0
