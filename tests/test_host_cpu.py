@@ -379,3 +379,28 @@ def test_status_word_is_one_per_device_and_its_check_waits_for_one_stream(monkey
     with pytest.raises(RuntimeError, match="timeout"):
         ops.check_status("cuda:3")
     assert len(waited) == 2 and int(word[0]) == 0
+
+
+def test_forward_takes_a_quantizer_that_is_no_registered_submodule():
+    """The patched forward reads wrapper.quantizer as an attribute: a subclass whose quantizer is a property, or a wrapper
+    with a plain object in its place, works as one with a registered submodule."""
+    from types import SimpleNamespace
+    from dirotq_b200 import backend
+    from dirotq_b200.wrapper import ActQuantWrapper
+
+    class Sub(ActQuantWrapper):
+        @property
+        def quantizer(self):
+            return SimpleNamespace(bits=16)
+
+        @quantizer.setter
+        def quantizer(self, value):
+            pass
+
+    lin = nn.Linear(8, 4)
+    x = torch.randn(2, 3, 8)
+    assert torch.equal(backend._fused_forward_b200(Sub(lin), x), lin(x))
+    plain = ActQuantWrapper(lin)
+    del plain.quantizer
+    object.__setattr__(plain, "quantizer", SimpleNamespace(bits=16))
+    assert torch.equal(backend._fused_forward_b200(plain, x), lin(x))
