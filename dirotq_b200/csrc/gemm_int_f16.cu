@@ -1067,14 +1067,9 @@ template <int BN, int AMODE, bool PAIR>
 static int launch_gf(const GfMaps& tm, const GemmIntF16Args& a, cudaStream_t st) {
   using Cfg = GfCfg<BN, AMODE == 2, PAIR>;
   auto k = gemm_int_f16_kernel<BN, AMODE, PAIR>;
-  static PerDeviceOnce attr_once;
+  static PerDeviceOnce attr_once, regs_once;
   if (int rc = set_max_dynamic_smem(attr_once, k, Cfg::SMEM_BYTES)) return rc;
-  // the register split is only sound if the kernel was compiled to the launch's share
-  static const bool regs_ok = [&] {
-    cudaFuncAttributes fa;
-    return cudaFuncGetAttributes(&fa, k) == cudaSuccess && fa.numRegs >= Cfg::REGS_LAUNCH;
-  }();
-  if (!regs_ok) return DIROTQ_E_UNSUPPORTED;
+  if (int rc = check_compiled_regs(regs_once, k, Cfg::REGS_LAUNCH)) return rc;
   if constexpr (PAIR) {
     const int64_t tiles = ((a.N + BN - 1) / BN) * ((a.M + 255) / 256);
     cudaLaunchConfig_t cfg = {};

@@ -560,14 +560,9 @@ static int launch_pair(const GemmFp4Args& a, cudaStream_t st) {
     twt = twq;
   }
   auto k = gemm_nvfp4_pair_kernel<BN, QOUT>;
-  static PerDeviceOnce attr_once;
+  static PerDeviceOnce attr_once, regs_once;
   if (int rc2 = set_max_dynamic_smem(attr_once, k, Cfg::SMEM_BYTES)) return rc2;
-  // the register split is only sound if the kernel was compiled to the launch's share
-  static const bool regs_ok = [&] {
-    cudaFuncAttributes fa;
-    return cudaFuncGetAttributes(&fa, k) == cudaSuccess && fa.numRegs >= Cfg::REGS_LAUNCH;
-  }();
-  if (!regs_ok) return DIROTQ_E_UNSUPPORTED;
+  if (int rc2 = check_compiled_regs(regs_once, k, Cfg::REGS_LAUNCH)) return rc2;
   const int tiles = (int)((a.M + 255) / 256) * (int)((a.N + BN - 1) / BN);
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(Cfg::THREADS);

@@ -28,6 +28,23 @@ inline int set_max_dynamic_smem(PerDeviceOnce& once, K kernel, int bytes) {
   return DIROTQ_OK;
 }
 
+// A register split between warpgroups (setmaxnreg) is only sound if the kernel was compiled to the launch's share.  Asked once
+// per device; a query that fails says nothing about the kernel and is asked again by the next launch.
+template <typename K>
+inline int check_compiled_regs(PerDeviceOnce& once, K kernel, int need) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) return DIROTQ_E_CUDA;
+  if (dev >= 64) return DIROTQ_E_UNSUPPORTED;
+  const unsigned long long bit = 1ull << dev;
+  if (!(once.done.load(std::memory_order_acquire) & bit)) {
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) return DIROTQ_E_CUDA;
+    if (fa.numRegs < need) return DIROTQ_E_UNSUPPORTED;
+    once.done.fetch_or(bit, std::memory_order_release);
+  }
+  return DIROTQ_OK;
+}
+
 // Launch with programmatic stream serialization allowed (see pdl_wait() in ptx.cuh).
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {

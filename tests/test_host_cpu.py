@@ -404,3 +404,45 @@ def test_forward_takes_a_quantizer_that_is_no_registered_submodule():
     del plain.quantizer
     object.__setattr__(plain, "quantizer", SimpleNamespace(bits=16))
     assert torch.equal(backend._fused_forward_b200(plain, x), lin(x))
+
+
+def test_a_failed_register_query_is_asked_again(tmp_path):
+    """launchers.cuh, check_compiled_regs against stand-ins for the two runtime calls: a query that fails refuses that
+    launch only; a kernel compiled to fewer registers is refused; the answer is kept per device."""
+    import shutil
+    import subprocess
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc")
+    src = tmp_path / "t.cu"
+    src.write_text(r'''
+#include <cuda_runtime.h>
+#include <cstdio>
+static int g_dev = 0, g_calls = 0, g_regs = 96;
+static cudaError_t g_answer = cudaErrorInitializationError;
+static cudaError_t fake_device(int* d) { *d = g_dev; return cudaSuccess; }
+static cudaError_t fake_attr(cudaFuncAttributes* fa, void (*)()) { ++g_calls; fa->numRegs = g_regs; return g_answer; }
+#define cudaGetDevice fake_device
+#define cudaFuncGetAttributes fake_attr
+#include "launchers.cuh"
+int main() {
+  dq::PerDeviceOnce once;
+  auto ask = [&] { return dq::check_compiled_regs(once, (void (*)())nullptr, 96); };
+  const int a = ask();                 // the query fails
+  g_answer = cudaSuccess;
+  const int b = ask(), c = ask();      // answered, then remembered
+  const int calls = g_calls;
+  g_dev = 1; g_regs = 95;
+  const int d = ask();                 // another device, too few registers
+  g_regs = 96;
+  const int e = ask();
+  printf("%d %d %d %d %d %d\n", a, b, c, calls, d, e);
+}
+''')
+    exe = tmp_path / "t"
+    subprocess.run([nvcc, "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", os.path.join(ROOT, "dirotq_b200", "csrc"),
+                    str(src), "-o", str(exe)], check=True, capture_output=True)
+    got = [int(v) for v in subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()]
+    hdr = open(os.path.join(ROOT, "include", "dirotq_b200.h")).read()
+    code = lambda name: int(re.search(name + r"\s*=\s*(-?\d+)", hdr).group(1))
+    assert got == [code("DIROTQ_E_CUDA"), 0, 0, 2, code("DIROTQ_E_UNSUPPORTED"), 0]
