@@ -104,6 +104,27 @@ def _buffer(owner, live: dict, M: int, place: tuple, make) -> torch.Tensor:
     return e[1]
 
 
+def _mark_built(owner, place: tuple):
+    """Something of `owner` that calls on other streams will read (packed weights, a resident 16-bit copy) has just been
+    queued on the current stream, inside a forward: the caller does not know of it and cannot order the streams."""
+    if place[0] is not None and not place[3]:
+        ev = torch.cuda.Event()
+        ev.record(torch.cuda.current_stream(place[0]))
+        owner.built = (ev, place[1])
+
+
+def _await_built(owner, place: tuple):
+    """Order the current stream behind what _mark_built noted.  (A capture cannot wait for work outside it; it starts behind a
+    synchronisation and after a call that built everything.)"""
+    ev, stream = owner.built
+    if place[3]:
+        return
+    if ev.query():
+        owner.built = None
+    elif stream != place[1]:
+        torch.cuda.current_stream(place[0]).wait_event(ev)
+
+
 def _drop_places(held: dict, gone):
     for p in [p for p in held if gone(p)]:
         held.pop(p, None)
@@ -213,6 +234,7 @@ class LayerState:
     chain_hits: int = 0
     chain_fed: bool = False                          # a producer's epilogue quantises for this layer
     panel_declined: bool = False                     # a large-batch call found the resident-panel budget spent
+    built: Optional[tuple] = None                    # see _mark_built
     _c: Optional[LinearC] = None
     _ws: Dict[tuple, tuple] = field(default_factory=dict)          # see _buffer
 
@@ -321,10 +343,13 @@ def linear_forward(st: LayerState, x2d: torch.Tensor, out: Optional[torch.Tensor
         half = bool(_lib.lib().dirotq_linear_uses_half_chunks(C.byref(st.c_struct())))
         st.folded.panel = ops.expand_weight_panel_f16(pk, st.folded, half)
         st._c = None
+        _mark_built(st, place)
         if st.shared is None:
             st._ws = {}                 # the workspace no longer needs room for a per-call panel
     elif CACHE_WEIGHT_PANEL == "auto" and st.folded is not None and st.folded.panel is None and M > PANEL_CACHE_MAX_ROWS:
         st.panel_declined = True        # over the budget: asked once, not on every call
+    if st.built is not None:
+        _await_built(st, place)
     watch = ops.status_watch(x2d.device)
     if WATCH_STATUS:
         watch.poll()                    # a wait that ran out in an earlier call surfaces here (no synchronisation)
@@ -608,6 +633,7 @@ class W4A16State:
     bias: Optional[torch.Tensor]
     dense: Optional[torch.Tensor] = None      # resident dequantised weight (bf16 [N, K]), see w4a16_forward
     declined: bool = False                    # a large-batch call found the budget for resident 16-bit copies spent
+    built: Optional[tuple] = None             # see _mark_built
 
 
 # Dequantised weights of W4A16 layers follow the policy of CACHE_WEIGHT_PANEL: resident (2 bytes per weight) for layers
@@ -631,6 +657,8 @@ def _w4a16_scratch(nbytes: int, device) -> torch.Tensor:
 def w4a16_forward(s16: W4A16State, x2d: torch.Tensor) -> torch.Tensor:
     """bf16 activations x 4-bit weight: x2d bf16 [M, K] -> bf16 [M, N]."""
     M = x2d.shape[0]
+    if s16.built is not None:
+        _await_built(s16, _place(x2d.device))
     nvfp4 = isinstance(s16.w, ops.PackedWeightNvfp4)
     resident = s16.dense is not None or CACHE_WEIGHT_PANEL is True
     if not resident and CACHE_WEIGHT_PANEL == "auto" and not s16.declined:
@@ -639,6 +667,7 @@ def w4a16_forward(s16: W4A16State, x2d: torch.Tensor) -> torch.Tensor:
     if resident:
         if s16.dense is None:
             s16.dense = ops.dequant_weight_nvfp4(s16.w) if nvfp4 else ops.dequant_weight_int4(s16.w)
+            _mark_built(s16, _place(x2d.device))
         return ops.gemm_bf16(x2d, s16.dense, s16.bias)
     K = s16.w.n_chunks * 64
     scratch = _w4a16_scratch(int(_lib.lib().dirotq_gemm_w4a16_workspace_bytes(s16.w.N, K)), x2d.device)
@@ -688,6 +717,8 @@ def _fused_forward_b200(self, x):
         s16 = getattr(self, "_b200_w4a16", None)
         if s16 is None and getattr(self, "_b200_explicit", None) is not None:
             s16 = prepare_w4a16(self, x.device, self._b200_explicit)     # synthetic layer: no dense weight
+            if s16 is not None:
+                _mark_built(s16, _place(x.device))
             object.__setattr__(self, "_b200_w4a16", s16)
         if s16 is None:
             return self.module(x).to(x.dtype)
@@ -698,6 +729,7 @@ def _fused_forward_b200(self, x):
     st = getattr(self, "_b200_state", None)
     if st is None:
         st = prepare_layer(self, x.device, getattr(self, "_b200_explicit", None))
+        _mark_built(st, _place(x.device))
         object.__setattr__(self, "_b200_state", st)
     x_dtype = x.dtype
     shp = x.shape

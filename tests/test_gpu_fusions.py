@@ -426,3 +426,23 @@ def test_same_layers_called_from_two_streams(quant):
         for g, w in zip(got[s], want[s]):
             assert all(torch.equal(a, b) for a, b in zip(g, w))
     ops.check_status()
+
+
+def test_first_calls_on_two_streams_share_what_the_first_builds():
+    """A layer prepared and given its resident panel inside its first forward, on one stream, and called at once on another."""
+    from dirotq_b200 import backend, dit, ops
+    from dirotq_b200.synth import synth_activations
+    x = synth_activations(640, 1152, torch.Generator().manual_seed(3)).cuda()
+    mk = lambda: dit.make_wrapped_linear(dit.LayerDef("proj", 1152, 4608, tail=64), "int4", 91, "cuda")
+    want = mk()(x)
+    torch.cuda.synchronize()
+    for _ in range(4):
+        w, (s1, s2) = mk(), (torch.cuda.Stream(), torch.cuda.Stream())
+        torch.cuda.synchronize()
+        with torch.cuda.stream(s1):
+            y1 = w(x)
+        with torch.cuda.stream(s2):
+            y2 = w(x)
+        torch.cuda.synchronize()
+        assert torch.equal(y1, want) and torch.equal(y2, want)
+    ops.check_status()

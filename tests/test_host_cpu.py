@@ -446,3 +446,38 @@ int main() {
     hdr = open(os.path.join(ROOT, "include", "dirotq_b200.h")).read()
     code = lambda name: int(re.search(name + r"\s*=\s*(-?\d+)", hdr).group(1))
     assert got == [code("DIROTQ_E_CUDA"), 0, 0, 2, code("DIROTQ_E_UNSUPPORTED"), 0]
+
+
+def test_what_a_forward_builds_is_awaited_by_other_streams(monkeypatch):
+    """A panel or a packed weight queued by the first forward on one stream: calls on another stream wait for it until it
+    has completed, calls on the same stream and calls in a capture do not."""
+    from types import SimpleNamespace
+    from dirotq_b200 import backend
+    done, waited = [False], []
+
+    class Event:
+        def record(self, stream):
+            self.stream = stream
+
+        def query(self):
+            return done[0]
+
+    class Stream:
+        def wait_event(self, ev):
+            waited.append(ev)
+
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: Stream())
+    owner = SimpleNamespace(built=None)
+    backend._mark_built(owner, (0, 11, 0, 0))
+    ev = owner.built[0]
+    backend._await_built(owner, (0, 11, 0, 0))
+    backend._await_built(owner, (0, 12, 0, 77))
+    assert not waited
+    backend._await_built(owner, (0, 12, 0, 0))
+    assert waited == [ev] and owner.built is not None
+    done[0] = True
+    backend._await_built(owner, (0, 12, 0, 0))
+    assert waited == [ev] and owner.built is None
+    backend._mark_built(owner, (None, 0, 0, 0))
+    assert owner.built is None
