@@ -8,8 +8,9 @@
 // n / 16 threads per row (several rows per CTA when that is fewer than 256), 16 values per thread in registers.  Four
 // stages at a time are register arithmetic: in pass p a thread holds the 16 values whose indices differ only in bits
 // 4p .. 4p+3, so the stages h = 2^(4p) .. 2^(4p+3) need no exchange; between passes the values trade places through
-// shared memory (rows of 16 floats padded to 17: conflict-free in every pass with four stages).  A thread writes only
-// the positions it read, so one barrier per exchange is enough.  4096 rows x 4608 channels, n = 4096: 98 -> 20 us (one
+// shared memory (rows of 16 floats padded to 17: conflict-free in the first two passes; in a third, whose lanes reach over
+// two rows, lanes 0 and 31 share a bank).  A thread writes only
+// the positions it read, so one barrier per exchange is enough.  4096 rows x 4608 channels, n = 4096: 98 -> 21 us (one
 // barrier pair and one shared-memory round trip per stage, with the butterfly's index arithmetic, before).
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -35,13 +36,34 @@ __device__ __forceinline__ void fwht_stages(float* v) {      // BITS stages over
   }
 }
 
+// A row of 16 or 32 transformed channels has one or two threads, 256 or 128 rows share a block, and the rest of a row is as
+// wide as ever: blocks of their own copy it (1152 channels, n = 16: 54 -> 2 us for 256 rows, 85 -> 26 for 32768).  Longer
+// transforms copy theirs in passing, which the loads of the transform hide (n = 8192 of 12288 channels, 32768 rows: 415 us,
+// 473 with blocks of their own; from n = 128 to 512 the two differ by a microsecond either way).
+constexpr bool copy_blocks_of(int logn) { return logn <= 5; }
+
 template <int LOGN>
 __global__ void __launch_bounds__(LOGN == 13 ? 512 : 256)
 hadamard_low_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int D, const __nv_bfloat16* __restrict__ flips,
-                    float inv_norm_is_exact, float norm, __nv_bfloat16* __restrict__ y) {
+                    float inv_norm_is_exact, float norm, __nv_bfloat16* __restrict__ y, int fwht_blocks, int copy_rows) {
   constexpr int N = 1 << LOGN, T = N / 16, THREADS = LOGN == 13 ? 512 : 256, ROWS = THREADS / T;
   constexpr int FULL = LOGN / 4, REM = LOGN % 4;              // passes of four stages, stages of the last pass
   __shared__ float sh[(FULL > 1 || REM) ? ROWS * T * 17 : 1];
+  if constexpr (copy_blocks_of(LOGN)) {
+    if ((int)blockIdx.x >= fwht_blocks) {                     // untouched channels of copy_rows rows
+      const int per = (D - N) >> 3;                           // 16-byte units per row
+      const int64_t r0 = (int64_t)((int)blockIdx.x - fwht_blocks) * copy_rows;
+      pdl_launch_dependents();
+      pdl_wait();
+      for (int i = threadIdx.x; i < copy_rows * per; i += THREADS) {
+        const int r = i / per;
+        if (r0 + r >= M) break;
+        const int64_t at = (r0 + r) * D + N + 8 * (i - r * per);
+        *reinterpret_cast<uint4*>(y + at) = *reinterpret_cast<const uint4*>(x + at);
+      }
+      return;
+    }
+  }
   const int t = threadIdx.x % T, lr = threadIdx.x / T;
   const int64_t row = (int64_t)blockIdx.x * ROWS + lr;
   const bool ok = row < M;
@@ -132,7 +154,8 @@ hadamard_low_kernel(const __nv_bfloat16* __restrict__ x, int64_t M, int D, const
       }
     }
     // untouched channels
-    for (int c = N + 8 * t; c < D; c += 8 * T) *reinterpret_cast<uint4*>(yr + c) = *reinterpret_cast<const uint4*>(xr + c);
+    if constexpr (!copy_blocks_of(LOGN))
+      for (int c = N + 8 * t; c < D; c += 8 * T) *reinterpret_cast<uint4*>(yr + c) = *reinterpret_cast<const uint4*>(xr + c);
   }
 }
 
@@ -141,9 +164,14 @@ static int launch_fwht(const void* x, int64_t M, int D, const void* flips, void*
   constexpr int THREADS = LOGN == 13 ? 512 : 256, ROWS = THREADS / ((1 << LOGN) / 16);
   const float norm = sqrtf((float)(1 << LOGN));
   const float inv_exact = (LOGN % 2 == 0) ? 1.f / norm : 0.f;     // power of four: the division is an exact scaling
-  return launch_pdl(hadamard_low_kernel<LOGN>, dim3((unsigned)((M + ROWS - 1) / ROWS)), dim3(THREADS), 0, st,
+  const int64_t fwht_blocks = (M + ROWS - 1) / ROWS;
+  const int per = (D - (1 << LOGN)) / 8;                      // 16-byte units to copy per row, four per thread and block
+  const int copy_rows = per > 0 && per < 4 * THREADS ? 4 * THREADS / per : 1;
+  const int64_t copy_blocks = copy_blocks_of(LOGN) && per > 0 ? (M + copy_rows - 1) / copy_rows : 0;
+  if (fwht_blocks + copy_blocks > 0x7fffffff) return DIROTQ_E_TOO_LARGE;
+  return launch_pdl(hadamard_low_kernel<LOGN>, dim3((unsigned)(fwht_blocks + copy_blocks)), dim3(THREADS), 0, st,
                     static_cast<const __nv_bfloat16*>(x), M, D, static_cast<const __nv_bfloat16*>(flips), inv_exact, norm,
-                    static_cast<__nv_bfloat16*>(y)) == cudaSuccess
+                    static_cast<__nv_bfloat16*>(y), (int)fwht_blocks, copy_rows) == cudaSuccess
              ? DIROTQ_OK : DIROTQ_E_CUDA;
 }
 

@@ -502,6 +502,21 @@ def test_hadamard_front_end_short_transforms(low_dim):
         assert torch.equal(y.view(torch.int16), O.hadamard_low(x, low_dim, flips, fp32=False).view(torch.int16)), M
 
 
+@pytest.mark.parametrize("D,low_dim", [(16, 16), (24, 16), (1152, 16), (1152, 32), (9232, 16)])
+@pytest.mark.parametrize("M", [1, 7, 257, 3000])
+def test_hadamard_front_end_copies_the_rest_of_short_transforms(D, low_dim, M):
+    """Transforms of 16 or 32 channels: blocks of their own copy the other channels -- none, one unit a row, several rows a
+    block, a row wider than a block's share, a last block partly past the end -- and nothing past the last row."""
+    from dirotq_b200 import ops
+    g = torch.Generator().manual_seed(D + M)
+    x = torch.randn(M, D, generator=g).to(torch.bfloat16)
+    flips = (torch.randint(0, 2, (low_dim,), generator=g).float() * 2 - 1).to(torch.bfloat16)
+    out = torch.full((M + 3, D), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.hadamard_low(x.cuda(), low_dim, flips.cuda(), out=out[:M])
+    ref = O.hadamard_low(x, low_dim, flips, fp32=False)
+    assert torch.equal(out[:M].cpu().view(torch.int16), ref.view(torch.int16)) and bool((out[M:] == 7.0).all())
+
+
 @pytest.mark.parametrize("quant", ["int4", "int8", "nvfp4"])
 def test_gelu_fused_into_the_gemm_epilogue(quant):
     """ff.net.0 = GELU(proj(x)): with the activation fused into the up-projection's epilogue the module returns
