@@ -261,6 +261,30 @@ def test_int_f16_gemm_wide_tiles(mode, M, N, D, tail):
     assert rel_l2(y[-(M % 128 or 128):], y_ref[-(M % 128 or 128):]) < 4e-3 and rel_l2(y[:, -8:], y_ref[:, -8:]) < 4e-3
 
 
+@pytest.mark.parametrize("pair", ["0", "1"])
+@pytest.mark.parametrize("mode,M,N,D,tail", [("sym", 1, 8, 64, 0), ("asym", 128, 136, 1152, 64), ("int8", 129, 264, 192, 72),
+                                             ("sym", 257, 264, 640, 8), ("int8", 257, 8, 1152, 0), ("asym", 1, 264, 192, 128)])
+def test_int_f16_gemm_forced_wide_tiles(monkeypatch, pair, mode, M, N, D, tail):
+    """The 256-wide kernels on one CTA and on CTA pairs where the launcher would not pick them, whatever its thresholds: one
+    row, one column block of 8, one operand stage, a pair whose second half is empty or holds a row, more stages than slots."""
+    monkeypatch.setenv("DIROTQ_GF_BN", "256")
+    monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
+    test_int_f16_gemm_edge_shapes(mode, M, N, D, tail)
+
+
+@pytest.mark.parametrize("pair", ["0", "1"])
+@pytest.mark.parametrize("quant,a_sym,H", [("int4", True, 5), ("int4", False, 70), ("int8", False, 7)])
+def test_int_f16_gemm_forced_wide_tiles_with_half_chunks(monkeypatch, pair, quant, a_sym, H):
+    """The same with two half-filled chunks per operand stage (short per-head groups, odd and even head counts)."""
+    from dirotq_b200 import backend
+    from dirotq_b200.wrapper import ActQuantWrapper
+    import test_gpu_models
+    monkeypatch.setenv("DIROTQ_GF_BN", "256")
+    monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
+    monkeypatch.setattr(ActQuantWrapper, "forward", backend._fused_forward_b200)
+    test_gpu_models.test_short_per_head_groups_share_operand_stages(quant, a_sym, H, 300, monkeypatch)
+
+
 def test_int_f16_gemm_empty_batch():
     from dirotq_b200 import ops
     fmt = ops.ActFormat(ops.INT4_SYM, 128, tail_len=64)
