@@ -95,9 +95,9 @@ template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
   static constexpr int RAW_A = 128 * 32 * GF_CPS * (A8 ? 2 : 1);   // 8-bit activation codes: two 128-byte boxes per row
   static constexpr int OFF_C = RAW_A;                      // [chunk][128] 8-byte records
   static constexpr int RAW_STAGE = OFF_C + GF_CPS * 128 * 8;
-  // Accumulators: two of 128 columns (the next tile's UMMAs overlap the epilogue); a 256-wide tile has one, and its
+  // Accumulators: two of 128 columns (the next tile's UMMAs overlap the epilogue); a wider tile has one, and its
   // UMMAs wait until the epilogue has read the previous tile out of tensor memory.
-  static constexpr int NACC = BN == 256 ? 1 : 2;
+  static constexpr int NACC = BN > 128 ? 1 : 2;
   // Operand stages in flight: every tensor-memory column the accumulators leave free holds activations
   // (32 columns per 64-wide chunk), as far as shared memory holds the weight tiles beside them.
   static constexpr int RAW_STAGES = GF_RAW_DEF;
@@ -675,7 +675,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
       if (PAIR && rank != 0) mbar_arrive_cluster_relaxed(map_to_rank(acce_bar(b), 0));
       else mbar_arrive(acce_bar(b));
     };
-    const bool qout = a.q_codes != nullptr;
+    const bool qout = BN != 192 && a.q_codes != nullptr;
     auto put_patch = [&](const uint32_t* w16, int col, int row) {     // 32 columns of the warp's 32 rows -> y
       if (lane == 0) bulk_wait_read0();              // the previous patch has left the staging buffer
       __syncwarp();
@@ -1109,11 +1109,17 @@ static int launch_gf(const GfMaps& tm, const GemmIntF16Args& a, cudaStream_t st)
 // per-stage barrier protocol does not depend on the width, and the wide tile's single accumulator is handed back before
 // anything else is done with it).  So 256 wherever it saves a quarter of the rounds (1152 -> 3456 at 32768 rows: 213 us
 // against 311; 1152 -> 4608 at 4096: 44 / 62), 128 where both need the same few (1152 x 1152 at 4096 rows: 23.0 / 25.3;
-// 2240 x 2240 at 1024: 28.7 / 30.5).  A 192-wide tile lay between the two everywhere and is gone.  DIROTQ_GF_BN overrides.
-static int pick_bn_f16(int64_t M, int64_t N) {
-  if (const char* e = getenv("DIROTQ_GF_BN")) return atoi(e) > 128 ? 256 : 128;
+// 2240 x 2240 at 1024: 28.7 / 30.5).  A round of 192-wide tiles takes 6/5 of a 128-wide one: ahead where it needs no more
+// rounds than 256 (1152 x 1152 at 12288 rows, four of either: 38.7 us against 40.3, 8-bit activations 38.2 / 42.2; 1152 -> 3456
+// at 3072: 29.9 / 31.0), never otherwise.  From five rounds on, where 256-wide tiles run on CTA pairs, only for short K (15360
+// rows: 1152 x 1152 45.8 / 47.7, 4608 -> 1152 139 / 137).  The quantise-out epilogue wants whole groups of 64 columns per
+// warp: not 192.  DIROTQ_GF_BN overrides.
+static int pick_bn_f16(int64_t M, int64_t N, int64_t k_total, bool qout) {
+  if (const char* e = getenv("DIROTQ_GF_BN")) return atoi(e) <= 128 ? 128 : atoi(e) <= 192 && !qout ? 192 : 256;
   const int64_t m_tiles = (M + 127) / 128, sms = num_sms();
-  const int64_t r256 = (m_tiles * ((N + 255) / 256) + sms - 1) / sms, r128 = (m_tiles * ((N + 127) / 128) + sms - 1) / sms;
+  auto rounds = [&](int64_t bn) { return (m_tiles * ((N + bn - 1) / bn) + sms - 1) / sms; };
+  const int64_t r256 = rounds(256), r192 = rounds(192), r128 = rounds(128);
+  if (!qout && r192 == r256 && 6 * r192 < 5 * r128 && (r256 <= 4 || k_total < 2048)) return 192;
   return 9 * r256 < 7 * r128 ? 256 : 128;
 }
 
@@ -1146,7 +1152,9 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
   if ((reinterpret_cast<uintptr_t>(a.bias) & 15) || (reinterpret_cast<uintptr_t>(a.cs) & 15) || (a.N & 7) ||
       (reinterpret_cast<uintptr_t>(a.a_const) & 15) || (reinterpret_cast<uintptr_t>(a.w_panel) & 15) || !a.w_panel)
     return DIROTQ_E_ALIGN;
-  const int BN = a.force_bn ? a.force_bn : pick_bn_f16(a.M, a.N);
+  const uint64_t n_stage = a.half_chunks ? (uint64_t)((a.n_chunks + 1) / 2) : (uint64_t)a.n_chunks;
+  const int64_t k_total = (int64_t)n_stage * 64 + ((a.kt + 63) / 64) * 64;
+  const int BN = a.force_bn ? a.force_bn : pick_bn_f16(a.M, a.N, k_total, a.q_codes != nullptr);
   const bool pair = BN == 256 && pick_pair_f16(a.M, a.N);
   if (a.q_codes) {
     if (a.N % 64 || a.q_len % 64 || a.q_len <= 0 || a.q_len > a.N || a.q_row_bytes < a.q_len / 2 || (a.q_row_bytes & 15) ||
@@ -1162,8 +1170,7 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
   int rc = make_tmap_2d_sw(&tm.xq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.xq, (uint64_t)a.x_row_bytes, (uint64_t)a.M,
                            (uint64_t)a.x_row_bytes, 32 * GF_CPS, 128, 32 * GF_CPS);
   if (rc) return rc;
-  const uint64_t n_stage = a.half_chunks ? (uint64_t)((a.n_chunks + 1) / 2) : (uint64_t)a.n_chunks;
-  if (a.raster == 0) a.raster = pick_raster_f16(BN, a.N, (int64_t)n_stage * 64 + ((a.kt + 63) / 64) * 64);
+  if (a.raster == 0) a.raster = pick_raster_f16(BN, a.N, k_total);
   rc = make_tmap_2d(&tm.wp, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.w_panel, n_stage * 64, (uint64_t)a.N, n_stage * 128, pair ? BN / 2 : BN);
   if (rc) return rc;
   // without an output tensor (quantise-out only) the map is never used: any valid address will do
@@ -1191,6 +1198,9 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
     case 256 * 4 + 0: return launch_gf<256, 0, false>(tm, a, st);
     case 256 * 4 + 1: return launch_gf<256, 1, false>(tm, a, st);
     case 256 * 4 + 2: return launch_gf<256, 2, false>(tm, a, st);
+    case 192 * 4 + 0: return launch_gf<192, 0, false>(tm, a, st);
+    case 192 * 4 + 1: return launch_gf<192, 1, false>(tm, a, st);
+    case 192 * 4 + 2: return launch_gf<192, 2, false>(tm, a, st);
     case 128 * 4 + 0: return launch_gf<128, 0, false>(tm, a, st);
     case 128 * 4 + 1: return launch_gf<128, 1, false>(tm, a, st);
     case 128 * 4 + 2: return launch_gf<128, 2, false>(tm, a, st);

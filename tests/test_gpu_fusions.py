@@ -446,3 +446,17 @@ def test_first_calls_on_two_streams_share_what_the_first_builds():
         torch.cuda.synchronize()
         assert torch.equal(y1, want) and torch.equal(y2, want)
     ops.check_status()
+
+
+def test_quantise_out_under_the_192_wide_switch(monkeypatch):
+    """The epilogue that quantises for the next layer needs whole groups per warp: it keeps to 256-wide tiles, same bits."""
+    from dirotq_b200 import backend, ops
+    from dirotq_b200.synth import synth_activations
+    root, ff, up, down = _pair(1472, 64, False, 89)
+    x = synth_activations(300, 384, torch.Generator().manual_seed(5)).reshape(1, 300, 384).cuda()
+    want = ff.net[2](ff.net[0](x))
+    monkeypatch.setenv("DIROTQ_GF_BN", "192")
+    assert torch.equal(ff.net[2](ff.net[0](x)), want)
+    assert backend.fuse_ffn_quantise(root, keep_hidden=False) == 1
+    assert torch.equal(ff.net[2](ff.net[0](x)), want) and down._b200_state.chain_hits == 1
+    ops.check_status()

@@ -272,6 +272,22 @@ def test_int_f16_gemm_forced_wide_tiles(monkeypatch, pair, mode, M, N, D, tail):
     test_int_f16_gemm_edge_shapes(mode, M, N, D, tail)
 
 
+@pytest.mark.parametrize("mode,M,N,D,tail", [("sym", 1, 8, 64, 0), ("asym", 128, 200, 1152, 64), ("int8", 129, 392, 192, 72),
+                                             ("sym", 257, 192, 640, 8), ("int8", 385, 200, 2240, 320)])
+def test_int_f16_gemm_192_wide_tiles(monkeypatch, mode, M, N, D, tail):
+    """192-wide tiles at their edges: a first and a last tile of 8 columns, whole tiles, one operand stage and more than the
+    ring holds.  A quantise-out call under the same switch takes 256-wide ones."""
+    monkeypatch.setenv("DIROTQ_GF_BN", "192")
+    test_int_f16_gemm_edge_shapes(mode, M, N, D, tail)
+
+
+@pytest.mark.parametrize("mode", ["sym", "asym", "int8"])
+@pytest.mark.parametrize("M,N,D,tail", [(3000, 1152, 192, 8), (1001, 3456, 640, 64)])
+def test_int_f16_gemm_unforced_192_wide_tiles(mode, M, N, D, tail):
+    """Sizes for which 192-wide tiles need as many rounds as 256-wide ones, and fewer than 128-wide ones."""
+    test_int_f16_gemm_edge_shapes(mode, M, N, D, tail)
+
+
 @pytest.mark.parametrize("pair", ["0", "1"])
 @pytest.mark.parametrize("quant,a_sym,H", [("int4", True, 5), ("int4", False, 70), ("int8", False, 7)])
 def test_int_f16_gemm_forced_wide_tiles_with_half_chunks(monkeypatch, pair, quant, a_sym, H):

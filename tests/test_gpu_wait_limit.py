@@ -52,6 +52,7 @@ def _rotate_quantize(mode, M, D):
 _KERNELS = {
     "int exact": ({}, lambda: _int_gemm("asym", 300, 264, 4608, 64, exact=True)),
     "int 128": ({"DIROTQ_GF_BN": "128"}, lambda: _int_gemm("sym", 300, 264, 12288, 320)),
+    "int 192": ({"DIROTQ_GF_BN": "192"}, lambda: _int_gemm("int8", 300, 264, 12288, 320)),
     "int 256": ({"DIROTQ_GF_BN": "256", "DIROTQ_GF_PAIR": "0"}, lambda: _int_gemm("asym", 300, 264, 12288, 320)),
     "int pair": ({"DIROTQ_GF_BN": "256", "DIROTQ_GF_PAIR": "1"}, lambda: _int_gemm("sym", 300, 264, 12288, 320)),
     "int pair, many tiles": ({"DIROTQ_GF_BN": "256", "DIROTQ_GF_PAIR": "1"}, lambda: _int_gemm("int8", 5000, 2056, 3072, 384)),
