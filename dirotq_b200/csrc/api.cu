@@ -419,7 +419,6 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
   a.y = static_cast<__nv_bfloat16*>(y);
   a.status = status;
   a.wait_limit_k = wait_limit_k();
-  a.force_bn = 0;
   a.act = act;
   a.half_chunks = hc;
   if (qo) {

@@ -39,8 +39,8 @@
 //   UMMA issuer    tcgen05.mma kind::f16 (A from TMEM, B from smem descriptor), 4 x K=16 per chunk, fp32
 //                  128 x BN accumulator in TMEM; the bf16 tail accumulates into the same tile
 //   8 epilogue warps  tcgen05.ld, * rs[m] * cs[n], + bias, bf16 in registers, accumulator handed back, then 32 x 32 staging
-//                  patches -> TMA stores.  128-wide tiles have two accumulators, 256-wide tiles one (the columns it leaves
-//                  hold eight stages of activations)
+//                  patches -> TMA stores.  128-wide tiles have two accumulators, wider ones one (the columns it leaves hold
+//                  eight stages of activations)
 // PAIR (256-wide tiles of long launches): clusters of two CTAs drive one tcgen05.mma.cta_group::2 on a 256 x 256 tile.  Each
 // CTA converts its own 128 rows into its own tensor memory, fetches half of the weight tile (the tensor core reads the other
 // half from the peer's shared memory) and runs the epilogue of its 128 rows.  One barrier per stage in the leader counts the
@@ -1154,7 +1154,7 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
     return DIROTQ_E_ALIGN;
   const uint64_t n_stage = a.half_chunks ? (uint64_t)((a.n_chunks + 1) / 2) : (uint64_t)a.n_chunks;
   const int64_t k_total = (int64_t)n_stage * 64 + ((a.kt + 63) / 64) * 64;
-  const int BN = a.force_bn ? a.force_bn : pick_bn_f16(a.M, a.N, k_total, a.q_codes != nullptr);
+  const int BN = pick_bn_f16(a.M, a.N, k_total, a.q_codes != nullptr);
   const bool pair = BN == 256 && pick_pair_f16(a.M, a.N);
   if (a.q_codes) {
     if (a.N % 64 || a.q_len % 64 || a.q_len <= 0 || a.q_len > a.N || a.q_row_bytes < a.q_len / 2 || (a.q_row_bytes & 15) ||

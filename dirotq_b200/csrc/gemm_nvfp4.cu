@@ -275,7 +275,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
 // tiles (one accumulator) takes 1.4 rounds of 256 x 128 ones (two) at K = 3072, 1.46 at 2240 and 1.63 at 1152, where its
 // hand-over weighs more: 256 wherever the rounds it saves are worth that (256 / 128 columns: 3072 -> 9216 at 16384 rows 286 /
 // 403 us, 2240 x 2240 69 / 95, 1152 -> 3456 at 32768 rows 111 / 128), 128 for the few rounds of short calls (1152 x 1152 at
-// 4096 rows 19.1 / 16.9, 3072 x 3072 at 512 rows 31.0 / 29.6).  DIROTQ_NVFP4_TILE = single | pair128 | pair256 forces one
+// 4096 rows 19.1 / 16.9, 3072 x 3072 at 512 rows 31.0 / 29.6).  From K = 2048 on the line is drawn at 10/7 = 1.43 rounds for all: between it
+// and the 1.46 of K = 2240 lie only pairs like 13 rounds against 9, worth 2 %.  DIROTQ_NVFP4_TILE = single | pair128 | pair256 forces one
 // form (measurements, tests).
 static int pick_nvfp4_tile(const GemmFp4Args& a) {
   if (const char* e = getenv("DIROTQ_NVFP4_TILE")) {

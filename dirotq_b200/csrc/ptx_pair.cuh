@@ -33,12 +33,12 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t ran
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// one arrival on an mbarrier that may live in the peer CTA (shared::cluster address)
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
-}
-// The same without memory ordering: for hand-offs whose payload is TENSOR memory (made complete by tcgen05.wait::ld /
-// wait::st before the arrival), not shared or global memory.  A cluster-scope release has to drain the thread's
+// One arrival on an mbarrier that may live in the peer CTA (shared::cluster address), without memory ordering: for hand-offs
+// whose payload is TENSOR memory, not shared or global memory.  Tensor-memory accesses of two threads are ordered by the
+// tcgen05 fences around the barrier, which itself has to order execution only; this is the pattern that the PTX ISA gives for
+// it (tcgen05, memory consistency model, synchronization between different threads): tcgen05.wait::ld or ::st,
+// tcgen05.fence::before_thread_sync and a relaxed cluster-scope arrival on this side, the barrier's wait and
+// tcgen05.fence::after_thread_sync on the other.  A cluster-scope release has to drain the thread's
 // earlier stores first and costs on the order of a microsecond per arrival on this kernel's critical path.
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
@@ -89,16 +89,11 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 
 // Completion of all pair UMMAs issued so far by this thread -> one arrival on the barrier at this shared-memory offset in
 // BOTH CTAs of the pair.  One commit of this form instead of two (the second to an address mapped from the peer), with a
-// stage's FP4 UMMAs in one block, took the NVFP4 GEMM from 150 to 130 us for 1152 -> 3456 at 32768 rows: what the issuing
-// thread does is time the pipe idles.
+// stage's FP4 UMMAs in one block, took the NVFP4 GEMM on 128-wide tiles from 150 to 130 us for 1152 -> 3456 at 32768 rows (which
+// now takes 256-wide ones): what the issuing thread does is time the pipe idles.
 __device__ __forceinline__ void umma_commit_pair_both(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(bar), "h"((uint16_t)3) : "memory");
-}
-// 32 rows x 16 bytes of EACH CTA's shared memory -> that CTA's TMEM lanes 0..31 (4 columns), replicated to all four
-// lane quarters; issued once by the leader
-__device__ __forceinline__ void tmem_cp_32x128b_x4_pair(uint32_t taddr, uint64_t sdesc) {
-  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
 }
 // E2M1 x E2M1 with UE4M3 scale factors, 256 x N x 64 over the pair: each CTA contributes its 128 rows of A, its
 // N/2 rows of B and holds its 128 x N half of the accumulator
