@@ -40,17 +40,25 @@ _HW_NVFP4_ACT_SCALE = 1.0   # static fp32 tensor scale of NVFP4 activations (UE4
 #   * inside a WorkspaceScope (dit.GraphedCall) the buffers belong to the scope, which whoever replays the graph keeps;
 #   * in a capture without a scope every call gets memory of the graph's own pool, cleared by the graph.
 # ---------------------------------------------------------------------------------------------------------------------
-_LOCAL = threading.local()
+class _Local(threading.local):
+    scope = None                                       # the WorkspaceScope this thread is in
+
+
+_LOCAL = _Local()
 _SCOPE_SERIAL = itertools.count(1)
 
 
 def _place(device) -> tuple:
     """Where a call runs, as far as scratch and the results held in it go: (device, stream, scope, capture)."""
-    if device.type != "cuda":
-        return (None, 0, 0, 0)
-    idx = device.index if device.index is not None else torch.cuda.current_device()
+    idx = device.index
+    if idx is None:
+        if device.type != "cuda":
+            return (None, 0, 0, 0)
+        idx = torch.cuda.current_device()
     stream = torch._C._cuda_getCurrentRawStream(idx)
-    scope = getattr(_LOCAL, "scope", None)
+    scope = _LOCAL.scope
+    if scope is None and not torch._C._cuda_isCurrentStreamCapturing():
+        return (idx, stream, 0, 0)
     capture = _lib.lib().dirotq_stream_capture_id(stream) if torch._C._cuda_isCurrentStreamCapturing() else 0
     return (idx, stream, 0 if scope is None else scope.serial, capture)
 
@@ -69,7 +77,7 @@ class WorkspaceScope:
         self._outer: list = []
 
     def __enter__(self):
-        self._outer.append(getattr(_LOCAL, "scope", None))
+        self._outer.append(_LOCAL.scope)
         _LOCAL.scope = self
         return self
 
@@ -92,15 +100,14 @@ class WorkspaceScope:
 
 
 def _buffer(owner, live: dict, M: int, place: tuple, make) -> torch.Tensor:
-    """The scratch buffer of `owner` (a layer or a sibling group) for a call of M rows at `place`."""
-    scope = getattr(_LOCAL, "scope", None)
+    """A scratch buffer of `owner` (a layer or a sibling group) for calls of M rows at `place`, where `live` -- outside scopes
+    and captures, place -> (rows, buffer) -- has none."""
+    scope = _LOCAL.scope
     if scope is not None and (place[3] == 0 or (id(owner), M) in scope._ws):
         return scope.buffer(owner, M, make)
     if place[3]:
         return make()
-    e = live.get(place[:2])
-    if e is None or e[0] != M:
-        e = live[place[:2]] = (M, make())              # keep one size; diffusion steps reuse the same M
+    e = live[place] = (M, make())                      # keep one size; diffusion steps reuse the same M
     return e[1]
 
 
@@ -108,21 +115,17 @@ def _mark_built(owner, place: tuple):
     """Something of `owner` that calls on other streams will read (packed weights, a resident 16-bit copy) has just been
     queued on the current stream, inside a forward: the caller does not know of it and cannot order the streams."""
     if place[0] is not None and not place[3]:
-        ev = torch.cuda.Event()
-        ev.record(torch.cuda.current_stream(place[0]))
-        owner.built = (ev, place[1])
+        owner.built = (place[1], {place[1]})           # the stream, and those known to run behind it
 
 
 def _await_built(owner, place: tuple):
-    """Order the current stream behind what _mark_built noted.  (A capture cannot wait for work outside it; it starts behind a
-    synchronisation and after a call that built everything.)"""
-    ev, stream = owner.built
-    if place[3]:
-        return
-    if ev.query():
-        owner.built = None
-    elif stream != place[1]:
-        torch.cuda.current_stream(place[0]).wait_event(ev)
+    """Order a stream that calls `owner` for the first time behind what _mark_built noted.  (A capture cannot wait for work
+    outside it; it starts behind a synchronisation and after a call that built everything.)"""
+    stream, behind = owner.built
+    if place[1] not in behind and not place[3]:
+        builder = torch.cuda.ExternalStream(stream, device=place[0]) if stream else torch.cuda.default_stream(place[0])
+        torch.cuda.current_stream(place[0]).wait_stream(builder)
+        behind.add(place[1])
 
 
 def _drop_places(held: dict, gone):
@@ -259,11 +262,15 @@ class LayerState:
     def workspace(self, M: int, device, place: Optional[tuple] = None) -> torch.Tensor:
         place = _place(torch.device(device)) if place is None else place
         grp = self.shared
+        live = self._ws if grp is None else grp.ws
+        e = live.get(place)
+        if e is not None and e[0] == M:
+            return e[1]
         # zero once: padding entries of the scale-factor tiles are never written afterwards
         make = lambda: torch.zeros(max([256] + [int(_lib.lib().dirotq_linear_workspace_bytes(C.byref(m.c_struct()), M))
                                                 for m in (grp.members if grp is not None and grp.members else [self])]),
                                    dtype=torch.uint8, device=device)
-        return _buffer(self, self._ws, M, place, make) if grp is None else _buffer(grp, grp.ws, M, place, make)
+        return _buffer(self if grp is None else grp, live, M, place, make)
 
 
 def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
@@ -316,7 +323,8 @@ def linear_forward(st: LayerState, x2d: torch.Tensor, out: Optional[torch.Tensor
     M = x2d.shape[0]
     if M == 0:
         return out if out is not None else torch.empty(0, st.out_features, dtype=torch.bfloat16, device=x2d.device)
-    place = _place(x2d.device)
+    dev = x2d.device
+    place = _place(dev)
     grp = st.shared
     if grp is not None and grp.fused is not None:
         # siblings fused into one layer: the first member called on a tensor runs it, the others take their columns
@@ -333,7 +341,7 @@ def linear_forward(st: LayerState, x2d: torch.Tensor, out: Optional[torch.Tensor
                 out.copy_(part)
                 return out
             return part
-    y = out if out is not None else torch.empty(M, st.out_features, dtype=torch.bfloat16, device=x2d.device)
+    y = out if out is not None else torch.empty(M, st.out_features, dtype=torch.bfloat16, device=dev)
     if st.hadamard_low_dim:
         x2d = ops.hadamard_low(x2d, st.hadamard_low_dim, st.hadamard_flips)
     if (CACHE_WEIGHT_PANEL == "auto" and st.folded is not None and st.folded.panel is None and not st.panel_declined and
@@ -348,13 +356,14 @@ def linear_forward(st: LayerState, x2d: torch.Tensor, out: Optional[torch.Tensor
             st._ws = {}                 # the workspace no longer needs room for a per-call panel
     elif CACHE_WEIGHT_PANEL == "auto" and st.folded is not None and st.folded.panel is None and M > PANEL_CACHE_MAX_ROWS:
         st.panel_declined = True        # over the budget: asked once, not on every call
-    if st.built is not None:
+    if st.built is not None and place[1] not in st.built[1]:
         _await_built(st, place)
-    watch = ops.status_watch(x2d.device)
+    watch = ops.status_watch(dev)
     if WATCH_STATUS:
         watch.poll()                    # a wait that ran out in an earlier call surfaces here (no synchronisation)
     lib = _lib.lib()
-    lin, yp, status, stream = C.byref(st.c_struct()), y.data_ptr(), watch.ptr, ops.stream_ptr()
+    lin, yp, status = C.byref(st.c_struct()), y.data_ptr(), watch.ptr
+    stream = place[1] if torch._C._cuda_getDevice() == place[0] else ops.stream_ptr()
     h = st.handed_at.pop(place, None) if st.handed_at else None
     if h is not None and h.key == _tensor_key(x2d):
         # the producer's epilogue left this tensor's codes, scales and 16-bit channels in the workspace
@@ -365,7 +374,11 @@ def linear_forward(st: LayerState, x2d: torch.Tensor, out: Optional[torch.Tensor
             ops.mark_written(out)
         return y
     h = grp.lookup(x2d, st.member_id, place) if grp is not None else None
-    ws = h.ws if h is not None else st.workspace(M, x2d.device, place)
+    if h is not None:
+        ws = h.ws
+    else:
+        e = (st._ws if grp is None else grp.ws).get(place)
+        ws = e[1] if e is not None and e[0] == M else st.workspace(M, dev, place)
     wsp, wsn = ws.data_ptr(), ws.numel()
     nxt = st.chain_next
     if nxt is not None and grp is None and not nxt.hadamard_low_dim:

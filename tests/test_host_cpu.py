@@ -449,35 +449,29 @@ int main() {
 
 
 def test_what_a_forward_builds_is_awaited_by_other_streams(monkeypatch):
-    """A panel or a packed weight queued by the first forward on one stream: calls on another stream wait for it until it
-    has completed, calls on the same stream and calls in a capture do not."""
+    """A panel or a packed weight queued by the first forward on one stream: the first call on any other stream waits for
+    that one, calls on the same stream, later ones and calls in a capture do not."""
     from types import SimpleNamespace
     from dirotq_b200 import backend
-    done, waited = [False], []
-
-    class Event:
-        def record(self, stream):
-            self.stream = stream
-
-        def query(self):
-            return done[0]
+    waited = []
 
     class Stream:
-        def wait_event(self, ev):
-            waited.append(ev)
+        def __init__(self, name):
+            self.name = name
 
-    monkeypatch.setattr(torch.cuda, "Event", Event)
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: Stream())
+        def wait_stream(self, other):
+            waited.append((self.name, other.name))
+
+    here = [0]
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda dev=None: Stream(here[0]))
+    monkeypatch.setattr(torch.cuda, "ExternalStream", lambda s, device=None: Stream(s))
+    monkeypatch.setattr(torch.cuda, "default_stream", lambda device=None: Stream("default"))
+    for builder, name in ((11, 11), (0, "default")):
+        owner, waited[:] = SimpleNamespace(built=None), []
+        backend._mark_built(owner, (0, builder, 0, 0))
+        for here[0], capture in ((builder, 0), (12, 77), (12, 0), (12, 0), (13, 0), (13, 0)):
+            backend._await_built(owner, (0, here[0], 0, capture))
+        assert waited == [(12, name), (13, name)]
     owner = SimpleNamespace(built=None)
-    backend._mark_built(owner, (0, 11, 0, 0))
-    ev = owner.built[0]
-    backend._await_built(owner, (0, 11, 0, 0))
-    backend._await_built(owner, (0, 12, 0, 77))
-    assert not waited
-    backend._await_built(owner, (0, 12, 0, 0))
-    assert waited == [ev] and owner.built is not None
-    done[0] = True
-    backend._await_built(owner, (0, 12, 0, 0))
-    assert waited == [ev] and owner.built is None
     backend._mark_built(owner, (None, 0, 0, 0))
     assert owner.built is None
