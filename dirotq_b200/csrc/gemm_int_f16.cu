@@ -563,15 +563,15 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
     }
   } else if (warp == W_MMA) {
     // ------------------------------ UMMA issuer ----------------------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       const uint32_t idesc_h = idesc_dense(ACC_F32, FMT_F16, FMT_F16, TILE_M, BN);
       const uint32_t idesc_bf = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, TILE_M, BN);
       int use = 0, stages = 0;
       bool ok = true;
       // loop-invariant pieces of the per-stage operands: barrier addresses are 8 bytes per slot apart, the weight
       // descriptor's low word holds the slot address >> 4, the activation slots are 32 tensor-memory columns apart
-      int es0 = 0;
-      uint32_t ph0 = 0;
+      int es = 0;
+      uint32_t ph = 0;
       const uint32_t expw0 = expw_bar(0);
       constexpr uint32_t kFullOff = 8u * 2 * GF_EXP_STAGES;      // expw_bar(s) - expf_bar(s)
       constexpr uint32_t kEmptyOff = 8u * GF_EXP_STAGES;         // expw_bar(s) - expe_bar(s)
@@ -579,75 +579,46 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
       const uint32_t bdesc_lo0 = (uint32_t)bdesc0, bdesc_hi = (uint32_t)(bdesc0 >> 32);
       constexpr uint32_t kDescStep = Cfg::EXP_STAGE >> 4;
       const uint32_t a_tmem0 = tmem_base + Cfg::TMEM_A0;
+      const int ns = n_main + n_tail;
       for (int t = first; t < total_tiles && ok; t += step) {
         const int buf = Cfg::NACC == 2 ? (use & 1) : 0;
         const uint32_t acc_ph = (uint32_t)(Cfg::NACC == 2 ? (use >> 1) & 1 : use & 1);
-        if (!mbar_wait_hot(acce_bar(buf), acc_ph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) { ok = false; break; }
+        if (!mbar_wait_hot_warp(acce_bar(buf), acc_ph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
-        // A UMMA occupies the issuing thread until the tensor pipe has taken it, so whatever else this thread
-        // does between UMMAs is time the pipe idles; a barrier test costs about a hundred cycles, hit or miss.
-        // So stages go two at a time: the four tests of a pair are issued back to back (their latencies
-        // overlap) and eight UMMAs follow without a break.
-        const int ns = n_main + n_tail;
-        for (int st = 0; st < ns && ok;) {
-          const bool two = st + 1 < ns;
-          // slot / phase of the pair's second stage (the first stage's again when the tile ends on a single one)
-          int es1 = es0;
-          uint32_t ph1 = ph0;
-          if (two && ++es1 == GF_EXP_STAGES) { es1 = 0; ph1 ^= 1u; }
-          const uint32_t w0 = expw0 + 8u * es0, w1 = expw0 + 8u * es1;       // expf / expe lie at fixed offsets from expw
-          if constexpr (PAIR) {
-            // one barrier per stage covers both operands in both CTAs
-            const uint32_t f0 = w0 - kFullOff, f1 = w1 - kFullOff;
-            const uint32_t rdy = mbar_test2(f0, ph0, f1, ph1);
-            if (rdy != 3u) {
-              if (!(rdy & 1u)) ok = mbar_wait_hot(f0, ph0, abort_flag, a.status, ERR_WAIT_FULL);
-              if (ok && !(rdy & 2u)) ok = mbar_wait_hot(f1, ph1, abort_flag, a.status, ERR_WAIT_FULL);
-              if (!ok) break;
-            }
-            tc_fence_after();
-            umma_f16_ts_x4_pair(d, a_tmem0 + 32u * es0, bdesc_lo0 + kDescStep * es0, bdesc_hi, st < n_main ? idesc_h : idesc_bf,
-                                st > 0 ? 1u : 0u);
-            umma_commit_pair_both(w0 - kEmptyOff);
-            if (two) {
-              umma_f16_ts_x4_pair(d, a_tmem0 + 32u * es1, bdesc_lo0 + kDescStep * es1, bdesc_hi,
-                                  st + 1 < n_main ? idesc_h : idesc_bf, 1u);
-              umma_commit_pair_both(w1 - kEmptyOff);
-            }
-          } else {
-            const uint32_t rdy = mbar_test4(w0, ph0, w0 - kFullOff, ph0, w1, ph1, w1 - kFullOff, ph1);
-            if (rdy != 15u) {
-              if (!(rdy & 1u)) ok = mbar_wait_hot(w0, ph0, abort_flag, a.status, ERR_WAIT_FULL);
-              if (ok && !(rdy & 2u)) ok = mbar_wait_hot(w0 - kFullOff, ph0, abort_flag, a.status, ERR_WAIT_FULL);
-              if (ok && !(rdy & 4u)) ok = mbar_wait_hot(w1, ph1, abort_flag, a.status, ERR_WAIT_FULL);
-              if (ok && !(rdy & 8u)) ok = mbar_wait_hot(w1 - kFullOff, ph1, abort_flag, a.status, ERR_WAIT_FULL);
-              if (!ok) break;
-            }
-            tc_fence_after();
-            umma_f16_ts_x4(d, a_tmem0 + 32u * es0, bdesc_lo0 + kDescStep * es0, bdesc_hi, st < n_main ? idesc_h : idesc_bf,
-                           st > 0 ? 1u : 0u);
-            umma_commit(w0 - kEmptyOff);
-            if (two) {
-              umma_f16_ts_x4(d, a_tmem0 + 32u * es1, bdesc_lo0 + kDescStep * es1, bdesc_hi,
-                             st + 1 < n_main ? idesc_h : idesc_bf, 1u);
-              umma_commit(w1 - kEmptyOff);
+        // What this warp does between UMMAs is time the pipe idles, and it has few of them queued.
+        for (int st = 0; st < ns; ++st) {
+          const uint32_t w = expw0 + 8u * es;                      // expf / expe lie at fixed offsets from expw
+          // pairs: one barrier per stage covers both operands in both CTAs
+          if (PAIR ? !mbar_wait_hot_warp(w - kFullOff, ph, abort_flag, a.status, ERR_WAIT_FULL)
+                   : !mbar_wait2_hot_warp(w, ph, w - kFullOff, ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+          tc_fence_after();
+          if (elect_one()) {
+            const uint32_t idesc = st < n_main ? idesc_h : idesc_bf;
+            if constexpr (PAIR) {
+              umma_f16_ts_x4_pair(d, a_tmem0 + 32u * es, bdesc_lo0 + kDescStep * es, bdesc_hi, idesc, st > 0 ? 1u : 0u);
+              umma_commit_pair_both(w - kEmptyOff);
+            } else {
+              umma_f16_ts_x4(d, a_tmem0 + 32u * es, bdesc_lo0 + kDescStep * es, bdesc_hi, idesc, st > 0 ? 1u : 0u);
+              umma_commit(w - kEmptyOff);
             }
           }
-          st += two ? 2 : 1;
-          stages += two ? 2 : 1;
-          es0 = es1;
-          ph0 = ph1;
-          if (++es0 == GF_EXP_STAGES) { es0 = 0; ph0 ^= 1u; }
+          __syncwarp();
+          ++stages;
+          if (++es == GF_EXP_STAGES) { es = 0; ph ^= 1u; }
         }
-        if (ok) {
+        if (!ok) break;
+        if (elect_one()) {
           if constexpr (PAIR) umma_commit_pair_both(accf_bar(buf));
           else umma_commit(accf_bar(buf));
-          ++use;
         }
+        __syncwarp();
+        ++use;
       }
-      abort_flag[AB_UMMA] = stages;
-      abort_flag[AB_ACC] = use;
+      if (lane == 0) {
+        abort_flag[AB_UMMA] = stages;
+        abort_flag[AB_ACC] = use;
+      }
     }
   }
   } else {

@@ -86,14 +86,14 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
   const int nkb_pad = n_main * 4;                // 64-element k-blocks per row tile in the SF buffers
 
   if (warp == 0) {
-    if (lane == 0) {
-      GfRing r;
-      int issued = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        const int mb = t / n_tiles, nb = t - mb * n_tiles;
-        for (int st = 0; st < n_main + n_tail; ++st) {
-          if (!mbar_wait(empty_bar(r.s), r.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+    GfRing r;
+    int issued = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      const int mb = t / n_tiles, nb = t - mb * n_tiles;
+      for (int st = 0; st < n_main + n_tail; ++st) {
+        if (!mbar_wait_warp(empty_bar(r.s), r.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+        if (elect_one()) {
           const uint32_t sA = smem_base + r.s * GF_STAGE_BYTES;
           const uint32_t sB = sA + GF_TILE_BYTES;
           if (st < n_main) {
@@ -108,32 +108,33 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
             tma_load_2d(sA, &tm_xt, full_bar(r.s), (st - n_main) * 64, mb * 128);
             tma_load_2d(sB, &tm_wt, full_bar(r.s), (st - n_main) * 64, nb * 128);
           }
-          ++issued;
-          r.next();
         }
+        __syncwarp();
+        ++issued;
+        r.next();
       }
-      abort_flag[AB_ISSUED] = issued;
     }
+    if (lane == 0) abort_flag[AB_ISSUED] = issued;
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc_f4 = idesc_nvf4(128, 128);
-      const uint32_t idesc_bf = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, 128, 128);
-      GfRing r;
-      int buf = 0;
-      uint32_t aph = 0;
-      uint32_t sf_slot = 0;
-      int stages = 0, accs = 0;
-      const uint64_t op_d0 = smem_desc_sw128(smem_base), sf_d0 = smem_desc_rows16(smem_base);
-      const uint32_t op_lo0 = (uint32_t)op_d0, op_hi = (uint32_t)(op_d0 >> 32);
-      const uint32_t sf_lo0 = (uint32_t)sf_d0, sf_hi = (uint32_t)(sf_d0 >> 32);
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-        if (!mbar_wait(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
+    const uint32_t idesc_f4 = idesc_nvf4(128, 128);
+    const uint32_t idesc_bf = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, 128, 128);
+    GfRing r;
+    int buf = 0;
+    uint32_t aph = 0;
+    uint32_t sf_slot = 0;
+    int stages = 0, accs = 0;
+    const uint64_t op_d0 = smem_desc_sw128(smem_base), sf_d0 = smem_desc_rows16(smem_base);
+    const uint32_t op_lo0 = (uint32_t)op_d0, op_hi = (uint32_t)(op_d0 >> 32);
+    const uint32_t sf_lo0 = (uint32_t)sf_d0, sf_hi = (uint32_t)(sf_d0 >> 32);
+    bool ok = true;
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      if (!mbar_wait_warp(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
+      tc_fence_after();
+      const uint32_t d = tmem_base + buf * 128;
+      for (int st = 0; st < n_main + n_tail; ++st) {
+        if (!mbar_wait_warp(full_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d = tmem_base + buf * 128;
-        for (int st = 0; st < n_main + n_tail; ++st) {
-          if (!mbar_wait(full_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
-          tc_fence_after();
+        if (elect_one()) {
           const uint32_t sA = smem_base + r.s * GF_STAGE_BYTES;
           const uint64_t adesc = smem_desc_sw128(sA), bdesc = smem_desc_sw128(sA + GF_TILE_BYTES);
           if (st < n_main) {
@@ -155,21 +156,25 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
               umma_nvf4(d, adesc + 2 * kb, bdesc + 2 * kb, idesc_f4, (st > 0 || kb > 0) ? 1u : 0u, sfa_t + kb * 4,
                         sfb_t + kb * 4);
             }
-            sf_slot ^= 1;
           } else {
             const uint32_t a_lo = op_lo0 + (uint32_t)r.s * (GF_STAGE_BYTES >> 4);
             umma_f16_ss_x4(d, a_lo, a_lo + (GF_TILE_BYTES >> 4), op_hi, idesc_bf, 1u);
           }
           umma_commit(empty_bar(r.s));
-          ++stages;
-          r.next();
         }
-        if (!ok) break;
-        umma_commit(accf_bar(buf));
-        ++accs;
-        buf ^= 1;
-        if (buf == 0) aph ^= 1;
+        __syncwarp();
+        if (st < n_main) sf_slot ^= 1;
+        ++stages;
+        r.next();
       }
+      if (!ok) break;
+      if (elect_one()) umma_commit(accf_bar(buf));
+      __syncwarp();
+      ++accs;
+      buf ^= 1;
+      if (buf == 0) aph ^= 1;
+    }
+    if (lane == 0) {
       abort_flag[AB_UMMA] = stages;
       abort_flag[AB_ACC] = accs;
     }

@@ -184,16 +184,16 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
   if (warp < Cfg::SF_WARP0) {
   reg_dealloc<Cfg::REGS_PROD>();
   if (warp == 0) {
-    if (lane == 0) {
-      GfRingT<STAGES> r;
-      int issued = 0;
-      bool ok = true;
-      for (int t = first; t < total_tiles && ok; t += step) {
-        const int mp = t / n_tiles, nb = t - mp * n_tiles;
-        const int row_a = mp * 256 + (int)rank * 128;            // this CTA's activation rows
-        const int row_b = nb * BN + (int)rank * (BN / 2);        // this CTA's half of the weight rows
-        for (int st = 0; st < n_main + n_tail; ++st) {
-          if (!mbar_wait(empty_bar(r.s), r.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+    GfRingT<STAGES> r;
+    int issued = 0;
+    bool ok = true;
+    for (int t = first; t < total_tiles && ok; t += step) {
+      const int mp = t / n_tiles, nb = t - mp * n_tiles;
+      const int row_a = mp * 256 + (int)rank * 128;            // this CTA's activation rows
+      const int row_b = nb * BN + (int)rank * (BN / 2);        // this CTA's half of the weight rows
+      for (int st = 0; st < n_main + n_tail; ++st) {
+        if (!mbar_wait_warp(empty_bar(r.s), r.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+        if (elect_one()) {
           const uint32_t sA = smem_base + r.s * Cfg::STAGE_BYTES;
           const uint32_t sB = sA + Cfg::A_BYTES;
           const uint32_t fb = map_to_rank(full_bar(r.s), 0);     // completions are counted in the leader
@@ -214,14 +214,15 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
             tma_load_2d_pair(sA, &tm_xt, fb, (st - n_main) * 64, row_a);
             tma_load_2d_pair(sB, &tm_wt, fb, (st - n_main) * 64, row_b);
           }
-          ++issued;
-          r.next();
         }
+        __syncwarp();
+        ++issued;
+        r.next();
       }
-      abort_flag[AB_ISSUED] = issued;
     }
+    if (lane == 0) abort_flag[AB_ISSUED] = issued;
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       const uint32_t idesc_f4 = idesc_nvf4(256, BN);
       const uint32_t idesc_bf = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, 256, BN);
       const uint64_t op_d0 = smem_desc_sw128(smem_base);
@@ -231,37 +232,41 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
       uint32_t aph = 0;
       bool ok = true;
       for (int t = first; t < total_tiles && ok; t += step) {
-        if (!mbar_wait(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
+        if (!mbar_wait_warp(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
         tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
         for (int st = 0; st < n_main + n_tail; ++st) {
           // one wait covers the operand bytes of both CTAs and the scale factors in both CTAs' tensor memory
-          if (!mbar_wait(full_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+          if (!mbar_wait_warp(full_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
-          // descriptors from loop-invariant words, a whole stage's UMMAs in one block: what this thread does between UMMAs
+          // descriptors from loop-invariant words, a whole stage's UMMAs in one block: what this warp does between UMMAs
           // is time the tensor pipe idles (an FP4 UMMA of a 128-wide tile keeps it busy for 64 cycles)
           const uint32_t a_lo = op_lo0 + (uint32_t)r.s * (Cfg::STAGE_BYTES >> 4), b_lo = a_lo + (Cfg::A_BYTES >> 4);
-          if (st < n_main) {
-            const uint32_t sfa_t = tmem_base + Cfg::SF_COL + r.s * Cfg::SF_SLOT, sfb_t = sfa_t + 16;
-            const int nkb = min(4, a.n_chunks - st * 4);
-            if (nkb == 4) {
-              umma_nvf4_x4_pair<BN / 32>(d, a_lo, b_lo, op_hi, idesc_f4, st > 0 ? 1u : 0u, sfa_t, sfb_t);
+          if (elect_one()) {
+            if (st < n_main) {
+              const uint32_t sfa_t = tmem_base + Cfg::SF_COL + r.s * Cfg::SF_SLOT, sfb_t = sfa_t + 16;
+              const int nkb = min(4, a.n_chunks - st * 4);
+              if (nkb == 4) {
+                umma_nvf4_x4_pair<BN / 32>(d, a_lo, b_lo, op_hi, idesc_f4, st > 0 ? 1u : 0u, sfa_t, sfb_t);
+              } else {
+                const uint64_t hi = (uint64_t)op_hi << 32;
+                for (int kb = 0; kb < nkb; ++kb)
+                  umma_nvf4_pair(d, hi | (a_lo + 2 * kb), hi | (b_lo + 2 * kb), idesc_f4, (st > 0 || kb > 0) ? 1u : 0u,
+                                 sfa_t + kb * 4, sfb_t + kb * (BN / 32));
+              }
             } else {
-              const uint64_t hi = (uint64_t)op_hi << 32;
-              for (int kb = 0; kb < nkb; ++kb)
-                umma_nvf4_pair(d, hi | (a_lo + 2 * kb), hi | (b_lo + 2 * kb), idesc_f4, (st > 0 || kb > 0) ? 1u : 0u,
-                               sfa_t + kb * 4, sfb_t + kb * (BN / 32));
+              umma_f16_ss_x4_pair(d, a_lo, b_lo, op_hi, idesc_bf, st > 0 ? 1u : 0u);
             }
-          } else {
-            umma_f16_ss_x4_pair(d, a_lo, b_lo, op_hi, idesc_bf, st > 0 ? 1u : 0u);
+            // the stage is free in BOTH CTAs once these UMMAs have read it
+            umma_commit_pair_both(empty_bar(r.s));
           }
-          // the stage is free in BOTH CTAs once these UMMAs have read it
-          umma_commit_pair_both(empty_bar(r.s));
+          __syncwarp();
           ++stages;
           r.next();
         }
         if (!ok) break;
-        umma_commit_pair_both(accf_bar(buf));
+        if (elect_one()) umma_commit_pair_both(accf_bar(buf));
+        __syncwarp();
         ++accs;
         if (NACC == 2) {
           buf ^= 1;
@@ -270,8 +275,10 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
           aph ^= 1;
         }
       }
-      abort_flag[AB_UMMA] = stages;
-      abort_flag[AB_ACC] = accs;
+      if (lane == 0) {
+        abort_flag[AB_UMMA] = stages;
+        abort_flag[AB_ACC] = accs;
+      }
     }
   }
   } else if (warp < Cfg::EPI_WARP0) {

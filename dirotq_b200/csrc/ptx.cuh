@@ -53,7 +53,34 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity, uint32_t
       : "memory");
   return ok != 0;
 }
-// Two phase tests issued back to back (see mbar_test4).
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// A poll of a sleeping wait: suspended in hardware, or, under a short limit (see AB_POLL), a plain test, since a suspended
+// poll may outlast its hint by many microseconds.
+__device__ __forceinline__ bool mbar_poll(uint32_t bar, uint32_t parity, int suspend_ns) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, l;\n\t"
+      "setp.ge.s32 l, %3, 20000;\n\t"
+      "@l mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "@!l mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(suspend_ns)
+      : "memory");
+  return ok != 0;
+}
+// Two phase tests issued back to back, so that their latencies overlap (a test costs about a hundred cycles even when the
+// phase has long completed).  Bit i of the result: barrier i's phase is complete.
 __device__ __forceinline__ uint32_t mbar_test2(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1) {
   uint32_t m;
   asm volatile(
@@ -68,30 +95,6 @@ __device__ __forceinline__ uint32_t mbar_test2(uint32_t b0, uint32_t p0, uint32_
       : "memory");
   return m;
 }
-// Four phase tests issued back to back, so that their latencies overlap (a test costs about a hundred
-// cycles even when the phase has long completed).  Bit i of the result: barrier i's phase is complete.
-__device__ __forceinline__ uint32_t mbar_test4(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2,
-                                               uint32_t b3, uint32_t p3) {
-  uint32_t m;
-  asm volatile(
-      "{\n\t.reg .pred q0, q1, q2, q3;\n\t.reg .u32 t0, t1, t2, t3;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 q0, [%1], %2;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 q1, [%3], %4;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 q2, [%5], %6;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 q3, [%7], %8;\n\t"
-      "selp.u32 t0, 1, 0, q0;\n\t"
-      "selp.u32 t1, 2, 0, q1;\n\t"
-      "selp.u32 t2, 4, 0, q2;\n\t"
-      "selp.u32 t3, 8, 0, q3;\n\t"
-      "or.b32 t0, t0, t1;\n\t"
-      "or.b32 t2, t2, t3;\n\t"
-      "or.b32 %0, t0, t2;\n\t}"
-      : "=r"(m)
-      : "r"(b0), "r"(p0), "r"(b1), "r"(p1), "r"(b2), "r"(p2), "r"(b3), "r"(p3)
-      : "memory");
-  return m;
-}
-
 // Shared words of a CTA's failure handling, behind its barriers.  Once any role gave up, all later waits of the CTA -- of
 // both CTAs of a pair, whose flags are raised together -- return at once; every role stops, and the CTA tears down what the
 // roles left in flight (see drain_ring).
@@ -146,10 +149,10 @@ __device__ __forceinline__ uint32_t tid_anew() {
 // are checked.  For one thread of a warp; a warp whose lanes all wait uses the forms below.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code) {
-  if (mbar_try(bar, parity)) return true;
+  if (mbar_test(bar, parity)) return true;
   const long long t0 = clock64();
   while (true) {
-    if (mbar_try(bar, parity, abort_flag[AB_POLL])) return true;
+    if (mbar_poll(bar, parity, abort_flag[AB_POLL])) return true;
     __nanosleep(128);            // keep pollers off the issue ports of the working warps
     if (abort_flag[AB_FLAG]) return false;
     if (abort_late(abort_flag, t0)) {
@@ -159,24 +162,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 
+// A short limit leaves no room for polls that do not look at the clock
+__device__ __forceinline__ bool hot_polls(volatile int* abort_flag) { return abort_flag[AB_POLL] >= 20000; }
 // Bounded wait for roles on the critical path (a stage hand-off every few hundred cycles): polls
 // back to back for a while -- a suspended waiter wakes up too late for such short intervals -- and
 // only then falls into the sleeping loop of mbar_wait.
 __device__ __forceinline__ bool mbar_wait_hot(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                               int* status, int code) {
+  if (mbar_test(bar, parity)) return true;
+  if (hot_polls(abort_flag)) {
 #pragma unroll 1
-  for (int i = 0; i < 4096; ++i)
-    if (mbar_try(bar, parity)) return true;
+    for (int i = 0; i < 4096; ++i)
+      if (mbar_try(bar, parity)) return true;
+  }
   return mbar_wait(bar, parity, abort_flag, status, code);
 }
 
 // The same for whole warps: one verdict for all lanes, by vote.  Lanes that poll for themselves could see a phase complete
 // and the flag raised, part each, and the warp would come apart in front of its next aligned instruction.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
-  if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
   const long long t0 = clock64();
   while (true) {
-    if (__all_sync(0xffffffffu, mbar_try(bar, parity, abort_flag[AB_POLL]))) return true;
+    if (__all_sync(0xffffffffu, mbar_poll(bar, parity, abort_flag[AB_POLL]))) return true;
     __nanosleep(128);
     const bool raised = abort_flag[AB_FLAG] != 0, late = abort_late(abort_flag, t0);
     if (__any_sync(0xffffffffu, raised || late)) {
@@ -186,10 +194,40 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
   }
 }
 __device__ __forceinline__ bool mbar_wait_hot_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+  if (hot_polls(abort_flag)) {
 #pragma unroll 1
-  for (int i = 0; i < 4096; ++i)
-    if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+    for (int i = 0; i < 4096; ++i)
+      if (__all_sync(0xffffffffu, mbar_try(bar, parity))) return true;
+  }
   return mbar_wait_warp(bar, parity, abort_flag, status, code);
+}
+
+// Two phases, tested back to back (the latencies of the tests overlap)
+__device__ __forceinline__ bool mbar_wait2_hot_warp(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, volatile int* abort_flag, int* status,
+                                                    int code) {
+  if (__all_sync(0xffffffffu, mbar_test2(b0, p0, b1, p1) == 3u)) return true;
+  if (hot_polls(abort_flag)) {
+#pragma unroll 1
+    for (int i = 0; i < 4096; ++i)
+      if (__all_sync(0xffffffffu, mbar_test2(b0, p0, b1, p1) == 3u)) return true;
+  }
+#pragma unroll 1
+  for (int i = 0; i < 2; ++i)
+    if (!mbar_wait_warp(i ? b1 : b0, i ? p1 : p0, abort_flag, status, code)) return false;
+  return true;
+}
+
+// One lane of a warp whose lanes are all here, the same one every time.  Issuer and producer warps run their loops with all
+// lanes (waits by vote) and let the elected lane issue: under elect.sync the compiler knows that one thread is active and keeps
+// descriptors and addresses in uniform registers.  The same loop run by `lane == 0` alone took 395 cycles per stage of four
+// UMMAs of 128 columns (nominal 256), this one 278 on CTA pairs and 304 on single CTAs; with 256 columns both are hidden behind
+// the UMMAs.  Rotation of 4096 x 1152 14.1 -> 11.9 us, of 1024 x 2240 14.1 -> 11.6; INT GEMM 4096 x 1152 x 1152 20.7 -> 19.4;
+// launches of many 256-wide tiles 0-3 %.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p) :: "memory");
+  return p != 0;
 }
 
 // Teardown after a wait ran out, once every role has stopped: wait (bounded) for one phase, and for those of the last `issued`

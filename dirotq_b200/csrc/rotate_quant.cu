@@ -647,18 +647,18 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   const uint32_t smem_base = smem_u32(smem);
 
   if (warp == 0) {
-    if (lane == 0) {
-      int s = 0;
-      uint32_t ph = 0;
-      int issued = 0;
-      bool ok = true;
-      for (int t = first; t < total_tiles && ok; t += step) {
-        const int mt = t / a.n_tiles, nb = t - mt * a.n_tiles;
-        const int mb = PAIR ? 2 * mt + (int)rank : mt;
-        int kb, ke;
-        tile_k_range(a, nb, kb, ke);
-        for (int kc = kb; kc < ke; ++kc) {
-          if (!mbar_wait(empty_bar(s), ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+    int s = 0;
+    uint32_t ph = 0;
+    int issued = 0;
+    bool ok = true;
+    for (int t = first; t < total_tiles && ok; t += step) {
+      const int mt = t / a.n_tiles, nb = t - mt * a.n_tiles;
+      const int mb = PAIR ? 2 * mt + (int)rank : mt;
+      int kb, ke;
+      tile_k_range(a, nb, kb, ke);
+      for (int kc = kb; kc < ke; ++kc) {
+        if (!mbar_wait_warp(empty_bar(s), ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+        if (elect_one()) {
           const uint32_t sa = smem_base + s * RQ_STAGE_BYTES;
           if constexpr (PAIR) {
             const uint32_t fb = map_to_rank(full_bar(s), 0);
@@ -670,14 +670,15 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
             tma_load_2d(sa, &tm_x, full_bar(s), kc * 64, mb * 128);
             tma_load_2d(sa + RQ_A_BYTES, &tm_u, full_bar(s), kc * 64, nb * a.BN);
           }
-          ++issued;
-          if (++s == RQ_STAGES) { s = 0; ph ^= 1; }
         }
+        __syncwarp();
+        ++issued;
+        if (++s == RQ_STAGES) { s = 0; ph ^= 1; }
       }
-      abort_flag[AB_ISSUED] = issued;
     }
+    if (lane == 0) abort_flag[AB_ISSUED] = issued;
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       const uint32_t idesc = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, PAIR ? 256 : 128, (uint32_t)a.BN);
       int s = 0, buf = 0, stages = 0, accs = 0;
       uint32_t ph = 0, aph = 0;
@@ -688,37 +689,42 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
         const int nb = t % a.n_tiles;
         int kb, ke;
         tile_k_range(a, nb, kb, ke);
-        if (!mbar_wait(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
+        if (!mbar_wait_warp(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * 256;
         for (int kc = kb; kc < ke; ++kc) {
-          if (!mbar_wait(full_bar(s), ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+          if (!mbar_wait_warp(full_bar(s), ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
-          // descriptors from loop-invariant words; the stage's four UMMAs in one block (what this thread does between
+          // descriptors from loop-invariant words; the stage's four UMMAs in one block (what this warp does between
           // UMMAs is time the tensor pipe idles)
           const uint32_t a_lo = op_lo0 + (uint32_t)s * (RQ_STAGE_BYTES >> 4);
-          if constexpr (PAIR) {
-            umma_f16_ss_x4_pair(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u);
-            umma_commit_pair_both(empty_bar(s));
-          } else {
-            umma_f16_ss_x4(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u);
-            umma_commit(empty_bar(s));
+          if (elect_one()) {
+            if constexpr (PAIR) {
+              umma_f16_ss_x4_pair(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u);
+              umma_commit_pair_both(empty_bar(s));
+            } else {
+              umma_f16_ss_x4(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u);
+              umma_commit(empty_bar(s));
+            }
           }
+          __syncwarp();
           ++stages;
           if (++s == RQ_STAGES) { s = 0; ph ^= 1; }
         }
         if (!ok) break;
-        if constexpr (PAIR) {
-          umma_commit_pair_both(accf_bar(buf));
-        } else {
-          umma_commit(accf_bar(buf));
+        if (elect_one()) {
+          if constexpr (PAIR) umma_commit_pair_both(accf_bar(buf));
+          else umma_commit(accf_bar(buf));
         }
+        __syncwarp();
         ++accs;
         buf ^= 1;
         if (buf == 0) aph ^= 1;
       }
-      abort_flag[AB_UMMA] = stages;
-      abort_flag[AB_ACC] = accs;
+      if (lane == 0) {
+        abort_flag[AB_UMMA] = stages;
+        abort_flag[AB_ACC] = accs;
+      }
     }
   } else {
     const int q = warp & 3, half = (warp - 2) >> 2;
