@@ -842,7 +842,7 @@ def gemm_algorithmic_bytes(M, N, lay, quant):
     """Bytes one W4A4 GEMM call must move: activation codes, scale data and tail, the weight's, bias, output."""
     if quant == "nvfp4":
         per_row = lay.code_row_bytes + lay.n_chunks * 4 + lay.tail_pitch * 2
-    else:   # codes + 8-byte records per chunk + bf16 scales read by the fold kernel + tail read, written and read again
+    else:   # long launches: codes + 8-byte records per chunk + bf16 scales read by the fold kernel + tail read, written, read again
         per_row = lay.code_row_bytes + lay.n_chunks * (8 + 2 + 8) + lay.tail_pitch * 2 * 3
     w_row = lay.code_row_bytes + lay.n_chunks * 8 + lay.tail_pitch * 2 + 2
     return float(M * per_row + N * w_row + 2 * M * N)

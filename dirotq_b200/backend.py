@@ -275,9 +275,10 @@ class LayerState:
 
 def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
     """Library kernels one forward of a wrapped linear launches.  A W4A16 layer (no LayerState): weight
-    dequantisation + GEMM.  W4A4: rotate/quantise + GEMM; the tensor-rate integer GEMM adds one preparation launch
-    (scale folding and, unless the layer keeps a resident panel, the weight-panel pre-pass); a sibling that reuses the
-    activations of the layer before it runs only its own GEMM (and pre-pass)."""
+    dequantisation + GEMM.  W4A4: rotate/quantise + GEMM; the tensor-rate integer GEMM adds one preparation launch where
+    the layer keeps no resident panel (the weight-panel pre-pass) or the call is long (scale folding; asked for the rows
+    of the last call, counted before any call); a sibling that reuses the activations of the layer before it runs only its
+    own GEMM (and preparation)."""
     if st is None:
         return 1 if (w4a16 is not None and w4a16.dense is not None) else 2    # resident dequantised weight: GEMM only
     if st.shared is not None and st.shared.fused is not None:
@@ -286,9 +287,9 @@ def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
     if st.chain_fed:
         n -= 1                              # its activations arrive quantised from the producer's epilogue
     if st.folded is not None:
-        # scale folding (first user of the activations only) and the weight-panel pre-pass (unless resident): one launch
-        # when both are due, else one each
-        fold = not (st.shared is not None and st.member_id > 0)
+        # scale folding and the weight-panel pre-pass: one launch when both are due
+        held = next(iter((st._ws if st.shared is None else st.shared.ws).values()), None)
+        fold = held is None or bool(_lib.lib().dirotq_linear_folds_scales(C.byref(st.c_struct()), held[0]))
         n += 1 if (fold or st.folded.panel is None) else 0
     follower = (st.shared is not None and st.member_id > 0) or st.chain_fed
     two_step = _rotates_then_quantises(st)

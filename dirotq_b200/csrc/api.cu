@@ -347,13 +347,12 @@ struct QuantOut {
   int n_kb64_pad;     // NVFP4 consumer: 64-column blocks per row of its scale-factor tile array
 };
 
-// skip_fold != 0: the workspace already holds the activation records and the scaled tail of these codes
-// (left there by an earlier call on the same activations).  qo != null: see QuantOut; y may then be null.
+// qo != null: see QuantOut; y may then be null.
 static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t n_chunks, const void* x_codes,
                                   const void* x_scales, const void* x_zeros, const void* w_codes, const void* w_mult,
                                   const void* w_panel, const float* w_colscale, const void* x_tail,
                                   const void* w_tail_scaled, int32_t tail_total, int32_t tail_pitch, const void* bias,
-                                  void* y, void* workspace, size_t workspace_bytes, int skip_fold, int act,
+                                  void* y, void* workspace, size_t workspace_bytes, int act,
                                   int32_t* status, void* stream, const QuantOut* qo = nullptr, const ActGeom* geom = nullptr) {
   if (a_mode != DIROTQ_INT4_SYM && a_mode != DIROTQ_INT4_ASYM && a_mode != DIROTQ_INT8_ASYM) return DIROTQ_E_UNSUPPORTED;
   if (M < 0 || N <= 0 || n_chunks <= 0 || !x_codes || !x_scales || !w_colscale || (!y && !qo) || !workspace)
@@ -379,26 +378,6 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
   __nv_bfloat16* tail_s = tail_total > 0 ? reinterpret_cast<__nv_bfloat16*>(ws + c.tail) : nullptr;
   const __nv_bfloat16* zeros_in = a_mode != DIROTQ_INT4_SYM ? static_cast<const __nv_bfloat16*>(x_zeros) : nullptr;
   const __nv_bfloat16* tail_in = tail_total > 0 ? static_cast<const __nv_bfloat16*>(x_tail) : nullptr;
-  if (!skip_fold && !w_panel) {
-    // both per-call preparations in one launch: activation scales folded into FMA operands, and the fp16 weight
-    // panel rebuilt in scratch (the weights stay 4-bit in memory)
-    int rc = launch_fold_act_and_expand(static_cast<const __nv_bfloat16*>(x_scales), zeros_in, n_chunks, M, ld_rows(M),
-                                        ws + c.rec, reinterpret_cast<float*>(ws + c.rs), tail_in, tail_s, tp,
-                                        static_cast<const uint8_t*>(w_codes), N, w_mult, ws + c.panel, st, hc);
-    if (rc) return rc;
-    w_panel = ws + c.panel;
-  } else {
-    if (!skip_fold) {
-      int rc = launch_fold_act_scales(static_cast<const __nv_bfloat16*>(x_scales), zeros_in, n_chunks, M, ld_rows(M),
-                                      ws + c.rec, reinterpret_cast<float*>(ws + c.rs), tail_in, tail_s, tp, st);
-      if (rc) return rc;
-    }
-    if (!w_panel) {
-      int rc = launch_expand_weight_panel(static_cast<const uint8_t*>(w_codes), n_chunks, N, w_mult, ws + c.panel, st, hc);
-      if (rc) return rc;
-      w_panel = ws + c.panel;
-    }
-  }
   GemmIntF16Args a;
   a.a_mode = a_mode;
   a.M = M;
@@ -406,12 +385,9 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
   a.n_chunks = n_chunks;
   a.xq = static_cast<const uint8_t*>(x_codes);
   a.x_row_bytes = (int64_t)n_chunks * (a_mode == DIROTQ_INT8_ASYM ? 64 : 32);
-  a.a_const = reinterpret_cast<const uint2*>(ws + c.rec);
-  a.rs = reinterpret_cast<const float*>(ws + c.rs);
-  a.ldm = f16_ld_act(M);
   a.w_panel = w_panel;
   a.cs = w_colscale;
-  a.xt = tail_s;
+  a.xt = tail_in;
   a.wt = static_cast<const __nv_bfloat16*>(w_tail_scaled);
   a.kt = tail_total;
   a.kt_pitch = tail_pitch;
@@ -433,6 +409,43 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
     a.q_mode = qo->mode;
     a.q_clip = qo->clip;
   }
+  const bool records = gemm_int_f16_wants_records(a);
+  if (records) {
+    if (!w_panel) {
+      // both per-call preparations in one launch: activation scales folded into FMA operands, and the fp16 weight
+      // panel rebuilt in scratch (the weights stay 4-bit in memory)
+      int rc = launch_fold_act_and_expand(static_cast<const __nv_bfloat16*>(x_scales), zeros_in, n_chunks, M, ld_rows(M),
+                                          ws + c.rec, reinterpret_cast<float*>(ws + c.rs), tail_in, tail_s, tp,
+                                          static_cast<const uint8_t*>(w_codes), N, w_mult, ws + c.panel, st, hc);
+      if (rc) return rc;
+    } else {
+      int rc = launch_fold_act_scales(static_cast<const __nv_bfloat16*>(x_scales), zeros_in, n_chunks, M, ld_rows(M),
+                                      ws + c.rec, reinterpret_cast<float*>(ws + c.rs), tail_in, tail_s, tp, st);
+      if (rc) return rc;
+    }
+    a.a_const = reinterpret_cast<const uint2*>(ws + c.rec);
+    a.rs = reinterpret_cast<const float*>(ws + c.rs);
+    a.ld_rec = f16_ld_act(M);
+    a.xt = tail_s;
+  } else {
+    if (!w_panel) {
+      int rc = launch_expand_weight_panel(static_cast<const uint8_t*>(w_codes), n_chunks, N, w_mult, ws + c.panel, st, hc);
+      if (rc) return rc;
+    }
+    const void* in[2] = {x_scales, x_zeros};
+    const size_t bytes = (size_t)n_chunks * (size_t)ld_rows(M) * 2;
+    for (int i = 0; i < (a_mode == DIROTQ_INT4_SYM ? 1 : 2); ++i)
+      if (reinterpret_cast<uintptr_t>(in[i]) & 15) {
+        // TMA fetches from 16-byte boundaries; this entry point takes scales anywhere (the records' scratch holds both copies)
+        uint8_t* copy = ws + c.rec + i * (((c.rs - c.rec) / 2) & ~size_t(255));
+        if (cudaMemcpyAsync(copy, in[i], bytes, cudaMemcpyDeviceToDevice, st) != cudaSuccess) return DIROTQ_E_CUDA;
+        in[i] = copy;
+      }
+    a.xs = static_cast<const __nv_bfloat16*>(in[0]);
+    a.xz = a_mode != DIROTQ_INT4_SYM ? static_cast<const __nv_bfloat16*>(in[1]) : nullptr;
+    a.ldm = ld_rows(M);
+  }
+  if (!w_panel) a.w_panel = ws + c.panel;
   return launch_gemm_int_f16(a, st);
 }
 
@@ -442,8 +455,8 @@ int dirotq_gemm_w4a4_int_f16(int32_t a_mode, int64_t M, int64_t N, int32_t n_chu
                              const void* w_tail_scaled, int32_t tail_total, int32_t tail_pitch, const void* bias, void* y,
                              void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
   return gemm_w4a4_int_f16_impl(a_mode, M, N, n_chunks, x_codes, x_scales, x_zeros, w_codes, w_mult, w_panel, w_colscale,
-                                x_tail, w_tail_scaled, tail_total, tail_pitch, bias, y, workspace, workspace_bytes, 0, 0,
-                                status, stream);
+                                x_tail, w_tail_scaled, tail_total, tail_pitch, bias, y, workspace, workspace_bytes, 0, status,
+                                stream);
 }
 
 static int gemm_w4a4_nvfp4_impl(int64_t M, int64_t N, int32_t n_chunks, const void* x_codes, const void* x_sf,
@@ -553,9 +566,7 @@ static bool produces_epilogue_codes(const dirotq_linear* lin, const ActGeom& g, 
   return consumer_mode == DIROTQ_INT4_SYM || consumer_mode == DIROTQ_INT4_ASYM;
 }
 
-// stages: 1 = rotate / quantise into the workspace, 2 = GEMM from the workspace, 3 = both; 4 (with 2) = the
-// workspace holds codes, scales and zero points written by someone else (a producer's epilogue): the per-call
-// folding of the scales, normally part of stage 1's bookkeeping, runs before the GEMM.
+// stages: 1 = rotate / quantise into the workspace, 2 = GEMM from the workspace, 3 = both.
 // qo != null: the GEMM's epilogue quantises its output into these buffers as well (16-bit-conversion INT path only).
 static int linear_stages(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace,
                          size_t workspace_bytes, int stages, int32_t* status, void* stream,
@@ -593,10 +604,9 @@ static int linear_stages(const dirotq_linear* lin, const void* x, int64_t M, voi
   if (lin->epilogue_act < 0 || lin->epilogue_act > 1) return DIROTQ_E_ARG;
   if (uses_f16_gemm(lin, g)) {
     if (!lin->w_colscale || (g.tail_total > 0 && !lin->w_tail_f16)) return DIROTQ_E_ARG;
-    // the activation-side folding belongs to the first stage: a GEMM-only call finds its results in place
     return gemm_w4a4_int_f16_impl(g.mode, M, lin->out_features, g.n_chunks, codes, scales, zeros, lin->w_codes,
                                   lin->w_mult, lin->w_panel_f16, lin->w_colscale, tail, lin->w_tail_f16, g.tail_total, g.tail_pitch,
-                                  lin->bias, y, ws + w.fold, w.total - w.fold, (stages & 5) ? 0 : 1, lin->epilogue_act,
+                                  lin->bias, y, ws + w.fold, w.total - w.fold, lin->epilogue_act,
                                   status, stream, qo, &g);
   }
   if (lin->epilogue_act != 0) return DIROTQ_E_UNSUPPORTED;
@@ -639,6 +649,18 @@ int dirotq_linear_uses_half_chunks(const dirotq_linear* lin) {
   return (uses_f16_gemm(lin, g) && half_chunk_geometry(g)) ? 1 : 0;
 }
 
+int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M) {
+  ActGeom g;
+  if (!lin || M <= 0 || make_geom(&lin->fmt, &g) || !uses_f16_gemm(lin, g)) return 0;
+  GemmIntF16Args a;
+  a.M = M;
+  a.N = lin->out_features;
+  a.n_chunks = g.n_chunks;
+  a.kt = g.tail_total;
+  a.half_chunks = half_chunk_geometry(g) ? 1 : 0;
+  return gemm_int_f16_wants_records(a) ? 1 : 0;
+}
+
 int dirotq_linear_chain_supported(const dirotq_linear* lin, const dirotq_linear* next) {
   if (!lin || !next) return 0;
   ActGeom g, gn;
@@ -677,7 +699,7 @@ int dirotq_linear_forward_chain(const dirotq_linear* lin, const void* x, int64_t
 
 int dirotq_linear_gemm_prequantised(const dirotq_linear* lin, int64_t M, void* y, void* workspace,
                                     size_t workspace_bytes, int32_t* status, void* stream) {
-  return linear_stages(lin, nullptr, M, y, workspace, workspace_bytes, 2 | 4, status, stream);
+  return linear_stages(lin, nullptr, M, y, workspace, workspace_bytes, 2, status, stream);
 }
 
 

@@ -93,7 +93,8 @@ template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
   static constexpr int B_EXP = BN_OWN * 128;               // BN_OWN rows x 64 halves
   static constexpr int EXP_STAGE = B_EXP;                  // only the weight operand is staged in shared memory
   static constexpr int RAW_A = 128 * 32 * GF_CPS * (A8 ? 2 : 1);   // 8-bit activation codes: two 128-byte boxes per row
-  static constexpr int OFF_C = RAW_A;                      // [chunk][128] 8-byte records
+  static constexpr int OFF_C = RAW_A;                      // pairs: [chunk][128] 8-byte records; else [chunk][128] bf16 scales
+  static constexpr int OFF_Z = OFF_C + GF_CPS * 128 * 2;   // and as many zero points
   static constexpr int RAW_STAGE = OFF_C + GF_CPS * 128 * 8;
   // Accumulators: two of 128 columns (the next tile's UMMAs overlap the epilogue); a wider tile has one, and its
   // UMMAs wait until the epilogue has read the previous tile out of tensor memory.
@@ -105,13 +106,18 @@ template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
   static constexpr int PIECES = BN / 32;                    // 16-column pieces of an epilogue warp
   static constexpr int TAB_WARP = PIECES * 8 * 8;           // per epilogue warp: {cs pair, bias pair} in bf16 per column pair
   static constexpr int TAB_BYTES = GF_EPI_WARPS * TAB_WARP;
+  // 1 / rs per row, for several tiles: the epilogue warps write a tile's once the accumulator before last has come, when
+  // every converter warp has at least released the raw stage RAW_STAGES before that tile's last one
+  static constexpr int ROW_TILES = 4;
+  static constexpr int ROW_BYTES = ROW_TILES * 128 * 4;
+  static_assert(ROW_TILES >= RAW_STAGES + 2, "a slot of the row table may still be in use");
   static constexpr int EXP_TMEM = (512 - NACC * BN) / 32;
   static constexpr int BAR_BYTES = 384;                     // barriers, tensor-memory address, failure words
-  static constexpr int EXP_SMEM = (232448 - 1024 - BAR_BYTES - STG_BYTES - TAB_BYTES - RAW_STAGES * RAW_STAGE) / EXP_STAGE;
+  static constexpr int EXP_SMEM = (232448 - 1024 - BAR_BYTES - STG_BYTES - TAB_BYTES - ROW_BYTES - RAW_STAGES * RAW_STAGE) / EXP_STAGE;
   static constexpr int EXP_CAP = EXP_TMEM < GF_EXP_MAX ? EXP_TMEM : GF_EXP_MAX;
   static constexpr int EXP_STAGES = EXP_CAP < EXP_SMEM ? EXP_CAP : EXP_SMEM;
-  static constexpr int SMEM_BYTES = EXP_STAGES * EXP_STAGE + RAW_STAGES * RAW_STAGE + STG_BYTES + TAB_BYTES + 1024 + BAR_BYTES;
-  static constexpr int NBARS = 2 * RAW_STAGES + 3 * EXP_STAGES + 4;
+  static constexpr int SMEM_BYTES = EXP_STAGES * EXP_STAGE + RAW_STAGES * RAW_STAGE + STG_BYTES + TAB_BYTES + ROW_BYTES + 1024 + BAR_BYTES;
+  static constexpr int NBARS = 2 * RAW_STAGES + 3 * EXP_STAGES + 4 + ROW_TILES;
   static_assert(NBARS * 8 + 4 + AB_WORDS * 4 <= BAR_BYTES && CONV_WARPS <= AB_WORDS - AB_WARP, "barrier area");
   static constexpr int TMEM_A0 = NACC * BN;                 // first column of the activation operand slots
   static constexpr int TMEM_COLS = 512;                     // accumulators + EXP_STAGES x 32 columns of A
@@ -121,7 +127,7 @@ template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
 };
 
 struct GfMaps {
-  CUtensorMap xq, wp, xt, wt, y;
+  CUtensorMap xq, xs, xz, wp, xt, wt, y;
 };
 
 template <int N> struct GfRing {
@@ -172,6 +178,42 @@ __device__ __forceinline__ uint32_t hmul2_2m4(uint32_t m) {
   uint32_t r;
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(m), "r"(0x2C002C00u));     // * 2^-4
   return r;
+}
+
+__device__ __forceinline__ uint32_t hmul2_m8(uint32_t m) {
+  uint32_t r;
+  asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(m), "r"(0x80088008u));     // * -8 * 2^-24
+  return r;
+}
+__device__ __forceinline__ uint32_t gf_lds16(uint32_t addr) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float gf_lds_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void gf_sts_f32(uint32_t addr, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t half_twice(float v) {
+  const __half2 h = __floats2half2_rn(v, v);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+// The power of two of a row (token or output channel) whose largest chunk scale is smax: rs = 2^(10 + E) for smax = 1.f * 2^E, so
+// that smax / rs lies in [2^-10, 2^-9).  Returns 1 / rs.
+__device__ __forceinline__ float row_inverse_power(float smax, float& rs) {
+  int E = (int)((__float_as_uint(smax) >> 23) & 0xFF) - 127;
+  E = max(-100, min(100, E));
+  rs = __uint_as_float((uint32_t)(127 + 10 + E) << 23);
+  return __uint_as_float((uint32_t)(127 - 10 - E) << 23);
+}
+// A chunk's multiplier and addend as fp16 pairs, { (s * 2^24 / rs) twice, -(z * s / rs) twice }, ready to be used as packed-FMA
+// operands; inv = 1 / rs (E >= -100 keeps inv * 2^24 finite).
+__device__ __forceinline__ uint2 chunk_record(float s, float z, float inv) {
+  return make_uint2(half_twice(s * (inv * 16777216.f)), half_twice(-z * s * inv));
 }
 
 // bf16 pair of { v0 * rs * cs0 + b0, v1 * rs * cs1 + b1 } from bf16 pairs cs and b; rs and cs are powers of two, so only the
@@ -259,7 +301,8 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   uint8_t* raw_area = smem + GF_EXP_STAGES * Cfg::EXP_STAGE;
   uint8_t* stg_area = raw_area + GF_RAW_STAGES * Cfg::RAW_STAGE;       // 1024-byte aligned
   uint8_t* tab_area = stg_area + Cfg::STG_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(tab_area + Cfg::TAB_BYTES);
+  uint8_t* row_area = tab_area + Cfg::TAB_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(row_area + Cfg::ROW_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + Cfg::NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -273,6 +316,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   auto expw_bar = [&](int s) { return bar0 + 8u * (2 * GF_RAW_STAGES + 2 * GF_EXP_STAGES + s); };   // weight tile landed
   auto accf_bar = [&](int b) { return bar0 + 8u * (2 * GF_RAW_STAGES + 3 * GF_EXP_STAGES + b); };
   auto acce_bar = [&](int b) { return bar0 + 8u * (2 * GF_RAW_STAGES + 3 * GF_EXP_STAGES + 2 + b); };
+  auto rows_bar = [&](int b) { return bar0 + 8u * (2 * GF_RAW_STAGES + 3 * GF_EXP_STAGES + 4 + b); };   // a tile's 1 / rs
 
   constexpr int W_MMA = GF_EPI_WARPS, W_TMA = GF_EPI_WARPS + 1, W_TMB = GF_EPI_WARPS + 2, W_CONV = GF_EPI_WARPS + 4;
   if (threadIdx.x == 0) {
@@ -284,6 +328,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
       mbar_init(expw_bar(s), 1);
     }
     for (int b = 0; b < 2; ++b) { mbar_init(accf_bar(b), 1); mbar_init(acce_bar(b), (PAIR ? 2 : 1) * GF_EPI_WARPS); }
+    for (int b = 0; b < Cfg::ROW_TILES; ++b) mbar_init(rows_bar(b), 4);
     abort_init(abort_flag, a.wait_limit_k, PAIR ? map_to_rank(bar0 + 8u * Cfg::NBARS + 4u, rank ^ 1) : 0u);
     fence_mbar_init();
     prefetch_tmap(&tm.xq);
@@ -298,7 +343,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   if constexpr (PAIR) cluster_sync_all();   // both CTAs' barriers exist before anything arrives on them remotely
   tc_fence_after();
   pdl_launch_dependents();
-  pdl_wait();                       // the kernels that produced the codes / records have completed
+  pdl_wait();                       // the kernels that produced the codes, scales or records have completed
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t exp_base = smem_u32(smem);
   const uint32_t raw_base = smem_u32(raw_area);
@@ -347,7 +392,22 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
     };
     auto exp_slot = [](int qq) { return qq % Cfg::EXP_STAGES; };
     auto exp_phase = [](int qq) { return (uint32_t)((qq / Cfg::EXP_STAGES) & 1); };
-    for (int t = first; t < total_tiles && ok; t += step) {
+    int tile_no = 0;
+    for (int t = first; t < total_tiles && ok; t += step, ++tile_no) {
+      float inv = 0.f;
+      if constexpr (!PAIR) {
+        const int rslot = tile_no % Cfg::ROW_TILES;
+        if (!mbar_wait_hot_warp(rows_bar(rslot), (uint32_t)((tile_no / Cfg::ROW_TILES) & 1), abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+        inv = gf_lds_f32(smem_u32(row_area) + (uint32_t)(rslot * 128 + rowA) * 4);
+      }
+      auto record = [&](uint32_t sraw, int j) {             // chunk j of a raw stage, this thread's row
+        if constexpr (PAIR) return gf_lds64(sraw + Cfg::OFF_C + j * 128 * 8 + rowA * 8);
+        const uint32_t at = sraw + (uint32_t)(j * 128 + rowA) * 2;
+        const float s = __uint_as_float(gf_lds16(at + Cfg::OFF_C) << 16);
+        if constexpr (ASYM) return chunk_record(s, __uint_as_float(gf_lds16(at + Cfg::OFF_Z) << 16), inv);
+        const uint32_t m = half_twice(s * (inv * 16777216.f));       // s has 8 bits: exact, so 8 s / rs may be taken from it
+        return make_uint2(m, hmul2_m8(m));
+      };
       for (int c = 0; c < n_raw && ok; c += GF_CPS) {
         if (!mbar_wait_hot_warp(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         const uint32_t sraw = raw_base + r.s * Cfg::RAW_STAGE;
@@ -362,8 +422,8 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
             // half chunks: the first 32 slots of chunks 2 jc and 2 jc + 1, each with its own record, side by side
             const int c0 = 2 * jc, c1 = 2 * jc + 1;
             const bool has1 = c1 < nv;
-            const uint2 ka0 = gf_lds64(sraw + Cfg::OFF_C + c0 * 128 * 8 + rowA * 8);
-            const uint2 ka1 = has1 ? gf_lds64(sraw + Cfg::OFF_C + c1 * 128 * 8 + rowA * 8) : make_uint2(0u, 0u);
+            const uint2 ka0 = record(sraw, c0);
+            const uint2 ka1 = has1 ? record(sraw, c1) : make_uint2(0u, 0u);
             const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
             if constexpr (A8) {
               const uint32_t rb0 = sraw + (c0 >> 1) * (128 * 128) + rowA * 128, rb1 = sraw + (c1 >> 1) * (128 * 128) + rowA * 128;
@@ -402,7 +462,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
               for (int i = 4; i < 8; ++i) expand_word(w8[i], xr1, ka1.x, mhi1, ka1.y, y1 + 4 * i);
             }
           } else {
-          const uint2 ka = gf_lds64(sraw + Cfg::OFF_C + jc * 128 * 8 + rowA * 8);
+          const uint2 ka = record(sraw, jc);
           if constexpr (A8) {
             // 8-bit codes: 64 bytes of this row = four 16-byte pieces of box jc >> 1.  A byte alone in a zero
             // half is the subnormal q * 2^-24, so (q - z) * s is one packed FMA again; the values are emitted
@@ -451,8 +511,8 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         if (lane == 0) mbar_arrive(rawe_bar(r.s));
         r.next();
       }
-      // tail: the activations' bf16 tile (already divided by rs) arrives in the raw ring and its rows are
-      // copied to TMEM like an expanded chunk
+      // tail: the activations' bf16 tile arrives in the raw ring; its rows, divided by rs (exact; for pairs the folding kernel
+      // has done that), go to TMEM like an expanded chunk
       for (int st = 0; st < n_tail && ok; ++st, ++q) {
         if (!mbar_wait_hot_warp(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         if (q % Cfg::GROUPS == grp) {
@@ -463,6 +523,14 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           for (int i = 0; i < 8; ++i) {
             const uint4 v = gf_lds128(rb + (uint32_t)((i ^ (rowA & 7)) << 4));
             y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
+          }
+          if constexpr (!PAIR) {
+            const __nv_bfloat162 inv2 = __float2bfloat162_rn(inv);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const __nv_bfloat162 h = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&y[i]), inv2);
+              y[i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
           }
           if (!mbar_wait_hot_warp(expe_bar(es), exp_phase(q) ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
           tc_fence_after();
@@ -498,7 +566,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         const int m0 = tm_ * TILE_M + (int)rank * 128;
         // the second half of a pair's last tile may lie past the end: codes arrive as zero fill, and the records (bulk
         // copies know no bounds) are those of the last row block; none of its rows is ever stored
-        const int64_t mrec = PAIR ? min((int64_t)m0, a.ldm - 128) : (int64_t)m0;
+        const int64_t mrec = PAIR ? min((int64_t)m0, a.ld_rec - 128) : (int64_t)m0;
         for (int c = 0; c < n_raw; c += GF_CPS) {
           if (!mbar_wait_hot(rawe_bar(r.s), r.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
           const uint32_t sb = raw_base + r.s * Cfg::RAW_STAGE;
@@ -507,15 +575,22 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           // 8-bit codes: the second 128-byte box is issued only when it holds a chunk (a box that lies
           // wholly outside the tensor is never requested; its bytes are not part of the count either)
           const bool second_box = A8 && nv > 2;
-          mbar_expect_tx(bar, (uint32_t)(Cfg::RAW_A - ((A8 && !second_box) ? 128 * 128 : 0) + nv * 128 * 8));
+          // boxes of scales are counted whole, zero fill included
+          mbar_expect_tx(bar, (uint32_t)(Cfg::RAW_A - ((A8 && !second_box) ? 128 * 128 : 0) +
+                                         (PAIR ? nv * 128 * 8 : (ASYM ? 2 : 1) * GF_CPS * 128 * 2)));
+          if constexpr (!PAIR) {
+            tma_load_2d(sb + Cfg::OFF_C, &tm.xs, bar, m0, c);
+            if constexpr (ASYM) tma_load_2d(sb + Cfg::OFF_Z, &tm.xz, bar, m0, c);
+          }
           if constexpr (A8) {
             tma_load_2d(sb, &tm.xq, bar, c * 64, m0);
             if (second_box) tma_load_2d(sb + 128 * 128, &tm.xq, bar, c * 64 + 128, m0);
           } else {
             tma_load_2d(sb, &tm.xq, bar, c * 32, m0);
           }
-          for (int j = 0; j < nv; ++j)
-            bulk_load(sb + Cfg::OFF_C + j * 128 * 8, a.a_const + ((int64_t)(c + j) * a.ldm + mrec), 128 * 8, bar);
+          if constexpr (PAIR)
+            for (int j = 0; j < nv; ++j)
+              bulk_load(sb + Cfg::OFF_C + j * 128 * 8, a.a_const + ((int64_t)(c + j) * a.ld_rec + mrec), 128 * 8, bar);
           ++issued;
           r.next();
         }
@@ -668,14 +743,47 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         w16[e] = *reinterpret_cast<const uint32_t*>(&h);
       }
     };
+    // Single CTAs: a row's power of two comes from its largest chunk scale.  These warps have time while a tile's UMMAs run, so
+    // they read the scales one tile ahead and leave 1 / rs for the converters in the tile's slot of a table (see ROW_TILES).
+    int rows_no = 0;
+    auto row_powers = [&](int t) {
+      int tm_, tn_;
+      tile_mn(t, tm_, tn_);
+      const int64_t r = (int64_t)tm_ * TILE_M + trow;
+      float smax = 0.f;
+      if (r < a.M) {
+        const uint16_t* s = reinterpret_cast<const uint16_t*>(a.xs) + r;
+#pragma unroll 1
+        for (int c = 0; c < n_raw; c += 24) {
+          uint32_t v24[24];
+#pragma unroll
+          for (int i = 0; i < 24; ++i) v24[i] = c + i < n_raw ? (uint32_t)__ldg(s + (int64_t)(c + i) * a.ldm) : 0u;
+#pragma unroll
+          for (int i = 0; i < 24; ++i) smax = fmaxf(smax, fabsf(__uint_as_float(v24[i] << 16)));
+        }
+      }
+      float rs;
+      const float inv = row_inverse_power(smax, rs);
+      if (ch == 0) {
+        const int rslot = rows_no % Cfg::ROW_TILES;
+        gf_sts_f32(smem_u32(row_area) + (uint32_t)(rslot * 128 + trow) * 4, inv);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(rows_bar(rslot));
+      }
+      ++rows_no;
+      return rs;
+    };
     int use = 0;
     bool ok = true;
+    float rs_next = 0.f;
+    if constexpr (!PAIR)
+      if (first < total_tiles) rs_next = row_powers(first);
     for (int t = first; t < total_tiles && ok; t += step) {
       int tm_, tn_;
       tile_mn(t, tm_, tn_);
       const int m0 = tm_ * TILE_M + (int)rank * 128, n0 = tn_ * BN;
       const int64_t row = (int64_t)m0 + trow;
-      const float rs = (row < a.M) ? __ldg(a.rs + row) : 0.f;
+      const float rs = !PAIR ? rs_next : (row < a.M) ? __ldg(a.rs + row) : 0.f;
       __syncwarp();                                  // every lane has read the previous tile's table
       for (int i = lane; i < Cfg::PIECES * 8; i += 32) { // one column pair each
         const int64_t col = (int64_t)n0 + ch * CW + 2 * i;
@@ -687,6 +795,8 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         }
         gf_sts64(tab + i * 8, cp, bp);
       }
+      if constexpr (!PAIR)
+        if (t + step < total_tiles) rs_next = row_powers(t + step);
       const int buf = Cfg::NACC == 2 ? (use & 1) : 0;
       const uint32_t acc_ph = (uint32_t)(Cfg::NACC == 2 ? (use >> 1) & 1 : use & 1);
       if (!mbar_wait_warp(accf_bar(buf), acc_ph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) { ok = false; break; }
@@ -776,7 +886,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   if constexpr (PAIR) cluster_sync_all();   // neither CTA retires while the other may still read its shared memory
   const int end_warp = (int)(tid_anew() >> 5);
   uint8_t* const end_bars = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(anew(smem_raw)) + 1023) & ~uintptr_t(1023)) +
-                            GF_EXP_STAGES * Cfg::EXP_STAGE + GF_RAW_STAGES * Cfg::RAW_STAGE + Cfg::STG_BYTES + Cfg::TAB_BYTES;
+                            GF_EXP_STAGES * Cfg::EXP_STAGE + GF_RAW_STAGES * Cfg::RAW_STAGE + Cfg::STG_BYTES + Cfg::TAB_BYTES + Cfg::ROW_BYTES;
   volatile int* const ab = reinterpret_cast<volatile int*>(end_bars + 8 * Cfg::NBARS) + 1;
   if (ab[AB_FLAG]) {                // a wait ran out (in both CTAs of a pair the flag is up)
     regs_even<Cfg::REGS_LAUNCH>(end_warp < GF_EPI_WARPS);
@@ -799,11 +909,6 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
 template <typename ST> __device__ __forceinline__ float scale_to_float(ST v);
 template <> __device__ __forceinline__ float scale_to_float<float>(float v) { return v; }
 template <> __device__ __forceinline__ float scale_to_float<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-
-__device__ __forceinline__ uint32_t half_twice(float v) {
-  const uint32_t h = __half_as_ushort(__float2half_rn(v));
-  return h | (h << 16);
-}
 
 // Block = ROWS rows x 256 / ROWS chunk phases (thread tid: row tid % ROWS, chunks c = tid / ROWS (mod 256 / ROWS)).
 // What this kernel takes is latency: two dependent passes over a few hundred bytes per thread.  So a thread's scales and zero
@@ -853,17 +958,13 @@ __device__ __forceinline__ void fold_scales_block(int block, const ST* __restric
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < P; ++k) smax = fmaxf(smax, part_max[k][lr]);
-  int E = (int)((__float_as_uint(smax) >> 23) & 0xFF) - 127;          // smax = 1.f * 2^E
-  E = max(-100, min(100, E));
-  const float inv = __uint_as_float((uint32_t)(127 - 10 - E) << 23);  // 2^(-10 - E): smax * inv in [2^-10, 2^-9)
+  float row_pow;
+  const float inv = row_inverse_power(smax, row_pow);
   if (part == 0) {
     inv_s[lr] = inv;
-    if (r < rows) rs[r] = __uint_as_float((uint32_t)(127 + 10 + E) << 23);
+    if (r < rows) rs[r] = row_pow;
   }
-  const float up = inv * 16777216.f;                                    // * 2^24 (E >= -100 keeps this finite)
-  auto record = [&](int c, float sc, float zp) {
-    rec[(int64_t)c * ld_rec + r] = make_uint2(half_twice(sc * up), half_twice(-zp * sc * inv));
-  };
+  auto record = [&](int c, float sc, float zp) { rec[(int64_t)c * ld_rec + r] = chunk_record(sc, zp, inv); };
   if (r < rows) {
 #pragma unroll
     for (int k = 0; k < KEEP; ++k)
@@ -1116,6 +1217,22 @@ static int pick_raster_f16(int BN, int64_t N, int64_t k_total) {
   return (int)(g < 4 ? 4 : g > 16 ? 16 : g);
 }
 
+// Whether a call reads activation records (and row powers of two, and a scaled tail) that the folding kernel has made, or the
+// scales themselves.  The folding kernel is 2-3 us of launch and latency; the converters' share of the same work is four to ten
+// instructions per row and chunk, which long launches, bound by the converters, feel.  Us, folding kernel + GEMM / GEMM alone: 256 x
+// 1152 x 1152 12.0 / 10.7, 4096 x 1152 x 1152 19.4 / 17.9, 1024 x 2240 x 6720 32.3 / 30.9, 4608 x 3072 x 3072 (three rounds) 63.8 /
+// 63.1; on pairs 32768 x 1152 x 3456 205 / 214, 4608 x 3072 x 12288 238 / 253.  A warp of the GEMM that makes the records for
+// the converters was slower than either (262): its polls and stores take from the same pipes.
+static bool picks_pair(const GemmIntF16Args& a, int* bn) {
+  const int64_t n_stage = a.half_chunks ? (a.n_chunks + 1) / 2 : a.n_chunks;
+  *bn = pick_bn_f16(a.M, a.N, n_stage * 64 + ((a.kt + 63) / 64) * 64, a.q_codes != nullptr);
+  return *bn == 256 && pick_pair_f16(a.M, a.N);
+}
+bool gemm_int_f16_wants_records(const GemmIntF16Args& a) {
+  int bn;
+  return picks_pair(a, &bn);
+}
+
 int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
   GemmIntF16Args a = a_in;
   if (a.M <= 0 || a.N <= 0) return DIROTQ_OK;
@@ -1125,8 +1242,9 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
     return DIROTQ_E_ALIGN;
   const uint64_t n_stage = a.half_chunks ? (uint64_t)((a.n_chunks + 1) / 2) : (uint64_t)a.n_chunks;
   const int64_t k_total = (int64_t)n_stage * 64 + ((a.kt + 63) / 64) * 64;
-  const int BN = pick_bn_f16(a.M, a.N, k_total, a.q_codes != nullptr);
-  const bool pair = BN == 256 && pick_pair_f16(a.M, a.N);
+  int BN;
+  const bool pair = picks_pair(a, &BN);
+  if (pair ? !a.a_const || !a.rs : !a.xs) return DIROTQ_E_ARG;
   if (a.q_codes) {
     if (a.N % 64 || a.q_len % 64 || a.q_len <= 0 || a.q_len > a.N || a.q_row_bytes < a.q_len / 2 || (a.q_row_bytes & 15) ||
         (a.q_len < a.N && (!a.q_tail || a.q_tail_pitch < a.N - a.q_len || (a.q_tail_pitch & 7) ||
@@ -1141,6 +1259,16 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
   int rc = make_tmap_2d_sw(&tm.xq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, a.xq, (uint64_t)a.x_row_bytes, (uint64_t)a.M,
                            (uint64_t)a.x_row_bytes, 32 * GF_CPS, 128, 32 * GF_CPS);
   if (rc) return rc;
+  tm.xs = tm.xz = tm.xq;
+  if (!pair) {
+    // scales (and zero points): [n_chunks, ldm] bf16, a stage's four chunks of 128 rows in one box
+    rc = make_tmap_2d_sw(&tm.xs, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.xs, (uint64_t)a.ldm, (uint64_t)a.n_chunks, (uint64_t)a.ldm * 2,
+                         128, GF_CPS, 0);
+    if (!rc && a.a_mode != DIROTQ_INT4_SYM)
+      rc = make_tmap_2d_sw(&tm.xz, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.xz, (uint64_t)a.ldm, (uint64_t)a.n_chunks,
+                           (uint64_t)a.ldm * 2, 128, GF_CPS, 0);
+    if (rc) return rc;
+  }
   if (a.raster == 0) a.raster = pick_raster_f16(BN, a.N, k_total);
   rc = make_tmap_2d(&tm.wp, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, a.w_panel, n_stage * 64, (uint64_t)a.N, n_stage * 128, pair ? BN / 2 : BN);
   if (rc) return rc;

@@ -226,7 +226,7 @@ class LinearPathStep(nn.Module):
 
     def kernel_launches_per_step(self) -> int:
         """Library kernels per step: rotate/quantise (or weight dequantise) + GEMM per linear, plus the
-        scale-folding kernel of the tensor-rate INT4 GEMM where a layer uses it."""
+        preparation kernel of the tensor-rate INT4 GEMM where a layer uses it."""
         from . import backend
         return sum(backend.kernel_launches(getattr(lyr, "_b200_state", None), getattr(lyr, "_b200_w4a16", None)) for lyr in self.layers)
 

@@ -210,8 +210,8 @@ int dirotq_gemm_w4a4_int(int32_t a_mode, int64_t M, int64_t N, int32_t n_chunks,
  * dirotq_gemm_w4a4_int_f16: a_mode DIROTQ_INT4_SYM, DIROTQ_INT4_ASYM or DIROTQ_INT8_ASYM; w_panel NULL: the panel
  *   is rebuilt from w_codes / w_mult in the workspace on every call (w_codes / w_mult may be NULL when w_panel
  *   is given); workspace of dirotq_gemm_w4a4_int_f16_workspace_bytes(M, N_panel, n_chunks, tail_pitch) bytes,
- *   256-byte aligned (per-call activation multipliers, the scaled copy of the tail and, for N_panel = N > 0,
- *   the panel; N_panel = 0 for callers that pass their own).
+ *   256-byte aligned (activation multipliers and the scaled copy of the tail, which long launches have made by a kernel of
+ *   their own, and, for N_panel = N > 0, the panel; N_panel = 0 for callers that pass their own).
  */
 size_t dirotq_fold_weight_records_bytes(int32_t n_chunks, int64_t N);
 int dirotq_fold_weight_scales_f16(int32_t n_chunks, int64_t N, const float* w_scales, const void* w_tail,
@@ -336,13 +336,14 @@ int dirotq_linear_gemm(const dirotq_linear* lin, int64_t M, void* y, void* works
  * quantised part and its 16-bit tail both multiples of 64 channels (the tail may be empty), no
  * rotation, no channel selection, width == lin->out_features, w_mult set.  Anything else: DIROTQ_E_UNSUPPORTED, nothing launched. */
 int dirotq_linear_uses_half_chunks(const dirotq_linear* lin);
+/* Whether a GEMM of `lin` on M rows launches the scale-folding kernel first (long launches of integer layers). */
+int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M);
 int dirotq_linear_chain_supported(const dirotq_linear* lin, const dirotq_linear* next);
 int dirotq_linear_forward_chain(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace,
                                 size_t workspace_bytes, const dirotq_linear* next, void* next_workspace,
                                 size_t next_workspace_bytes, int32_t* status, void* stream);
 /* The GEMM of `lin` on codes / scales / zero points that a producer's epilogue wrote into `workspace`
- * (dirotq_linear_forward_chain): like dirotq_linear_gemm, plus the per-call folding of the scales
- * that dirotq_linear_forward does in its first half. */
+ * (dirotq_linear_forward_chain); the same as dirotq_linear_gemm. */
 int dirotq_linear_gemm_prequantised(const dirotq_linear* lin, int64_t M, void* y, void* workspace,
                                     size_t workspace_bytes, int32_t* status, void* stream);
 

@@ -1,0 +1,68 @@
+"""The two ways a row's scales reach the 16-bit-conversion GEMM -- records of the folding kernel (CTA pairs), or the scales
+themselves (single CTAs) -- give the same bits, from any scales and from any address; and the rotation kernel's packed
+quantiser agrees with the oracle where a group lies far from zero or is clipped."""
+import dataclasses
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# rows and widths around the tiles (128 rows, a stage of four 64-slot chunks, a tail of 64), one to five chunks, ragged ends
+@pytest.mark.parametrize("M,D,tail", [(1, 128, 8), (129, 320, 0), (257, 384, 72), (300, 1152, 64), (520, 4608, 320)])
+@pytest.mark.parametrize("mode", ["sym", "asym", "int8"])
+def test_both_scale_routes_give_the_same_bits(mode, M, D, tail, monkeypatch):
+    from dirotq_b200 import ops
+    from test_gpu_gemm import _setup_int
+    m = {"sym": ops.INT4_SYM, "asym": ops.INT4_ASYM, "int8": ops.INT8_ASYM}[mode]
+    x, act, dec, qw, sw, pk, w_tail, bias = _setup_int(ops, M, 264, ops.ActFormat(m, D, tail_len=tail), 71)
+    lay = act.layout
+    # rows 2^-24 .. 2^24 apart, and groups of one row 2^-12 apart: scales whose records are subnormal or zero
+    s = act.scales[: lay.n_scales * act.ldm * 2].view(torch.bfloat16).view(lay.n_scales, act.ldm)
+    rows = torch.arange(act.ldm, device="cuda")
+    s *= torch.exp2(((rows * 7) % 49 - 24).float()).to(torch.bfloat16)
+    s[::2] *= torch.exp2(-((rows * 5) % 13).float()).to(torch.bfloat16)
+    s[:, M // 2] = 0
+    wt = ops.pad_tail_weight(w_tail, lay.tail_pitch, 264, "cuda")
+    folded = ops.fold_weight_scales_f16(pk, wt, lay.tail_total)
+    run = lambda a: ops.gemm_w4a4_int_f16(a, pk, folded, bias.cuda())
+    out = {}
+    for bn, pair in (("256", "1"), ("128", "0"), ("192", "0"), ("256", "0")):
+        monkeypatch.setenv("DIROTQ_GF_BN", bn)
+        monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
+        out[bn, pair] = run(act)
+    ops.check_status()
+    assert torch.isfinite(out["256", "1"].float()).all()
+    for k, y in out.items():
+        assert torch.equal(y, out["256", "1"]), k
+
+    def shifted(t):                                   # the same values at an address that is no multiple of 16
+        if t is None:
+            return None
+        buf = torch.empty(t.numel() + 16, dtype=torch.uint8, device="cuda")[2:2 + t.numel()]
+        return buf.copy_(t)
+    moved = dataclasses.replace(act, scales=shifted(act.scales), zeros=shifted(act.zeros))
+    assert moved.scales.data_ptr() % 16
+    for bn, pair in (("128", "0"), ("256", "1")):
+        monkeypatch.setenv("DIROTQ_GF_BN", bn)
+        monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
+        assert torch.equal(run(moved), out["256", "1"])
+    ops.check_status()
+
+
+@pytest.mark.parametrize("M,D,tail", [(5, 128, 0), (131, 320, 40), (300, 1152, 64)])
+@pytest.mark.parametrize("mode,clip", [("sym", 1.0), ("sym", 0.3), ("asym", 1.0), ("asym", 0.3)])
+def test_rotation_epilogue_quantises_groups_far_from_zero_as_the_oracle(mode, clip, M, D, tail):
+    from gpu_helpers import assert_act_matches_oracle
+    from dirotq_b200 import ops
+    g = torch.Generator().manual_seed(72)
+    x = torch.randn(M, D, generator=g)
+    x[::3] += torch.tensor([3.0, -40.0, 700.0])[torch.arange(D) // 64 % 3]      # offsets from within to far outside the spread
+    x[1, :64] = 0
+    x[2, 64:128] = -1e-7
+    x = x.to(torch.bfloat16)
+    fmt = ops.ActFormat(ops.INT4_SYM if mode == "sym" else ops.INT4_ASYM, D, tail_len=tail, clip_ratio=clip)
+    buf = ops.rotate_quantize(x.cuda(), torch.eye(D).to(torch.bfloat16).cuda(), fmt)     # x_rot is x itself
+    ops.check_status()
+    assert_act_matches_oracle(buf, x)
