@@ -295,8 +295,11 @@ def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
     two_step = _rotates_then_quantises(st)
     if two_step and not follower:
         n += 1                              # rotation into scratch, then the quantise kernel
-    if (st.rot_t is None or two_step) and st.layout.tail_total > 0 and not follower:
-        n += 1                              # the quantise kernel copies the passthrough channels in a launch of its own
+    f, lay = st.fmt, st.layout
+    rides = (f.num_heads == 0 and st.perm_idx is None and not (lay.q_len | lay.tail_total) % 8 and
+             (f.group_size == 64 or f.mode in (ops.NVFP4_HW, ops.NVFP4_REF)))
+    if (st.rot_t is None or two_step) and lay.tail_total > 0 and not follower and not rides:
+        n += 1                              # the passthrough channels, where the quantise kernel does not copy them too
     if st.hadamard_low_dim:
         n += 1
     return n

@@ -73,6 +73,7 @@ struct QuantArgs {
   uint8_t* sf;             // NVFP4_HW tiled bytes
   __nv_bfloat16* zeros;
   __nv_bfloat16* tail;
+  unsigned quant_blocks;   // blocks from here on copy the passthrough channels
 };
 
 struct PackIntArgs {

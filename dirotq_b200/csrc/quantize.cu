@@ -5,6 +5,7 @@
 #include <cuda_bf16.h>
 #include "layout.cuh"
 #include "launchers.cuh"
+#include "ptx.cuh"
 #include "quant_math.cuh"
 
 namespace dq {
@@ -70,11 +71,33 @@ static __device__ __noinline__ void quant_int_block_slow(const __nv_bfloat16* x,
   }
 }
 
+// Passthrough channels of the hidden layout, eight per thread (16-byte loads and stores): the last blocks of a quantise launch.
+// (A launch of their own behind the quantiser's, and both without programmatic dependent launch, cost short layers more than
+// the copy: see launch_quantize.)
+__device__ __forceinline__ void copy_tail_vec_block(const QuantArgs& a, unsigned block) {
+  const ActGeom& g = a.g;
+  const int per_row = g.tail_pitch >> 3;
+  const int64_t total = a.M * per_row;
+  const int64_t tid = (int64_t)block * blockDim.x + threadIdx.x;
+  if (tid >= total) return;
+  const int64_t row = tid / per_row;
+  const int t = (int)(tid - row * per_row) * 8;
+  uint4 val = make_uint4(0u, 0u, 0u, 0u);
+  if (t < g.tail_total) val = __ldg(reinterpret_cast<const uint4*>(a.x + row * a.x_pitch + g.q_len + t));
+  *reinterpret_cast<uint4*>(a.tail + row * g.tail_pitch + t) = val;
+}
+
 // One thread = one block of 32 code slots of one row.  The 2*cpg threads that share a group sit
 // on consecutive lanes (aligned), so the group extrema need log2(2*cpg) shuffles.
 template <int MODE>
 __global__ void __launch_bounds__(256) quant_int_kernel(const QuantArgs a) {
   const ActGeom& g = a.g;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (blockIdx.x >= a.quant_blocks) {
+    copy_tail_vec_block(a, blockIdx.x - a.quant_blocks);
+    return;
+  }
   const int bpr = g.n_chunks * 2;                      // 32-slot blocks per row
   const int64_t total = a.M * bpr;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -210,6 +233,8 @@ __global__ void __launch_bounds__(256) quant_int_kernel(const QuantArgs a) {
 template <int MODE>
 __global__ void __launch_bounds__(256) quant_int_token_kernel(const QuantArgs a) {
   const ActGeom& g = a.g;
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t row = blockIdx.x;
   const __nv_bfloat16* xr = a.x + row * a.x_pitch;
   float mx = 0.f, mn = 0.f;
@@ -247,6 +272,12 @@ __global__ void __launch_bounds__(256) quant_int_token_kernel(const QuantArgs a)
 template <int MODE>
 __global__ void __launch_bounds__(256) quant_nvfp4_kernel(const QuantArgs a) {
   const ActGeom& g = a.g;
+  pdl_launch_dependents();
+  pdl_wait();
+  if (blockIdx.x >= a.quant_blocks) {
+    copy_tail_vec_block(a, blockIdx.x - a.quant_blocks);
+    return;
+  }
   const int64_t total = a.M * g.n_chunks;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= total) return;
@@ -367,6 +398,8 @@ __global__ void __launch_bounds__(256) quant_nvfp4_kernel(const QuantArgs a) {
 // Passthrough channels -> tail buffer [M, tail_pitch] (pad columns zero).
 __global__ void __launch_bounds__(256) copy_tail_kernel(const QuantArgs a) {
   const ActGeom& g = a.g;
+  pdl_launch_dependents();
+  pdl_wait();
   const int64_t total = a.M * g.tail_pitch;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= total) return;
@@ -384,55 +417,50 @@ __global__ void __launch_bounds__(256) copy_tail_kernel(const QuantArgs a) {
 }
 
 
-// Passthrough channels of the hidden layout, eight per thread (16-byte loads and stores).
 __global__ void __launch_bounds__(256) copy_tail_vec_kernel(const QuantArgs a) {
-  const ActGeom& g = a.g;
-  const int per_row = g.tail_pitch >> 3;
-  const int64_t total = a.M * per_row;
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= total) return;
-  const int64_t row = tid / per_row;
-  const int t = (int)(tid - row * per_row) * 8;
-  uint4 val = make_uint4(0u, 0u, 0u, 0u);
-  if (t < g.tail_total) val = __ldg(reinterpret_cast<const uint4*>(a.x + row * a.x_pitch + g.q_len + t));
-  *reinterpret_cast<uint4*>(a.tail + row * g.tail_pitch + t) = val;
+  pdl_launch_dependents();
+  pdl_wait();
+  copy_tail_vec_block(a, blockIdx.x);
 }
 
-int launch_quantize(const QuantArgs& a, cudaStream_t st) {
+// The passthrough channels ride in the quantiser's launch where they are 16-byte pieces of the hidden layout and the quantiser
+// is one of the block kernels with the usual groups; else they take a launch behind it.  All of them are launched with
+// programmatic serialization, as the kernels before and after them are: a Hadamard layer 4608 -> 1152 of 4096 rows (transform,
+// quantiser, GEMM) 93.4 -> 88.4 us with both.
+int launch_quantize(const QuantArgs& a_in, cudaStream_t st) {
+  QuantArgs a = a_in;
   const ActGeom& g = a.g;
   if (a.M <= 0) return DIROTQ_OK;
-  const int threads = 256;
+  const unsigned threads = 256;
   if (is_nvfp4(g.mode) && g.H > 0) return DIROTQ_E_UNSUPPORTED;   // per-head NVFP4 exists only fused with its rotation
-  if (is_nvfp4(g.mode)) {
-    int64_t total = a.M * g.n_chunks;
-    unsigned blocks = (unsigned)((total + threads - 1) / threads);
-    if (g.mode == DIROTQ_NVFP4_REF) quant_nvfp4_kernel<MODE_NVFP4_REF><<<blocks, threads, 0, st>>>(a);
-    else quant_nvfp4_kernel<MODE_NVFP4_HW><<<blocks, threads, 0, st>>>(a);
-  } else if (g.per_token) {
+  const bool tail = g.tail_total > 0 && a.tail;
+  const bool vec = tail && g.H == 0 && !a.perm && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (a.x_pitch & 7) == 0 &&
+                   (reinterpret_cast<uintptr_t>(a.tail) & 15) == 0 && g.q_len % 8 == 0 && g.tail_total % 8 == 0 &&
+                   g.tail_pitch % 8 == 0;
+  const bool merged = vec && !g.per_token && (is_nvfp4(g.mode) || g.group == 64);
+  const unsigned tail_blocks = vec ? (unsigned)((a.M * (g.tail_pitch / 8) + threads - 1) / threads)
+                                   : tail ? (unsigned)((a.M * g.tail_pitch + threads - 1) / threads) : 0u;
+  auto go = [&](void (*k)(QuantArgs), unsigned blocks) { return launch_pdl(k, dim3(blocks), dim3(threads), 0, st, a); };
+  cudaError_t rc;
+  if (g.per_token) {
     if (a.M > 0x7fffffff) return DIROTQ_E_TOO_LARGE;
-    if (g.mode == DIROTQ_INT4_SYM) quant_int_token_kernel<MODE_INT4_SYM><<<(unsigned)a.M, threads, 0, st>>>(a);
-    else if (g.mode == DIROTQ_INT4_ASYM) quant_int_token_kernel<MODE_INT4_ASYM><<<(unsigned)a.M, threads, 0, st>>>(a);
-    else quant_int_token_kernel<MODE_INT8_ASYM><<<(unsigned)a.M, threads, 0, st>>>(a);
+    a.quant_blocks = (unsigned)a.M;
+    rc = go(g.mode == DIROTQ_INT4_SYM ? quant_int_token_kernel<MODE_INT4_SYM>
+            : g.mode == DIROTQ_INT4_ASYM ? quant_int_token_kernel<MODE_INT4_ASYM> : quant_int_token_kernel<MODE_INT8_ASYM>, a.quant_blocks);
   } else {
-    int64_t total = a.M * g.n_chunks * 2;
-    unsigned blocks = (unsigned)((total + threads - 1) / threads);
-    if (g.mode == DIROTQ_INT4_SYM) quant_int_kernel<MODE_INT4_SYM><<<blocks, threads, 0, st>>>(a);
-    else if (g.mode == DIROTQ_INT4_ASYM) quant_int_kernel<MODE_INT4_ASYM><<<blocks, threads, 0, st>>>(a);
-    else quant_int_kernel<MODE_INT8_ASYM><<<blocks, threads, 0, st>>>(a);
-  }
-  if (g.tail_total > 0 && a.tail) {
-    const bool vec = g.H == 0 && !a.perm && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (a.x_pitch & 7) == 0 &&
-                     (reinterpret_cast<uintptr_t>(a.tail) & 15) == 0 && g.q_len % 8 == 0 && g.tail_total % 8 == 0 &&
-                     g.tail_pitch % 8 == 0;
-    if (vec) {
-      int64_t total = a.M * (g.tail_pitch / 8);
-      copy_tail_vec_kernel<<<(unsigned)((total + threads - 1) / threads), threads, 0, st>>>(a);
-    } else {
-      int64_t total = a.M * g.tail_pitch;
-      copy_tail_kernel<<<(unsigned)((total + threads - 1) / threads), threads, 0, st>>>(a);
+    const int64_t total = a.M * g.n_chunks * (is_nvfp4(g.mode) ? 1 : 2);
+    a.quant_blocks = (unsigned)((total + threads - 1) / threads);
+    const unsigned blocks = a.quant_blocks + (merged ? tail_blocks : 0u);
+    switch (g.mode) {
+      case DIROTQ_NVFP4_REF: rc = go(quant_nvfp4_kernel<MODE_NVFP4_REF>, blocks); break;
+      case DIROTQ_NVFP4_HW: rc = go(quant_nvfp4_kernel<MODE_NVFP4_HW>, blocks); break;
+      case DIROTQ_INT4_SYM: rc = go(quant_int_kernel<MODE_INT4_SYM>, blocks); break;
+      case DIROTQ_INT4_ASYM: rc = go(quant_int_kernel<MODE_INT4_ASYM>, blocks); break;
+      default: rc = go(quant_int_kernel<MODE_INT8_ASYM>, blocks); break;
     }
   }
-  return cudaGetLastError() == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
+  if (rc == cudaSuccess && tail && !merged) rc = go(vec ? copy_tail_vec_kernel : copy_tail_kernel, tail_blocks);
+  return rc == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
 }
 
 }  // namespace dq

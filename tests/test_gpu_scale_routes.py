@@ -1,6 +1,7 @@
 """The two ways a row's scales reach the 16-bit-conversion GEMM -- records of the folding kernel (CTA pairs), or the scales
 themselves (single CTAs) -- give the same bits, from any scales and from any address; and the rotation kernel's packed
-quantiser agrees with the oracle where a group lies far from zero or is clipped."""
+quantiser agrees with the oracle where a group lies far from zero or is clipped; 16-bit channels copied in the quantiser's
+launch or behind it."""
 import dataclasses
 
 import pytest
@@ -66,3 +67,16 @@ def test_rotation_epilogue_quantises_groups_far_from_zero_as_the_oracle(mode, cl
     buf = ops.rotate_quantize(x.cuda(), torch.eye(D).to(torch.bfloat16).cuda(), fmt)     # x_rot is x itself
     ops.check_status()
     assert_act_matches_oracle(buf, x)
+
+
+# the quantise-only kernels copy the 16-bit channels in their own launch (groups of 64, NVFP4; whole 16-byte pieces) or a launch behind
+@pytest.mark.parametrize("M", [1, 33, 515])
+@pytest.mark.parametrize("mode,group,D,tail", [("INT4_SYM", 64, 136, 8), ("INT4_ASYM", 64, 4608, 512), ("INT4_SYM", 64, 136, 12),
+                                               ("INT4_SYM", 32, 136, 8), ("INT8_ASYM", 64, 192, 64), ("NVFP4_HW", 16, 136, 8),
+                                               ("NVFP4_HW", 16, 1152, 20), ("INT4_SYM", -1, 136, 8)])
+def test_quantise_only_kernels_copy_the_16_bit_channels(mode, group, D, tail, M):
+    from gpu_helpers import assert_act_matches_oracle
+    from dirotq_b200 import ops
+    x = torch.randn(M, D, generator=torch.Generator().manual_seed(73)).to(torch.bfloat16)
+    fmt = ops.ActFormat(getattr(ops, mode), D, tail_len=tail, group_size=group)
+    assert_act_matches_oracle(ops.quantize_act(x.cuda(), fmt), x)
