@@ -277,11 +277,11 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
 
 // Tile choice.  CTA pairs (gemm_nvfp4_pair.cu) halve the weight bytes each SM pulls through L2 per flop; up to 128 rows a
 // pair would idle half of itself, so the single-CTA 128 x 128 kernel of this file keeps those.  A round of 256 x 256 pair
-// tiles (one accumulator) takes 1.4 rounds of 256 x 128 ones (two) at K = 3072, 1.46 at 2240 and 1.63 at 1152, where its
-// hand-over weighs more: 256 wherever the rounds it saves are worth that (256 / 128 columns: 3072 -> 9216 at 16384 rows 286 /
-// 403 us, 2240 x 2240 69 / 95, 1152 -> 3456 at 32768 rows 111 / 128), 128 for the few rounds of short calls (1152 x 1152 at
-// 4096 rows 19.1 / 16.9, 3072 x 3072 at 512 rows 31.0 / 29.6).  From K = 2048 on the line is drawn at 10/7 = 1.43 rounds for all: between it
-// and the 1.46 of K = 2240 lie only pairs like 13 rounds against 9, worth 2 %.  DIROTQ_NVFP4_TILE = single | pair128 | pair256 forces one
+// tiles (one accumulator) takes 1.4 rounds of 256 x 128 ones (two) at every K now that the issuer is not bound by its own
+// instructions (at K = 1152 it was 1.63): 256 wherever the rounds it saves are worth that (256 / 128 columns: 3072 -> 9216 at 16384 rows
+// 286 / 403 us, 2240 x 2240 53 / 75, 1152 -> 3456 at 4096 rows, four rounds against six, 19.1 / 19.9, 1152 x 1152 at 12288, the same, 19.9 /
+// 20.3), 128 for the few rounds of short calls (1152 x 1152 at 4096 rows 11.6 / 10.3, at 8192, three against four, 17.3 / 16.7; 2240 x
+// 2240 at 1024 10.6 / 10.0).  The line is drawn at 10/7 = 1.43 rounds.  DIROTQ_NVFP4_TILE = single | pair128 | pair256 forces one
 // form (measurements, tests).
 static int pick_nvfp4_tile(const GemmFp4Args& a) {
   if (const char* e = getenv("DIROTQ_NVFP4_TILE")) {
@@ -290,9 +290,9 @@ static int pick_nvfp4_tile(const GemmFp4Args& a) {
     if (!strcmp(e, "pair256")) return 256;
   }
   if (a.M <= 128) return 0;
-  const int64_t K = (int64_t)a.n_chunks * 64 + a.kt, pairs = num_sms() / 2, mp = (a.M + 255) / 256;
+  const int64_t pairs = num_sms() / 2, mp = (a.M + 255) / 256;
   const int64_t r256 = (mp * ((a.N + 255) / 256) + pairs - 1) / pairs, r128 = (mp * ((a.N + 127) / 128) + pairs - 1) / pairs;
-  return (K >= 2048 ? 10 * r256 < 7 * r128 : 8 * r256 < 5 * r128) ? 256 : 128;
+  return 10 * r256 < 7 * r128 ? 256 : 128;
 }
 
 int launch_gemm_nvfp4(const GemmFp4Args& a, cudaStream_t st) {
