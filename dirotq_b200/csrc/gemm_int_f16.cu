@@ -30,8 +30,8 @@
 //     from TMEM, B from smem.
 //
 // Data flow per persistent CTA (128 x BN output tiles, K walked in 64-wide chunks):
-//   TMA (A)        4-bit codes (four chunks = 128 B per row per stage, 128-byte swizzle) + per-row records of
-//                  the chunk's multipliers (bulk copies) -> "raw" ring
+//   TMA (A)        4-bit codes (four chunks = 128 B per row per stage, 128-byte swizzle) + the chunks' scales and zero
+//                  points, or (pairs) the records a folding kernel made of them (bulk copies) -> "raw" ring
 //   TMA (B)        one BN x 64 fp16 tile of the panel (or of the bf16 tail weights) per operand stage, straight
 //                  into the stage's 128-byte-swizzled K-major slot as soon as the UMMAs that read it retire
 //   converter warps  two groups of four taking alternate chunks; a warp expands 32 activation rows into TMEM
