@@ -872,8 +872,9 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           minmax_bf16x16(wk + 24, mx, mn);
           p = int_asym_params<true>(mx, mn, a.q_clip, 15.f);
           const float rcp = __frcp_rn(p.scale);
-          dst[0] = int_asym_planar32_packed(wk, rcp, p.zero);
-          dst[1] = int_asym_planar32_packed(wk + 16, rcp, p.zero);
+          const bool packs = int_asym_packs(mx, mn, rcp, p.zero);
+          dst[0] = int_asym_planar32(wk, p.scale, rcp, p.zero, packs);
+          dst[1] = int_asym_planar32(wk + 16, p.scale, rcp, p.zero, packs);
           a.q_zeros[(int64_t)chunk * a.q_ldm + row] = __float2bfloat16_rn(p.zero);
         }
         a.q_scales[(int64_t)chunk * a.q_ldm + row] = __float2bfloat16_rn(p.scale);

@@ -172,9 +172,14 @@ __device__ __forceinline__ uint4 int_sym_planar32_packed(const uint32_t* p, floa
   }
   return make_uint4(out[0], out[1], out[2], out[3]);
 }
-// The asymmetric 4-bit form of the same: code = clamp(rint(bf16(x / s)) + zero, 0, 15).  On packed bf16 pairs: adding
-// 192 rounds the quotient (|q| <= 15.1) half-even to an integer (bf16 spacing is 1 in [128, 256)); adding (zero - 192)
-// gives rint(q) + zero exactly (both are integers below 2^8); clamp; adding 128 leaves the code in the low mantissa bits.
+// The asymmetric 4-bit form of the same: code = clamp(bf16(rint(bf16(x / s)) + zero), 0, 15).  On packed bf16 pairs: adding
+// 192 rounds the quotient half-even to an integer (bf16 spacing is 1 in [128, 256)); adding (zero - 192) gives rint(q) + zero
+// exactly (both are integers below 2^8); clamp; adding 128 leaves the code in the low mantissa bits.  Only for groups that
+// int_asym_packs allows: the range of a group need not include zero (int_asym_params), so a group whose mean lies far from
+// zero has quotients and a zero point of any size, and 192 + q would leave [128, 256).
+__device__ __forceinline__ bool int_asym_packs(float mx, float mn, float rcp_s, float zero) {
+  return fmaxf(fabsf(mx), fabsf(mn)) * rcp_s <= 60.f && fabsf(zero) <= 60.f;     // false for NaN
+}
 __device__ __forceinline__ uint4 int_asym_planar32_packed(const uint32_t* p, float rcp_s, float zero) {
   const __nv_bfloat162 c192 = __floats2bfloat162_rn(192.f, 192.f), c0 = __floats2bfloat162_rn(0.f, 0.f),
                        c15 = __floats2bfloat162_rn(15.f, 15.f), c128 = __floats2bfloat162_rn(128.f, 128.f),
@@ -226,6 +231,25 @@ __device__ __forceinline__ uint2 int_asym_byte8_fast(const float* v, float s, fl
     w[j >> 2] |= (int_bits(q) & 0xFFu) << (8 * (j & 3));
   }
   return make_uint2(w[0], w[1]);
+}
+// Planar-32 codes of any asymmetric group, `packs` = int_asym_packs of the group: one value at a time where the packed
+// rounding does not hold.  The test costs the quantise-only kernel 1 % (16384 x 12288 129.0 -> 130.8 us).
+__device__ __forceinline__ uint4 int_asym_planar32(const uint32_t* p, float s, float rcp_s, float zero, bool packs) {
+  if (packs) return int_asym_planar32_packed(p, rcp_s, zero);
+  uint32_t out[4];
+#pragma unroll
+  for (int wd = 0; wd < 4; ++wd) {
+    uint32_t acc = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int j = 4 * wd + k;
+      const uint32_t a = p[j >> 1], b = p[8 + (j >> 1)];
+      const float fa = __uint_as_float((j & 1) ? (a & 0xFFFF0000u) : (a << 16)), fb = __uint_as_float((j & 1) ? (b & 0xFFFF0000u) : (b << 16));
+      acc |= (int_asym_code_fast(fa, s, rcp_s, zero, 15.f) | (int_asym_code_fast(fb, s, rcp_s, zero, 15.f) << 4)) << (8 * k);
+    }
+    out[wd] = acc;
+  }
+  return make_uint4(out[0], out[1], out[2], out[3]);
 }
 // four bytes holding 4-bit values -> four nibbles in the low 16 bits
 __device__ __forceinline__ uint32_t squeeze_nibbles(uint32_t b) {

@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(256) quant_int_kernel(const QuantArgs a) {
   const bool vec_ok = (a.perm == nullptr) && ((c0 & 7) == 0) && ((a.x_pitch & 7) == 0) &&
                       ((reinterpret_cast<uintptr_t>(a.x) & 15) == 0) && (c0 + 32 <= g.D);
   // Whole groups of a 4-bit layer (the common case) stay on the packed bf16 pairs as loaded: extrema by packed max / min,
-  // codes by int_sym_planar32_packed / int_asym_planar32_packed, no conversion to fp32 beyond the multiply.  The choice is the same for
+  // codes by int_sym_planar32_packed / int_asym_planar32, no conversion to fp32 beyond the multiply.  The choice is the same for
   // every thread of a group; the shuffles below run outside it, on all lanes of the warp.
   const bool packed_path = (MODE == MODE_INT4_SYM || MODE == MODE_INT4_ASYM) && vec_ok && glen == 64 * g.cpg;
   uint32_t w[16];
@@ -192,7 +192,8 @@ __global__ void __launch_bounds__(256) quant_int_kernel(const QuantArgs a) {
   if (packed_path) {
     const float rcp = __frcp_rn(p.scale);
     *reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)b * 16) =
-        (MODE == MODE_INT4_SYM) ? int_sym_planar32_packed(w, rcp, g.clip < 1.f) : int_asym_planar32_packed(w, rcp, p.zero);
+        (MODE == MODE_INT4_SYM) ? int_sym_planar32_packed(w, rcp, g.clip < 1.f)
+                                : int_asym_planar32(w, p.scale, rcp, p.zero, int_asym_packs(mx, mn, rcp, p.zero));
   } else if (nvalid == 32) {
     // full block: the division-free exact forms (reciprocal multiply, see quant_math.cuh)
     const float rcp = __frcp_rn(p.scale);

@@ -100,6 +100,7 @@ __device__ __forceinline__ void epi_int_hidden(const RotArgs& a, uint32_t taddr,
     if (col >= g.D) break;
     if (((turn++) % (uint32_t)wpq) != (uint32_t)half) continue;
     uint32_t r[64];
+    __syncwarp();                                 // lanes may have quantised the chunk before in different ways
     tmem_ld32(taddr + c0, r);
     tmem_ld32(taddr + c0 + 32, r + 32);
     tmem_wait_ld();
@@ -150,22 +151,9 @@ __device__ __forceinline__ void epi_int_hidden(const RotArgs& a, uint32_t taddr,
       dst[1] = int_sym_planar32_packed(xb + 16, rcp, clamp);
     } else if constexpr (MODE == MODE_INT4_ASYM) {
       uint4* dst = reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)chunk * 32);
-      if (fmaxf(fabsf(mx), fabsf(mn)) * rcp <= 60.f && fabsf(p.zero) <= 60.f) {
-        dst[0] = int_asym_planar32_packed(xb, rcp, p.zero);
-        dst[1] = int_asym_planar32_packed(xb + 16, rcp, p.zero);
-      } else {                                    // a group far from zero, or clipped: quotients that the packed rounding does not take
-        uint32_t n8[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          float v8[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v8[e] = val(8 * i + e);
-          const uint2 b = int_asym_byte8_fast(v8, p.scale, rcp, p.zero, maxq);
-          n8[i] = squeeze_nibbles(b.x) | (squeeze_nibbles(b.y) << 16);
-        }
-        dst[0] = planar32_from_nib8(n8[0], n8[1], n8[2], n8[3]);
-        dst[1] = planar32_from_nib8(n8[4], n8[5], n8[6], n8[7]);
-      }
+      const bool packs = int_asym_packs(mx, mn, rcp, p.zero);
+      dst[0] = int_asym_planar32(xb, p.scale, rcp, p.zero, packs);
+      dst[1] = int_asym_planar32(xb + 16, p.scale, rcp, p.zero, packs);
     } else {
       uint4* dst = reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)chunk * 64);
 #pragma unroll
@@ -295,6 +283,7 @@ __device__ __forceinline__ void epi_nvfp4_hidden(const RotArgs& a, uint32_t tadd
 // 32 columns starting at a column that is only 8-aligned (heads of 72 channels): four
 // naturally aligned 8-column reads, one wait.
 __device__ __forceinline__ void ld32_by8(uint32_t taddr, uint32_t* r) {
+  __syncwarp();                                   // lanes may have quantised the block before in different ways
   tmem_ld8(taddr, r);
   tmem_ld8(taddr + 8, r + 8);
   tmem_ld8(taddr + 16, r + 16);
@@ -384,7 +373,7 @@ __device__ __forceinline__ void epi_int_perhead(const RotArgs& a, uint32_t taddr
             for (int i = 0; i < 16; ++i) pw[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
           }
           if constexpr (MODE == MODE_INT4_SYM) c4 = int_sym_planar32_packed(pw, rcp, g.clip < 1.f);
-          else c4 = int_asym_planar32_packed(pw, rcp, p.zero);
+          else c4 = int_asym_planar32(pw, p.scale, rcp, p.zero, int_asym_packs(mx, mn, rcp, p.zero));
           const int nv = d_q - 32 * b;
           if (nv < 32) {
             const uint4 m4 = planar32_valid_mask(nv);
@@ -447,6 +436,7 @@ __device__ __forceinline__ void epi_int_perhead(const RotArgs& a, uint32_t taddr
     if (a.tail) {
       for (int c8 = d_q & ~7; c8 < d; c8 += 8) {
         uint32_t r[8];
+        __syncwarp();
         tmem_ld8(taddr + cb + c8, r);
         tmem_wait_ld();
         if (row_ok) {

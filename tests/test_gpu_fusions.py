@@ -107,6 +107,28 @@ def test_epilogue_quantises_for_the_down_projection(quant, a_sym, M, inner, tail
     assert_act_matches_oracle(buf, hidden.reshape(M, -1))
 
 
+@pytest.mark.parametrize("M", [129, 12929])                     # single CTAs, CTA pairs
+def test_epilogue_quantises_groups_far_from_zero(M):
+    """Biases that put groups of the hidden tensor far from zero (GELU is the identity there)."""
+    from dirotq_b200 import backend, ops
+    from dirotq_b200.synth import synth_activations
+    from gpu_helpers import assert_act_matches_oracle
+    root, ff, up, down = _pair(1536, 128, False, 77)
+    x = synth_activations(M, 384, torch.Generator().manual_seed(4)).reshape(1, M, 384).cuda()
+    hidden = ff.net[0](x)
+    ff.net[2](hidden)
+    away = hidden.float().std() * torch.tensor([0.0, 40.0, 300.0, 10.0], device="cuda")
+    up._b200_state.bias += away[torch.arange(1536, device="cuda") // 64 % 4].to(torch.bfloat16)
+    assert backend.fuse_ffn_quantise(root) == 1
+    hidden = ff.net[0](x)
+    sd = down._b200_state
+    regions, _ = _regions(sd, M)
+    ws = sd.workspace(M, x.device)
+    view = lambda k: ws[regions[k][1]:regions[k][1] + regions[k][2]] if regions[k][2] else None
+    ops.check_status()
+    assert_act_matches_oracle(ops.ActBuffers(sd.fmt, sd.layout, M, view(0), view(1), view(2), view(3)), hidden.reshape(M, -1))
+
+
 def test_hidden_tensor_not_written_when_nobody_else_reads_it():
     from dirotq_b200 import backend, ops
     from dirotq_b200.synth import synth_activations

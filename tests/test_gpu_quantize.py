@@ -131,6 +131,27 @@ def test_fused_rotate_quantize_per_head(H, d, hlen, mode):
     assert_act_matches_oracle(buf, x_rot.cpu())
 
 
+# Asymmetric groups whose mean lies from within to far outside their spread (quotients and zero points up to thousands), also
+# clipped: the quantise-only kernel and the per-head rotation epilogue (heads of three, one and four 32-column blocks)
+@pytest.mark.parametrize("H,d,tail", [(0, 64, 0), (0, 64, 40), (16, 72, 9), (10, 32, 4), (3, 128, 16)])
+@pytest.mark.parametrize("rotated", [False, True])
+@pytest.mark.parametrize("clip", [1.0, 0.3])
+def test_asymmetric_groups_far_from_zero(H, d, tail, rotated, clip):
+    ops = _ops()
+    from gpu_helpers import assert_act_matches_oracle
+    M, D = 131, (H * d if H else 5 * d)
+    x = torch.randn(M, D, generator=torch.Generator().manual_seed(74))
+    x[::3] += torch.tensor([3.0, -40.0, 700.0, 20.0])[torch.arange(D) // d % 4]
+    x = x.to(torch.bfloat16)
+    fmt = ops.ActFormat(ops.INT4_ASYM, D, tail_len=tail, num_heads=H, head_dim=d if H else 0, clip_ratio=clip)
+    if rotated:
+        buf = ops.rotate_quantize(x.cuda(), torch.eye(D).to(torch.bfloat16).cuda(), fmt)         # x_rot is x itself
+    else:
+        buf = ops.quantize_act(x.cuda(), fmt)
+    ops.check_status()
+    assert_act_matches_oracle(buf, x)
+
+
 def test_pack_weight_int4_matches_reference_rtn():
     ops = _ops()
     g = load_golden("weights")
