@@ -69,6 +69,7 @@ SIGNATURES = {
     "dirotq_linear_workspace_bytes": (_SZ, [C.POINTER(LinearC), _I64]),
     "dirotq_linear_forward": (C.c_int, [C.POINTER(LinearC), _P, _I64, _P, _P, _SZ, _P, _P]),
     "dirotq_linear_gemm": (C.c_int, [C.POINTER(LinearC), _I64, _P, _P, _SZ, _P, _P]),
+    "dirotq_linear_sibling": (C.c_int, [C.POINTER(LinearC), _P, _I64, _P, _P, _SZ, C.POINTER(_I32), _P, _P]),
     "dirotq_expand_weight_panel_f16_layout": (C.c_int, [_I32, _I64, _P, _P, _P, _I32, _P]),
     "dirotq_linear_uses_half_chunks": (C.c_int, [C.POINTER(LinearC)]),
     "dirotq_linear_folds_scales": (C.c_int, [C.POINTER(LinearC), _I64]),

@@ -134,11 +134,12 @@ def _drop_places(held: dict, gone):
 
 
 class _Held:
-    """A quantised tensor in a workspace: the tensor, what identifies it, and who has used it."""
-    __slots__ = ("x", "key", "seen", "ws", "y_all")
+    """A quantised tensor in a workspace: the tensor, what identifies it, who has used it, and (`records`, an int32 that the
+    library keeps) whether the folded scales that long GEMMs read lie beside the codes."""
+    __slots__ = ("x", "key", "seen", "ws", "y_all", "records")
 
-    def __init__(self, x, key, seen, ws=None, y_all=None):
-        self.x, self.key, self.seen, self.ws, self.y_all = x, key, seen, ws, y_all
+    def __init__(self, x, key, seen, ws=None, y_all=None, records=None):
+        self.x, self.key, self.seen, self.ws, self.y_all, self.records = x, key, seen, ws, y_all, records
 
 
 def _tensor_key(x: torch.Tensor) -> tuple:
@@ -192,14 +193,14 @@ class SharedActivation:
             self.held.pop(place, None)
         return h
 
-    def store(self, x: torch.Tensor, member_id: int, place: Optional[tuple] = None, ws=None, y_all=None) -> _Held:
+    def store(self, x: torch.Tensor, member_id: int, place: Optional[tuple] = None, ws=None, y_all=None, records=None) -> _Held:
         place = _place(x.device) if place is None else place
         self.misses += 1
         if place in self.held:
             self.incomplete += 1
         if place[3]:
             self.forget(lambda p: p[3] not in (0, place[3]))       # captures that are over
-        h = self.held[place] = _Held(x, _tensor_key(x), {member_id}, ws, y_all)
+        h = self.held[place] = _Held(x, _tensor_key(x), {member_id}, ws, y_all, records)
         return h
 
     def forget(self, gone):
@@ -281,7 +282,7 @@ def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
     dequantisation + GEMM.  W4A4: rotate/quantise + GEMM; the tensor-rate integer GEMM adds one preparation launch where
     the layer keeps no resident panel (the weight-panel pre-pass) or the call is long (scale folding; asked for the rows
     of the last call, counted before any call); a sibling that reuses the activations of the layer before it runs only its
-    own GEMM (and preparation)."""
+    own GEMM (and preparation; scales that an earlier sibling has folded are not folded again)."""
     if st is None:
         return 1 if (w4a16 is not None and w4a16.dense is not None) else 2    # resident dequantised weight: GEMM only
     if st.shared is not None and st.shared.fused is not None:
@@ -291,8 +292,7 @@ def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
         n -= 1                              # its activations arrive quantised from the producer's epilogue
     if st.folded is not None:
         # scale folding and the weight-panel pre-pass: one launch when both are due
-        held = next(iter((st._ws if st.shared is None else st.shared.ws).values()), None)
-        fold = held is None or bool(_lib.lib().dirotq_linear_folds_scales(C.byref(st.c_struct()), held[0]))
+        fold = _reads_records(st) and not (st.shared is not None and any(_reads_records(m) for m in st.shared.members[:st.member_id]))
         n += 1 if (fold or st.folded.panel is None) else 0
     follower = (st.shared is not None and st.member_id > 0) or st.chain_fed
     two_step = _rotates_then_quantises(st)
@@ -306,6 +306,12 @@ def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
     if st.hadamard_low_dim:
         n += 1
     return n
+
+
+def _reads_records(st: LayerState) -> bool:
+    """Whether this integer layer's GEMM reads folded scales."""
+    held = next(iter((st._ws if st.shared is None else st.shared.ws).values()), None)
+    return held is None or bool(_lib.lib().dirotq_linear_folds_scales(C.byref(st.c_struct()), held[0]))
 
 
 def _rotates_then_quantises(st: LayerState) -> bool:
@@ -408,14 +414,16 @@ def _linear(st: LayerState, x: torch.Tensor, M: int, shape: tuple, out: Optional
             nxt.forget(lambda p: p[3] not in (0, place[3]))        # captures that are over
         nxt.handed_at[place] = _Held(y, _tensor_key(y), (), nws)
         return y
-    if h is not None:
-        check(lib.dirotq_linear_gemm(lin, M, yp, wsp, wsn, status, stream), "dirotq_linear_gemm")
+    if grp is not None:
+        records = C.c_int32(0) if h is None else h.records
+        check(lib.dirotq_linear_sibling(lin, xp if h is None else None, M, yp, wsp, wsn, C.byref(records), status, stream),
+              "dirotq_linear_sibling")
+        if h is None:
+            grp.store(x, st.member_id, place, ws, records=records)
     else:
         rc = lib.dirotq_linear_forward(lin, xp, M, yp, wsp, wsn, status, stream)
         if rc:
             check(rc, "dirotq_linear_forward")
-        if grp is not None:
-            grp.store(x, st.member_id, place, ws)
     if out is not None:
         ops.mark_written(out)
     return y

@@ -347,13 +347,15 @@ struct QuantOut {
   int n_kb64_pad;     // NVFP4 consumer: 64-column blocks per row of its scale-factor tile array
 };
 
-// qo != null: see QuantOut; y may then be null.
+// qo != null: see QuantOut; y may then be null.  have != null (host memory): whether the workspace holds the records and
+// the scaled tail of these codes from an earlier call; set where this call makes them.
 static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t n_chunks, const void* x_codes,
                                   const void* x_scales, const void* x_zeros, const void* w_codes, const void* w_mult,
                                   const void* w_panel, const float* w_colscale, const void* x_tail,
                                   const void* w_tail_scaled, int32_t tail_total, int32_t tail_pitch, const void* bias,
                                   void* y, void* workspace, size_t workspace_bytes, int act,
-                                  int32_t* status, void* stream, const QuantOut* qo = nullptr, const ActGeom* geom = nullptr) {
+                                  int32_t* status, void* stream, const QuantOut* qo = nullptr, const ActGeom* geom = nullptr,
+                                  int32_t* have = nullptr) {
   if (a_mode != DIROTQ_INT4_SYM && a_mode != DIROTQ_INT4_ASYM && a_mode != DIROTQ_INT8_ASYM) return DIROTQ_E_UNSUPPORTED;
   if (M < 0 || N <= 0 || n_chunks <= 0 || !x_codes || !x_scales || !w_colscale || (!y && !qo) || !workspace)
     return DIROTQ_E_ARG;
@@ -410,7 +412,12 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
     a.q_clip = qo->clip;
   }
   const bool records = gemm_int_f16_wants_records(a);
-  if (records) {
+  if (records && have && *have) {
+    if (!w_panel) {
+      int rc = launch_expand_weight_panel(static_cast<const uint8_t*>(w_codes), n_chunks, N, w_mult, ws + c.panel, st, hc);
+      if (rc) return rc;
+    }
+  } else if (records) {
     if (!w_panel) {
       // both per-call preparations in one launch: activation scales folded into FMA operands, and the fp16 weight
       // panel rebuilt in scratch (the weights stay 4-bit in memory)
@@ -423,10 +430,7 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
                                       ws + c.rec, reinterpret_cast<float*>(ws + c.rs), tail_in, tail_s, tp, st);
       if (rc) return rc;
     }
-    a.a_const = reinterpret_cast<const uint2*>(ws + c.rec);
-    a.rs = reinterpret_cast<const float*>(ws + c.rs);
-    a.ld_rec = f16_ld_act(M);
-    a.xt = tail_s;
+    if (have) *have = 1;
   } else {
     if (!w_panel) {
       int rc = launch_expand_weight_panel(static_cast<const uint8_t*>(w_codes), n_chunks, N, w_mult, ws + c.panel, st, hc);
@@ -444,6 +448,12 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
     a.xs = static_cast<const __nv_bfloat16*>(in[0]);
     a.xz = a_mode != DIROTQ_INT4_SYM ? static_cast<const __nv_bfloat16*>(in[1]) : nullptr;
     a.ldm = ld_rows(M);
+  }
+  if (records) {
+    a.a_const = reinterpret_cast<const uint2*>(ws + c.rec);
+    a.rs = reinterpret_cast<const float*>(ws + c.rs);
+    a.ld_rec = f16_ld_act(M);
+    a.xt = tail_s;
   }
   if (!w_panel) a.w_panel = ws + c.panel;
   return launch_gemm_int_f16(a, st);
@@ -568,9 +578,10 @@ static bool produces_epilogue_codes(const dirotq_linear* lin, const ActGeom& g, 
 
 // stages: 1 = rotate / quantise into the workspace, 2 = GEMM from the workspace, 3 = both.
 // qo != null: the GEMM's epilogue quantises its output into these buffers as well (16-bit-conversion INT path only).
+// have: see gemm_w4a4_int_f16_impl.
 static int linear_stages(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace,
                          size_t workspace_bytes, int stages, int32_t* status, void* stream,
-                         const QuantOut* qo = nullptr) {
+                         const QuantOut* qo = nullptr, int32_t* have = nullptr) {
   if (!lin || !workspace || ((stages & 1) && !x) || ((stages & 2) && !y && !qo)) return DIROTQ_E_ARG;
   ActGeom g;
   WsCarve w;
@@ -607,7 +618,7 @@ static int linear_stages(const dirotq_linear* lin, const void* x, int64_t M, voi
     return gemm_w4a4_int_f16_impl(g.mode, M, lin->out_features, g.n_chunks, codes, scales, zeros, lin->w_codes,
                                   lin->w_mult, lin->w_panel_f16, lin->w_colscale, tail, lin->w_tail_f16, g.tail_total, g.tail_pitch,
                                   lin->bias, y, ws + w.fold, w.total - w.fold, lin->epilogue_act,
-                                  status, stream, qo, &g);
+                                  status, stream, qo, &g, have);
   }
   if (lin->epilogue_act != 0) return DIROTQ_E_UNSUPPORTED;
   return dirotq_gemm_w4a4_int(g.mode, M, lin->out_features, g.n_chunks, codes, scales, zeros, lin->w_codes,
@@ -625,10 +636,18 @@ int dirotq_linear_gemm(const dirotq_linear* lin, int64_t M, void* y, void* works
   return linear_stages(lin, nullptr, M, y, workspace, workspace_bytes, 2, status, stream);
 }
 
+// Long launches fold their activation scales by a kernel, 14 MB at 32768 x 1152: one for all siblings of a tensor, whichever
+// of them first needs it, and not one each.
+int dirotq_linear_sibling(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace, size_t workspace_bytes,
+                          int32_t* records, int32_t* status, void* stream) {
+  if (!records) return DIROTQ_E_ARG;
+  if (x) *records = 0;
+  return linear_stages(lin, x, M, y, workspace, workspace_bytes, x ? 3 : 2, status, stream, nullptr, records);
+}
+
 // A following layer can take its activations from the producer's epilogue when its quantiser needs nothing but the
 // producer's output row: 4-bit integer groups of 64 over the leading channels, the rest (a multiple of 64, possibly
-// none) kept in 16 bits, no rotation, no channel selection, and the 16-bit-conversion GEMM (whose per-call folding
-// step reads the scales back).
+// none) kept in 16 bits, no rotation, no channel selection, and the 16-bit-conversion GEMM, as in the producer.
 static int next_takes_epilogue_codes(const dirotq_linear* lin, const dirotq_linear* next, const ActGeom& gn) {
   if (next->rot_t || next->perm_idx) return 0;
   if (gn.H != 0 || gn.per_token || gn.q_len % 64 != 0 || gn.tail_total % 64 != 0) return 0;

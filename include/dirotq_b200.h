@@ -323,6 +323,13 @@ int dirotq_linear_forward(const dirotq_linear* lin, const void* x, int64_t M, vo
 int dirotq_linear_gemm(const dirotq_linear* lin, int64_t M, void* y, void* workspace, size_t workspace_bytes,
                        int32_t* status, void* stream);
 
+/* dirotq_linear_forward (x given) and dirotq_linear_gemm (x NULL) for layers that share activations in one workspace, as above.
+ * The GEMM of a long call reads records that a folding kernel makes of the activation scales, in the workspace; *records (the
+ * caller's, host memory, one per workspace) says whether it holds those of its codes, so that only the first of the layers
+ * that needs them makes them.  Cleared where x is given; not to be changed otherwise. */
+int dirotq_linear_sibling(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace,
+                          size_t workspace_bytes, int32_t* records, int32_t* status, void* stream);
+
 /* Producer -> consumer hand-off inside a feed-forward pair (up-projection with its fused GELU, then
  * the down-projection; the reference runs them as two ActQuantWrapper forwards with the activation
  * between them, models/pixart-sigma/model_utils.py:120-127, utils/quant_utils.py:255-326): the

@@ -121,3 +121,25 @@ def dense_reference_weight(w, ld) -> torch.Tensor:
         H, d, hl = ld.heads, ld.head_dim, ld.tail
         return torch.cat([low.reshape(N, H, d - hl), tail.reshape(N, H, hl)], dim=2).reshape(N, H * d)
     return torch.cat([low, tail], dim=1)
+
+
+def kernels_of(fn):
+    """Kernel launches of fn(), counted in a captured graph; what fn builds lazily exists by then."""
+    from cuda.bindings import runtime as rt
+    from dirotq_b200 import backend
+    with backend.WorkspaceScope(), torch.no_grad():
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            fn()
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            fn()
+    raw = rt.cudaGraph_t(graph.raw_cuda_graph())
+    err, _, n = rt.cudaGraphGetNodes(raw)
+    assert err == rt.cudaError_t.cudaSuccess
+    err, nodes, n = rt.cudaGraphGetNodes(raw, n)
+    assert err == rt.cudaError_t.cudaSuccess
+    kinds = [rt.cudaGraphNodeGetType(node)[1] for node in nodes[:n]]
+    return sum(k == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for k in kinds)

@@ -454,6 +454,52 @@ def test_sibling_layers_share_one_rotate_quantise_pass(quant):
     ops.check_status()
 
 
+# 1152 outputs of 16000 rows run on CTA pairs, which read folded scales; 128 on single CTAs, which fold their own
+@pytest.mark.parametrize("quant,a_sym", [("int4", True), ("int4", False), ("int8", True)])
+@pytest.mark.parametrize("widths,folds", [((1152, 1152, 1152), 1), ((128, 1152, 1152), 1), ((1152, 128, 1152), 1), ((128, 128), 0)])
+@pytest.mark.parametrize("panel", ["auto", False])
+def test_siblings_on_pairs_fold_their_scales_once(quant, a_sym, widths, folds, panel, monkeypatch):
+    """Every member's output equals the unshared layer's, whichever member needs the folded scales first, and the folding kernel
+    runs once for the group (without a resident panel it rides in the first pre-pass that needs it)."""
+    from dirotq_b200 import backend, dit, ops
+    from dirotq_b200.synth import synth_activations
+    from gpu_helpers import kernels_of
+    monkeypatch.setattr(backend, "CACHE_WEIGHT_PANEL", panel)
+    M, D = 16000, 128
+
+    def build(share):
+        attn, ws = nn.Module(), []
+        for i, (leaf, N) in enumerate(zip(("to_q", "to_k", "to_v"), widths)):
+            w = dit.make_wrapped_linear(dit.LayerDef("attn1." + leaf, D, N, tail=64), quant, 37 + i, "cuda", a_sym=a_sym)
+            if ws:
+                w.rotation = ws[0].rotation.clone()
+            attn.add_module(leaf, w)
+            ws.append(w)
+        root = nn.Module()
+        root.add_module("attn1", attn)
+        monkeypatch.setattr(backend, "SHARE_SIBLING_ACTIVATIONS", share)
+        backend.preconvert_rotations_to_device(root, "cuda")
+        return ws
+
+    ws, alone = build(True), build(False)
+    assert ws[0]._b200_state.shared is not None and alone[0]._b200_state.shared is None
+    x = synth_activations(M, D, torch.Generator().manual_seed(11)).reshape(1, M, D).cuda()
+    want = [w(x) for w in alone]
+    for _ in range(2):
+        for y, ref in zip([w(x) for w in ws], want):
+            assert torch.equal(y, ref)
+    ops.check_status()
+    prepasses = len(widths) if panel is False else 0
+    n = kernels_of(lambda: [w(x) for w in ws])
+    assert n == 1 + len(widths) + (prepasses if prepasses else folds)
+    assert n == sum(backend.kernel_launches(w._b200_state) for w in ws)
+    # another input through the same workspace
+    x2 = x * 1.5
+    for y, w in zip([w(x2) for w in ws], alone):
+        assert torch.equal(y, w(x2))
+
+
+
 @pytest.mark.parametrize("name", ["hadamard_int4_sym", "hadamard_int4_sym_n128"])
 def test_hadamard_layers(name):
     """use_hadamard layers: the FWHT front end is bit-identical to the reference's fp32 butterflies, so the
