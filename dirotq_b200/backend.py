@@ -242,6 +242,7 @@ class LayerState:
     chain_fed: bool = False                          # a producer's epilogue quantises for this layer
     panel_declined: bool = False                     # a large-batch call found the resident-panel budget spent
     built: Optional[tuple] = None                    # see _mark_built
+    rows: int = 0                                    # of the last call
     _c: Optional[LinearC] = None
     _ws: Dict[tuple, tuple] = field(default_factory=dict)          # see _buffer
 
@@ -309,9 +310,15 @@ def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
 
 
 def _reads_records(st: LayerState) -> bool:
-    """Whether this integer layer's GEMM reads folded scales."""
-    held = next(iter((st._ws if st.shared is None else st.shared.ws).values()), None)
-    return held is None or bool(_lib.lib().dirotq_linear_folds_scales(C.byref(st.c_struct()), held[0]))
+    """Whether this integer layer's GEMM reads folded scales, for the rows of its last call (before any call: counted as if)."""
+    lib = _lib.lib()
+    asked = lib.dirotq_linear_chain_folds_scales if _hands_on(st) else lib.dirotq_linear_folds_scales
+    return st.rows == 0 or bool(asked(C.byref(st.c_struct()), st.rows))
+
+
+def _hands_on(st: LayerState) -> bool:
+    """Whether this layer's GEMM also quantises its output for the layer behind it."""
+    return st.chain_next is not None and st.shared is None and not st.chain_next.hadamard_low_dim
 
 
 def _rotates_then_quantises(st: LayerState) -> bool:
@@ -346,6 +353,7 @@ def _linear(st: LayerState, x: torch.Tensor, M: int, shape: tuple, out: Optional
     dev = x.device
     place = _place(dev)
     grp = st.shared
+    st.rows = M
     if grp is not None and grp.fused is not None:
         # siblings fused into one layer: the first member called on a tensor runs it, the others take their columns
         if grp.incomplete > 2:
@@ -402,8 +410,8 @@ def _linear(st: LayerState, x: torch.Tensor, M: int, shape: tuple, out: Optional
         e = (st._ws if grp is None else grp.ws).get(place)
         ws = e[1] if e is not None and e[0] == M else st.workspace(M, dev, place)
     wsp, wsn = ws.data_ptr(), ws.numel()
-    nxt = st.chain_next
-    if nxt is not None and grp is None and not nxt.hadamard_low_dim:
+    if st.chain_next is not None and _hands_on(st):
+        nxt = st.chain_next
         nws = nxt.workspace(M, dev, place)
         check(lib.dirotq_linear_forward_chain(lin, xp, M, yp if st.chain_keep_output else None, wsp, wsn,
                                               C.byref(nxt.c_struct()), nws.data_ptr(), nws.numel(), status, stream),

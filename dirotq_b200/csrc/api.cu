@@ -411,7 +411,7 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
     a.q_mode = qo->mode;
     a.q_clip = qo->clip;
   }
-  const bool records = gemm_int_f16_wants_records(a);
+  const bool records = gemm_int_f16_wants_records(a, qo != nullptr);
   if (records && have && *have) {
     if (!w_panel) {
       int rc = launch_expand_weight_panel(static_cast<const uint8_t*>(w_codes), n_chunks, N, w_mult, ws + c.panel, st, hc);
@@ -668,7 +668,7 @@ int dirotq_linear_uses_half_chunks(const dirotq_linear* lin) {
   return (uses_f16_gemm(lin, g) && half_chunk_geometry(g)) ? 1 : 0;
 }
 
-int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M) {
+static int folds_scales(const dirotq_linear* lin, int64_t M, bool quantise_out) {
   ActGeom g;
   if (!lin || M <= 0 || make_geom(&lin->fmt, &g) || !uses_f16_gemm(lin, g)) return 0;
   GemmIntF16Args a;
@@ -677,8 +677,10 @@ int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M) {
   a.n_chunks = g.n_chunks;
   a.kt = g.tail_total;
   a.half_chunks = half_chunk_geometry(g) ? 1 : 0;
-  return gemm_int_f16_wants_records(a) ? 1 : 0;
+  return gemm_int_f16_wants_records(a, quantise_out) ? 1 : 0;
 }
+int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M) { return folds_scales(lin, M, false); }
+int dirotq_linear_chain_folds_scales(const dirotq_linear* lin, int64_t M) { return folds_scales(lin, M, true); }
 
 int dirotq_linear_chain_supported(const dirotq_linear* lin, const dirotq_linear* next) {
   if (!lin || !next) return 0;

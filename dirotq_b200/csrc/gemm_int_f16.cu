@@ -1224,14 +1224,14 @@ static int pick_raster_f16(int BN, int64_t N, int64_t k_total) {
 // 1152 x 1152 12.0 / 10.7, 4096 x 1152 x 1152 19.4 / 17.9, 1024 x 2240 x 6720 32.3 / 30.9, 4608 x 3072 x 3072 (three rounds) 63.8 /
 // 63.1; on pairs 32768 x 1152 x 3456 205 / 214, 4608 x 3072 x 12288 238 / 253.  A warp of the GEMM that makes the records for
 // the converters was slower than either (262): its polls and stores take from the same pipes.
-static bool picks_pair(const GemmIntF16Args& a, int* bn) {
+static bool picks_pair(const GemmIntF16Args& a, bool quantise_out, int* bn) {
   const int64_t n_stage = a.half_chunks ? (a.n_chunks + 1) / 2 : a.n_chunks;
-  *bn = pick_bn_f16(a.M, a.N, n_stage * 64 + ((a.kt + 63) / 64) * 64, a.q_codes != nullptr);
+  *bn = pick_bn_f16(a.M, a.N, n_stage * 64 + ((a.kt + 63) / 64) * 64, quantise_out);
   return *bn == 256 && pick_pair_f16(a.M, a.N);
 }
-bool gemm_int_f16_wants_records(const GemmIntF16Args& a) {
+bool gemm_int_f16_wants_records(const GemmIntF16Args& a, bool quantise_out) {
   int bn;
-  return picks_pair(a, &bn);
+  return picks_pair(a, quantise_out, &bn);
 }
 
 int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
@@ -1244,7 +1244,7 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
   const uint64_t n_stage = a.half_chunks ? (uint64_t)((a.n_chunks + 1) / 2) : (uint64_t)a.n_chunks;
   const int64_t k_total = (int64_t)n_stage * 64 + ((a.kt + 63) / 64) * 64;
   int BN;
-  const bool pair = picks_pair(a, &BN);
+  const bool pair = picks_pair(a, a.q_codes != nullptr, &BN);
   if (pair ? !a.a_const || !a.rs : !a.xs) return DIROTQ_E_ARG;
   if (a.q_codes) {
     if (a.N % 64 || a.q_len % 64 || a.q_len <= 0 || a.q_len > a.N || a.q_row_bytes < a.q_len / 2 || (a.q_row_bytes & 15) ||

@@ -343,8 +343,10 @@ int dirotq_linear_sibling(const dirotq_linear* lin, const void* x, int64_t M, vo
  * quantised part and its 16-bit tail both multiples of 64 channels (the tail may be empty), no
  * rotation, no channel selection, width == lin->out_features, w_mult set.  Anything else: DIROTQ_E_UNSUPPORTED, nothing launched. */
 int dirotq_linear_uses_half_chunks(const dirotq_linear* lin);
-/* Whether a GEMM of `lin` on M rows launches the scale-folding kernel first (long launches of integer layers). */
+/* Whether a GEMM of `lin` on M rows launches the scale-folding kernel first (long launches of integer layers): alone, or as
+ * the producer of dirotq_linear_forward_chain, whose quantising epilogue does not take every tile width. */
 int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M);
+int dirotq_linear_chain_folds_scales(const dirotq_linear* lin, int64_t M);
 int dirotq_linear_chain_supported(const dirotq_linear* lin, const dirotq_linear* next);
 int dirotq_linear_forward_chain(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace,
                                 size_t workspace_bytes, const dirotq_linear* next, void* next_workspace,

@@ -156,6 +156,25 @@ def test_hidden_tensor_not_written_when_nobody_else_reads_it():
     assert torch.equal(y_other.reshape(M, -1), y_plain)
 
 
+@pytest.mark.parametrize("M", [300, 15360, 20000])      # 15360: 192-wide single CTAs alone, 256-wide pairs when quantising
+def test_launch_counts_follow_the_last_call(M):
+    """kernel_launches against the kernels of a captured pass: alone, as a pair that hands its activations on, after calls of
+    other sizes on other streams."""
+    from dirotq_b200 import backend
+    from dirotq_b200.synth import synth_activations
+    from gpu_helpers import kernels_of
+    root, ff, up, down = _pair(1152, 128, True, 79)
+    x = synth_activations(M, 384, torch.Generator().manual_seed(3)).reshape(1, M, 384).cuda()
+    counted = lambda: sum(backend.kernel_launches(w._b200_state) for w in (up, down))
+    for other in (16500, 200):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            ff.net[2](ff.net[0](x.new_zeros(1, other, 384)))
+        torch.cuda.synchronize()
+        assert kernels_of(lambda: ff.net[2](ff.net[0](x))) == counted()
+    assert backend.fuse_ffn_quantise(root) == 1
+    assert kernels_of(lambda: ff.net[2](ff.net[0](x))) == counted()
+
+
 def test_unsupported_pairs_are_left_alone():
     from dirotq_b200 import backend, dit
     # a rotated down-projection needs the whole row before it can quantise: no hand-off
