@@ -24,7 +24,8 @@ def test_both_scale_routes_give_the_same_bits(mode, M, D, tail, monkeypatch):
     rows = torch.arange(act.ldm, device="cuda")
     s *= torch.exp2(((rows * 7) % 49 - 24).float()).to(torch.bfloat16)
     s[::2] *= torch.exp2(-((rows * 5) % 13).float()).to(torch.bfloat16)
-    s[:, M // 2] = 0
+    if M > 1:
+        s[:, M // 2] = 0
     wt = ops.pad_tail_weight(w_tail, lay.tail_pitch, 264, "cuda")
     folded = ops.fold_weight_scales_f16(pk, wt, lay.tail_total)
     run = lambda a: ops.gemm_w4a4_int_f16(a, pk, folded, bias.cuda())
@@ -49,6 +50,46 @@ def test_both_scale_routes_give_the_same_bits(mode, M, D, tail, monkeypatch):
         monkeypatch.setenv("DIROTQ_GF_BN", bn)
         monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
         assert torch.equal(run(moved), out["256", "1"])
+    ops.check_status()
+
+
+# Nine tiles and more per CTA: the table of row powers, four tiles deep and written one tile ahead, goes round more than twice.
+# One operand stage per tile (converter groups take alternate tiles), two (a chunk and the tail), five.
+@pytest.mark.parametrize("D,tail", [(64, 0), (128, 64), (320, 0)])
+@pytest.mark.parametrize("mode", ["sym", "asym", "int8"])
+def test_row_powers_of_many_tiles_per_cta(mode, D, tail, monkeypatch):
+    from dirotq_b200 import ops
+    from test_gpu_gemm import _setup_int
+    M, N = 34300, 1032                               # 268 x 5 tiles of 256 columns on 148 SMs
+    m = {"sym": ops.INT4_SYM, "asym": ops.INT4_ASYM, "int8": ops.INT8_ASYM}[mode]
+    x, act, dec, qw, sw, pk, w_tail, bias = _setup_int(ops, M, N, ops.ActFormat(m, D, tail_len=tail), 75)
+    lay = act.layout
+    s = act.scales[: lay.n_scales * act.ldm * 2].view(torch.bfloat16).view(lay.n_scales, act.ldm)
+    rows = torch.arange(act.ldm, device="cuda")
+    s *= torch.exp2(((rows // 3 * 7) % 49 - 24).float()).to(torch.bfloat16)     # a wrong tile's or row's power shows
+    folded = ops.fold_weight_scales_f16(pk, ops.pad_tail_weight(w_tail, lay.tail_pitch, N, "cuda"), lay.tail_total)
+    bias = bias.cuda()
+    out = {}
+    for bn, pair in (("256", "1"), ("128", "0"), ("192", "0"), ("256", "0")):
+        monkeypatch.setenv("DIROTQ_GF_BN", bn)
+        monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
+        out[bn, pair] = ops.gemm_w4a4_int_f16(act, pk, folded, bias)
+    ops.check_status()
+    for k, y in out.items():
+        assert torch.equal(y, out["256", "1"]), k
+
+
+def test_unforced_call_of_five_single_cta_rounds(monkeypatch):
+    """15360 x 1152 x 1152: 192-wide tiles on single CTAs, five rounds, by the dispatch's own choice."""
+    from dirotq_b200 import ops
+    from test_gpu_gemm import _setup_int
+    x, act, dec, qw, sw, pk, w_tail, bias = _setup_int(ops, 15360, 1152, ops.ActFormat(ops.INT4_ASYM, 1152, tail_len=64), 76)
+    lay = act.layout
+    folded = ops.fold_weight_scales_f16(pk, ops.pad_tail_weight(w_tail, lay.tail_pitch, 1152, "cuda"), lay.tail_total)
+    y = ops.gemm_w4a4_int_f16(act, pk, folded, bias.cuda())
+    monkeypatch.setenv("DIROTQ_GF_BN", "256")
+    monkeypatch.setenv("DIROTQ_GF_PAIR", "1")
+    assert torch.equal(y, ops.gemm_w4a4_int_f16(act, pk, folded, bias.cuda()))
     ops.check_status()
 
 
