@@ -10,8 +10,10 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-# rows and widths around the tiles (128 rows, a stage of four 64-slot chunks, a tail of 64), one to five chunks, ragged ends
-@pytest.mark.parametrize("M,D,tail", [(1, 128, 8), (129, 320, 0), (257, 384, 72), (300, 1152, 64), (520, 4608, 320)])
+# rows and widths around the tiles (128 rows, a stage of four 64-slot chunks, a tail of 64), one to five chunks, ragged ends; rows
+# around an octet of scales, 100 and 192 chunks (96 of them are in flight when the epilogue warps read a tile's scales)
+@pytest.mark.parametrize("M,D,tail", [(1, 128, 8), (129, 320, 0), (257, 384, 72), (300, 1152, 64), (520, 4608, 320), (39, 6464, 64),
+                                      (137, 12288, 0)])
 @pytest.mark.parametrize("mode", ["sym", "asym", "int8"])
 def test_both_scale_routes_give_the_same_bits(mode, M, D, tail, monkeypatch):
     from dirotq_b200 import ops
