@@ -84,9 +84,11 @@ template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
   // Warpgroups: epilogue (warps 0..7), issuer and the two producers (8..11, the last one idle), converters (12..19).  The
   // launch gives every thread 96 registers; the producers' and converters' groups hand some back to the epilogue's, which
   // holds a quarter row of the tile (64 registers of bf16 pairs) besides the piece in work and the one being fetched.
-  // (128 / 48 / 88 spills nowhere; with 136 / 48 / 80 the converters' votes cost 52 bytes a thread and 2 % of a long call.)
+  // On pairs the issuer's whole-warp form spills with 128 / 48 / 88 (52 bytes a thread stored, 124 loaded) and not with 120 / 80 / 80:
+  // 32768 x 1152 x 3456 205 -> 201 us, 16384 x 2240 x 2240 122.5 -> 120, half chunks 160 -> 157.  Single CTAs spill 24 bytes with
+  // the former and are slower all the same with 120 or 128 / 64 to 80 / 80: 4096 x 4608 x 1152 50.0 -> 52.0.
   static constexpr int THREADS = (GF_EPI_WARPS + 4 + CONV_WARPS) * 32;
-  static constexpr int REGS_LAUNCH = 96, REGS_EPI = 128, REGS_PROD = 48, REGS_CONV = 88;
+  static constexpr int REGS_LAUNCH = 96, REGS_EPI = PAIR ? 120 : 128, REGS_PROD = PAIR ? 80 : 48, REGS_CONV = PAIR ? 80 : 88;
   static_assert(GF_EPI_WARPS * REGS_EPI + 4 * REGS_PROD + CONV_WARPS * REGS_CONV <= THREADS / 32 * REGS_LAUNCH,
                 "setmaxnreg draws on the registers of the launch");
   static constexpr int BN_OWN = PAIR ? BN / 2 : BN;         // weight rows this CTA fetches
