@@ -56,9 +56,12 @@ struct GpCfg {
   // Warpgroups: producer and issuer (warps 0, 1; 2 and 3 idle), movers (4..7), epilogue (8..15).  The launch gives every
   // thread 128 registers; the first two groups hand some back to the epilogue's, which holds a quarter row of the tile
   // (128 accumulators of a 256-wide one; with 128 registers it spilled 350 bytes a thread).
+  // 128-wide tiles leave what is over to the issuer, whose whole-warp form spills with 56 (36 bytes stored, 116 loaded; 8 / 36 with 72):
+  // 512 x 3072 x 3072 11.9 -> 11.1 us, 1024 x 2240 x 2240 11.1 -> 10.2, 4096 x 1152 x 1152 11.1 -> 10.7.  256-wide ones have no use for
+  // it (32768 x 1152 x 3456 98.7 / 99.5).
   static constexpr int SF_WARP0 = 4, EPI_WARP0 = SF_WARP0 + SF_WARPS;
   static constexpr int THREADS = (EPI_WARP0 + EPI_WARPS) * 32;
-  static constexpr int REGS_LAUNCH = 128, REGS_EPI = 184, REGS_PROD = 56, REGS_SF = 72;
+  static constexpr int REGS_LAUNCH = 128, REGS_EPI = 184, REGS_PROD = BN == 128 ? 72 : 56, REGS_SF = 72;
   static_assert(EPI_WARPS * REGS_EPI + SF_WARP0 * REGS_PROD + SF_WARPS * REGS_SF <= THREADS / 32 * REGS_LAUNCH,
                 "setmaxnreg draws on the registers of the launch");
   static constexpr int STG_BYTES = EPI_WARPS * 2 * 2048;    // per epilogue warp: two 32 rows x 32 bf16 staging patches
