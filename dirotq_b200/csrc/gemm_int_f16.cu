@@ -1208,16 +1208,17 @@ static int launch_gf(const GfMaps& tm, const GemmIntF16Args& a, cudaStream_t st)
   return launch_pdl(k, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, st, tm, a) == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
 }
 
-// Column-tile width.  The persistent grid runs ceil(tiles / SMs) rounds, and a round of 256-wide tiles takes 9/7 of a round
-// of 128-wide ones whatever K is: 8.5 us against 6.6 at K = 1152, 16.6 / 12.9 at 2240, 21.1 / 16.7 at 3072 (the issuer's
-// per-stage barrier protocol does not depend on the width, and the wide tile's single accumulator is handed back before
-// anything else is done with it).  So 256 wherever it saves a quarter of the rounds (1152 -> 3456 at 32768 rows: 213 us
-// against 311; 1152 -> 4608 at 4096: 44 / 62), 128 where both need the same few (1152 x 1152 at 4096 rows: 23.0 / 25.3;
-// 2240 x 2240 at 1024: 28.7 / 30.5).  A round of 192-wide tiles takes 6/5 of a 128-wide one: ahead where it needs no more
-// rounds than 256 (1152 x 1152 at 12288 rows, four of either: 38.7 us against 40.3, 8-bit activations 38.2 / 42.2; 1152 -> 3456
-// at 3072: 29.9 / 31.0), never otherwise.  From five rounds on, where 256-wide tiles run on CTA pairs, only for short K (15360
-// rows: 1152 x 1152 45.8 / 47.7, 4608 -> 1152 139 / 137).  The quantise-out epilogue wants whole groups of 64 columns per
-// warp: not 192.  DIROTQ_GF_BN overrides.
+// Column-tile width.  The persistent grid runs ceil(tiles / SMs) rounds, and a round of 256-wide tiles takes about 9/7 of a
+// round of 128-wide ones whatever K is (the converters' work for a stage does not depend on the width, and the wide tile's
+// single accumulator is handed back before anything else is done with it).  So 256 wherever it saves a quarter of the rounds (us,
+// 256 / 128 columns: 1152 -> 3456 at 32768 rows 213 / 298, 1152 -> 4608 at 4096 37.7 / 56.5), 128 where both need the same few
+// (1152 x 1152 at 4096 rows, two of either: 20.5 / 18.4; 2240 x 2240 at 1024, one: 18.4 / 17.2).  A round of
+// 192-wide tiles takes 6/5 of a 128-wide one: ahead where it needs no more rounds than 256 (192 / 256: 1152 x 1152 at 12288 rows,
+// four of either, 33.6 / 36.1, 8-bit activations 34.0 / 37.3; 1152 -> 3456 at 3072 26.6 / 28.7).  From five rounds on, where
+// 256-wide tiles run on CTA pairs behind the folding kernel, for short K: 1152 x 1152 at 15360 rows 40.1 / 47.1.  That line was
+// drawn when both forms paid the folding kernel (4608 -> 1152 139 / 137); now that single CTAs do not, 192 is ahead there too,
+// 127 / 138, 8-bit 134 / 142.  The quantise-out epilogue wants whole groups of 64 columns per warp: not 192.
+// DIROTQ_GF_BN overrides.
 static int pick_bn_f16(int64_t M, int64_t N, int64_t k_total, bool qout) {
   if (const char* e = getenv("DIROTQ_GF_BN")) return atoi(e) <= 128 ? 128 : atoi(e) <= 192 && !qout ? 192 : 256;
   const int64_t m_tiles = (M + 127) / 128, sms = num_sms();
@@ -1227,10 +1228,11 @@ static int pick_bn_f16(int64_t M, int64_t N, int64_t k_total, bool qout) {
   return 9 * r256 < 7 * r128 ? 256 : 128;
 }
 
-// CTA pairs halve the weight traffic of a 256-wide tile and issue one UMMA for two SMs: 204 us against 213 for 1152 -> 3456 at
-// 32768 rows, 185 / 190 for 3072 -> 9216 at 4608.  Their tiles are twice as tall, so the last round is coarser, and a stage's
-// hand-off crosses the pair: 26.1 us against 25.3 for 1152 x 1152 at 4096 rows (two rounds), 44.7 / 44.4 for 1152 -> 4608 (four),
-// level at 32768 x 1152 (nine).  Hence only from five rounds on.  DIROTQ_GF_PAIR overrides (0 or 1).
+// CTA pairs halve the weight traffic of a 256-wide tile and issue one UMMA for two SMs (us, pair with its folding kernel / single:
+// 1152 -> 3456 at 32768 rows 201 / 213, 1152 -> 4608 259 / 277, 3072 -> 9216 at 4608 176 / 184, 8-bit 184 / 194).  Their tiles are
+// twice as tall, so the last round is coarser, and a stage's hand-off crosses the pair: 22.9 / 20.5 for 1152 x 1152 at 4096 rows (two
+// rounds), 39.3 / 37.7 for 1152 -> 4608 (four), 77.0 / 75.8 for 32768 x 1152 (nine).  Hence only from five rounds on.  DIROTQ_GF_PAIR
+// overrides (0 or 1).
 static bool pick_pair_f16(int64_t M, int64_t N) {
   if (const char* e = getenv("DIROTQ_GF_PAIR")) return atoi(e) != 0;
   return ((M + 127) / 128) * ((N + 255) / 256) > 4 * (int64_t)num_sms();
@@ -1250,11 +1252,12 @@ static int pick_raster_f16(int BN, int64_t N, int64_t k_total) {
 }
 
 // Whether a call reads activation records (and row powers of two, and a scaled tail) that the folding kernel has made, or the
-// scales themselves.  The folding kernel is 2-3 us of launch and latency; the converters' share of the same work is four to ten
-// instructions per row and chunk, which long launches, bound by the converters, feel.  Us, folding kernel + GEMM / GEMM alone: 256 x
-// 1152 x 1152 12.0 / 10.7, 4096 x 1152 x 1152 19.4 / 17.9, 1024 x 2240 x 6720 32.3 / 30.9, 4608 x 3072 x 3072 (three rounds) 63.8 /
-// 63.1; on pairs 32768 x 1152 x 3456 205 / 214, 4608 x 3072 x 12288 238 / 253.  A warp of the GEMM that makes the records for
-// the converters was slower than either (262): its polls and stores take from the same pipes.
+// scales themselves: the former on CTA pairs, the latter in every launch of single CTAs, 128- and 192-wide ones of any length
+// included.  The folding kernel is 2-3 us of launch and latency; the converters' share of the same work is four to ten instructions
+// per row and chunk, which the long launches on pairs, bound by the converters, feel.  Us, folding kernel + GEMM (256 columns) / GEMM
+// alone: 1536 x 12288 x 3072 82.3 / 78.2, and before its scales were read by 16-byte loads (2-8 % more than now) 4608 x 3072 x 3072
+// (three rounds) 63.9 / 62.3, 8192 x 2240 x 2240 64.3 / 61.8, 12288 x 4608 x 1152 115.9 / 112.6, 4096 x 1152 x 4608 39.7 / 38.5; on pairs 32768 x 1152 x 3456 205 / 214, 4608 x 3072 x 12288 238 / 253.  A warp of the GEMM that makes the records for the converters was slower than either (262): its polls and stores take from the
+// same pipes.
 static bool picks_pair(const GemmIntF16Args& a, bool quantise_out, int* bn) {
   const int64_t n_stage = a.half_chunks ? (a.n_chunks + 1) / 2 : a.n_chunks;
   *bn = pick_bn_f16(a.M, a.N, n_stage * 64 + ((a.kt + 63) / 64) * 64, quantise_out);
