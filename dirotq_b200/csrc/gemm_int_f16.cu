@@ -1256,8 +1256,9 @@ static int pick_raster_f16(int BN, int64_t N, int64_t k_total) {
 // included.  The folding kernel is 2-3 us of launch and latency; the converters' share of the same work is four to ten instructions
 // per row and chunk, which the long launches on pairs, bound by the converters, feel.  Us, folding kernel + GEMM (256 columns) / GEMM
 // alone: 1536 x 12288 x 3072 82.3 / 78.2, and before its scales were read by 16-byte loads (2-8 % more than now) 4608 x 3072 x 3072
-// (three rounds) 63.9 / 62.3, 8192 x 2240 x 2240 64.3 / 61.8, 12288 x 4608 x 1152 115.9 / 112.6, 4096 x 1152 x 4608 39.7 / 38.5; on pairs 32768 x 1152 x 3456 205 / 214, 4608 x 3072 x 12288 238 / 253.  A warp of the GEMM that makes the records for the converters was slower than either (262): its polls and stores take from the
-// same pipes.
+// (three rounds) 63.9 / 62.3, 8192 x 2240 x 2240 64.3 / 61.8, 12288 x 4608 x 1152 115.9 / 112.6, 4096 x 1152 x 4608 39.7 / 38.5;
+// on pairs 32768 x 1152 x 3456 205 / 214, 4608 x 3072 x 12288 238 / 253.  A warp of the GEMM that makes the records for the
+// converters was slower than either (262): its polls and stores take from the same pipes.
 static bool picks_pair(const GemmIntF16Args& a, bool quantise_out, int* bn) {
   const int64_t n_stage = a.half_chunks ? (a.n_chunks + 1) / 2 : a.n_chunks;
   *bn = pick_bn_f16(a.M, a.N, n_stage * 64 + ((a.kt + 63) / 64) * 64, quantise_out);
