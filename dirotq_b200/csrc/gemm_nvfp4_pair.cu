@@ -458,10 +458,8 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
           uint32_t sfw = 0;
 #pragma unroll
           for (int gi = 0; gi < 4; ++gi) {
-            float eff;
-            const uint8_t sbyte = nvfp4_hw_scale(amax_bf16x16(w + 8 * gi), a.q_clip, a.q_T, &eff);
-            uint2 cc = make_uint2(0u, 0u);
-            if (eff > 0.f) cc = nvfp4_hw_group_packed(w + 8 * gi, eff);
+            uint2 cc;
+            const uint8_t sbyte = nvfp4_hw_group(w + 8 * gi, a.q_clip, a.q_T, cc);
             packed[2 * gi] = cc.x;
             packed[2 * gi + 1] = cc.y;
             sfw |= (uint32_t)sbyte << (8 * gi);

@@ -114,6 +114,11 @@ struct RotArgs {
   int m_tiles;
   int K;                  // contraction length (== g.D for a rotation)
   int band;               // 0 = dense rotation, else head_dim of a block-diagonal rotation
+  // per-head layouts: a group's last block of 32 slots where it is not full.  Masks of its valid slots, as bf16 pairs and as
+  // code bytes (the planar nibbles of the 4-bit modes, one byte a slot in 8 bits)
+  int ragged;
+  uint32_t pair_mask[16];
+  uint32_t code_mask[8];
   const __nv_bfloat16* bias;  // plain-GEMM epilogue only
   __nv_bfloat16* x_rot;   // optional [M, D]
   uint8_t* codes;

@@ -147,70 +147,78 @@ __device__ __forceinline__ uint32_t int_sym_nib8_packed(const uint32_t* p, float
 // paired with value 16 + j BEFORE the packed rounding, so that the two nibbles of byte j come out of one register
 // (no re-ordering of nibbles afterwards).  The two quotients of a pair are one packed fp32 multiply.  `clamp` is
 // needed only when the scale was clipped (clip_ratio < 1): with scale = bf16(amax / 7) no quotient exceeds 7.03.
+__device__ __forceinline__ uint64_t mul_f32x2(uint32_t lo, uint32_t hi, uint64_t k) {
+  uint64_t q;
+  asm("{\n\t.reg .b64 x;\n\tmov.b64 x, {%1, %2};\n\tmul.rn.f32x2 %0, x, %3;\n\t}" : "=l"(q) : "r"(lo), "r"(hi), "l"(k));
+  return q;
+}
+__device__ __forceinline__ uint64_t twice_f32(float v) { return ((uint64_t)__float_as_uint(v) << 32) | __float_as_uint(v); }
+// Four words whose halves hold, in their low bytes, the nibbles (with anything above them) of slots j (low half) and 16 + j
+// (high half), j = 0 .. 3 -> the four planar-32 bytes.  Bytes are gathered before they are masked: six instructions, 1.5 per
+// pair of codes, where masking, folding and shifting each word took four to five.
+__device__ __forceinline__ uint32_t planar_bytes(const uint32_t* c) {
+  const uint32_t c01 = __byte_perm(c[0], c[1], 0x6240), c23 = __byte_perm(c[2], c[3], 0x6240);
+  const uint32_t lo = __byte_perm(c01, c23, 0x5410), hi = __byte_perm(c01, c23, 0x7632);
+  return (lo & 0x0F0F0F0Fu) | ((hi << 4) & 0xF0F0F0F0u);
+}
 __device__ __forceinline__ uint4 int_sym_planar32_packed(const uint32_t* p, float rcp_s, bool clamp) {
   const __nv_bfloat162 lo2 = __floats2bfloat162_rn(-8.f, -8.f), hi2 = __floats2bfloat162_rn(7.f, 7.f),
                        magic = __floats2bfloat162_rn(192.f, 192.f);
-  const uint64_t rr = ((uint64_t)__float_as_uint(rcp_s) << 32) | __float_as_uint(rcp_s);
+  const uint64_t rr = twice_f32(rcp_s);
   uint32_t out[4];
 #pragma unroll
   for (int wd = 0; wd < 4; ++wd) {
-    uint32_t acc = 0;
+    uint32_t c[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int j = 4 * wd + k;                          // byte j: slots j and 16 + j
       const uint32_t a = p[j >> 1], b = p[8 + (j >> 1)];
-      const uint32_t fa = (j & 1) ? (a & 0xFFFF0000u) : (a << 16), fb = (j & 1) ? (b & 0xFFFF0000u) : (b << 16);
-      uint64_t q;
-      asm("{\n\t.reg .b64 x;\n\tmov.b64 x, {%1, %2};\n\tmul.rn.f32x2 %0, x, %3;\n\t}" : "=l"(q) : "r"(fa), "r"(fb), "l"(rr));
+      const uint64_t q = mul_f32x2((j & 1) ? (a & 0xFFFF0000u) : (a << 16), (j & 1) ? (b & 0xFFFF0000u) : (b << 16), rr);
       __nv_bfloat162 r = __floats2bfloat162_rn(__uint_as_float((uint32_t)q), __uint_as_float((uint32_t)(q >> 32)));
       if (clamp) r = __hmin2(__hmax2(r, lo2), hi2);
       r = __hadd2(r, magic);
-      const uint32_t c = *reinterpret_cast<const uint32_t*>(&r) & 0x000F000Fu;
-      acc |= ((c & 0xFu) | (c >> 12)) << (8 * k);
+      c[k] = *reinterpret_cast<const uint32_t*>(&r);
     }
-    out[wd] = acc;
+    out[wd] = planar_bytes(c);
   }
   return make_uint4(out[0], out[1], out[2], out[3]);
 }
 // The asymmetric 4-bit form of the same: code = clamp(bf16(rint(bf16(x / s)) + zero), 0, 15).  On packed bf16 pairs: adding
-// 192 rounds the quotient half-even to an integer (bf16 spacing is 1 in [128, 256)); adding (zero - 192) gives rint(q) + zero
-// exactly (both are integers below 2^8); clamp; adding 128 leaves the code in the low mantissa bits.  Only for groups that
+// 192 rounds the quotient half-even to an integer (bf16 spacing is 1 in [128, 256)); adding (zero - 64) gives rint(q) + zero + 128
+// exactly (an integer in [8, 248]); the clamp to [128, 143] leaves the code in the low mantissa bits.  Only for groups that
 // int_asym_packs allows: the range of a group need not include zero (int_asym_params), so a group whose mean lies far from
 // zero has quotients and a zero point of any size, and 192 + q would leave [128, 256).
 __device__ __forceinline__ bool int_asym_packs(float mx, float mn, float rcp_s, float zero) {
   return fmaxf(fabsf(mx), fabsf(mn)) * rcp_s <= 60.f && fabsf(zero) <= 60.f;     // false for NaN
 }
 __device__ __forceinline__ uint4 int_asym_planar32_packed(const uint32_t* p, float rcp_s, float zero) {
-  const __nv_bfloat162 c192 = __floats2bfloat162_rn(192.f, 192.f), c0 = __floats2bfloat162_rn(0.f, 0.f),
-                       c15 = __floats2bfloat162_rn(15.f, 15.f), c128 = __floats2bfloat162_rn(128.f, 128.f),
-                       zm = __floats2bfloat162_rn(zero - 192.f, zero - 192.f);
-  const uint64_t rr = ((uint64_t)__float_as_uint(rcp_s) << 32) | __float_as_uint(rcp_s);
+  const __nv_bfloat162 c192 = __floats2bfloat162_rn(192.f, 192.f), c128 = __floats2bfloat162_rn(128.f, 128.f),
+                       c143 = __floats2bfloat162_rn(143.f, 143.f), zm = __floats2bfloat162_rn(zero - 64.f, zero - 64.f);
+  const uint64_t rr = twice_f32(rcp_s);
   uint32_t out[4];
 #pragma unroll
   for (int wd = 0; wd < 4; ++wd) {
-    uint32_t acc = 0;
+    uint32_t c[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int j = 4 * wd + k;
       const uint32_t a = p[j >> 1], b = p[8 + (j >> 1)];
-      const uint32_t fa = (j & 1) ? (a & 0xFFFF0000u) : (a << 16), fb = (j & 1) ? (b & 0xFFFF0000u) : (b << 16);
-      uint64_t q;
-      asm("{\n\t.reg .b64 x;\n\tmov.b64 x, {%1, %2};\n\tmul.rn.f32x2 %0, x, %3;\n\t}" : "=l"(q) : "r"(fa), "r"(fb), "l"(rr));
+      const uint64_t q = mul_f32x2((j & 1) ? (a & 0xFFFF0000u) : (a << 16), (j & 1) ? (b & 0xFFFF0000u) : (b << 16), rr);
       __nv_bfloat162 r = __floats2bfloat162_rn(__uint_as_float((uint32_t)q), __uint_as_float((uint32_t)(q >> 32)));
       r = __hadd2(__hadd2(r, c192), zm);
-      r = __hadd2(__hmin2(__hmax2(r, c0), c15), c128);
-      const uint32_t c = *reinterpret_cast<const uint32_t*>(&r) & 0x000F000Fu;
-      acc |= ((c & 0xFu) | (c >> 12)) << (8 * k);
+      r = __hmin2(__hmax2(r, c128), c143);               // a NaN gives way to 128: code 0
+      c[k] = *reinterpret_cast<const uint32_t*>(&r);
     }
-    out[wd] = acc;
+    out[wd] = planar_bytes(c);
   }
   return make_uint4(out[0], out[1], out[2], out[3]);
 }
-// largest and smallest of sixteen packed bf16 values
-__device__ __forceinline__ void minmax_bf16x16(const uint32_t* w, float& mx, float& mn) {
+// largest and smallest of 2 N packed bf16 values
+template <int N>
+__device__ __forceinline__ void minmax_bf16(const uint32_t* w, float& mx, float& mn) {
   __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&w[0]), lo = hi;
 #pragma unroll
-  for (int i = 1; i < 8; ++i) {
+  for (int i = 1; i < N; ++i) {
     const __nv_bfloat162 x = *reinterpret_cast<const __nv_bfloat162*>(&w[i]);
     hi = __hmax2(hi, x);
     lo = __hmin2(lo, x);
@@ -219,6 +227,7 @@ __device__ __forceinline__ void minmax_bf16x16(const uint32_t* w, float& mx, flo
   mx = fmaxf(mx, fmaxf(__uint_as_float(h << 16), __uint_as_float(h & 0xFFFF0000u)));
   mn = fminf(mn, fminf(__uint_as_float(l << 16), __uint_as_float(l & 0xFFFF0000u)));
 }
+__device__ __forceinline__ void minmax_bf16x16(const uint32_t* w, float& mx, float& mn) { minmax_bf16<8>(w, mx, mn); }
 // asymmetric: codes in [0, maxq]; returned as eight bytes in two words
 __device__ __forceinline__ uint2 int_asym_byte8_fast(const float* v, float s, float rcp_s, float zero, float maxq) {
   (void)s;
@@ -231,6 +240,52 @@ __device__ __forceinline__ uint2 int_asym_byte8_fast(const float* v, float s, fl
     w[j >> 2] |= (int_bits(q) & 0xFFu) << (8 * (j & 3));
   }
   return make_uint2(w[0], w[1]);
+}
+// The same from packed bf16 pairs, sixteen values (eight words) -> sixteen bytes in order.  Where quotients and zero point stay
+// within 512 (`packs`, int_asym_packs8), rint(q) is the low bits of q + 1.5 * 2^23, the zero point is added to it as an
+// integer, and the conversion saturates two sums at a time: the reference rounds a sum above 256 to bf16 before it clamps to
+// 255, which changes nothing.  Five instructions a value instead of twelve: 16384 x 12288 quantise-only 177 -> 136 us.  The
+// maximum sends a NaN to code 0.
+__device__ __forceinline__ bool int_asym_packs8(float mx, float mn, float rcp_s, float zero) {
+  return fmaxf(fabsf(mx), fabsf(mn)) * rcp_s <= 512.f && fabsf(zero) <= 512.f;   // false for NaN
+}
+__device__ __forceinline__ uint4 int_asym_byte16_packed(const uint32_t* p, float s, float rcp_s, float zero, bool packs) {
+  uint32_t out[4];
+  if (packs) {
+    const uint64_t rr = twice_f32(rcp_s);
+    const int32_t zi = (int32_t)zero - 0x4B400000;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      int32_t v[4];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const uint32_t a = p[2 * i + k];
+        const uint64_t q = mul_f32x2(a << 16, a & 0xFFFF0000u, rr);
+        const __nv_bfloat162 r = __floats2bfloat162_rn(__uint_as_float((uint32_t)q), __uint_as_float((uint32_t)(q >> 32)));
+        const uint32_t rb = *reinterpret_cast<const uint32_t*>(&r);
+        v[2 * k] = (int32_t)__float_as_uint(fmaxf(__uint_as_float(rb << 16) + 12582912.f, 12580864.f)) + zi;
+        v[2 * k + 1] = (int32_t)__float_as_uint(fmaxf(__uint_as_float(rb & 0xFFFF0000u) + 12582912.f, 12580864.f)) + zi;
+      }
+      uint32_t w;
+      asm("{\n\t.reg .b32 t;\n\tcvt.pack.sat.u8.s32.b32 t, %4, %3, 0;\n\tcvt.pack.sat.u8.s32.b32 %0, %2, %1, t;\n\t}"
+          : "=r"(w) : "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]));
+      out[i] = w;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        v[2 * k] = __uint_as_float(p[4 * i + k] << 16);
+        v[2 * k + 1] = __uint_as_float(p[4 * i + k] & 0xFFFF0000u);
+      }
+      const uint2 b = int_asym_byte8_fast(v, s, rcp_s, zero, 255.f);
+      out[2 * i] = b.x;
+      out[2 * i + 1] = b.y;
+    }
+  }
+  return make_uint4(out[0], out[1], out[2], out[3]);
 }
 // Planar-32 codes of any asymmetric group, `packs` = int_asym_packs of the group: one value at a time where the packed
 // rounding does not hold.  The test costs the quantise-only kernel 1 % (16384 x 12288 129.0 -> 130.8 us).
@@ -405,6 +460,73 @@ __device__ __forceinline__ float amax_bf16x16(const uint32_t* w) {
     m = *reinterpret_cast<const uint32_t*>(&x);
   }
   return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u));
+}
+
+// the same, NaN where one of them is
+__device__ __forceinline__ float amax_nan_bf16x16(const uint32_t* w) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t a = w[i] & 0x7FFF7FFFu;
+    const __nv_bfloat162 x = __hmax2_nan(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&m));
+    m = *reinterpret_cast<const uint32_t*>(&x);
+  }
+  const uint32_t o = __byte_perm(m, m, 0x1032);
+  const __nv_bfloat162 x = __hmax2_nan(*reinterpret_cast<const __nv_bfloat162*>(&m), *reinterpret_cast<const __nv_bfloat162*>(&o));
+  return __uint_as_float(*reinterpret_cast<const uint32_t*>(&x) << 16);
+}
+
+// A whole group under a power-of-two tensor scale (nvfp4_pow2_tensor_scale): scale byte and sixteen codes from eight words of
+// packed bf16 pairs, by the hardware's conversion to E2M1 pairs.  It rounds ties to even, the reference to the lower value
+// (toward -inf, no negative zero).  With p = thr * eff of at most 7 significant bits and |x| of 8, |x| / eff is equal to a threshold or at
+// least 2^-8 thr >= 2^-10 away from it, and fl32(x * fl32(1 / eff)) is off by less than 2^-19; so subtracting 2^-14 -- in the
+// multiply's own rounding, an FMA -- turns every tie toward -inf and moves nothing else across a threshold.  What comes out as a
+// negative zero (zero itself among it) is cleared.  Three instructions a value where seven compares and their count took
+// eleven to twelve: 16384 x 12288 quantise-only 141 -> 112 us, rotation of 32768 x 1152 69.2 -> 65.1.  Groups with infinities or NaN, and tensor scales outside 2^-60 .. 2^60, keep the compares.
+static __device__ __noinline__ uint2 nvfp4_hw_group_compare(uint4 a, uint4 b, float eff) {
+  const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  return nvfp4_hw_group_packed(w, eff);
+}
+__device__ __forceinline__ uint8_t nvfp4_hw_group(const uint32_t* w, float clip, float T, uint2& codes) {
+  float eff = 0.f;
+  codes = make_uint2(0u, 0u);
+  const float amax = amax_nan_bf16x16(w);
+  const uint32_t tb = __float_as_uint(T);
+  if (amax < INFINITY && tb >= 0x21800000u && tb <= 0x5D800000u) {
+    if (amax == 0.f) return 0;
+    // nvfp4_hw_scale with the division by a power of two as a multiplication
+    const float r = fminf(fmaxf(__fmul_rn(__fdiv_rn(__fmul_rn(amax, clip), 6.f), __uint_as_float(0x7F000000u - tb)), 0.001953125f), 448.f);
+    const uint8_t sb = (uint8_t)__nv_cvt_float_to_fp8(r, __NV_SATFINITE, __NV_E4M3);
+    eff = __fmul_rn(e4m3_to_float(sb), T);
+    const uint64_t rr = twice_f32(__frcp_rn(eff)), nudge = twice_f32(-0x1p-14f);
+    uint32_t out[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t f[8];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        uint64_t q;
+        asm("{\n\t.reg .b64 x;\n\tmov.b64 x, {%1, %2};\n\tfma.rn.f32x2 %0, x, %3, %4;\n\t}"
+            : "=l"(q) : "r"(w[4 * h + k] << 16), "r"(w[4 * h + k] & 0xFFFF0000u), "l"(rr), "l"(nudge));
+        f[2 * k] = (uint32_t)q;
+        f[2 * k + 1] = (uint32_t)(q >> 32);
+      }
+      uint32_t c;
+      asm("{\n\t.reg .b8 b0, b1, b2, b3;\n\t"
+          "cvt.rn.satfinite.e2m1x2.f32 b0, %2, %1;\n\tcvt.rn.satfinite.e2m1x2.f32 b1, %4, %3;\n\t"
+          "cvt.rn.satfinite.e2m1x2.f32 b2, %6, %5;\n\tcvt.rn.satfinite.e2m1x2.f32 b3, %8, %7;\n\t"
+          "mov.b32 %0, {b0, b1, b2, b3};\n\t}"
+          : "=r"(c)
+          : "f"(__uint_as_float(f[0])), "f"(__uint_as_float(f[1])), "f"(__uint_as_float(f[2])), "f"(__uint_as_float(f[3])),
+            "f"(__uint_as_float(f[4])), "f"(__uint_as_float(f[5])), "f"(__uint_as_float(f[6])), "f"(__uint_as_float(f[7])));
+      out[h] = c & (((c & 0x77777777u) + 0x77777777u) | 0x77777777u);
+    }
+    codes = make_uint2(out[0], out[1]);
+    return sb;
+  }
+  const uint8_t sb = nvfp4_hw_scale(amax_bf16x16(w), clip, T, &eff);
+  if (eff > 0.f) codes = nvfp4_hw_group_compare(make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]), eff);
+  return sb;
 }
 
 }  // namespace dq

@@ -126,10 +126,10 @@ __global__ void __launch_bounds__(256) quant_int_kernel(const QuantArgs a) {
   const int c0 = src_col(g, grp, e0);
   const bool vec_ok = (a.perm == nullptr) && ((c0 & 7) == 0) && ((a.x_pitch & 7) == 0) &&
                       ((reinterpret_cast<uintptr_t>(a.x) & 15) == 0) && (c0 + 32 <= g.D);
-  // Whole groups of a 4-bit layer (the common case) stay on the packed bf16 pairs as loaded: extrema by packed max / min,
-  // codes by int_sym_planar32_packed / int_asym_planar32, no conversion to fp32 beyond the multiply.  The choice is the same for
-  // every thread of a group; the shuffles below run outside it, on all lanes of the warp.
-  const bool packed_path = (MODE == MODE_INT4_SYM || MODE == MODE_INT4_ASYM) && vec_ok && glen == 64 * g.cpg;
+  // Whole groups (the common case) stay on the packed bf16 pairs as loaded: extrema by packed max / min, codes by
+  // int_sym_planar32_packed, int_asym_planar32 or int_asym_byte16_packed, no conversion to fp32 beyond the multiply.  The choice is
+  // the same for every thread of a group; the shuffles below run outside it, on all lanes of the warp.
+  const bool packed_path = vec_ok && glen == 64 * g.cpg;
   uint32_t w[16];
   float mx = -INFINITY, mn = INFINITY;
   if (packed_path) {
@@ -191,9 +191,16 @@ __global__ void __launch_bounds__(256) quant_int_kernel(const QuantArgs a) {
   if (!live) return;
   if (packed_path) {
     const float rcp = __frcp_rn(p.scale);
-    *reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)b * 16) =
-        (MODE == MODE_INT4_SYM) ? int_sym_planar32_packed(w, rcp, g.clip < 1.f)
-                                : int_asym_planar32(w, p.scale, rcp, p.zero, int_asym_packs(mx, mn, rcp, p.zero));
+    if constexpr (MODE == MODE_INT8_ASYM) {
+      uint4* dst = reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)b * 32);
+      const bool packs = int_asym_packs8(mx, mn, rcp, p.zero);
+      dst[0] = int_asym_byte16_packed(w, p.scale, rcp, p.zero, packs);
+      dst[1] = int_asym_byte16_packed(w + 8, p.scale, rcp, p.zero, packs);
+    } else {
+      *reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)b * 16) =
+          (MODE == MODE_INT4_SYM) ? int_sym_planar32_packed(w, rcp, g.clip < 1.f)
+                                  : int_asym_planar32(w, p.scale, rcp, p.zero, int_asym_packs(mx, mn, rcp, p.zero));
+    }
   } else if (nvalid == 32) {
     // full block: the division-free exact forms (reciprocal multiply, see quant_math.cuh)
     const float rcp = __frcp_rn(p.scale);
@@ -300,7 +307,7 @@ __global__ void __launch_bounds__(256) quant_nvfp4_kernel(const QuantArgs a) {
   uint32_t sfw = 0;
   if constexpr (MODE == MODE_NVFP4_HW) {
     // whole chunk inside the quantised region, 16-byte aligned, power-of-two tensor scale: everything on packed bf16
-    // pairs as loaded, no conversion to fp32 (see nvfp4_hw_group_packed)
+    // pairs as loaded (see nvfp4_hw_group)
     if (a.perm == nullptr && (a.x_pitch & 7) == 0 && c0 + 64 <= g.q_len && (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 &&
         nvfp4_pow2_tensor_scale(g.T)) {
       uint32_t w[32];
@@ -311,10 +318,8 @@ __global__ void __launch_bounds__(256) quant_nvfp4_kernel(const QuantArgs a) {
       }
 #pragma unroll
       for (int gi = 0; gi < 4; ++gi) {
-        float eff;
-        const uint8_t sb = nvfp4_hw_scale(amax_bf16x16(w + 8 * gi), g.clip, g.T, &eff);
-        uint2 c = make_uint2(0u, 0u);
-        if (eff > 0.f) c = nvfp4_hw_group_packed(w + 8 * gi, eff);
+        uint2 c;
+        const uint8_t sb = nvfp4_hw_group(w + 8 * gi, g.clip, g.T, c);
         packed[2 * gi] = c.x;
         packed[2 * gi + 1] = c.y;
         sfw |= (uint32_t)sb << (8 * gi);

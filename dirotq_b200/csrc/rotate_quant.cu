@@ -45,12 +45,15 @@ template <bool PAIR> struct RqStage {
 #ifndef RQ_WPQ_PERHEAD
 #define RQ_WPQ_PERHEAD 4
 #endif
+constexpr int RQ_TAIL_STAGED = 16;              // high channels per head that go through the staging patch, at most
 template <int EPI, bool PAIR = false> struct RqCfg {
   static constexpr int WPQ = (EPI == 2 /* EPI_NVFP4_HIDDEN */) ? RQ_WPQ_NVFP4 : (EPI == 3 || EPI == 4 /* per-head */) ? RQ_WPQ_PERHEAD : 2;
   static constexpr int EPI_WARPS = 4 * WPQ;
   static constexpr int THREADS = (2 + EPI_WARPS) * 32;
-  // plain-GEMM epilogue (EPI_ROT_ONLY = 0): a 32 x 32 bf16 staging patch per epilogue warp for its TMA stores
-  static constexpr int STG_BYTES = (EPI == 0) ? EPI_WARPS * 2048 : 0;
+  // per epilogue warp: EPI_ROT_ONLY (0) a 32 x 32 bf16 staging patch for its TMA stores, EPI_INT_PERHEAD (3) the high
+  // channels of a head of its 32 rows
+  static constexpr int STG_WARP = EPI == 0 ? 2048 : EPI == 3 ? 32 * RQ_TAIL_STAGED * 2 : 0;
+  static constexpr int STG_BYTES = EPI_WARPS * STG_WARP;
   static constexpr int SMEM_BYTES = RqStage<PAIR>::STAGES * RqStage<PAIR>::STAGE_BYTES + STG_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
 
@@ -72,17 +75,15 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-// 32 code slots -> 16 bytes; byte j = slot j | slot 16+j << 4
-__device__ __forceinline__ uint4 pack_planar32(const uint32_t* q) {
-  uint32_t w[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint32_t x = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) x |= ((q[4 * i + j] & 0xF) | ((q[16 + 4 * i + j] & 0xF) << 4)) << (8 * j);
-    w[i] = x;
+// 32 bytes of codes of one row: a whole sector in one store where the code buffer starts on a sector (rows are multiples of
+// 32 bytes).  Lanes hold different rows, so a store is one request per lane whatever its width.
+__device__ __forceinline__ void store_codes32(uint8_t* dst, bool whole, uint4 lo, uint4 hi) {
+  if (whole) {
+    st_global_32(dst, lo, hi);
+  } else {
+    reinterpret_cast<uint4*>(dst)[0] = lo;
+    reinterpret_cast<uint4*>(dst)[1] = hi;
   }
-  return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // ---- epilogues: thread = one row of the tile; `taddr` already points at this warp's lanes.
@@ -93,7 +94,7 @@ __device__ __forceinline__ uint4 pack_planar32(const uint32_t* q) {
 template <int MODE>
 __device__ __forceinline__ void epi_int_hidden(const RotArgs& a, uint32_t taddr, int64_t row, int n0, int half, uint32_t& turn, int wpq = 2) {
   const ActGeom& g = a.g;
-  const bool row_ok = row < a.M;
+  const bool row_ok = row < a.M, whole = (reinterpret_cast<uintptr_t>(a.codes) & 31) == 0;
   constexpr float maxq = (MODE == MODE_INT4_SYM) ? 7.f : (MODE == MODE_INT4_ASYM ? 15.f : 255.f);
   for (int c0 = 0; c0 < a.BN; c0 += 64) {
     const int col = n0 + c0;
@@ -143,28 +144,21 @@ __device__ __forceinline__ void epi_int_hidden(const RotArgs& a, uint32_t taddr,
     else p = int_asym_params<true>(mx, mn, g.clip, maxq);
     const float rcp = __frcp_rn(p.scale);
     if (!row_ok) continue;
-    auto val = [&](int j) { return __uint_as_float((j & 1) ? xb[j >> 1] & 0xFFFF0000u : xb[j >> 1] << 16); };
     if constexpr (MODE == MODE_INT4_SYM) {
-      uint4* dst = reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)chunk * 32);
       const bool clamp = g.clip < 1.f || !(p.scale < INFINITY);      // else no quotient passes 7.03
-      dst[0] = int_sym_planar32_packed(xb, rcp, clamp);
-      dst[1] = int_sym_planar32_packed(xb + 16, rcp, clamp);
+      store_codes32(a.codes + row * g.code_row_bytes + (int64_t)chunk * 32, whole, int_sym_planar32_packed(xb, rcp, clamp),
+                    int_sym_planar32_packed(xb + 16, rcp, clamp));
     } else if constexpr (MODE == MODE_INT4_ASYM) {
-      uint4* dst = reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)chunk * 32);
       const bool packs = int_asym_packs(mx, mn, rcp, p.zero);
-      dst[0] = int_asym_planar32(xb, p.scale, rcp, p.zero, packs);
-      dst[1] = int_asym_planar32(xb + 16, p.scale, rcp, p.zero, packs);
+      store_codes32(a.codes + row * g.code_row_bytes + (int64_t)chunk * 32, whole, int_asym_planar32(xb, p.scale, rcp, p.zero, packs),
+                    int_asym_planar32(xb + 16, p.scale, rcp, p.zero, packs));
     } else {
-      uint4* dst = reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)chunk * 64);
+      uint8_t* dst = a.codes + row * g.code_row_bytes + (int64_t)chunk * 64;
+      const bool packs = int_asym_packs8(mx, mn, rcp, p.zero);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        float v16[16];
-#pragma unroll
-        for (int e = 0; e < 16; ++e) v16[e] = val(16 * i + e);
-        const uint2 b0 = int_asym_byte8_fast(v16, p.scale, rcp, p.zero, maxq);
-        const uint2 b1 = int_asym_byte8_fast(v16 + 8, p.scale, rcp, p.zero, maxq);
-        dst[i] = make_uint4(b0.x, b0.y, b1.x, b1.y);
-      }
+      for (int i = 0; i < 2; ++i)
+        store_codes32(dst + 32 * i, whole, int_asym_byte16_packed(xb + 16 * i, p.scale, rcp, p.zero, packs),
+                      int_asym_byte16_packed(xb + 16 * i + 8, p.scale, rcp, p.zero, packs));
     }
     a.scales[(int64_t)chunk * a.ldm + row] = __float2bfloat16_rn(p.scale);
     if constexpr (MODE != MODE_INT4_SYM) a.zeros[(int64_t)chunk * a.ldm + row] = __float2bfloat16_rn(p.zero);
@@ -188,11 +182,33 @@ __device__ __forceinline__ void epi_nvfp4_hidden(const RotArgs& a, uint32_t tadd
     const int nq = max(0, min(64, g.q_len - col));
     const int chunk = col >> 6;
     uint32_t sfw = 0;
+    if constexpr (MODE == MODE_NVFP4_HW) {
+      if (nq == 64 && pow2_T && a.codes && !a.x_rot) {
+        // a whole chunk under a power-of-two tensor scale: two groups at a time on packed pairs (nvfp4_hw_group)
+#pragma unroll 1
+        for (int gp = 0; gp < 2; ++gp) {
+          uint32_t r[32];
+          __syncwarp();                           // lanes may have quantised the groups before in different ways
+          tmem_ld32(taddr + c0 + 32 * gp, r);
+          tmem_wait_ld();
+          uint32_t w[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) w[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+          uint2 k0, k1;
+          const uint32_t s0 = nvfp4_hw_group(w, g.clip, g.T, k0), s1 = nvfp4_hw_group(w + 8, g.clip, g.T, k1);
+          sfw |= (s0 | s1 << 8) << (16 * gp);
+          if (row_ok) *reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)chunk * 32 + gp * 16) = make_uint4(k0.x, k0.y, k1.x, k1.y);
+        }
+        if (row_ok) *reinterpret_cast<uint32_t*>(a.sf + sf_offset(row, chunk * 4, n_kb64_pad)) = sfw;
+        continue;
+      }
+    }
 #pragma unroll 1
     for (int gi = 0; gi < 4; ++gi) {
       const int gcol = col + 16 * gi;
       if (gcol >= g.D) break;
       uint32_t r[16];
+      __syncwarp();
       tmem_ld16(taddr + c0 + 16 * gi, r);
       tmem_wait_ld();
       // the rotated values, rounded to bf16 and packed in pairs: what the quantiser is defined on
@@ -209,11 +225,9 @@ __device__ __forceinline__ void epi_nvfp4_hidden(const RotArgs& a, uint32_t tadd
       const int nvalid = max(0, min(16, nq - 16 * gi));
       if constexpr (MODE == MODE_NVFP4_HW) {
         if (nvalid == 16 && pow2_T) {
-          // whole group, power-of-two tensor scale: decided on the packed pairs (nvfp4_hw_group_packed)
-          float eff = 0.f;
-          const uint8_t sb = nvfp4_hw_scale(amax_bf16x16(w), g.clip, g.T, &eff);
-          uint2 c = make_uint2(0u, 0u);
-          if (eff > 0.f) c = nvfp4_hw_group_packed(w, eff);
+          // whole group, power-of-two tensor scale
+          uint2 c;
+          const uint8_t sb = nvfp4_hw_group(w, g.clip, g.T, c);
           sfw |= (uint32_t)sb << (8 * gi);
           if (row_ok) *reinterpret_cast<uint2*>(a.codes + row * g.code_row_bytes + (int64_t)chunk * 32 + gi * 8) = c;
           continue;
@@ -280,43 +294,137 @@ __device__ __forceinline__ void epi_nvfp4_hidden(const RotArgs& a, uint32_t tadd
   }
 }
 
-// 32 columns starting at a column that is only 8-aligned (heads of 72 channels): four
-// naturally aligned 8-column reads, one wait.
-__device__ __forceinline__ void ld32_by8(uint32_t taddr, uint32_t* r) {
-  __syncwarp();                                   // lanes may have quantised the block before in different ways
-  tmem_ld8(taddr, r);
-  tmem_ld8(taddr + 8, r + 8);
-  tmem_ld8(taddr + 16, r + 16);
-  tmem_ld8(taddr + 24, r + 24);
-  tmem_wait_ld();
-}
-
-// Planar-32 codes (byte j = slots j and 16 + j): the nibbles of the first nv slots.
-__device__ __forceinline__ uint4 planar32_valid_mask(int nv) {
-  const int nlo = min(nv, 16), nhi = max(nv - 16, 0);
-  uint32_t w[4];
-#pragma unroll
-  for (int wd = 0; wd < 4; ++wd) {
-    const int lc = min(max(nlo - 4 * wd, 0), 4), hc = min(max(nhi - 4 * wd, 0), 4);
-    const uint32_t lm = lc == 4 ? 0xFFFFFFFFu : ((1u << (8 * lc)) - 1u), hm = hc == 4 ? 0xFFFFFFFFu : ((1u << (8 * hc)) - 1u);
-    w[wd] = (0x0F0F0F0Fu & lm) | (0xF0F0F0F0u & hm);
-  }
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
-// Per-head layout: head h = tile columns [hh*d, hh*d + d): first d_q quantised as ONE group,
-// last hlen passthrough.  Two passes over TMEM (extrema, then codes) keep registers small.
-template <int MODE>
-__device__ __forceinline__ void epi_int_perhead(const RotArgs& a, uint32_t taddr, int64_t row, int n0, int half, uint32_t& turn, int wpq = 2) {
+// Per-head layout: head h = tile columns [hh*d, hh*d + d): first d_q quantised as ONE group, last hlen passthrough.
+// What bounds it are this epilogue's instructions and, where a head's high channels are an odd number of 2-byte stores, their
+// requests (a lane is a row: every store is one request per lane).  So: bf16 pairs throughout, the ragged last block handled with
+// masks from the launch's arguments, a whole code sector per store, and odd tails through a patch of shared memory, so that
+// consecutive lanes store consecutive channels.  A group of at most two blocks of 32 keeps its words between extrema and codes;
+// a longer one reads tensor memory twice.  Us, before and now: 32768 x 16 heads of 72 (9 high) 61.4 / 36.9, 16384 x 70 of 32 (4 high)
+// 51.6 / 35.2, in 8 bits 75.4 / 40.6, 18432 x 24 of 128 (16 high) 47.1 / 41.4, NVFP4 63.5 / 49.6; floors by bytes 15 to 25.
+// NB: blocks of 32 slots of a group (1, 2; 0 = any number)
+template <int MODE, int NB>
+__device__ __forceinline__ void perhead_group(const RotArgs& a, uint32_t tcol, int64_t row, bool row_ok, int h, bool whole) {
   const ActGeom& g = a.g;
-  const bool row_ok = row < a.M;
   constexpr float maxq = (MODE == MODE_INT4_SYM) ? 7.f : (MODE == MODE_INT4_ASYM ? 15.f : 255.f);
+  const int nblk = NB ? NB : (g.group + 31) >> 5;
+  const bool wide = (g.d & 31) == 0;
+  uint32_t pw[NB == 2 ? 32 : 16];
+  auto load_block = [&](int b, uint32_t* p) {
+    uint32_t r[32];
+    __syncwarp();                                 // lanes may have quantised the block before in different ways
+    if (wide) {
+      tmem_ld32(tcol + 32 * b, r);
+    } else {                                      // columns that are only 8-aligned (heads of 72 channels)
+      tmem_ld8(tcol + 32 * b, r);
+      tmem_ld8(tcol + 32 * b + 8, r + 8);
+      tmem_ld8(tcol + 32 * b + 16, r + 16);
+      tmem_ld8(tcol + 32 * b + 24, r + 24);
+    }
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) p[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));   // the rounding of x_rot
+  };
+  float mx = -INFINITY, mn = INFINITY;
+  auto extrema = [&](const uint32_t* p, bool last) {
+    if (!last || !a.ragged) {
+      minmax_bf16<16>(p, mx, mn);
+    } else {
+      const uint32_t fill = __byte_perm(p[0], p[0], 0x1010);          // slot 0 of the block (always valid) twice
+      uint32_t pm[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) pm[i] = (p[i] & a.pair_mask[i]) | (fill & ~a.pair_mask[i]);
+      minmax_bf16<16>(pm, mx, mn);
+    }
+  };
+  if constexpr (NB == 1) {
+    load_block(0, pw);
+    extrema(pw, true);
+  } else if constexpr (NB == 2) {
+    load_block(0, pw);
+    load_block(1, pw + 16);
+    extrema(pw, false);
+    extrema(pw + 16, true);
+  } else {
+#pragma unroll 1
+    for (int b = 0; b < nblk; ++b) {
+      load_block(b, pw);
+      extrema(pw, b + 1 == nblk);
+    }
+  }
+  GroupParams p;
+  if constexpr (MODE == MODE_INT4_SYM) p = int_sym_params<true>(mx, mn, g.clip, maxq);
+  else p = int_asym_params<true>(mx, mn, g.clip, maxq);
+  const float rcp = __frcp_rn(p.scale);
+  const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
+  if constexpr (MODE != MODE_INT8_ASYM) {
+    const bool packs = MODE == MODE_INT4_SYM ? g.clip < 1.f : int_asym_packs(mx, mn, rcp, p.zero);
+    auto codes = [&](const uint32_t* w, bool last) {
+      uint4 c;
+      if constexpr (MODE == MODE_INT4_SYM) c = int_sym_planar32_packed(w, rcp, packs);
+      else c = int_asym_planar32(w, p.scale, rcp, p.zero, packs);
+      if (last && a.ragged) c = make_uint4(c.x & a.code_mask[0], c.y & a.code_mask[1], c.z & a.code_mask[2], c.w & a.code_mask[3]);
+      return c;
+    };
+    uint8_t* dst = a.codes + row * g.code_row_bytes + (int64_t)h * g.cpg * 32;
+    if constexpr (NB != 0) {
+      const uint4 c0 = codes(pw, NB == 1), c1 = NB == 2 ? codes(pw + 16, true) : z4;
+      if (row_ok) store_codes32(dst, whole, c0, c1);
+    } else {
+#pragma unroll 1
+      for (int c = 0; c < g.cpg; ++c) {
+        load_block(2 * c, pw);
+        const uint4 c0 = codes(pw, 2 * c + 1 == nblk);
+        uint4 c1 = z4;
+        if (2 * c + 1 < nblk) {
+          load_block(2 * c + 1, pw);
+          c1 = codes(pw, 2 * c + 2 == nblk);
+        }
+        if (row_ok) store_codes32(dst + 32 * c, whole, c0, c1);
+      }
+    }
+  } else {
+    const bool packs = int_asym_packs8(mx, mn, rcp, p.zero);
+    uint8_t* dst = a.codes + row * g.code_row_bytes + (int64_t)h * g.cpg * 64;
+    auto put = [&](int b, const uint32_t* w, bool last) {
+      uint4 c0 = int_asym_byte16_packed(w, p.scale, rcp, p.zero, packs), c1 = int_asym_byte16_packed(w + 8, p.scale, rcp, p.zero, packs);
+      if (last && a.ragged) {
+        c0 = make_uint4(c0.x & a.code_mask[0], c0.y & a.code_mask[1], c0.z & a.code_mask[2], c0.w & a.code_mask[3]);
+        c1 = make_uint4(c1.x & a.code_mask[4], c1.y & a.code_mask[5], c1.z & a.code_mask[6], c1.w & a.code_mask[7]);
+      }
+      if (row_ok) store_codes32(dst + 32 * b, whole, c0, c1);
+    };
+    if constexpr (NB != 0) {
+      put(0, pw, NB == 1);
+      if constexpr (NB == 2) put(1, pw + 16, true);
+    } else {
+#pragma unroll 1
+      for (int b = 0; b < nblk; ++b) {
+        load_block(b, pw);
+        put(b, pw, b + 1 == nblk);
+      }
+    }
+    if (row_ok)
+      for (int b = nblk; b < 2 * g.cpg; ++b) store_codes32(dst + 32 * b, whole, z4, z4);
+  }
+  if (row_ok) {
+    for (int c = 0; c < g.cpg; ++c) {
+      a.scales[(int64_t)(h * g.cpg + c) * a.ldm + row] = __float2bfloat16_rn(p.scale);
+      if constexpr (MODE != MODE_INT4_SYM) a.zeros[(int64_t)(h * g.cpg + c) * a.ldm + row] = __float2bfloat16_rn(p.zero);
+    }
+  }
+}
+
+template <int MODE>
+__device__ __forceinline__ void epi_int_perhead(const RotArgs& a, uint32_t taddr, int64_t row, int lane, int n0, int half, uint32_t& turn,
+                                                uint32_t stg) {
+  const ActGeom& g = a.g;
+  const bool row_ok = row < a.M, whole = (reinterpret_cast<uintptr_t>(a.codes) & 31) == 0;
+  constexpr uint32_t WPQ = RqCfg<EPI_INT_PERHEAD>::WPQ;
   const int d = g.d, d_q = g.group;
-  const int nblk = (d_q + 31) >> 5;
-  for (int cb = 0; cb < a.BN; cb += d) {
-    const int h = (n0 + cb) / d;
-    if (h >= g.H) break;
-    if (((turn++) % (uint32_t)wpq) != (uint32_t)half) continue;
+  const bool staged = g.hlen <= RQ_TAIL_STAGED && ((g.hlen | g.tail_pitch) & 3) != 0;
+  int h = n0 / d;
+  for (int cb = 0; cb < a.BN && h < g.H; cb += d, ++h) {
+    if (((turn++) % WPQ) != (uint32_t)half) continue;
     if (a.x_rot) {
       for (int c8 = 0; c8 < d; c8 += 8) {
         uint32_t r[8];
@@ -331,130 +439,51 @@ __device__ __forceinline__ void epi_int_perhead(const RotArgs& a, uint32_t taddr
       }
     }
     if (!a.codes) continue;
-    float mx = -INFINITY, mn = INFINITY;
-    GroupParams p;
-    if constexpr (MODE != MODE_INT8_ASYM) {
-      // 4-bit modes, on packed bf16 pairs: a block of 32 columns becomes 16 words (one conversion per pair = the bf16
-      // rounding of x_rot), the extrema are packed min / max, the codes come out in the planar layout directly
-      // (quant_math.cuh).  A ragged last block takes part with its invalid slots replaced (extrema) or cleared (codes).
-      // A head of one block (SANA: 28 of 32 columns) keeps its words between the two passes.
-      uint32_t pw[16];
-      for (int b = 0; b < nblk; ++b) {
-        uint32_t r[32];
-        ld32_by8(taddr + cb + 32 * b, r);
+    if (d_q <= 32) perhead_group<MODE, 1>(a, taddr + cb, row, row_ok, h, whole);
+    else if (d_q <= 64) perhead_group<MODE, 2>(a, taddr + cb, row, row_ok, h, whole);
+    else perhead_group<MODE, 0>(a, taddr + cb, row, row_ok, h, whole);
+    if (!a.tail) continue;
+#pragma unroll 1
+    for (int c8 = d_q & ~7; c8 < d; c8 += 8) {
+      uint32_t r[8];
+      __syncwarp();
+      tmem_ld8(taddr + cb + c8, r);
+      tmem_wait_ld();
+      const int t0 = c8 - d_q;                                  // tail index of r[0] within the head (may be negative)
+      if (staged) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) pw[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-        const int nv = min(32, d_q - 32 * b);
-        if (nv == 32) {
-          minmax_bf16x16(pw, mx, mn);
-          minmax_bf16x16(pw + 8, mx, mn);
+        for (int j = 0; j < 8; ++j)
+          if (t0 + j >= 0)
+            asm volatile("st.shared.u16 [%0], %1;" ::"r"(stg + (uint32_t)(lane * g.hlen + t0 + j) * 2),
+                         "h"(__bfloat16_as_ushort(__float2bfloat16_rn(__uint_as_float(r[j])))) : "memory");
+      } else if (row_ok) {
+        __nv_bfloat16* tr = a.tail + row * g.tail_pitch + h * g.hlen;
+        if (t0 >= 0 && ((t0 | g.hlen | g.tail_pitch) & 7) == 0) {        // a whole, 16-byte aligned octet of tail channels
+          *reinterpret_cast<uint4*>(tr + t0) =
+              make_uint4(pack_bf16x2(__uint_as_float(r[0]), __uint_as_float(r[1])), pack_bf16x2(__uint_as_float(r[2]), __uint_as_float(r[3])),
+                         pack_bf16x2(__uint_as_float(r[4]), __uint_as_float(r[5])), pack_bf16x2(__uint_as_float(r[6]), __uint_as_float(r[7])));
+        } else if (t0 == -4 && ((g.hlen | g.tail_pitch) & 3) == 0) {     // the octet's upper half starts the head's tail
+          *reinterpret_cast<uint2*>(tr) = make_uint2(pack_bf16x2(__uint_as_float(r[4]), __uint_as_float(r[5])),
+                                                     pack_bf16x2(__uint_as_float(r[6]), __uint_as_float(r[7])));
         } else {
-          const uint32_t fill = (pw[0] << 16) | (pw[0] & 0xFFFFu);      // slot 0 of the block (always valid) twice
-          uint32_t pm[16];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const uint32_t vm = (2 * i + 1 < nv) ? 0xFFFFFFFFu : ((2 * i < nv) ? 0x0000FFFFu : 0u);
-            pm[i] = (pw[i] & vm) | (fill & ~vm);
-          }
-          minmax_bf16x16(pm, mx, mn);
-          minmax_bf16x16(pm + 8, mx, mn);
+          for (int j = 0; j < 8; ++j)
+            if (t0 + j >= 0) tr[t0 + j] = __float2bfloat16_rn(__uint_as_float(r[j]));
         }
-      }
-      if constexpr (MODE == MODE_INT4_SYM) p = int_sym_params<true>(mx, mn, g.clip, maxq);
-      else p = int_asym_params<true>(mx, mn, g.clip, maxq);
-      const float rcp = __frcp_rn(p.scale);
-      for (int b = 0; b < 2 * g.cpg; ++b) {
-        uint4 c4 = make_uint4(0u, 0u, 0u, 0u);
-        if (b < nblk) {
-          if (nblk > 1) {
-            uint32_t r[32];
-            ld32_by8(taddr + cb + 32 * b, r);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) pw[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-          }
-          if constexpr (MODE == MODE_INT4_SYM) c4 = int_sym_planar32_packed(pw, rcp, g.clip < 1.f);
-          else c4 = int_asym_planar32(pw, p.scale, rcp, p.zero, int_asym_packs(mx, mn, rcp, p.zero));
-          const int nv = d_q - 32 * b;
-          if (nv < 32) {
-            const uint4 m4 = planar32_valid_mask(nv);
-            c4 = make_uint4(c4.x & m4.x, c4.y & m4.y, c4.z & m4.z, c4.w & m4.w);
-          }
-        }
-        if (row_ok)
-          *reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + ((int64_t)h * g.cpg * 64 + 32 * b) / 2) = c4;
-      }
-    } else {
-    for (int b = 0; b < nblk; ++b) {
-      uint32_t r[32];
-      ld32_by8(taddr + cb + 32 * b, r);
-#pragma unroll
-      for (int j = 0; j < 32; ++j)
-        if (32 * b + j < d_q) {
-          float f = rnd<true>(__uint_as_float(r[j]));
-          mx = fmaxf(mx, f);
-          mn = fminf(mn, f);
-        }
-    }
-    p = int_asym_params<true>(mx, mn, g.clip, maxq);
-    const float rcp = __frcp_rn(p.scale);
-    for (int b = 0; b < 2 * g.cpg; ++b) {
-      // 8-bit mode: eight codes per pair of words by the division-free exact form (guarded reciprocal, quant_math.cuh);
-      // an octet that straddles the end of the group is computed whole and its invalid bytes cleared
-      uint2 b8[4] = {make_uint2(0u, 0u), make_uint2(0u, 0u), make_uint2(0u, 0u), make_uint2(0u, 0u)};
-      if (b < nblk) {
-        uint32_t r[32];
-        ld32_by8(taddr + cb + 32 * b, r);
-        float f[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) f[j] = rnd<true>(__uint_as_float(r[j]));
-#pragma unroll
-        for (int o = 0; o < 4; ++o) {
-          const int nvo = d_q - (32 * b + 8 * o);                // valid values of this octet
-          if (nvo > 0) {
-            b8[o] = int_asym_byte8_fast(f + 8 * o, p.scale, rcp, p.zero, maxq);
-            if (nvo < 8) {
-              const uint32_t lo_m = nvo >= 4 ? 0xFFFFFFFFu : ((1u << (8 * nvo)) - 1u);
-              const uint32_t hi_m = nvo > 4 ? ((1u << (8 * (nvo - 4))) - 1u) : 0u;
-              b8[o] = make_uint2(b8[o].x & lo_m, b8[o].y & hi_m);
-            }
-          }
-        }
-      }
-      if (row_ok) {
-        uint4* dst = reinterpret_cast<uint4*>(a.codes + row * g.code_row_bytes + (int64_t)h * g.cpg * 64 + 32 * b);
-        dst[0] = make_uint4(b8[0].x, b8[0].y, b8[1].x, b8[1].y);
-        dst[1] = make_uint4(b8[2].x, b8[2].y, b8[3].x, b8[3].y);
       }
     }
-    }
-    if (row_ok) {
-      for (int c = 0; c < g.cpg; ++c) {
-        a.scales[(int64_t)(h * g.cpg + c) * a.ldm + row] = __float2bfloat16_rn(p.scale);
-        if constexpr (MODE != MODE_INT4_SYM) a.zeros[(int64_t)(h * g.cpg + c) * a.ldm + row] = __float2bfloat16_rn(p.zero);
-      }
-    }
-    if (a.tail) {
-      for (int c8 = d_q & ~7; c8 < d; c8 += 8) {
-        uint32_t r[8];
-        __syncwarp();
-        tmem_ld8(taddr + cb + c8, r);
-        tmem_wait_ld();
-        if (row_ok) {
-          __nv_bfloat16* tr = a.tail + row * g.tail_pitch + h * g.hlen;
-          const int t0 = c8 - d_q;                                  // tail index of r[0] within the head (may be negative)
-          if (t0 >= 0 && ((t0 | g.hlen | g.tail_pitch) & 7) == 0) {        // a whole, 16-byte aligned octet of tail channels
-            *reinterpret_cast<uint4*>(tr + t0) =
-                make_uint4(pack_bf16x2(__uint_as_float(r[0]), __uint_as_float(r[1])), pack_bf16x2(__uint_as_float(r[2]), __uint_as_float(r[3])),
-                           pack_bf16x2(__uint_as_float(r[4]), __uint_as_float(r[5])), pack_bf16x2(__uint_as_float(r[6]), __uint_as_float(r[7])));
-          } else if (t0 == -4 && ((g.hlen | g.tail_pitch) & 3) == 0) {     // the octet's upper half starts the head's tail
-            *reinterpret_cast<uint2*>(tr) = make_uint2(pack_bf16x2(__uint_as_float(r[4]), __uint_as_float(r[5])),
-                                                       pack_bf16x2(__uint_as_float(r[6]), __uint_as_float(r[7])));
-          } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              if (c8 + j >= d_q) tr[c8 + j - d_q] = __float2bfloat16_rn(__uint_as_float(r[j]));
-          }
-        }
+    if (staged) {
+      // 32 rows x hlen channels, now consecutive channels by consecutive lanes (e / hlen by multiplication: e < 32 x 16)
+      __syncwarp();
+      const int64_t row0 = row - lane;
+      const uint32_t inv = 65536u / (uint32_t)g.hlen + 1u;
+      __nv_bfloat16* const t = a.tail + row0 * g.tail_pitch + h * g.hlen;
+#pragma unroll 1
+      for (int e = lane; e < 32 * g.hlen; e += 32) {
+        const int r = (int)(((uint32_t)e * inv) >> 16);
+        uint16_t v;
+        asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(stg + (uint32_t)e * 2) : "memory");
+        if (row0 + r < a.M) t[r * g.tail_pitch + (e - r * g.hlen)] = __ushort_as_bfloat16(v);
       }
     }
   }
@@ -473,9 +502,43 @@ __device__ __forceinline__ void epi_nvfp4_perhead(const RotArgs& a, uint32_t tad
     const int h = (n0 + cb) / d;
     if (h >= g.H) break;
     if (((turn++) % (uint32_t)wpq) != (uint32_t)half) continue;
+    if (pow2_T && a.codes && !a.x_rot) {
+      // blocks of 16 by nvfp4_hw_group, two at a time from an even block on: 16-byte code stores, two scale bytes
 #pragma unroll 1
-    for (int c16 = 0; c16 < d; c16 += 16) {
+      for (int c16 = 0; c16 < d_q;) {
+        const int slot = h * d_q + c16;                         // first code slot (a multiple of 16)
+        uint8_t* dst = a.codes + row * g.code_row_bytes + (slot >> 1);
+        uint8_t* sf = a.sf + sf_offset(row, slot >> 4, n_kb64_pad);
+        const bool two = !(slot & 16) && c16 + 32 <= d_q;
+        uint32_t r[32];
+        __syncwarp();                                           // lanes may have quantised the blocks before in different ways
+        tmem_ld16(taddr + cb + c16, r);
+        if (two) tmem_ld16(taddr + cb + c16 + 16, r + 16);
+        tmem_wait_ld();
+        uint32_t w[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (i < 8 || two) w[i] = pack_bf16x2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+        uint2 k0, k1;
+        const uint32_t s0 = nvfp4_hw_group(w, g.clip, g.T, k0);
+        if (two) {
+          const uint32_t s1 = nvfp4_hw_group(w + 8, g.clip, g.T, k1);
+          if (row_ok) {
+            *reinterpret_cast<uint4*>(dst) = make_uint4(k0.x, k0.y, k1.x, k1.y);
+            *reinterpret_cast<uint16_t*>(sf) = (uint16_t)(s0 | s1 << 8);
+          }
+        } else if (row_ok) {
+          *reinterpret_cast<uint2*>(dst) = k0;
+          *sf = (uint8_t)s0;
+        }
+        c16 += two ? 32 : 16;
+      }
+    }
+    const int c_rest = pow2_T && a.codes && !a.x_rot ? d_q : 0;
+#pragma unroll 1
+    for (int c16 = c_rest; c16 < d; c16 += 16) {
       uint32_t r[16];
+      __syncwarp();
       tmem_ld16(taddr + cb + c16, r);
       tmem_wait_ld();
       uint32_t w[8];                       // the rotated values, rounded to bf16 and packed in pairs
@@ -490,13 +553,12 @@ __device__ __forceinline__ void epi_nvfp4_perhead(const RotArgs& a, uint32_t tad
       if (!a.codes) continue;
       if (c16 < d_q) {
         const int slot = h * d_q + c16;                       // first code slot of this block (a multiple of 16)
-        float eff = 0.f;
         uint8_t sb;
-        uint2 c = make_uint2(0u, 0u);
+        uint2 c;
         if (pow2_T) {
-          sb = nvfp4_hw_scale(amax_bf16x16(w), g.clip, g.T, &eff);
-          if (eff > 0.f) c = nvfp4_hw_group_packed(w, eff);
+          sb = nvfp4_hw_group(w, g.clip, g.T, c);
         } else {
+          float eff = 0.f;
           float v[16];
           float amax = 0.f;
 #pragma unroll
@@ -726,11 +788,11 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       const int64_t row = (int64_t)mb * 128 + q * 32 + lane;
       const int n0 = nb * a.BN;
       if constexpr (EPI == EPI_ROT_ONLY)
-        epi_rot_only(a, &tm_y, smem_u32(stg_area) + (warp - 2) * 2048, taddr, mb * 128 + q * 32, lane, n0, half, turn);
+        epi_rot_only(a, &tm_y, smem_u32(stg_area) + (warp - 2) * RqCfg<EPI>::STG_WARP, taddr, mb * 128 + q * 32, lane, n0, half, turn);
       else if constexpr (EPI == EPI_INT_HIDDEN) epi_int_hidden<MODE>(a, taddr, row, n0, half, turn);
       else if constexpr (EPI == EPI_NVFP4_HIDDEN) epi_nvfp4_hidden<MODE>(a, taddr, row, n0, half, turn, RqCfg<EPI>::WPQ);
       else if constexpr (EPI == EPI_NVFP4_PERHEAD) epi_nvfp4_perhead(a, taddr, row, n0, half, turn, RqCfg<EPI>::WPQ);
-      else epi_int_perhead<MODE>(a, taddr, row, n0, half, turn, RqCfg<EPI>::WPQ);
+      else epi_int_perhead<MODE>(a, taddr, row, lane, n0, half, turn, smem_u32(stg_area) + (warp - 2) * RqCfg<EPI>::STG_WARP);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
@@ -877,6 +939,17 @@ int pick_bn(const ActGeom& g, int64_t M) {
   return best;
 }
 
+static void ragged_masks(const ActGeom& g, RotArgs& a) {
+  const int nv = g.group & 31;
+  a.ragged = nv != 0;
+  for (int j = 0; j < 32 && nv; ++j) {
+    if (j >= nv) continue;
+    a.pair_mask[j >> 1] |= 0xFFFFu << (16 * (j & 1));
+    if (g.mode == DIROTQ_INT8_ASYM) a.code_mask[j >> 2] |= 0xFFu << (8 * (j & 3));
+    else a.code_mask[(j & 15) >> 2] |= (j < 16 ? 0xFu : 0xF0u) << (8 * (j & 3));
+  }
+}
+
 int launch_rotate_quantize(const ActGeom& g, const void* x, const void* rot_t, int64_t M, RotArgs a, cudaStream_t st) {
   if (M <= 0) return DIROTQ_OK;
   a.g = g;
@@ -899,6 +972,7 @@ int launch_rotate_quantize(const ActGeom& g, const void* x, const void* rot_t, i
   if (!rot_only && g.H > 0) {
     // 32-column TMEM reads of a head's group must stay inside the head
     if (((g.group + 31) / 32) * 32 > g.d) return DIROTQ_E_UNSUPPORTED;
+    ragged_masks(g, a);
   }
   if (!rot_only && g.H == 0 && !is_nvfp4(g.mode) && g.group != 64) return DIROTQ_E_UNSUPPORTED;
   if (!rot_only && g.per_token) return DIROTQ_E_UNSUPPORTED;     // a row's scale needs the whole rotated row: rotate, then quantise
