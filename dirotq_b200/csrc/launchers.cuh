@@ -110,6 +110,7 @@ struct RotArgs {
   int64_t M;
   int64_t ldm;
   int BN;
+  int bn_last;            // width of the last column of tiles
   int n_tiles;
   int m_tiles;
   int K;                  // contraction length (== g.D for a rotation)

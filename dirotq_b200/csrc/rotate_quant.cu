@@ -60,6 +60,19 @@ template <int EPI, bool PAIR = false> struct RqCfg {
 enum : int { EPI_ROT_ONLY = 0, EPI_INT_HIDDEN = 1, EPI_NVFP4_HIDDEN = 2, EPI_INT_PERHEAD = 3, EPI_NVFP4_PERHEAD = 4 };
 
 
+// Tile t: row block and column block.  Where the last column block is narrower than the others, a row block's columns start one
+// further than those of the row block before, so that a CTA, which takes every gridDim-th tile, meets narrow tiles in turn
+// even where the grid and the number of columns have a common factor.
+__device__ __forceinline__ void tile_at(const RotArgs& a, int t, int& mt, int& nb) {
+  mt = t / a.n_tiles;
+  nb = t - mt * a.n_tiles;
+  if (a.bn_last != a.BN) {
+    nb += mt % a.n_tiles;
+    if (nb >= a.n_tiles) nb -= a.n_tiles;
+  }
+}
+__device__ __forceinline__ int tile_width(const RotArgs& a, int nb) { return nb + 1 == a.n_tiles ? a.bn_last : a.BN; }
+
 __device__ __forceinline__ void tile_k_range(const RotArgs& a, int nb, int& kb, int& ke) {
   const int kchunks = (a.K + 63) / 64;
   if (a.band == 0) { kb = 0; ke = kchunks; return; }
@@ -700,8 +713,10 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     int issued = 0;
     bool ok = true;
     for (int t = first; t < total_tiles && ok; t += step) {
-      const int mt = t / a.n_tiles, nb = t - mt * a.n_tiles;
+      int mt, nb;
+      tile_at(a, t, mt, nb);
       const int mb = PAIR ? 2 * mt + (int)rank : mt;
+      const int row_u = nb * a.BN + (int)rank * (tile_width(a, nb) >> 1);   // of a pair, each CTA fetches half of the tile's rows
       int kb, ke;
       tile_k_range(a, nb, kb, ke);
       for (int kc = kb; kc < ke; ++kc) {
@@ -712,11 +727,11 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
             const uint32_t fb = map_to_rank(full_bar(s), 0);
             if (rank == 0) mbar_expect_tx(full_bar(s), 2u * (RQ_A_BYTES + bn_own * 128));
             tma_load_2d_pair(sa, &tm_x, fb, kc * 64, mb * 128);
-            tma_load_2d_pair(sa + RQ_A_BYTES, &tm_u, fb, kc * 64, nb * a.BN + (int)rank * bn_own);
+            tma_load_2d_pair(sa + RQ_A_BYTES, &tm_u, fb, kc * 64, row_u);
           } else {
             mbar_expect_tx(full_bar(s), RQ_A_BYTES + a.BN * 128);
             tma_load_2d(sa, &tm_x, full_bar(s), kc * 64, mb * 128);
-            tma_load_2d(sa + RQ_A_BYTES, &tm_u, full_bar(s), kc * 64, nb * a.BN);
+            tma_load_2d(sa + RQ_A_BYTES, &tm_u, full_bar(s), kc * 64, row_u);
           }
         }
         __syncwarp();
@@ -727,14 +742,15 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     if (lane == 0) abort_flag[AB_ISSUED] = issued;
   } else if (warp == 1) {
     if (rank == 0) {
-      const uint32_t idesc = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, PAIR ? 256 : 128, (uint32_t)a.BN);
       int s = 0, buf = 0, stages = 0, accs = 0;
       uint32_t ph = 0, aph = 0;
       bool ok = true;
       const uint64_t op_d0 = smem_desc_sw128(smem_base);
       const uint32_t op_lo0 = (uint32_t)op_d0, op_hi = (uint32_t)(op_d0 >> 32);
       for (int t = first; t < total_tiles && ok; t += step) {
-        const int nb = t % a.n_tiles;
+        int mt, nb;
+        tile_at(a, t, mt, nb);
+        const uint32_t idesc = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, PAIR ? 256 : 128, (uint32_t)tile_width(a, nb));
         int kb, ke;
         tile_k_range(a, nb, kb, ke);
         if (!mbar_wait_warp(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
@@ -780,7 +796,8 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     uint32_t aph = 0, turn = 0;
     const uint32_t acce_leader = PAIR ? map_to_rank(acce_bar(0), 0) : 0u;
     for (int t = first; t < total_tiles; t += step) {
-      const int mt = t / a.n_tiles, nb = t - mt * a.n_tiles;
+      int mt, nb;
+      tile_at(a, t, mt, nb);
       const int mb = PAIR ? 2 * mt + (int)rank : mt;
       if (!mbar_wait_warp(accf_bar(buf), aph, abort_flag, a.status, ERR_WAIT_ACC_FULL)) break;
       tc_fence_after();
@@ -918,8 +935,16 @@ static int launch_rq(const CUtensorMap& tx, const CUtensorMap& tu, const CUtenso
 // layouts: a multiple of 64; the persistent grid runs ceil(tiles / SMs) rounds, and a round costs a part that grows with
 // the tile width (the UMMAs) plus a part that does not (the per-stage barrier protocol of the issuer, the same for every
 // width).  Measured at D = 1152, 32768 rows: 6.03 / 6.68 / 7.59 us per round for 128 / 192 / 256 columns, i.e. the fixed
-// part is worth about 370 columns; the choice minimises rounds x (width + 370) -- padding of D and a nearly empty last
-// round both count (32768 rows of a 1152-wide layer take 256: 68 us against 74 with 192; a 4096-row shard takes 128).
+// part is worth about 370 columns; the choice minimises rounds x (width + 370) less what narrow last columns save -- padding
+// of D and a nearly empty last round both count (32768 rows of a 1152-wide layer take 256: 68 us against 74 with 192; a 4096-row
+// shard takes 128).
+// The last column of tiles is only as wide as D needs, rounded up to 64 (1152 columns were five tiles of 256, and are four and a
+// half): 32768 x 1152 63.9 -> 62.3 us, 32768 x 4608 -> 1152 in bf16 246 -> 242.  The shared-memory pipe, which the operands
+// pass twice, keeps the gain below the UMMAs saved.
+static int last_width(int D, int bn) {
+  const int w = ((D % bn) + 63) & ~63;
+  return w == 0 || w > bn ? bn : w;
+}
 int pick_bn(const ActGeom& g, int64_t M) {
   if (g.H > 0) {
     int best = 0;
@@ -933,7 +958,8 @@ int pick_bn(const ActGeom& g, int64_t M) {
   int64_t best_cost = -1;
   for (int i = 0; i < 3; ++i) {
     const int64_t tiles = m_tiles * ceil_div(g.D, cand[i]);
-    const int64_t cost = ((tiles + sms - 1) / sms) * (cand[i] + 370);
+    const int64_t n_tiles = ceil_div(g.D, cand[i]), rounds = (tiles + sms - 1) / sms;
+    const int64_t cost = rounds * (cand[i] + 370) - rounds / n_tiles * (cand[i] - last_width(g.D, cand[i]));
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = cand[i]; }
   }
   return best;
@@ -967,6 +993,7 @@ int launch_rotate_quantize(const ActGeom& g, const void* x, const void* rot_t, i
   a.BN = pick_bn(g_tile, M);
   if (a.BN <= 0) return DIROTQ_E_UNSUPPORTED;
   a.n_tiles = ceil_div(g.D, a.BN);
+  a.bn_last = last_width(g.D, a.BN);
   a.m_tiles = (int)((M + 127) / 128);
   a.band = g.H > 0 ? g.d : 0;
   if (!rot_only && g.H > 0) {
@@ -1021,6 +1048,7 @@ int launch_gemm_bf16(const void* x, const void* w_t, int64_t M, int64_t N, int64
   a.ldm = ld_rows(M);
   a.BN = pick_bn(a.g, M);
   a.n_tiles = ceil_div((int)N, a.BN);
+  a.bn_last = last_width((int)N, a.BN);
   a.m_tiles = (int)((M + 127) / 128);
   a.band = 0;
   a.x_rot = static_cast<__nv_bfloat16*>(y);
