@@ -182,6 +182,28 @@ __device__ __forceinline__ uint32_t hmul2_2m4(uint32_t m) {
   return r;
 }
 
+// 32 codes of one row, as loaded, -> 16 fp16 pairs of (code - z) * s, by the record k of their chunk: 16 planar bytes ...
+template <bool ASYM>
+__device__ __forceinline__ void expand_nibbles32(uint4 p, uint2 k, uint32_t* y) {
+  const uint32_t mhi = hmul2_2m4(k.x), xr = ASYM ? 0u : 0x00080008u;
+  expand_word(p.x, xr, k.x, mhi, k.y, y);
+  expand_word(p.y, xr, k.x, mhi, k.y, y + 4);
+  expand_word(p.z, xr, k.x, mhi, k.y, y + 8);
+  expand_word(p.w, xr, k.x, mhi, k.y, y + 12);
+}
+// ... or 32 bytes: a byte alone in a zero half is the subnormal q * 2^-24, so (q - z) * s is one packed FMA again; the values
+// are emitted in the K order the 4-bit weight expansion produces (see expand_word)
+__device__ __forceinline__ void expand_bytes32(const uint4* p, uint2 k, uint32_t* y) {
+  const uint32_t w[8] = {p[0].x, p[0].y, p[0].z, p[0].w, p[1].x, p[1].y, p[1].z, p[1].w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    y[4 * i] = hfma2_u(__byte_perm(w[i], 0u, 0x4240), k.x, k.y);
+    y[4 * i + 1] = hfma2_u(__byte_perm(w[4 + i], 0u, 0x4240), k.x, k.y);
+    y[4 * i + 2] = hfma2_u(__byte_perm(w[i], 0u, 0x4341), k.x, k.y);
+    y[4 * i + 3] = hfma2_u(__byte_perm(w[4 + i], 0u, 0x4341), k.x, k.y);
+  }
+}
+
 __device__ __forceinline__ uint32_t hmul2_m8(uint32_t m) {
   uint32_t r;
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(m), "r"(0x80088008u));     // * -8 * 2^-24
@@ -416,141 +438,124 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         const uint32_t m = half_twice(s * (inv * 16777216.f));       // s has 8 bits: exact, so 8 s / rs may be taken from it
         return make_uint2(m, hmul2_m8(m));
       };
+      // A stage's values, in registers, go to tensor memory as soon as the slot is free.  (The empty statement keeps the expansion in
+      // front of the wait: the compiler would move it behind, onto the path between "slot free" and "stage ready".)
+      auto deliver = [&](int qq, uint32_t (&y)[32]) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(y[i]));
+        const int es = exp_slot(qq);
+        if (!mbar_wait_hot_warp(expe_bar(es), exp_phase(qq) ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { q = qq; return false; }
+        tc_fence_after();
+        tmem_st32(tmem_base + ((uint32_t)(quarter * 32) << 16) + Cfg::TMEM_A0 + es * 32, y);
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) exp_ready(es);
+        return true;
+      };
+      auto release_raw = [&]() {                              // what this warp needs of the raw stage is in registers
+        __syncwarp();
+        if (lane == 0) mbar_arrive(rawe_bar(r.s));
+        r.next();
+      };
       for (int c = 0; c < n_raw && ok; c += GF_CPS) {
         if (!mbar_wait_hot_warp(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         const uint32_t sraw = raw_base + r.s * Cfg::RAW_STAGE;
         const int nv = min(GF_CPS, n_raw - c);
         const int njc = hc ? (nv + 1) >> 1 : nv;               // operand stages this raw stage feeds
-        for (int jc = 0; jc < njc; ++jc, ++q) {
-          if (q % Cfg::GROUPS != grp) continue;
-          // The row is expanded into registers before the slot is known to be free, so that only the
-          // tensor-memory store remains on the path between "slot free" and "stage ready".
-          uint32_t y1[32];
-          if (hc) {
-            // half chunks: the first 32 slots of chunks 2 jc and 2 jc + 1, each with its own record, side by side
-            const int c0 = 2 * jc, c1 = 2 * jc + 1;
-            const bool has1 = c1 < nv;
-            const uint2 ka0 = record(sraw, c0);
-            const uint2 ka1 = has1 ? record(sraw, c1) : make_uint2(0u, 0u);
-            const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
-            if constexpr (A8) {
-              const uint32_t rb0 = sraw + (c0 >> 1) * (128 * 128) + rowA * 128, rb1 = sraw + (c1 >> 1) * (128 * 128) + rowA * 128;
-              uint4 pq[4];
-#pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                pq[u] = gf_lds128(rb0 + ((((c0 & 1) * 4 + u) ^ (rowA & 7)) << 4));
-                pq[2 + u] = has1 ? gf_lds128(rb1 + ((((c1 & 1) * 4 + u) ^ (rowA & 7)) << 4)) : z4;
-              }
-              const uint32_t w16[16] = {pq[0].x, pq[0].y, pq[0].z, pq[0].w, pq[1].x, pq[1].y, pq[1].z, pq[1].w,
-                                        pq[2].x, pq[2].y, pq[2].z, pq[2].w, pq[3].x, pq[3].y, pq[3].z, pq[3].w};
-#pragma unroll
-              for (int h = 0; h < 2; ++h) {
-                const uint2 ka = h ? ka1 : ka0;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                  const uint32_t wl = w16[8 * h + i], wh = w16[8 * h + 4 + i];
-                  uint32_t* y = y1 + 16 * h + 4 * i;
-                  y[0] = hfma2_u(__byte_perm(wl, 0u, 0x4240), ka.x, ka.y);
-                  y[1] = hfma2_u(__byte_perm(wh, 0u, 0x4240), ka.x, ka.y);
-                  y[2] = hfma2_u(__byte_perm(wl, 0u, 0x4341), ka.x, ka.y);
-                  y[3] = hfma2_u(__byte_perm(wh, 0u, 0x4341), ka.x, ka.y);
-                }
-              }
-            } else {
-              const uint32_t rb = sraw + rowA * 128;
-              const int sw = rowA & 7;
-              const uint4 pa0 = gf_lds128(rb + (((2 * c0) ^ sw) << 4));
-              const uint4 pa1 = has1 ? gf_lds128(rb + (((2 * c1) ^ sw) << 4)) : z4;
-              const uint32_t w8[8] = {pa0.x, pa0.y, pa0.z, pa0.w, pa1.x, pa1.y, pa1.z, pa1.w};
-              const uint32_t xr1 = ASYM ? 0u : 0x00080008u;
-              const uint32_t mhi0 = hmul2_2m4(ka0.x), mhi1 = hmul2_2m4(ka1.x);
-#pragma unroll
-              for (int i = 0; i < 4; ++i) expand_word(w8[i], xr1, ka0.x, mhi0, ka0.y, y1 + 4 * i);
-#pragma unroll
-              for (int i = 4; i < 8; ++i) expand_word(w8[i], xr1, ka1.x, mhi1, ka1.y, y1 + 4 * i);
-            }
-          } else {
-          const uint2 ka = record(sraw, jc);
+        const int q0 = q, j0 = (grp ^ q) & 1, j1 = j0 + 2;     // this group's: j0 and j1, where they exist
+        q += njc;
+        if (j0 >= njc) { release_raw(); continue; }
+        uint32_t y[32];
+        if (hc) {
+          // half chunks: the first 32 slots of chunks 2 j0 and 2 j0 + 1, each with its own record, side by side
+          const int c0 = 2 * j0, c1 = 2 * j0 + 1;
+          const bool has1 = c1 < nv;
+          const uint2 ka0 = record(sraw, c0);
+          const uint2 ka1 = has1 ? record(sraw, c1) : make_uint2(0u, 0u);
+          const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
           if constexpr (A8) {
-            // 8-bit codes: 64 bytes of this row = four 16-byte pieces of box jc >> 1.  A byte alone in a zero
-            // half is the subnormal q * 2^-24, so (q - z) * s is one packed FMA again; the values are emitted
-            // in the K order the 4-bit weight expansion produces (see expand_word).
-            const uint32_t rb = sraw + (jc >> 1) * (128 * 128) + rowA * 128;
-            uint4 pq[4];
+            const uint32_t rb0 = sraw + (c0 >> 1) * (128 * 128) + rowA * 128, rb1 = sraw + (c1 >> 1) * (128 * 128) + rowA * 128;
+            uint4 p0[4], p1[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) pq[u] = gf_lds128(rb + ((((jc & 1) * 4 + u) ^ (rowA & 7)) << 4));
-            const uint32_t w16[16] = {pq[0].x, pq[0].y, pq[0].z, pq[0].w, pq[1].x, pq[1].y, pq[1].z, pq[1].w,
-                                      pq[2].x, pq[2].y, pq[2].z, pq[2].w, pq[3].x, pq[3].y, pq[3].z, pq[3].w};
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const uint32_t wl = w16[8 * h + i], wh = w16[8 * h + 4 + i];
-                uint32_t* y = y1 + 16 * h + 4 * i;
-                y[0] = hfma2_u(__byte_perm(wl, 0u, 0x4240), ka.x, ka.y);
-                y[1] = hfma2_u(__byte_perm(wh, 0u, 0x4240), ka.x, ka.y);
-                y[2] = hfma2_u(__byte_perm(wl, 0u, 0x4341), ka.x, ka.y);
-                y[3] = hfma2_u(__byte_perm(wh, 0u, 0x4341), ka.x, ka.y);
-              }
+            for (int u = 0; u < 2; ++u) {
+              p0[u] = gf_lds128(rb0 + ((((c0 & 1) * 4 + u) ^ (rowA & 7)) << 4));
+              p1[u] = has1 ? gf_lds128(rb1 + ((((c1 & 1) * 4 + u) ^ (rowA & 7)) << 4)) : z4;
+            }
+            release_raw();
+            expand_bytes32(p0, ka0, y);
+            expand_bytes32(p1, ka1, y + 16);
           } else {
-            // two 16-byte pieces of the swizzled 128-byte raw row
             const uint32_t rb = sraw + rowA * 128;
             const int sw = rowA & 7;
-            const uint4 pa0 = gf_lds128(rb + (((2 * jc) ^ sw) << 4));
-            const uint4 pa1 = gf_lds128(rb + (((2 * jc + 1) ^ sw) << 4));
-            const uint32_t w8[8] = {pa0.x, pa0.y, pa0.z, pa0.w, pa1.x, pa1.y, pa1.z, pa1.w};
-            const uint32_t mhi = hmul2_2m4(ka.x);
-            const uint32_t xr1 = ASYM ? 0u : 0x00080008u;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) expand_word(w8[i], xr1, ka.x, mhi, ka.y, y1 + 4 * i);
+            const uint4 p0 = gf_lds128(rb + (((2 * c0) ^ sw) << 4));
+            const uint4 p1 = has1 ? gf_lds128(rb + (((2 * c1) ^ sw) << 4)) : z4;
+            release_raw();
+            expand_nibbles32<ASYM>(p0, ka0, y);
+            expand_nibbles32<ASYM>(p1, ka1, y + 16);
           }
-          }
-          const int es = exp_slot(q);
-          if (!mbar_wait_hot_warp(expe_bar(es), exp_phase(q) ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
-          tc_fence_after();
-          tmem_st32(tmem_base + ((uint32_t)(quarter * 32) << 16) + Cfg::TMEM_A0 + es * 32, y1);
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) exp_ready(es);
+          if (!deliver(q0 + j0, y)) { ok = false; break; }
+          continue;
         }
-        if (!ok) break;
-        __syncwarp();
-        if (lane == 0) mbar_arrive(rawe_bar(r.s));
-        r.next();
+        // (Single CTAs, with the weight producer as a whole warp and the issuer's early tests, us: 512 x 12288 x 3072 64.3 -> 56.5, 4096 x
+        // 4608 x 1152 50.4 -> 44, 1024 x 2240 x 2240 17.2 -> 15.6; long launches on pairs, which the UMMAs bound, 0.5 %.)
+        // 4-bit codes: two 16-byte pieces of the swizzled 128-byte raw row; 8-bit codes: 64 bytes of this row = four pieces of box
+        // j >> 1.  Both stages' codes are read before the first is expanded, and the raw stage goes back to its producer.
+        constexpr int PC = A8 ? 4 : 2;
+        auto fetch = [&](int j, uint4 (&p)[PC]) {
+#pragma unroll
+          for (int u = 0; u < PC; ++u)
+            p[u] = A8 ? gf_lds128(sraw + (j >> 1) * (128 * 128) + rowA * 128 + ((((j & 1) * 4 + u) ^ (rowA & 7)) << 4))
+                      : gf_lds128(sraw + rowA * 128 + (((2 * j + u) ^ (rowA & 7)) << 4));
+        };
+        auto expand = [&](const uint4 (&p)[PC], uint2 k) {
+          if constexpr (A8) {
+            expand_bytes32(p, k, y);
+            expand_bytes32(p + 2, k, y + 16);
+          } else {
+            expand_nibbles32<ASYM>(p[0], k, y);
+            expand_nibbles32<ASYM>(p[1], k, y + 16);
+          }
+        };
+        uint4 p0[PC], p1[PC];
+        const uint2 k0 = record(sraw, j0);
+        fetch(j0, p0);
+        uint2 k1 = make_uint2(0u, 0u);
+        if (j1 < njc) {
+          k1 = record(sraw, j1);
+          fetch(j1, p1);
+        }
+        release_raw();
+        expand(p0, k0);
+        if (!deliver(q0 + j0, y)) { ok = false; break; }
+        if (j1 < njc) {
+          expand(p1, k1);
+          if (!deliver(q0 + j1, y)) { ok = false; break; }
+        }
       }
       // tail: the activations' bf16 tile arrives in the raw ring; its rows, divided by rs (exact; for pairs the folding kernel
       // has done that), go to TMEM like an expanded chunk
-      for (int st = 0; st < n_tail && ok; ++st, ++q) {
+      for (int st = 0; st < n_tail && ok; ++st) {
         if (!mbar_wait_hot_warp(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
-        if (q % Cfg::GROUPS == grp) {
-          const int es = exp_slot(q);
-          const uint32_t rb = raw_base + r.s * Cfg::RAW_STAGE + rowA * 128;
-          uint32_t y[32];
+        const int qq = q++;
+        if (((qq ^ grp) & 1) != 0) { release_raw(); continue; }
+        const uint32_t rb = raw_base + r.s * Cfg::RAW_STAGE + rowA * 128;
+        uint32_t y[32];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const uint4 v = gf_lds128(rb + (uint32_t)((i ^ (rowA & 7)) << 4));
-            y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
-          }
-          if constexpr (!PAIR) {
-            const __nv_bfloat162 inv2 = __float2bfloat162_rn(inv);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              const __nv_bfloat162 h = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&y[i]), inv2);
-              y[i] = *reinterpret_cast<const uint32_t*>(&h);
-            }
-          }
-          if (!mbar_wait_hot_warp(expe_bar(es), exp_phase(q) ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
-          tc_fence_after();
-          tmem_st32(tmem_base + ((uint32_t)(quarter * 32) << 16) + Cfg::TMEM_A0 + es * 32, y);
-          tmem_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) exp_ready(es);
+        for (int i = 0; i < 8; ++i) {
+          const uint4 v = gf_lds128(rb + (uint32_t)((i ^ (rowA & 7)) << 4));
+          y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(rawe_bar(r.s));
-        r.next();
+        release_raw();
+        if constexpr (!PAIR) {
+          const __nv_bfloat162 inv2 = __float2bfloat162_rn(inv);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            const __nv_bfloat162 h = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&y[i]), inv2);
+            y[i] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+        }
+        if (!deliver(qq, y)) { ok = false; break; }
       }
     }
     if (PAIR && lane == 0) {
@@ -616,41 +621,47 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
     }
   } else if (warp == W_TMB) {
     // ------------------------------ weight-tile producer ---------------------------------------
-    // Operand stage q's weight tile goes straight into slot q % EXP_STAGES as soon as the slot is free.
-    if (lane == 0) {
-      int q = 0;
-      bool ok = true;
-      for (int t = first; t < total_tiles && ok; t += step) {
-        int tm_, tn_;
-        tile_mn(t, tm_, tn_);
-        const int n0 = tn_ * BN;
-        for (int st = 0; st < n_main + n_tail; ++st, ++q) {
-          const int es = q % GF_EXP_STAGES;
-          if (!mbar_wait_hot(expe_bar(es), (uint32_t)(((q / GF_EXP_STAGES) & 1) ^ 1), abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+    // Operand stage q's weight tile goes straight into slot q % EXP_STAGES as soon as the slot is free.  A whole warp waits and its
+    // elected lane issues, as in the issuer: in one lane this loop took 450 cycles a stage, more than the four UMMAs of a 128-wide
+    // tile, and was what such launches waited for.
+    GfRing<GF_EXP_STAGES> e;
+    int issued = 0;
+    bool ok = true;
+    const uint32_t full_lead = PAIR ? map_to_rank(expf_bar(0), 0) : 0u;   // the bytes of both halves are counted in the leader
+    const int ns = n_main + n_tail;
+    for (int t = first; t < total_tiles && ok; t += step) {
+      int tm_, tn_;
+      tile_mn(t, tm_, tn_);
+      const int row_b = tn_ * BN + (int)rank * Cfg::BN_OWN;               // of a pair, this CTA's half of the weight rows
+      for (int st = 0; st < ns; ++st) {
+        if (!mbar_wait_hot_warp(expe_bar(e.s), e.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+        if (elect_one()) {
+          const uint32_t dst = exp_base + e.s * Cfg::EXP_STAGE;
           if constexpr (PAIR) {
-            // this CTA's half of the weight rows; the bytes of both halves are counted in the leader
-            const uint32_t bar = map_to_rank(expf_bar(es), 0);
-            const int row_b = n0 + (int)rank * Cfg::BN_OWN;
-            if (rank == 0) mbar_expect_tx(expf_bar(es), 2 * Cfg::B_EXP);
-            if (st < n_main) tma_load_2d_pair(exp_base + es * Cfg::EXP_STAGE, &tm.wp, bar, st * 64, row_b);
-            else tma_load_2d_pair(exp_base + es * Cfg::EXP_STAGE, &tm.wt, bar, (st - n_main) * 64, row_b);
-            continue;
+            const uint32_t bar = full_lead + 8u * e.s;
+            if (rank == 0) mbar_expect_tx(expf_bar(e.s), 2 * Cfg::B_EXP);
+            if (st < n_main) tma_load_2d_pair(dst, &tm.wp, bar, st * 64, row_b);
+            else tma_load_2d_pair(dst, &tm.wt, bar, (st - n_main) * 64, row_b);
+          } else {
+            const uint32_t bar = expw_bar(e.s);
+            mbar_expect_tx(bar, Cfg::B_EXP);                   // the box is counted whole, zero fill included
+            if (st < n_main) tma_load_2d(dst, &tm.wp, bar, st * 64, row_b);
+            else tma_load_2d(dst, &tm.wt, bar, (st - n_main) * 64, row_b);
           }
-          const uint32_t bar = expw_bar(es);
-          mbar_expect_tx(bar, Cfg::B_EXP);                     // the box is counted whole, zero fill included
-          if (st < n_main) tma_load_2d(exp_base + es * Cfg::EXP_STAGE, &tm.wp, bar, st * 64, n0);
-          else tma_load_2d(exp_base + es * Cfg::EXP_STAGE, &tm.wt, bar, (st - n_main) * 64, n0);
         }
+        __syncwarp();
+        ++issued;
+        e.next();
       }
-      abort_flag[AB_ISSUED2] = q;
     }
+    if (lane == 0) abort_flag[AB_ISSUED2] = issued;
   } else if (warp == W_MMA) {
     // ------------------------------ UMMA issuer ----------------------------------------------
     if (rank == 0) {
       const uint32_t idesc_h = idesc_dense(ACC_F32, FMT_F16, FMT_F16, TILE_M, BN);
       const uint32_t idesc_bf = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, TILE_M, BN);
       int use = 0, stages = 0;
-      bool ok = true;
+      bool ok = true, ready = false;                               // ready: the next stage's barriers are known to be complete
       // loop-invariant pieces of the per-stage operands: barrier addresses are 8 bytes per slot apart, the weight
       // descriptor's low word holds the slot address >> 4, the activation slots are 32 tensor-memory columns apart
       int es = 0;
@@ -669,26 +680,25 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         if (!mbar_wait_hot_warp(acce_bar(buf), acc_ph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
-        // What this warp does between UMMAs is time the pipe idles, and it has few of them queued.
+        // What this warp does between UMMAs is time the pipe idles, and it has few of them queued: so the next stage's barriers
+        // are tested within this one's block (umma_f16_ts_stage): waiting, issuing and looping took 150 + 180 + 100 cycles.
         for (int st = 0; st < ns; ++st) {
           const uint32_t w = expw0 + 8u * es;                      // expf / expe lie at fixed offsets from expw
           // pairs: one barrier per stage covers both operands in both CTAs
-          if (PAIR ? !mbar_wait_hot_warp(w - kFullOff, ph, abort_flag, a.status, ERR_WAIT_FULL)
-                   : !mbar_wait2_hot_warp(w, ph, w - kFullOff, ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+          if (!ready && (PAIR ? !mbar_wait_hot_warp(w - kFullOff, ph, abort_flag, a.status, ERR_WAIT_FULL)
+                              : !mbar_wait2_hot_warp(w, ph, w - kFullOff, ph, abort_flag, a.status, ERR_WAIT_FULL))) { ok = false; break; }
           tc_fence_after();
+          const uint32_t a_t = a_tmem0 + 32u * es, b_lo = bdesc_lo0 + kDescStep * es;
+          if (++es == GF_EXP_STAGES) { es = 0; ph ^= 1u; }
+          const uint32_t wn = expw0 + 8u * es;
+          uint32_t next = 0u;
           if (elect_one()) {
             const uint32_t idesc = st < n_main ? idesc_h : idesc_bf;
-            if constexpr (PAIR) {
-              umma_f16_ts_x4_pair(d, a_tmem0 + 32u * es, bdesc_lo0 + kDescStep * es, bdesc_hi, idesc, st > 0 ? 1u : 0u);
-              umma_commit_pair_both(w - kEmptyOff);
-            } else {
-              umma_f16_ts_x4(d, a_tmem0 + 32u * es, bdesc_lo0 + kDescStep * es, bdesc_hi, idesc, st > 0 ? 1u : 0u);
-              umma_commit(w - kEmptyOff);
-            }
+            if constexpr (PAIR) next = umma_f16_ts_stage_pair(d, a_t, b_lo, bdesc_hi, idesc, st > 0 ? 1u : 0u, w - kEmptyOff, wn - kFullOff, ph);
+            else next = umma_f16_ts_stage(d, a_t, b_lo, bdesc_hi, idesc, st > 0 ? 1u : 0u, w - kEmptyOff, wn, ph, wn - kFullOff);
           }
-          __syncwarp();
+          ready = __any_sync(0xffffffffu, next != 0u);
           ++stages;
-          if (++es == GF_EXP_STAGES) { es = 0; ph ^= 1u; }
         }
         if (!ok) break;
         if (elect_one()) {

@@ -126,16 +126,19 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
     const uint64_t op_d0 = smem_desc_sw128(smem_base), sf_d0 = smem_desc_rows16(smem_base);
     const uint32_t op_lo0 = (uint32_t)op_d0, op_hi = (uint32_t)(op_d0 >> 32);
     const uint32_t sf_lo0 = (uint32_t)sf_d0, sf_hi = (uint32_t)(sf_d0 >> 32);
-    bool ok = true;
+    bool ok = true, ready = false;                     // ready: the next stage is known to be full
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
       if (!mbar_wait_warp(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
       tc_fence_after();
       const uint32_t d = tmem_base + buf * 128;
       for (int st = 0; st < n_main + n_tail; ++st) {
-        if (!mbar_wait_warp(full_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+        if (!ready && !mbar_wait_warp(full_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         tc_fence_after();
+        const int slot = r.s;
+        r.next();
+        uint32_t next = 0u;
         if (elect_one()) {
-          const uint32_t sA = smem_base + r.s * GF_STAGE_BYTES;
+          const uint32_t sA = smem_base + slot * GF_STAGE_BYTES;
           const uint64_t adesc = smem_desc_sw128(sA), bdesc = smem_desc_sw128(sA + GF_TILE_BYTES);
           if (st < n_main) {
             const uint32_t sfa_s = sA + 2 * GF_TILE_BYTES, sfb_s = sfa_s + GF_SF_BYTES;
@@ -143,8 +146,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
             const int nkb = min(4, a.n_chunks - st * 4);
             if (nkb == 4) {
               // a whole stage: descriptors from loop-invariant words, eight copies + four UMMAs in one block
-              const uint32_t a_lo = op_lo0 + (uint32_t)r.s * (GF_STAGE_BYTES >> 4);
-              const uint32_t sf_lo = sf_lo0 + (uint32_t)r.s * (GF_STAGE_BYTES >> 4);
+              const uint32_t a_lo = op_lo0 + (uint32_t)slot * (GF_STAGE_BYTES >> 4);
+              const uint32_t sf_lo = sf_lo0 + (uint32_t)slot * (GF_STAGE_BYTES >> 4);
               umma_nvf4_stage4(d, a_lo, a_lo + (GF_TILE_BYTES >> 4), op_hi, idesc_f4, st > 0 ? 1u : 0u, sfa_t, sfb_t,
                                sf_lo + (2 * GF_TILE_BYTES >> 4), sf_lo + ((2 * GF_TILE_BYTES + GF_SF_BYTES) >> 4), sf_hi);
             } else {
@@ -156,16 +159,15 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_consta
               umma_nvf4(d, adesc + 2 * kb, bdesc + 2 * kb, idesc_f4, (st > 0 || kb > 0) ? 1u : 0u, sfa_t + kb * 4,
                         sfb_t + kb * 4);
             }
+            umma_commit(empty_bar(slot));
           } else {
-            const uint32_t a_lo = op_lo0 + (uint32_t)r.s * (GF_STAGE_BYTES >> 4);
-            umma_f16_ss_x4(d, a_lo, a_lo + (GF_TILE_BYTES >> 4), op_hi, idesc_bf, 1u);
+            const uint32_t a_lo = op_lo0 + (uint32_t)slot * (GF_STAGE_BYTES >> 4);
+            next = umma_f16_ss_stage(d, a_lo, a_lo + (GF_TILE_BYTES >> 4), op_hi, idesc_bf, 1u, empty_bar(slot), full_bar(r.s), r.ph);
           }
-          umma_commit(empty_bar(r.s));
         }
-        __syncwarp();
+        ready = __any_sync(0xffffffffu, next != 0u);
         if (st < n_main) sf_slot ^= 1;
         ++stages;
-        r.next();
       }
       if (!ok) break;
       if (elect_one()) umma_commit(accf_bar(buf));

@@ -233,39 +233,40 @@ gemm_nvfp4_pair_kernel(const __grid_constant__ CUtensorMap tm_xq, const __grid_c
       GfRingT<STAGES> r;
       int buf = 0, stages = 0, accs = 0;
       uint32_t aph = 0;
-      bool ok = true;
+      bool ok = true, ready = false;                         // ready: the next stage is known to be full
       for (int t = first; t < total_tiles && ok; t += step) {
         if (!mbar_wait_warp(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
         tc_fence_after();
         const uint32_t d = tmem_base + buf * BN;
         for (int st = 0; st < n_main + n_tail; ++st) {
           // one wait covers the operand bytes of both CTAs and the scale factors in both CTAs' tensor memory
-          if (!mbar_wait_warp(full_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+          if (!ready && !mbar_wait_warp(full_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
-          // descriptors from loop-invariant words, a whole stage's UMMAs in one block: what this warp does between UMMAs
-          // is time the tensor pipe idles (an FP4 UMMA of a 128-wide tile keeps it busy for 64 cycles)
+          // descriptors from loop-invariant words; a whole stage's UMMAs, their commit (the stage is free in BOTH CTAs once they have
+          // read it) and a test of the next stage's barrier in one block: what this warp does between UMMAs is time the tensor
+          // pipe idles (an FP4 UMMA of a 128-wide tile keeps it busy for 64 cycles)
           const uint32_t a_lo = op_lo0 + (uint32_t)r.s * (Cfg::STAGE_BYTES >> 4), b_lo = a_lo + (Cfg::A_BYTES >> 4);
+          const uint32_t sfa_t = tmem_base + Cfg::SF_COL + r.s * Cfg::SF_SLOT, sfb_t = sfa_t + 16, done = empty_bar(r.s);
+          r.next();
+          uint32_t next = 0u;
           if (elect_one()) {
             if (st < n_main) {
-              const uint32_t sfa_t = tmem_base + Cfg::SF_COL + r.s * Cfg::SF_SLOT, sfb_t = sfa_t + 16;
               const int nkb = min(4, a.n_chunks - st * 4);
               if (nkb == 4) {
-                umma_nvf4_x4_pair<BN / 32>(d, a_lo, b_lo, op_hi, idesc_f4, st > 0 ? 1u : 0u, sfa_t, sfb_t);
+                next = umma_nvf4_stage_pair<BN / 32>(d, a_lo, b_lo, op_hi, idesc_f4, st > 0 ? 1u : 0u, sfa_t, sfb_t, done, full_bar(r.s), r.ph);
               } else {
                 const uint64_t hi = (uint64_t)op_hi << 32;
                 for (int kb = 0; kb < nkb; ++kb)
                   umma_nvf4_pair(d, hi | (a_lo + 2 * kb), hi | (b_lo + 2 * kb), idesc_f4, (st > 0 || kb > 0) ? 1u : 0u,
                                  sfa_t + kb * 4, sfb_t + kb * (BN / 32));
+                umma_commit_pair_both(done);
               }
             } else {
-              umma_f16_ss_x4_pair(d, a_lo, b_lo, op_hi, idesc_bf, st > 0 ? 1u : 0u);
+              next = umma_f16_ss_stage_pair(d, a_lo, b_lo, op_hi, idesc_bf, st > 0 ? 1u : 0u, done, full_bar(r.s), r.ph);
             }
-            // the stage is free in BOTH CTAs once these UMMAs have read it
-            umma_commit_pair_both(empty_bar(r.s));
           }
-          __syncwarp();
+          ready = __any_sync(0xffffffffu, next != 0u);
           ++stages;
-          r.next();
         }
         if (!ok) break;
         if (elect_one()) umma_commit_pair_both(accf_bar(buf));

@@ -374,21 +374,28 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64
 }
 // The four K = 16 UMMAs of one 64-wide operand stage in one block: A from tensor memory (8 columns per step), B through a
 // shared-memory descriptor whose low word advances by 2 (32 bytes) per step; `accum0` = 0 clears the accumulator first.
-__device__ __forceinline__ void umma_f16_ts_x4(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc_lo, uint32_t bdesc_hi,
-                                               uint32_t idesc, uint32_t accum0) {
+__device__ __forceinline__ uint32_t umma_f16_ts_stage(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc_lo, uint32_t bdesc_hi, uint32_t idesc,
+                                                      uint32_t accum0, uint32_t done, uint32_t next, uint32_t nph, uint32_t next2) {
+  uint32_t r;
   asm volatile(
-      "{\n\t.reg .pred p, t;\n\t.reg .b64 d0, d1, d2, d3;\n\t.reg .b32 l1, l2, l3, a1, a2, a3;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
+      "{\n\t.reg .pred p, t, q, q2;\n\t.reg .b64 d0, d1, d2, d3;\n\t.reg .b32 l1, l2, l3, a1, a2, a3;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
       "setp.eq.b32 t, 0, 0;\n\t"
-      "add.u32 l1, %2, 2;\n\tadd.u32 l2, %2, 4;\n\tadd.u32 l3, %2, 6;\n\t"
-      "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
-      "mov.b64 d0, {%2, %3};\n\tmov.b64 d1, {l1, %3};\n\tmov.b64 d2, {l2, %3};\n\tmov.b64 d3, {l3, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], d0, %4, p;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], d1, %4, t;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], d2, %4, t;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], d3, %4, t;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(bdesc_lo), "r"(bdesc_hi), "r"(idesc), "r"(accum0)
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%8], %9;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 q2, [%10], %9;\n\t"
+      "add.u32 l1, %3, 2;\n\tadd.u32 l2, %3, 4;\n\tadd.u32 l3, %3, 6;\n\t"
+      "add.u32 a1, %2, 8;\n\tadd.u32 a2, %2, 16;\n\tadd.u32 a3, %2, 24;\n\t"
+      "mov.b64 d0, {%3, %4};\n\tmov.b64 d1, {l1, %4};\n\tmov.b64 d2, {l2, %4};\n\tmov.b64 d3, {l3, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], d0, %5, p;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], d1, %5, t;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], [a2], d2, %5, t;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], [a3], d3, %5, t;\n\t"
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t"
+      "and.pred q, q, q2;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(d_tmem), "r"(a_tmem), "r"(bdesc_lo), "r"(bdesc_hi), "r"(idesc), "r"(accum0), "r"(done), "r"(next), "r"(nph), "r"(next2)
       : "memory");
+  return r;
 }
 __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
   asm volatile(
@@ -406,24 +413,32 @@ __device__ __forceinline__ void umma_nvf4(uint32_t d_tmem, uint64_t adesc, uint6
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum), "r"(sfa_tmem), "r"(sfb_tmem)
       : "memory");
 }
-// The four K = 16 UMMAs of one 64-wide operand stage, both operands through shared-memory descriptors given as low words
-// (address >> 4, advancing by 2 = 32 bytes per step) and one common high word; `accum0` = 0 clears the accumulator first.
-__device__ __forceinline__ void umma_f16_ss_x4(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
-                                               uint32_t accum0) {
+// One 64-wide operand stage in one block: the four K = 16 UMMAs, the commit that frees the stage (on `done`), and a test of the
+// NEXT stage's barrier (`next`, parity `nph`), whose latency the UMMAs' issue hides; returns whether that phase is complete.
+// Both operands through shared-memory descriptors given as low words (address >> 4, advancing by 2 = 32 bytes per step) and one
+// common high word; `accum0` = 0 clears the accumulator first.
+__device__ __forceinline__ uint32_t umma_f16_ss_stage(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                                      uint32_t accum0, uint32_t done, uint32_t next, uint32_t nph) {
+  uint32_t r;
   asm volatile(
-      "{\n\t.reg .pred p, t;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
+      "{\n\t.reg .pred p, t, q;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
       "setp.eq.b32 t, 0, 0;\n\t"
-      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t"
-      "add.u32 x, %1, 2;\n\tadd.u32 y, %2, 2;\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, t;\n\t"
-      "add.u32 x, %1, 4;\n\tadd.u32 y, %2, 4;\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, t;\n\t"
-      "add.u32 x, %1, 6;\n\tadd.u32 y, %2, 6;\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, t;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accum0)
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%8], %9;\n\t"
+      "mov.b64 da, {%2, %4};\n\tmov.b64 db, {%3, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %5, p;\n\t"
+      "add.u32 x, %2, 2;\n\tadd.u32 y, %3, 2;\n\tmov.b64 da, {x, %4};\n\tmov.b64 db, {y, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %5, t;\n\t"
+      "add.u32 x, %2, 4;\n\tadd.u32 y, %3, 4;\n\tmov.b64 da, {x, %4};\n\tmov.b64 db, {y, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %5, t;\n\t"
+      "add.u32 x, %2, 6;\n\tadd.u32 y, %3, 6;\n\tmov.b64 da, {x, %4};\n\tmov.b64 db, {y, %4};\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%1], da, db, %5, t;\n\t"
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%7];\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accum0), "r"(done), "r"(next), "r"(nph)
       : "memory");
+  return r;
 }
 // One whole NVFP4 operand stage (four 64-element k-blocks) in one block: eight scale-factor copies shared memory ->
 // tensor memory (4 columns per k-block and operand), then four block-scaled UMMAs.  Descriptors are given as low

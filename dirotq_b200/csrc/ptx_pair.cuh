@@ -105,66 +105,85 @@ __device__ __forceinline__ void umma_nvf4_pair(uint32_t d_tmem, uint64_t adesc, 
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum), "r"(sfa_tmem), "r"(sfb_tmem)
       : "memory");
 }
-// Four of these in one block: descriptors as low words (advancing by 2 = 32 bytes per k-block) with one high word, the
-// scale factors 4 (activations) and SFB (weights) columns apart; `accum0` = 0 clears the accumulator first.
+// A whole operand stage in one block: the four UMMAs, the commit that frees the stage in both CTAs (on `done`), and a test of the
+// NEXT stage's barrier (`next`, parity `nph`), whose latency the UMMAs' issue hides; returns whether that phase is complete.
+// Descriptors as low words (address >> 4, advancing by 2 = 32 bytes per step) with one high word; `accum0` = 0 clears the
+// accumulator first.  FP4: the scale factors 4 (activations) and SFB (weights) columns apart.
 template <int SFB>
-__device__ __forceinline__ void umma_nvf4_x4_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
-                                                  uint32_t accum0, uint32_t sfa, uint32_t sfb) {
+__device__ __forceinline__ uint32_t umma_nvf4_stage_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                                         uint32_t accum0, uint32_t sfa, uint32_t sfb, uint32_t done, uint32_t next,
+                                                         uint32_t nph) {
+  uint32_t r;
   asm volatile(
-      "{\n\t.reg .pred p, t;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y, u, v;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
+      "{\n\t.reg .pred p, t, q;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y, u, v;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
       "setp.eq.b32 t, 0, 0;\n\t"
-      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], da, db, %4, [%6], [%7], p;\n\t"
-      "add.u32 x, %1, 2;\n\tadd.u32 y, %2, 2;\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t"
-      "add.u32 u, %6, 4;\n\tadd.u32 v, %7, %8;\n\t"
-      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], da, db, %4, [u], [v], t;\n\t"
-      "add.u32 x, %1, 4;\n\tadd.u32 y, %2, 4;\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t"
-      "add.u32 u, %6, 8;\n\tadd.u32 v, %7, %9;\n\t"
-      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], da, db, %4, [u], [v], t;\n\t"
-      "add.u32 x, %1, 6;\n\tadd.u32 y, %2, 6;\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t"
-      "add.u32 u, %6, 12;\n\tadd.u32 v, %7, %10;\n\t"
-      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], da, db, %4, [u], [v], t;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accum0), "r"(sfa), "r"(sfb), "n"(SFB), "n"(2 * SFB), "n"(3 * SFB)
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%8], %9;\n\t"
+      "mov.b64 da, {%2, %4};\n\tmov.b64 db, {%3, %4};\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%1], da, db, %5, [%11], [%12], p;\n\t"
+      "add.u32 x, %2, 2;\n\tadd.u32 y, %3, 2;\n\tmov.b64 da, {x, %4};\n\tmov.b64 db, {y, %4};\n\t"
+      "add.u32 u, %11, 4;\n\tadd.u32 v, %12, %13;\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%1], da, db, %5, [u], [v], t;\n\t"
+      "add.u32 x, %2, 4;\n\tadd.u32 y, %3, 4;\n\tmov.b64 da, {x, %4};\n\tmov.b64 db, {y, %4};\n\t"
+      "add.u32 u, %11, 8;\n\tadd.u32 v, %12, %14;\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%1], da, db, %5, [u], [v], t;\n\t"
+      "add.u32 x, %2, 6;\n\tadd.u32 y, %3, 6;\n\tmov.b64 da, {x, %4};\n\tmov.b64 db, {y, %4};\n\t"
+      "add.u32 u, %11, 12;\n\tadd.u32 v, %12, %15;\n\t"
+      "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%1], da, db, %5, [u], [v], t;\n\t"
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%7], %10;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accum0), "r"(done), "r"(next), "r"(nph), "h"((uint16_t)3), "r"(sfa),
+        "r"(sfb), "n"(SFB), "n"(2 * SFB), "n"(3 * SFB)
       : "memory");
+  return r;
 }
-// The four K = 16 pair UMMAs of one 64-wide bf16 operand stage, both operands through shared-memory descriptors given as
-// low words (address >> 4, advancing by 2 = 32 bytes per step) and one common high word; `accum0` = 0 clears the
-// accumulator first.
-__device__ __forceinline__ void umma_f16_ss_x4_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
-                                                    uint32_t accum0) {
+__device__ __forceinline__ uint32_t umma_f16_ss_stage_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc,
+                                                           uint32_t accum0, uint32_t done, uint32_t next, uint32_t nph) {
+  uint32_t r;
   asm volatile(
-      "{\n\t.reg .pred p, t;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
+      "{\n\t.reg .pred p, t, q;\n\t.reg .b64 da, db;\n\t.reg .b32 x, y;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
       "setp.eq.b32 t, 0, 0;\n\t"
-      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, p;\n\t"
-      "add.u32 x, %1, 2;\n\tadd.u32 y, %2, 2;\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, t;\n\t"
-      "add.u32 x, %1, 4;\n\tadd.u32 y, %2, 4;\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, t;\n\t"
-      "add.u32 x, %1, 6;\n\tadd.u32 y, %2, 6;\n\tmov.b64 da, {x, %3};\n\tmov.b64 db, {y, %3};\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %4, t;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accum0)
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%8], %9;\n\t"
+      "mov.b64 da, {%2, %4};\n\tmov.b64 db, {%3, %4};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%1], da, db, %5, p;\n\t"
+      "add.u32 x, %2, 2;\n\tadd.u32 y, %3, 2;\n\tmov.b64 da, {x, %4};\n\tmov.b64 db, {y, %4};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%1], da, db, %5, t;\n\t"
+      "add.u32 x, %2, 4;\n\tadd.u32 y, %3, 4;\n\tmov.b64 da, {x, %4};\n\tmov.b64 db, {y, %4};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%1], da, db, %5, t;\n\t"
+      "add.u32 x, %2, 6;\n\tadd.u32 y, %3, 6;\n\tmov.b64 da, {x, %4};\n\tmov.b64 db, {y, %4};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%1], da, db, %5, t;\n\t"
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%7], %10;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accum0), "r"(done), "r"(next), "r"(nph), "h"((uint16_t)3)
       : "memory");
+  return r;
 }
-// The four K = 16 pair UMMAs of one 64-wide operand stage, A from the tensor memory of both CTAs (each holds its own 128
-// rows at the same columns, 8 per step), B through a shared-memory descriptor (each CTA holds N/2 rows at the same offset).
-__device__ __forceinline__ void umma_f16_ts_x4_pair(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc_lo, uint32_t bdesc_hi,
-                                                    uint32_t idesc, uint32_t accum0) {
+// A from the tensor memory of both CTAs (each holds its own 128 rows at the same columns, 8 per step), B through a shared-memory
+// descriptor (each CTA holds N/2 rows at the same offset)
+__device__ __forceinline__ uint32_t umma_f16_ts_stage_pair(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc_lo, uint32_t bdesc_hi,
+                                                           uint32_t idesc, uint32_t accum0, uint32_t done, uint32_t next, uint32_t nph) {
+  uint32_t r;
   asm volatile(
-      "{\n\t.reg .pred p, t;\n\t.reg .b64 d0, d1, d2, d3;\n\t.reg .b32 l1, l2, l3, a1, a2, a3;\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
+      "{\n\t.reg .pred p, t, q;\n\t.reg .b64 d0, d1, d2, d3;\n\t.reg .b32 l1, l2, l3, a1, a2, a3;\n\t"
+      "setp.ne.b32 p, %6, 0;\n\t"
       "setp.eq.b32 t, 0, 0;\n\t"
-      "add.u32 l1, %2, 2;\n\tadd.u32 l2, %2, 4;\n\tadd.u32 l3, %2, 6;\n\t"
-      "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
-      "mov.b64 d0, {%2, %3};\n\tmov.b64 d1, {l1, %3};\n\tmov.b64 d2, {l2, %3};\n\tmov.b64 d3, {l3, %3};\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], d0, %4, p;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], d1, %4, t;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a2], d2, %4, t;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a3], d3, %4, t;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(bdesc_lo), "r"(bdesc_hi), "r"(idesc), "r"(accum0)
+      "mbarrier.test_wait.parity.shared::cta.b64 q, [%8], %9;\n\t"
+      "add.u32 l1, %3, 2;\n\tadd.u32 l2, %3, 4;\n\tadd.u32 l3, %3, 6;\n\t"
+      "add.u32 a1, %2, 8;\n\tadd.u32 a2, %2, 16;\n\tadd.u32 a3, %2, 24;\n\t"
+      "mov.b64 d0, {%3, %4};\n\tmov.b64 d1, {l1, %4};\n\tmov.b64 d2, {l2, %4};\n\tmov.b64 d3, {l3, %4};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%1], [%2], d0, %5, p;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%1], [a1], d1, %5, t;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%1], [a2], d2, %5, t;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%1], [a3], d3, %5, t;\n\t"
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%7], %10;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(d_tmem), "r"(a_tmem), "r"(bdesc_lo), "r"(bdesc_hi), "r"(idesc), "r"(accum0), "r"(done), "r"(next), "r"(nph), "h"((uint16_t)3)
       : "memory");
+  return r;
 }
 
 }  // namespace dq

@@ -744,7 +744,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     if (rank == 0) {
       int s = 0, buf = 0, stages = 0, accs = 0;
       uint32_t ph = 0, aph = 0;
-      bool ok = true;
+      bool ok = true, ready = false;                       // ready: the next stage is known to be full
       const uint64_t op_d0 = smem_desc_sw128(smem_base);
       const uint32_t op_lo0 = (uint32_t)op_d0, op_hi = (uint32_t)(op_d0 >> 32);
       for (int t = first; t < total_tiles && ok; t += step) {
@@ -757,23 +757,21 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * 256;
         for (int kc = kb; kc < ke; ++kc) {
-          if (!mbar_wait_warp(full_bar(s), ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+          if (!ready && !mbar_wait_warp(full_bar(s), ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
-          // descriptors from loop-invariant words; the stage's four UMMAs in one block (what this warp does between
-          // UMMAs is time the tensor pipe idles)
-          const uint32_t a_lo = op_lo0 + (uint32_t)s * (RQ_STAGE_BYTES >> 4);
-          if (elect_one()) {
-            if constexpr (PAIR) {
-              umma_f16_ss_x4_pair(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u);
-              umma_commit_pair_both(empty_bar(s));
-            } else {
-              umma_f16_ss_x4(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u);
-              umma_commit(empty_bar(s));
-            }
-          }
-          __syncwarp();
-          ++stages;
+          // descriptors from loop-invariant words; the stage's four UMMAs, their commit and a test of the next stage's barrier in
+          // one block (what this warp does between UMMAs is time the tensor pipe idles)
+          const uint32_t a_lo = op_lo0 + (uint32_t)s * (RQ_STAGE_BYTES >> 4), done = empty_bar(s);
           if (++s == RQ_STAGES) { s = 0; ph ^= 1; }
+          uint32_t next = 0u;
+          if (elect_one()) {
+            if constexpr (PAIR)
+              next = umma_f16_ss_stage_pair(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u, done, full_bar(s), ph);
+            else
+              next = umma_f16_ss_stage(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u, done, full_bar(s), ph);
+          }
+          ready = __any_sync(0xffffffffu, next != 0u);
+          ++stages;
         }
         if (!ok) break;
         if (elect_one()) {
