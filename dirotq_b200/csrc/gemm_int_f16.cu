@@ -453,7 +453,9 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         if (lane == 0) exp_ready(es);
         return true;
       };
-      auto release_raw = [&]() {                              // what this warp needs of the raw stage is in registers
+      // Only once instructions that use what was read have been issued: an arrival overtakes shared-memory loads that still wait in
+      // their queue, behind stores of the quantising epilogue for instance, and the next copy would overwrite what they read.
+      auto release_raw = [&]() {
         __syncwarp();
         if (lane == 0) mbar_arrive(rawe_bar(r.s));
         r.next();
@@ -482,7 +484,6 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
               p0[u] = gf_lds128(rb0 + ((((c0 & 1) * 4 + u) ^ (rowA & 7)) << 4));
               p1[u] = has1 ? gf_lds128(rb1 + ((((c1 & 1) * 4 + u) ^ (rowA & 7)) << 4)) : z4;
             }
-            release_raw();
             expand_bytes32(p0, ka0, y);
             expand_bytes32(p1, ka1, y + 16);
           } else {
@@ -490,17 +491,17 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
             const int sw = rowA & 7;
             const uint4 p0 = gf_lds128(rb + (((2 * c0) ^ sw) << 4));
             const uint4 p1 = has1 ? gf_lds128(rb + (((2 * c1) ^ sw) << 4)) : z4;
-            release_raw();
             expand_nibbles32<ASYM>(p0, ka0, y);
             expand_nibbles32<ASYM>(p1, ka1, y + 16);
           }
           if (!deliver(q0 + j0, y)) { ok = false; break; }
+          release_raw();
           continue;
         }
         // (Single CTAs, with the weight producer as a whole warp and the issuer's early tests, us: 512 x 12288 x 3072 64.3 -> 56.5, 4096 x
         // 4608 x 1152 50.4 -> 44, 1024 x 2240 x 2240 17.2 -> 15.6; long launches on pairs, which the UMMAs bound, 0.5 %.)
         // 4-bit codes: two 16-byte pieces of the swizzled 128-byte raw row; 8-bit codes: 64 bytes of this row = four pieces of box
-        // j >> 1.  Both stages' codes are read before the first is expanded, and the raw stage goes back to its producer.
+        // j >> 1.  Both stages' codes are read before the first is expanded.
         constexpr int PC = A8 ? 4 : 2;
         auto fetch = [&](int j, uint4 (&p)[PC]) {
 #pragma unroll
@@ -525,13 +526,13 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           k1 = record(sraw, j1);
           fetch(j1, p1);
         }
-        release_raw();
         expand(p0, k0);
         if (!deliver(q0 + j0, y)) { ok = false; break; }
         if (j1 < njc) {
           expand(p1, k1);
           if (!deliver(q0 + j1, y)) { ok = false; break; }
         }
+        release_raw();
       }
       // tail: the activations' bf16 tile arrives in the raw ring; its rows, divided by rs (exact; for pairs the folding kernel
       // has done that), go to TMEM like an expanded chunk
@@ -546,7 +547,6 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           const uint4 v = gf_lds128(rb + (uint32_t)((i ^ (rowA & 7)) << 4));
           y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
         }
-        release_raw();
         if constexpr (!PAIR) {
           const __nv_bfloat162 inv2 = __float2bfloat162_rn(inv);
 #pragma unroll
@@ -556,6 +556,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           }
         }
         if (!deliver(qq, y)) { ok = false; break; }
+        release_raw();
       }
     }
     if (PAIR && lane == 0) {
