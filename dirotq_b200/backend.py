@@ -310,10 +310,11 @@ def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
 
 
 def _reads_records(st: LayerState) -> bool:
-    """Whether this integer layer's GEMM reads folded scales, for the rows of its last call (before any call: counted as if)."""
-    lib = _lib.lib()
-    asked = lib.dirotq_linear_chain_folds_scales if _hands_on(st) else lib.dirotq_linear_folds_scales
-    return st.rows == 0 or bool(asked(C.byref(st.c_struct()), st.rows))
+    """Whether this integer layer's GEMM reads folded scales, for the rows of its last call (before any call: counted as if):
+    members of a group that share activations without being one GEMM, in long calls."""
+    if st.shared is None or _hands_on(st):
+        return False
+    return st.rows == 0 or bool(_lib.lib().dirotq_linear_folds_scales(C.byref(st.c_struct()), st.rows))
 
 
 def _hands_on(st: LayerState) -> bool:

@@ -411,8 +411,8 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
     a.q_mode = qo->mode;
     a.q_clip = qo->clip;
   }
-  const bool records = gemm_int_f16_wants_records(a, qo != nullptr);
-  if (records && have && *have) {
+  const bool records = have && gemm_int_f16_takes_records(a, qo != nullptr);
+  if (records && *have) {
     if (!w_panel) {
       int rc = launch_expand_weight_panel(static_cast<const uint8_t*>(w_codes), n_chunks, N, w_mult, ws + c.panel, st, hc);
       if (rc) return rc;
@@ -430,7 +430,7 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
                                       ws + c.rec, reinterpret_cast<float*>(ws + c.rs), tail_in, tail_s, tp, st);
       if (rc) return rc;
     }
-    if (have) *have = 1;
+    *have = 1;
   } else {
     if (!w_panel) {
       int rc = launch_expand_weight_panel(static_cast<const uint8_t*>(w_codes), n_chunks, N, w_mult, ws + c.panel, st, hc);
@@ -668,19 +668,15 @@ int dirotq_linear_uses_half_chunks(const dirotq_linear* lin) {
   return (uses_f16_gemm(lin, g) && half_chunk_geometry(g)) ? 1 : 0;
 }
 
-static int folds_scales(const dirotq_linear* lin, int64_t M, bool quantise_out) {
+int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M) {
   ActGeom g;
   if (!lin || M <= 0 || make_geom(&lin->fmt, &g) || !uses_f16_gemm(lin, g)) return 0;
   GemmIntF16Args a;
   a.M = M;
   a.N = lin->out_features;
-  a.n_chunks = g.n_chunks;
-  a.kt = g.tail_total;
-  a.half_chunks = half_chunk_geometry(g) ? 1 : 0;
-  return gemm_int_f16_wants_records(a, quantise_out) ? 1 : 0;
+  return gemm_int_f16_takes_records(a, false) ? 1 : 0;
 }
-int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M) { return folds_scales(lin, M, false); }
-int dirotq_linear_chain_folds_scales(const dirotq_linear* lin, int64_t M) { return folds_scales(lin, M, true); }
+int dirotq_linear_chain_folds_scales(const dirotq_linear*, int64_t) { return 0; }
 
 int dirotq_linear_chain_supported(const dirotq_linear* lin, const dirotq_linear* next) {
   if (!lin || !next) return 0;

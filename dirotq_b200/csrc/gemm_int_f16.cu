@@ -29,20 +29,20 @@
 //     per row = one TMEM lane) store the fp16 values straight into tensor memory, and the UMMA takes A
 //     from TMEM, B from smem.
 //
-// Data flow per persistent CTA (128 x BN output tiles, K walked in 64-wide chunks):
+// Data flow per persistent CTA (128 x BN output tiles, K walked in 64-wide units, one or two to an operand stage):
 //   TMA (A)        4-bit codes (four chunks = 128 B per row per stage, 128-byte swizzle) + the chunks' scales and zero
-//                  points, or (pairs) the records a folding kernel made of them (bulk copies) -> "raw" ring
-//   TMA (B)        one BN x 64 fp16 tile of the panel (or of the bf16 tail weights) per operand stage, straight
-//                  into the stage's 128-byte-swizzled K-major slot as soon as the UMMAs that read it retire
-//   converter warps  two groups of four taking alternate chunks; a warp expands 32 activation rows into TMEM
+//                  points, or (REC) the records a folding kernel made of them (bulk copies) -> "raw" ring
+//   TMA (B)        BN x 64 fp16 tiles of the panel (or of the bf16 tail weights), one per unit, straight into the stage's
+//                  128-byte-swizzled K-major slot as soon as the UMMAs that read it retire
+//   converter warps  two groups of four taking alternate stages; a warp expands 32 activation rows into TMEM
 //                  (tcgen05.st); for a tail stage it copies the bf16 rows from the raw ring instead
 //   UMMA issuer    tcgen05.mma kind::f16 (A from TMEM, B from smem descriptor), 4 x K=16 per chunk, fp32
 //                  128 x BN accumulator in TMEM; the bf16 tail accumulates into the same tile
 //   8 epilogue warps  tcgen05.ld, * rs[m] * cs[n], + bias, bf16 in registers, accumulator handed back, then 32 x 32 staging
 //                  patches -> TMA stores.  128-wide tiles have two accumulators, wider ones one (the columns it leaves hold
-//                  eight stages of activations)
-// PAIR (256-wide tiles of long launches): clusters of two CTAs drive one tcgen05.mma.cta_group::2 on a 256 x 256 tile.  Each
-// CTA converts its own 128 rows into its own tensor memory, fetches half of the weight tile (the tensor core reads the other
+//                  eight units of activations)
+// PAIR (192- and 256-wide tiles): clusters of two CTAs drive one tcgen05.mma.cta_group::2 on a 256-row tile, which halves the
+// weight traffic and issues one UMMA for two SMs.  Each CTA converts its own 128 rows into its own tensor memory, fetches half of the weight tile (the tensor core reads the other
 // half from the peer's shared memory) and runs the epilogue of its 128 rows.  One barrier per stage in the leader counts the
 // weight bytes of both CTAs and one arrival per converter warp of both (from the peer without memory ordering: their payload
 // is tensor memory); commits arrive in both CTAs; accumulator-empty in the leader counts the epilogue warps of both.
@@ -77,32 +77,40 @@ constexpr int GF_EPI_WARPS = 8;
 
 // A chunk of a 128-row tile is four conversion units of 32 rows (a thread per row = TMEM lane); a group is
 // the four warps that cover the four lane quarters.
-template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
+template <int BN, bool A8 = false, bool PAIR = false, bool REC = false> struct GfCfg {
+  // 64-wide pieces of K ("units") per operand stage.  A stage costs every role a wait (a barrier test takes 110 cycles even when the
+  // phase is complete) and the issuer, all in all, 270 cycles besides its UMMAs, which narrow tiles do not hide: two units (us, one /
+  // two: 512 x 12288 x 3072 on 128 columns 56.5 / 48.7, 4096 x 4608 x 1152 44 / 39.3, 4096 x 1152 x 1152 16.8 / 15.6; 8192 x 2240 x
+  // 2240 on 192 67.6 / 65.5).  256-wide tiles do hide them and would rather have eight small stages in flight than four large ones (16384 x
+  // 2240 x 2240 113.9 / 117.2, 32768 x 1152 x 3456 197 / 206).
+  static constexpr int UNITS = BN == 256 ? 1 : 2;
   static constexpr int GROUP_WARPS = 4;
   static constexpr int GROUPS = GF_GROUPS;
   static constexpr int CONV_WARPS = GROUPS * GROUP_WARPS;
   // Warpgroups: epilogue (warps 0..7), issuer and the two producers (8..11, the last one idle), converters (12..19).  The
   // launch gives every thread 96 registers; the producers' and converters' groups hand some back to the epilogue's, which
   // holds a quarter row of the tile (64 registers of bf16 pairs) besides the piece in work and the one being fetched.
-  // On pairs the issuer's whole-warp form spills with 128 / 48 / 88 (52 bytes a thread stored, 124 loaded) and not with 120 / 80 / 80:
-  // 32768 x 1152 x 3456 205 -> 201 us, 16384 x 2240 x 2240 122.5 -> 120, half chunks 160 -> 157.  Single CTAs spill 24 bytes with
-  // the former and are slower all the same with 120 or 128 / 64 to 80 / 80: 4096 x 4608 x 1152 50.0 -> 52.0.
+  // Epilogue / issuer and producers / converters.  On pairs 128 / 48 / 88 spills 52 bytes a thread in the issuer and 120 / 80 / 80 does
+  // not (32768 x 1152 x 3456 205 -> 201 us); 8-bit converters hold twice the codes and take 88 from the producers (32768 x 1152 x 3456
+  // 208.9 with 80 / 80, 210.5 with 112 / 80 / 88, 206.9 with 120 / 64 / 88).  128-wide tiles spill 24 bytes with 128 / 48 / 88 and are no
+  // faster with 128 / 64 / 80 or 120 / 80 / 80 (1024 x 2240 x 2240 14.3 / 14.8).
   static constexpr int THREADS = (GF_EPI_WARPS + 4 + CONV_WARPS) * 32;
-  static constexpr int REGS_LAUNCH = 96, REGS_EPI = PAIR ? 120 : 128, REGS_PROD = PAIR ? 80 : 48, REGS_CONV = PAIR ? 80 : 88;
+  static constexpr int REGS_LAUNCH = 96, REGS_EPI = PAIR ? 120 : 128, REGS_PROD = !PAIR ? 48 : A8 ? 64 : 80, REGS_CONV = PAIR && !A8 ? 80 : 88;
   static_assert(GF_EPI_WARPS * REGS_EPI + 4 * REGS_PROD + CONV_WARPS * REGS_CONV <= THREADS / 32 * REGS_LAUNCH,
                 "setmaxnreg draws on the registers of the launch");
   static constexpr int BN_OWN = PAIR ? BN / 2 : BN;         // weight rows this CTA fetches
   static constexpr int B_EXP = BN_OWN * 128;               // BN_OWN rows x 64 halves
-  static constexpr int EXP_STAGE = B_EXP;                  // only the weight operand is staged in shared memory
+  static constexpr int EXP_STAGE = UNITS * B_EXP;          // only the weight operand is staged in shared memory
+  static constexpr int A_COLS = UNITS * 32;                // tensor-memory columns of a stage's activations
   static constexpr int RAW_A = 128 * 32 * GF_CPS * (A8 ? 2 : 1);   // 8-bit activation codes: two 128-byte boxes per row
-  static constexpr int OFF_C = RAW_A;                      // pairs: [chunk][128] 8-byte records; else [chunk][128] bf16 scales
+  static constexpr int OFF_C = RAW_A;                      // REC: [chunk][128] 8-byte records; else [chunk][128] bf16 scales
   static constexpr int OFF_Z = OFF_C + GF_CPS * 128 * 2;   // and as many zero points
   static constexpr int RAW_STAGE = OFF_C + GF_CPS * 128 * 8;
   // Accumulators: two of 128 columns (the next tile's UMMAs overlap the epilogue); a wider tile has one, and its
   // UMMAs wait until the epilogue has read the previous tile out of tensor memory.
   static constexpr int NACC = BN > 128 ? 1 : 2;
   // Operand stages in flight: every tensor-memory column the accumulators leave free holds activations
-  // (32 columns per 64-wide chunk), as far as shared memory holds the weight tiles beside them.
+  // (32 columns per unit), as far as shared memory holds the weight tiles beside them.
   static constexpr int RAW_STAGES = GF_RAW_DEF;
   static constexpr int STG_BYTES = GF_EPI_WARPS * 2048;     // per epilogue warp: 32 rows x 32 bf16 output staging
   static constexpr int PIECES = BN / 32;                    // 16-column pieces of an epilogue warp
@@ -113,7 +121,7 @@ template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
   static constexpr int ROW_TILES = 4;
   static constexpr int ROW_BYTES = ROW_TILES * 128 * 4;
   static_assert(ROW_TILES >= RAW_STAGES + 2, "a slot of the row table may still be in use");
-  static constexpr int EXP_TMEM = (512 - NACC * BN) / 32;
+  static constexpr int EXP_TMEM = (512 - NACC * BN) / A_COLS;
   static constexpr int BAR_BYTES = 384;                     // barriers, tensor-memory address, failure words
   static constexpr int EXP_SMEM = (232448 - 1024 - BAR_BYTES - STG_BYTES - TAB_BYTES - ROW_BYTES - RAW_STAGES * RAW_STAGE) / EXP_STAGE;
   static constexpr int EXP_CAP = EXP_TMEM < GF_EXP_MAX ? EXP_TMEM : GF_EXP_MAX;
@@ -122,8 +130,8 @@ template <int BN, bool A8 = false, bool PAIR = false> struct GfCfg {
   static constexpr int NBARS = 2 * RAW_STAGES + 3 * EXP_STAGES + 4 + ROW_TILES;
   static_assert(NBARS * 8 + 4 + AB_WORDS * 4 <= BAR_BYTES && CONV_WARPS <= AB_WORDS - AB_WARP, "barrier area");
   static constexpr int TMEM_A0 = NACC * BN;                 // first column of the activation operand slots
-  static constexpr int TMEM_COLS = 512;                     // accumulators + EXP_STAGES x 32 columns of A
-  static_assert(NACC * BN + EXP_STAGES * 32 <= 512 && EXP_STAGES >= 2, "tensor memory");
+  static constexpr int TMEM_COLS = 512;                     // accumulators + EXP_STAGES x A_COLS columns of A
+  static_assert(NACC * BN + EXP_STAGES * A_COLS <= 512 && EXP_STAGES >= 2, "tensor memory");
   static_assert(SMEM_BYTES <= 232448, "shared memory");
   static_assert(RAW_A >= 128 * 128 && GF_CPS == 4, "a raw stage must hold one 128 x 64 bf16 tail tile of the activations");
 };
@@ -264,8 +272,8 @@ __device__ __forceinline__ uint32_t scale_pair(uint32_t v0, uint32_t v1, float r
 }
 
 // After a wait ran out, by all threads (of both CTAs of a pair) once the roles have stopped: await what is in flight.
-template <int BN, bool A8, bool PAIR>
-__device__ __forceinline__ void gf_teardown(uint8_t* bars, int* status) {
+template <int BN, bool A8, bool PAIR, typename F>
+__device__ __forceinline__ void gf_teardown(uint8_t* bars, F half_of, int* status) {
   using Cfg = GfCfg<BN, A8, PAIR>;
   constexpr int GF_EXP_STAGES = Cfg::EXP_STAGES, GF_RAW_STAGES = Cfg::RAW_STAGES;
   constexpr int W_MMA = GF_EPI_WARPS, W_TMA = GF_EPI_WARPS + 1, W_TMB = GF_EPI_WARPS + 2, W_CONV = GF_EPI_WARPS + 4;
@@ -299,7 +307,7 @@ __device__ __forceinline__ void gf_teardown(uint8_t* bars, int* status) {
       for (int n = ab[AB_WARP + cw]; n < upto; ++n)
         if (n % Cfg::GROUPS == grp) mbar_arrive_cluster_relaxed(fb + 8u * (n % GF_EXP_STAGES));
     }
-    if (warp == W_TMB && one && cta == 0) drain_pair_ring(expf, GF_EXP_STAGES, own, peer, upto, Cfg::B_EXP, status);
+    if (warp == W_TMB && one && cta == 0) drain_pair_ring(expf, GF_EXP_STAGES, own, peer, upto, half_of, status);
   } else if (warp == W_TMB && one) {
     drain_ring(expw, GF_EXP_STAGES, own, status);
   }
@@ -320,7 +328,7 @@ __device__ __forceinline__ void gf_teardown(uint8_t* bars, int* status) {
 
 // AMODE: 0 = signed 4-bit activation codes, 1 = unsigned 4-bit with zero points, 2 = unsigned 8-bit with zero points
 // PAIR: see the head of this file
-template <int BN, int AMODE, bool PAIR>
+template <int BN, int AMODE, bool PAIR, bool REC>
 __global__ void __launch_bounds__(GfCfg<BN, AMODE == 2, PAIR>::THREADS, 1)
 gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   constexpr bool ASYM = AMODE != 0, A8 = AMODE == 2;
@@ -379,9 +387,12 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   const uint32_t raw_base = smem_u32(raw_area);
 
   const int n_raw = a.n_chunks;                                    // chunks of codes in the raw stream
-  const bool hc = a.half_chunks != 0;                              // two half-padded chunks per operand stage
-  const int n_main = hc ? (a.n_chunks + 1) >> 1 : a.n_chunks;      // operand stages of codes
+  const bool hc = a.half_chunks != 0;                              // two half-padded chunks per unit
+  const int n_main = hc ? (a.n_chunks + 1) >> 1 : a.n_chunks;      // units of codes
   const int n_tail = (a.kt + 63) >> 6;
+  constexpr int UNITS = Cfg::UNITS;
+  const int s_main = (n_main + UNITS - 1) / UNITS, ns = s_main + (n_tail + UNITS - 1) / UNITS;    // operand stages
+  auto units_of = [&](int st) { return UNITS == 1 ? 1 : min(2, st < s_main ? n_main - 2 * st : n_tail - 2 * (st - s_main)); };
   const int n_tiles_n = (int)((a.N + BN - 1) / BN);
   constexpr int TILE_M = PAIR ? 256 : 128;
   const int n_tiles_m = (int)((a.M + TILE_M - 1) / TILE_M);
@@ -413,6 +424,8 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
     const int grp = cw / GW;
     const int quarter = warp & 3;
     const int rowA = quarter * 32 + lane;
+    constexpr bool LATE = A8 && UNITS == 2;
+    const uint32_t never = (uint32_t)a.half_chunks & 0x100u;      // half_chunks is 0 or 1
     GfRing<GF_RAW_STAGES> r;
     int q = 0;
     bool ok = true;
@@ -425,89 +438,114 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
     int tile_no = 0;
     for (int t = first; t < total_tiles && ok; t += step, ++tile_no) {
       float inv = 0.f;
-      if constexpr (!PAIR) {
+      if constexpr (!REC) {
         const int rslot = tile_no % Cfg::ROW_TILES;
         if (!mbar_wait_hot_warp(rows_bar(rslot), (uint32_t)((tile_no / Cfg::ROW_TILES) & 1), abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         inv = gf_lds_f32(smem_u32(row_area) + (uint32_t)(rslot * 128 + rowA) * 4);
       }
       auto record = [&](uint32_t sraw, int j) {             // chunk j of a raw stage, this thread's row
-        if constexpr (PAIR) return gf_lds64(sraw + Cfg::OFF_C + j * 128 * 8 + rowA * 8);
+        if constexpr (REC) return gf_lds64(sraw + Cfg::OFF_C + j * 128 * 8 + rowA * 8);
         const uint32_t at = sraw + (uint32_t)(j * 128 + rowA) * 2;
         const float s = __uint_as_float(gf_lds16(at + Cfg::OFF_C) << 16);
         if constexpr (ASYM) return chunk_record(s, __uint_as_float(gf_lds16(at + Cfg::OFF_Z) << 16), inv);
         const uint32_t m = half_twice(s * (inv * 16777216.f));       // s has 8 bits: exact, so 8 s / rs may be taken from it
         return make_uint2(m, hmul2_m8(m));
       };
-      // A stage's values, in registers, go to tensor memory as soon as the slot is free.  (The empty statement keeps the expansion in
-      // front of the wait: the compiler would move it behind, onto the path between "slot free" and "stage ready".)
-      auto deliver = [&](int qq, uint32_t (&y)[32]) {
+      // Only once what was read has arrived in registers: an arrival overtakes shared-memory loads that still wait in their queue, behind
+      // stores of the quantising epilogue for instance, and the next copy would overwrite what they read.  Either instructions
+      // that use it have been issued, or the arrival's own address depends on it (`read`, a word of every load, under a mask that
+      // is zero for reasons the compiler does not know).
+      auto release_raw = [&](uint32_t read = 0u) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(rawe_bar(r.s) + (read & never));
+        r.next();
+      };
+      // A unit's values, in registers, go to tensor memory, the first of a stage as soon as the slot is free.  (The empty statement
+      // keeps the expansion in front of the wait: the compiler would move it behind, onto the path between "slot free" and
+      // "stage ready".)
+      auto slot_free = [&](int qq, uint32_t (&y)[32]) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) asm volatile("" : "+r"(y[i]));
-        const int es = exp_slot(qq);
-        if (!mbar_wait_hot_warp(expe_bar(es), exp_phase(qq) ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { q = qq; return false; }
+        if (!mbar_wait_hot_warp(expe_bar(exp_slot(qq)), exp_phase(qq) ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { q = qq; return false; }
         tc_fence_after();
-        tmem_st32(tmem_base + ((uint32_t)(quarter * 32) << 16) + Cfg::TMEM_A0 + es * 32, y);
+        return true;
+      };
+      auto put = [&](int qq, int unit, uint32_t (&y)[32]) {
+        tmem_st32(tmem_base + ((uint32_t)(quarter * 32) << 16) + Cfg::TMEM_A0 + exp_slot(qq) * Cfg::A_COLS + unit * 32, y);
+      };
+      auto stage_done = [&](int qq) {
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) exp_ready(es);
-        return true;
-      };
-      // Only once instructions that use what was read have been issued: an arrival overtakes shared-memory loads that still wait in
-      // their queue, behind stores of the quantising epilogue for instance, and the next copy would overwrite what they read.
-      auto release_raw = [&]() {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(rawe_bar(r.s));
-        r.next();
+        if (lane == 0) exp_ready(exp_slot(qq));
       };
       for (int c = 0; c < n_raw && ok; c += GF_CPS) {
         if (!mbar_wait_hot_warp(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
         const uint32_t sraw = raw_base + r.s * Cfg::RAW_STAGE;
         const int nv = min(GF_CPS, n_raw - c);
-        const int njc = hc ? (nv + 1) >> 1 : nv;               // operand stages this raw stage feeds
-        const int q0 = q, j0 = (grp ^ q) & 1, j1 = j0 + 2;     // this group's: j0 and j1, where they exist
-        q += njc;
-        if (j0 >= njc) { release_raw(); continue; }
+        const int nu = hc ? (nv + 1) >> 1 : nv, nst = (nu + UNITS - 1) / UNITS;   // units and operand stages this raw stage feeds
+        const int j = (grp ^ q) & 1, qq = q + j;               // this group's first stage of them, if there is one
+        q += nst;
+        if (j >= nst) { release_raw(); continue; }
+        const int u0 = UNITS * j, u1 = UNITS == 2 ? u0 + 1 : u0 + 2;    // its units: of one stage, or of two stages
+        const bool two = u1 < nu;
         uint32_t y[32];
         if (hc) {
-          // half chunks: the first 32 slots of chunks 2 j0 and 2 j0 + 1, each with its own record, side by side
-          const int c0 = 2 * j0, c1 = 2 * j0 + 1;
-          const bool has1 = c1 < nv;
-          const uint2 ka0 = record(sraw, c0);
-          const uint2 ka1 = has1 ? record(sraw, c1) : make_uint2(0u, 0u);
-          const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
-          if constexpr (A8) {
-            const uint32_t rb0 = sraw + (c0 >> 1) * (128 * 128) + rowA * 128, rb1 = sraw + (c1 >> 1) * (128 * 128) + rowA * 128;
-            uint4 p0[4], p1[4];
+          // half chunks: the first 32 slots of chunks 2 u and 2 u + 1, each with its own record, side by side
+          constexpr int PC = A8 ? 2 : 1;
+          auto fetch = [&](int ch, uint4 (&p)[PC]) {           // (slots past the last chunk: codes 0 under a record of zeros)
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              p0[u] = gf_lds128(rb0 + ((((c0 & 1) * 4 + u) ^ (rowA & 7)) << 4));
-              p1[u] = has1 ? gf_lds128(rb1 + ((((c1 & 1) * 4 + u) ^ (rowA & 7)) << 4)) : z4;
+            for (int u = 0; u < PC; ++u)
+              p[u] = ch >= nv ? make_uint4(0u, 0u, 0u, 0u)
+                     : A8     ? gf_lds128(sraw + (ch >> 1) * (128 * 128) + rowA * 128 + ((((ch & 1) * 4 + u) ^ (rowA & 7)) << 4))
+                              : gf_lds128(sraw + rowA * 128 + (((2 * ch) ^ (rowA & 7)) << 4));
+            return ch < nv ? record(sraw, ch) : make_uint2(0u, 0u);
+          };
+          auto expand = [&](const uint4 (&p)[PC], uint2 k, uint32_t* d) {
+            if constexpr (A8) expand_bytes32(p, k, d);
+            else expand_nibbles32<ASYM>(p[0], k, d);
+          };
+          uint4 p0[PC], p1[PC], p2[PC], p3[PC];
+          const uint2 k0 = fetch(2 * u0, p0), k1 = fetch(2 * u0 + 1, p1);
+          uint2 k2, k3;
+          auto fetch1 = [&]() {
+            if constexpr (UNITS == 2) { k2 = fetch(2, p2), k3 = fetch(3, p3); }
+          };
+          if constexpr (!LATE) {
+            fetch1();
+            uint32_t read = k0.x ^ k1.x;
+#pragma unroll
+            for (int i = 0; i < PC; ++i) read ^= p0[i].x ^ p1[i].x;
+            if constexpr (UNITS == 2) {
+              read ^= k2.x ^ k3.x;
+#pragma unroll
+              for (int i = 0; i < PC; ++i) read ^= p2[i].x ^ p3[i].x;
             }
-            expand_bytes32(p0, ka0, y);
-            expand_bytes32(p1, ka1, y + 16);
-          } else {
-            const uint32_t rb = sraw + rowA * 128;
-            const int sw = rowA & 7;
-            const uint4 p0 = gf_lds128(rb + (((2 * c0) ^ sw) << 4));
-            const uint4 p1 = has1 ? gf_lds128(rb + (((2 * c1) ^ sw) << 4)) : z4;
-            expand_nibbles32<ASYM>(p0, ka0, y);
-            expand_nibbles32<ASYM>(p1, ka1, y + 16);
+            release_raw(read);
           }
-          if (!deliver(q0 + j0, y)) { ok = false; break; }
-          release_raw();
+          expand(p0, k0, y);
+          expand(p1, k1, y + 16);
+          if (!slot_free(qq, y)) { ok = false; break; }
+          put(qq, 0, y);
+          if (UNITS == 2 && two) {
+            if constexpr (LATE) fetch1();
+            expand(p2, k2, y);
+            expand(p3, k3, y + 16);
+            put(qq, 1, y);
+          }
+          if constexpr (LATE) release_raw();
+          stage_done(qq);
           continue;
         }
-        // (Single CTAs, with the weight producer as a whole warp and the issuer's early tests, us: 512 x 12288 x 3072 64.3 -> 56.5, 4096 x
-        // 4608 x 1152 50.4 -> 44, 1024 x 2240 x 2240 17.2 -> 15.6; long launches on pairs, which the UMMAs bound, 0.5 %.)
         // 4-bit codes: two 16-byte pieces of the swizzled 128-byte raw row; 8-bit codes: 64 bytes of this row = four pieces of box
-        // j >> 1.  Both stages' codes are read before the first is expanded.
+        // u0 >> 1.  Both units' codes are read before the first is expanded; 8-bit codes, twice the registers, one after the
+        // other in stages of two units.
         constexpr int PC = A8 ? 4 : 2;
-        auto fetch = [&](int j, uint4 (&p)[PC]) {
+        auto fetch = [&](int u, uint4 (&p)[PC]) {
 #pragma unroll
-          for (int u = 0; u < PC; ++u)
-            p[u] = A8 ? gf_lds128(sraw + (j >> 1) * (128 * 128) + rowA * 128 + ((((j & 1) * 4 + u) ^ (rowA & 7)) << 4))
-                      : gf_lds128(sraw + rowA * 128 + (((2 * j + u) ^ (rowA & 7)) << 4));
+          for (int i = 0; i < PC; ++i)
+            p[i] = A8 ? gf_lds128(sraw + (u >> 1) * (128 * 128) + rowA * 128 + ((((u & 1) * 4 + i) ^ (rowA & 7)) << 4))
+                      : gf_lds128(sraw + rowA * 128 + (((2 * u + i) ^ (rowA & 7)) << 4));
         };
         auto expand = [&](const uint4 (&p)[PC], uint2 k) {
           if constexpr (A8) {
@@ -519,44 +557,72 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           }
         };
         uint4 p0[PC], p1[PC];
-        const uint2 k0 = record(sraw, j0);
-        fetch(j0, p0);
+        const uint2 k0 = record(sraw, u0);
+        fetch(u0, p0);
         uint2 k1 = make_uint2(0u, 0u);
-        if (j1 < njc) {
-          k1 = record(sraw, j1);
-          fetch(j1, p1);
+        auto fetch1 = [&]() {
+          if (two) {
+            k1 = record(sraw, u1);
+            fetch(u1, p1);
+          }
+        };
+        if constexpr (!LATE) {
+          fetch1();
+          uint32_t read = k0.x ^ k1.x;
+#pragma unroll
+          for (int i = 0; i < PC; ++i) read ^= two ? p0[i].x ^ p1[i].x : p0[i].x;
+          release_raw(read);
         }
         expand(p0, k0);
-        if (!deliver(q0 + j0, y)) { ok = false; break; }
-        if (j1 < njc) {
-          expand(p1, k1);
-          if (!deliver(q0 + j1, y)) { ok = false; break; }
-        }
-        release_raw();
-      }
-      // tail: the activations' bf16 tile arrives in the raw ring; its rows, divided by rs (exact; for pairs the folding kernel
-      // has done that), go to TMEM like an expanded chunk
-      for (int st = 0; st < n_tail && ok; ++st) {
-        if (!mbar_wait_hot_warp(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
-        const int qq = q++;
-        if (((qq ^ grp) & 1) != 0) { release_raw(); continue; }
-        const uint32_t rb = raw_base + r.s * Cfg::RAW_STAGE + rowA * 128;
-        uint32_t y[32];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint4 v = gf_lds128(rb + (uint32_t)((i ^ (rowA & 7)) << 4));
-          y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
-        }
-        if constexpr (!PAIR) {
-          const __nv_bfloat162 inv2 = __float2bfloat162_rn(inv);
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const __nv_bfloat162 h = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&y[i]), inv2);
-            y[i] = *reinterpret_cast<const uint32_t*>(&h);
+        if (!slot_free(qq, y)) { ok = false; break; }
+        put(qq, 0, y);
+        if constexpr (UNITS == 2) {
+          if constexpr (LATE) fetch1();
+          if (two) {
+            expand(p1, k1);
+            put(qq, 1, y);
+          }
+          if constexpr (LATE) release_raw();
+          stage_done(qq);
+        } else {
+          stage_done(qq);
+          if (two) {
+            expand(p1, k1);
+            if (!slot_free(qq + 2, y)) { ok = false; break; }
+            put(qq + 2, 0, y);
+            stage_done(qq + 2);
           }
         }
-        if (!deliver(qq, y)) { ok = false; break; }
-        release_raw();
+      }
+      // tail: the activations' bf16 tiles arrive in the raw ring, a unit each; their rows, divided by rs (exact; with records the
+      // folding kernel has done that), go to TMEM like expanded chunks
+      for (int st = 0; st < n_tail && ok; st += UNITS) {
+        const int qq = q++;
+        const bool mine = ((qq ^ grp) & 1) == 0;
+        for (int u = 0; u < min(UNITS, n_tail - st); ++u) {
+          if (!mbar_wait_hot_warp(rawf_bar(r.s), r.ph, abort_flag, a.status, ERR_WAIT_FULL)) { q = qq; ok = false; break; }
+          if (!mine) { release_raw(); continue; }
+          const uint32_t rb = raw_base + r.s * Cfg::RAW_STAGE + rowA * 128;
+          uint32_t y[32];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const uint4 v = gf_lds128(rb + (uint32_t)((i ^ (rowA & 7)) << 4));
+            y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
+          }
+          if constexpr (!REC) {
+            const __nv_bfloat162 inv2 = __float2bfloat162_rn(inv);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              const __nv_bfloat162 h = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(&y[i]), inv2);
+              y[i] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+          }
+          if (u == 0 && !slot_free(qq, y)) { ok = false; break; }
+          put(qq, u, y);
+          release_raw();
+        }
+        if (!ok) break;
+        if (mine) stage_done(qq);
       }
     }
     if (PAIR && lane == 0) {
@@ -580,7 +646,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         const int m0 = tm_ * TILE_M + (int)rank * 128;
         // the second half of a pair's last tile may lie past the end: codes arrive as zero fill, and the records (bulk
         // copies know no bounds) are those of the last row block; none of its rows is ever stored
-        const int64_t mrec = PAIR ? min((int64_t)m0, a.ld_rec - 128) : (int64_t)m0;
+        const int64_t mrec = REC ? min((int64_t)m0, a.ld_rec - 128) : (int64_t)m0;
         for (int c = 0; c < n_raw; c += GF_CPS) {
           if (!mbar_wait_hot(rawe_bar(r.s), r.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
           const uint32_t sb = raw_base + r.s * Cfg::RAW_STAGE;
@@ -591,8 +657,8 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           const bool second_box = A8 && nv > 2;
           // boxes of scales are counted whole, zero fill included
           mbar_expect_tx(bar, (uint32_t)(Cfg::RAW_A - ((A8 && !second_box) ? 128 * 128 : 0) +
-                                         (PAIR ? nv * 128 * 8 : (ASYM ? 2 : 1) * GF_CPS * 128 * 2)));
-          if constexpr (!PAIR) {
+                                         (REC ? nv * 128 * 8 : (ASYM ? 2 : 1) * GF_CPS * 128 * 2)));
+          if constexpr (!REC) {
             tma_load_2d(sb + Cfg::OFF_C, &tm.xs, bar, m0, c);
             if constexpr (ASYM) tma_load_2d(sb + Cfg::OFF_Z, &tm.xz, bar, m0, c);
           }
@@ -602,7 +668,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           } else {
             tma_load_2d(sb, &tm.xq, bar, c * 32, m0);
           }
-          if constexpr (PAIR)
+          if constexpr (REC)
             for (int j = 0; j < nv; ++j)
               bulk_load(sb + Cfg::OFF_C + j * 128 * 8, a.a_const + ((int64_t)(c + j) * a.ld_rec + mrec), 128 * 8, bar);
           ++issued;
@@ -629,7 +695,6 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
     int issued = 0;
     bool ok = true;
     const uint32_t full_lead = PAIR ? map_to_rank(expf_bar(0), 0) : 0u;   // the bytes of both halves are counted in the leader
-    const int ns = n_main + n_tail;
     for (int t = first; t < total_tiles && ok; t += step) {
       int tm_, tn_;
       tile_mn(t, tm_, tn_);
@@ -638,16 +703,18 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         if (!mbar_wait_hot_warp(expe_bar(e.s), e.ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
         if (elect_one()) {
           const uint32_t dst = exp_base + e.s * Cfg::EXP_STAGE;
+          const int nu = units_of(st), x = (st < s_main ? st : st - s_main) * (UNITS * 64);
+          const CUtensorMap* const map = st < s_main ? &tm.wp : &tm.wt;
           if constexpr (PAIR) {
             const uint32_t bar = full_lead + 8u * e.s;
-            if (rank == 0) mbar_expect_tx(expf_bar(e.s), 2 * Cfg::B_EXP);
-            if (st < n_main) tma_load_2d_pair(dst, &tm.wp, bar, st * 64, row_b);
-            else tma_load_2d_pair(dst, &tm.wt, bar, (st - n_main) * 64, row_b);
+            if (rank == 0) mbar_expect_tx(expf_bar(e.s), (uint32_t)(2 * nu * Cfg::B_EXP));
+            tma_load_2d_pair(dst, map, bar, x, row_b);
+            if (nu == 2) tma_load_2d_pair(dst + Cfg::B_EXP, map, bar, x + 64, row_b);
           } else {
             const uint32_t bar = expw_bar(e.s);
-            mbar_expect_tx(bar, Cfg::B_EXP);                   // the box is counted whole, zero fill included
-            if (st < n_main) tma_load_2d(dst, &tm.wp, bar, st * 64, row_b);
-            else tma_load_2d(dst, &tm.wt, bar, (st - n_main) * 64, row_b);
+            mbar_expect_tx(bar, (uint32_t)(nu * Cfg::B_EXP));  // boxes are counted whole, zero fill included
+            tma_load_2d(dst, map, bar, x, row_b);
+            if (nu == 2) tma_load_2d(dst + Cfg::B_EXP, map, bar, x + 64, row_b);
           }
         }
         __syncwarp();
@@ -674,7 +741,6 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
       const uint32_t bdesc_lo0 = (uint32_t)bdesc0, bdesc_hi = (uint32_t)(bdesc0 >> 32);
       constexpr uint32_t kDescStep = Cfg::EXP_STAGE >> 4;
       const uint32_t a_tmem0 = tmem_base + Cfg::TMEM_A0;
-      const int ns = n_main + n_tail;
       for (int t = first; t < total_tiles && ok; t += step) {
         const int buf = Cfg::NACC == 2 ? (use & 1) : 0;
         const uint32_t acc_ph = (uint32_t)(Cfg::NACC == 2 ? (use >> 1) & 1 : use & 1);
@@ -689,14 +755,22 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           if (!ready && (PAIR ? !mbar_wait_hot_warp(w - kFullOff, ph, abort_flag, a.status, ERR_WAIT_FULL)
                               : !mbar_wait2_hot_warp(w, ph, w - kFullOff, ph, abort_flag, a.status, ERR_WAIT_FULL))) { ok = false; break; }
           tc_fence_after();
-          const uint32_t a_t = a_tmem0 + 32u * es, b_lo = bdesc_lo0 + kDescStep * es;
+          uint32_t a_t = a_tmem0 + (uint32_t)Cfg::A_COLS * es, b_lo = bdesc_lo0 + kDescStep * es;
           if (++es == GF_EXP_STAGES) { es = 0; ph ^= 1u; }
           const uint32_t wn = expw0 + 8u * es;
           uint32_t next = 0u;
           if (elect_one()) {
-            const uint32_t idesc = st < n_main ? idesc_h : idesc_bf;
-            if constexpr (PAIR) next = umma_f16_ts_stage_pair(d, a_t, b_lo, bdesc_hi, idesc, st > 0 ? 1u : 0u, w - kEmptyOff, wn - kFullOff, ph);
-            else next = umma_f16_ts_stage(d, a_t, b_lo, bdesc_hi, idesc, st > 0 ? 1u : 0u, w - kEmptyOff, wn, ph, wn - kFullOff);
+            const uint32_t idesc = st < s_main ? idesc_h : idesc_bf;
+            uint32_t acc = st > 0 ? 1u : 0u;
+            if (units_of(st) == 2) {
+              if constexpr (PAIR) umma_f16_ts_x4_pair(d, a_t, b_lo, bdesc_hi, idesc, acc);
+              else umma_f16_ts_x4(d, a_t, b_lo, bdesc_hi, idesc, acc);
+              a_t += 32u;
+              b_lo += Cfg::B_EXP >> 4;
+              acc = 1u;
+            }
+            if constexpr (PAIR) next = umma_f16_ts_stage_pair(d, a_t, b_lo, bdesc_hi, idesc, acc, w - kEmptyOff, wn - kFullOff, ph);
+            else next = umma_f16_ts_stage(d, a_t, b_lo, bdesc_hi, idesc, acc, w - kEmptyOff, wn, ph, wn - kFullOff);
           }
           ready = __any_sync(0xffffffffu, next != 0u);
           ++stages;
@@ -762,7 +836,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         w16[e] = *reinterpret_cast<const uint32_t*>(&h);
       }
     };
-    // Single CTAs: a row's power of two comes from its largest chunk scale.  These warps have time while a tile's UMMAs run, so
+    // Without records a row's power of two comes from its largest chunk scale.  These warps have time while a tile's UMMAs run, so
     // they read the scales one tile ahead and leave 1 / rs for the converters in the tile's slot of a table (see ROW_TILES).  The
     // first tile waits for it: 16-byte loads, eight rows of eight chunks each per warp instruction, 96 chunks in flight.  With
     // 2-byte loads of a row per lane, 24 in flight, every call began with a chain of them: 512 x 12288 x 3072 79.5 -> 63.9 us, 4096 x
@@ -772,7 +846,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
       int tm_, tn_;
       tile_mn(t, tm_, tn_);
       // this lane: rows r8 .. r8 + 7 of the warp's 32, chunks lane / 4 + 8 i (scales are 16-byte aligned, ldm a multiple of eight)
-      const int64_t r8 = (int64_t)tm_ * TILE_M + q * 32 + (lane & 3) * 8;
+      const int64_t r8 = (int64_t)tm_ * TILE_M + (int)rank * 128 + q * 32 + (lane & 3) * 8;
       const __nv_bfloat16* const s8 = a.xs + r8;
       uint32_t m[4] = {0u, 0u, 0u, 0u};
 #pragma unroll 1
@@ -818,14 +892,14 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
     int use = 0;
     bool ok = true;
     float rs_next = 0.f;
-    if constexpr (!PAIR)
+    if constexpr (!REC)
       if (first < total_tiles) rs_next = row_powers(first);
     for (int t = first; t < total_tiles && ok; t += step) {
       int tm_, tn_;
       tile_mn(t, tm_, tn_);
       const int m0 = tm_ * TILE_M + (int)rank * 128, n0 = tn_ * BN;
       const int64_t row = (int64_t)m0 + trow;
-      const float rs = !PAIR ? rs_next : (row < a.M) ? __ldg(a.rs + row) : 0.f;
+      const float rs = !REC ? rs_next : (row < a.M) ? __ldg(a.rs + row) : 0.f;
       __syncwarp();                                  // every lane has read the previous tile's table
       for (int i = lane; i < Cfg::PIECES * 8; i += 32) { // one column pair each
         const int64_t col = (int64_t)n0 + ch * CW + 2 * i;
@@ -837,7 +911,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         }
         gf_sts64(tab + i * 8, cp, bp);
       }
-      if constexpr (!PAIR)
+      if constexpr (!REC)
         if (t + step < total_tiles) rs_next = row_powers(t + step);
       const int buf = Cfg::NACC == 2 ? (use & 1) : 0;
       const uint32_t acc_ph = (uint32_t)(Cfg::NACC == 2 ? (use >> 1) & 1 : use & 1);
@@ -933,7 +1007,13 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
   volatile int* const ab = reinterpret_cast<volatile int*>(end_bars + 8 * Cfg::NBARS) + 1;
   if (ab[AB_FLAG]) {                // a wait ran out (in both CTAs of a pair the flag is up)
     regs_even<Cfg::REGS_LAUNCH>(end_warp < GF_EPI_WARPS);
-    gf_teardown<BN, A8, PAIR>(end_bars, a.status);
+    // bytes that each CTA of a pair fetches for stage q of the kernel-wide sequence
+    auto half_of = [&](int q) {
+      constexpr int U = Cfg::UNITS;
+      const int nm = a.half_chunks ? (a.n_chunks + 1) >> 1 : a.n_chunks, nt = (a.kt + 63) >> 6, sm = (nm + U - 1) / U, st = q % (sm + (nt + U - 1) / U);
+      return (uint32_t)(min(U, st < sm ? nm - U * st : nt - U * (st - sm)) * Cfg::B_EXP);
+    };
+    gf_teardown<BN, A8, PAIR>(end_bars, half_of, a.status);
   }
   if (end_warp == W_MMA) {
     __syncwarp();
@@ -1178,10 +1258,10 @@ int launch_fold_weight_scales(const float* s, int n_chunks, int64_t N, int64_t l
   return cudaGetLastError() == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
 }
 
-template <int BN, int AMODE, bool PAIR>
+template <int BN, int AMODE, bool PAIR, bool REC = false>
 static int launch_gf(const GfMaps& tm, const GemmIntF16Args& a, cudaStream_t st) {
   using Cfg = GfCfg<BN, AMODE == 2, PAIR>;
-  auto k = gemm_int_f16_kernel<BN, AMODE, PAIR>;
+  auto k = gemm_int_f16_kernel<BN, AMODE, PAIR, REC>;
   static PerDeviceOnce attr_once, regs_once;
   if (int rc = set_max_dynamic_smem(attr_once, k, Cfg::SMEM_BYTES)) return rc;
   if (int rc = check_compiled_regs(regs_once, k, Cfg::REGS_LAUNCH)) return rc;
@@ -1219,34 +1299,28 @@ static int launch_gf(const GfMaps& tm, const GemmIntF16Args& a, cudaStream_t st)
   return launch_pdl(k, dim3(grid), dim3(Cfg::THREADS), Cfg::SMEM_BYTES, st, tm, a) == cudaSuccess ? DIROTQ_OK : DIROTQ_E_CUDA;
 }
 
-// Column-tile width.  The persistent grid runs ceil(tiles / SMs) rounds, and a round of 256-wide tiles takes about 9/7 of a
-// round of 128-wide ones whatever K is (the converters' work for a stage does not depend on the width, and the wide tile's
-// single accumulator is handed back before anything else is done with it).  So 256 wherever it saves a quarter of the rounds (us,
-// 256 / 128 columns: 1152 -> 3456 at 32768 rows 213 / 298, 1152 -> 4608 at 4096 37.7 / 56.5), 128 where both need the same few
-// (1152 x 1152 at 4096 rows, two of either: 20.5 / 18.4; 2240 x 2240 at 1024, one: 18.4 / 17.2).  A round of
-// 192-wide tiles takes 6/5 of a 128-wide one: ahead where it needs no more rounds than 256 (192 / 256: 1152 x 1152 at 12288 rows,
-// four of either, 33.6 / 36.1, 8-bit activations 34.0 / 37.3; 1152 -> 3456 at 3072 26.6 / 28.7).  From five rounds on, where
-// 256-wide tiles run on CTA pairs behind the folding kernel, for short K: 1152 x 1152 at 15360 rows 40.1 / 47.1.  That line was
-// drawn when both forms paid the folding kernel (4608 -> 1152 139 / 137); now that single CTAs do not, 192 is ahead there too,
-// 127 / 138, 8-bit 134 / 142.  The quantise-out epilogue wants whole groups of 64 columns per warp: not 192.
-// DIROTQ_GF_BN overrides.
-static int pick_bn_f16(int64_t M, int64_t N, int64_t k_total, bool qout) {
+// Column-tile width.  The persistent grid runs whole rounds of tiles, over 148 CTAs with 128-wide tiles and 74 CTA pairs (256 rows) with
+// wider ones.  A round takes 225 / 250 / 320 ns per 64-wide unit of K (128 / 192 / 256 columns) and 1.0 / 1.4 / 1.5 us besides: what a
+// stage costs the roles hardly depends on the width, the UMMAs do, and a wide tile's single accumulator has to be handed back.
+// Launch, first loads and last epilogue add 4.5 / 5.5 / 6 us.  The smallest sum is taken; measured (us, 128 / 192 / 256 columns): 256 x
+// 1152 x 1152 9.4 / 11.1 / 12.7, 1024 x 2240 x 2240 14.3 / 16.8 / 18.9, 4096 x 4608 x 1152 39.3 / 43.8 / 53.3, 3995 x 1152 x 4608 45.5 / 41.0 /
+// 37.3, 8192 x 2240 x 2240 75 / 65.5 / 59.4, 32768 x 1152 x 1152 85.6 / 71.7 / 73.3, 4608 x 3072 x 3072 73.8 / 60.6 / 59.4.
+// Calls of at most 128 rows would leave half of each pair idle.  The quantise-out epilogue wants whole groups of 64 columns per
+// warp: not 192.  DIROTQ_GF_BN overrides.
+static int pick_bn_f16(int64_t M, int64_t N, int64_t units, bool qout) {
   if (const char* e = getenv("DIROTQ_GF_BN")) return atoi(e) <= 128 ? 128 : atoi(e) <= 192 && !qout ? 192 : 256;
-  const int64_t m_tiles = (M + 127) / 128, sms = num_sms();
-  auto rounds = [&](int64_t bn) { return (m_tiles * ((N + bn - 1) / bn) + sms - 1) / sms; };
-  const int64_t r256 = rounds(256), r192 = rounds(192), r128 = rounds(128);
-  if (!qout && r192 == r256 && 6 * r192 < 5 * r128 && (r256 <= 4 || k_total < 2048)) return 192;
-  return 9 * r256 < 7 * r128 ? 256 : 128;
-}
-
-// CTA pairs halve the weight traffic of a 256-wide tile and issue one UMMA for two SMs (us, pair with its folding kernel / single:
-// 1152 -> 3456 at 32768 rows 201 / 213, 1152 -> 4608 259 / 277, 3072 -> 9216 at 4608 176 / 184, 8-bit 184 / 194).  Their tiles are
-// twice as tall, so the last round is coarser, and a stage's hand-off crosses the pair: 22.9 / 20.5 for 1152 x 1152 at 4096 rows (two
-// rounds), 39.3 / 37.7 for 1152 -> 4608 (four), 77.0 / 75.8 for 32768 x 1152 (nine).  Hence only from five rounds on.  DIROTQ_GF_PAIR
-// overrides (0 or 1).
-static bool pick_pair_f16(int64_t M, int64_t N) {
-  if (const char* e = getenv("DIROTQ_GF_PAIR")) return atoi(e) != 0;
-  return ((M + 127) / 128) * ((N + 255) / 256) > 4 * (int64_t)num_sms();
+  if (M <= 128) return 128;
+  static const int width[3] = {128, 192, 256}, unit_ns[3] = {225, 250, 320}, tile_ns[3] = {1000, 1400, 1500}, call_ns[3] = {4500, 5500, 6000};
+  const int64_t m128 = (M + 127) / 128, m256 = (M + 255) / 256, sms = num_sms();
+  int best = 128;
+  int64_t best_ns = -1;
+  for (int i = 0; i < 3; ++i) {
+    if (qout && width[i] == 192) continue;
+    const int64_t n = (N + width[i] - 1) / width[i], slots = i ? sms / 2 : sms, rounds = ((i ? m256 : m128) * n + slots - 1) / slots;
+    const int64_t ns = rounds * (units * unit_ns[i] + tile_ns[i]) + call_ns[i];
+    if (best_ns < 0 || ns < best_ns) { best_ns = ns; best = width[i]; }
+  }
+  return best;
 }
 
 // Column tiles per rasterisation group.  With n fastest over the whole width, the CTAs of one round read every weight
@@ -1262,22 +1336,16 @@ static int pick_raster_f16(int BN, int64_t N, int64_t k_total) {
   return (int)(g < 4 ? 4 : g > 16 ? 16 : g);
 }
 
-// Whether a call reads activation records (and row powers of two, and a scaled tail) that the folding kernel has made, or the
-// scales themselves: the former on CTA pairs, the latter in every launch of single CTAs, 128- and 192-wide ones of any length
-// included.  The folding kernel is 2-3 us of launch and latency; the converters' share of the same work is four to ten instructions
-// per row and chunk, which the long launches on pairs, bound by the converters, feel.  Us, folding kernel + GEMM (256 columns) / GEMM
-// alone: 1536 x 12288 x 3072 82.3 / 78.2, and before its scales were read by 16-byte loads (2-8 % more than now) 4608 x 3072 x 3072
-// (three rounds) 63.9 / 62.3, 8192 x 2240 x 2240 64.3 / 61.8, 12288 x 4608 x 1152 115.9 / 112.6, 4096 x 1152 x 4608 39.7 / 38.5;
-// on pairs 32768 x 1152 x 3456 205 / 214, 4608 x 3072 x 12288 238 / 253.  A warp of the GEMM that makes the records for the
-// converters was slower than either (262): its polls and stores take from the same pipes.
-static bool picks_pair(const GemmIntF16Args& a, bool quantise_out, int* bn) {
-  const int64_t n_stage = a.half_chunks ? (a.n_chunks + 1) / 2 : a.n_chunks;
-  *bn = pick_bn_f16(a.M, a.N, n_stage * 64 + ((a.kt + 63) / 64) * 64, quantise_out);
-  return *bn == 256 && pick_pair_f16(a.M, a.N);
-}
-bool gemm_int_f16_wants_records(const GemmIntF16Args& a, bool quantise_out) {
-  int bn;
-  return picks_pair(a, quantise_out, &bn);
+// Whether siblings that share activations without being one GEMM read records (and row powers of two, and a scaled tail) that the
+// folding kernel makes once for all of them; other calls read the scales themselves.  The folding kernel is 2-3 us of launch and
+// latency, its share of the work in the GEMM four to ten instructions per row and chunk of the converters, which have time for them (us,
+// folding kernel + GEMM / GEMM alone, 256 columns: 32768 x 1152 x 3456 199.5 / 197.4, 16384 x 2240 x 2240 120.0 / 113.9, 4608 x 3072 x
+// 3072 63.1 / 59.4, x 12288 232.5 / 230.4; before the converters read a raw stage at once the long launches were 2-4 % slower alone).
+// For long launches (more than four rounds of 148 tiles) of three siblings the two come out even, and a group keeps its records.
+bool gemm_int_f16_takes_records(const GemmIntF16Args& a, bool quantise_out) {
+  if (const char* e = getenv("DIROTQ_GF_BN"))
+    return pick_bn_f16(a.M, a.N, 1, quantise_out) == 256 && !(getenv("DIROTQ_GF_PAIR") && atoi(getenv("DIROTQ_GF_PAIR")) == 0);
+  return a.N > 128 && ((a.M + 127) / 128) * ((a.N + 255) / 256) > 4 * (int64_t)num_sms();
 }
 
 int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
@@ -1289,9 +1357,10 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
     return DIROTQ_E_ALIGN;
   const uint64_t n_stage = a.half_chunks ? (uint64_t)((a.n_chunks + 1) / 2) : (uint64_t)a.n_chunks;
   const int64_t k_total = (int64_t)n_stage * 64 + ((a.kt + 63) / 64) * 64;
-  int BN;
-  const bool pair = picks_pair(a, a.q_codes != nullptr, &BN);
-  if (pair ? !a.a_const || !a.rs : !a.xs) return DIROTQ_E_ARG;
+  const bool rec = a.a_const != nullptr;
+  const int BN = rec ? 256 : pick_bn_f16(a.M, a.N, k_total / 64, a.q_codes != nullptr);
+  const bool pair = BN > 128;
+  if (rec ? !a.rs : !a.xs) return DIROTQ_E_ARG;
   if (a.q_codes) {
     if (a.N % 64 || a.q_len % 64 || a.q_len <= 0 || a.q_len > a.N || a.q_row_bytes < a.q_len / 2 || (a.q_row_bytes & 15) ||
         (a.q_len < a.N && (!a.q_tail || a.q_tail_pitch < a.N - a.q_len || (a.q_tail_pitch & 7) ||
@@ -1307,7 +1376,7 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
                            (uint64_t)a.x_row_bytes, 32 * GF_CPS, 128, 32 * GF_CPS);
   if (rc) return rc;
   tm.xs = tm.xz = tm.xq;
-  if (!pair) {
+  if (!rec) {
     // scales (and zero points): [n_chunks, ldm] bf16, a stage's four chunks of 128 rows in one box
     rc = make_tmap_2d_sw(&tm.xs, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.xs, (uint64_t)a.ldm, (uint64_t)a.n_chunks, (uint64_t)a.ldm * 2,
                          128, GF_CPS, 0);
@@ -1333,20 +1402,13 @@ int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {
     tm.wt = tm.wp;
   }
   const int amode = a.a_mode == DIROTQ_INT4_SYM ? 0 : a.a_mode == DIROTQ_INT4_ASYM ? 1 : 2;
-  if (BN == 256 && pair) {
-    switch (amode) {
-      case 0: return launch_gf<256, 0, true>(tm, a, st);
-      case 1: return launch_gf<256, 1, true>(tm, a, st);
-      case 2: return launch_gf<256, 2, true>(tm, a, st);
-    }
-  }
   switch (BN * 4 + amode) {
-    case 256 * 4 + 0: return launch_gf<256, 0, false>(tm, a, st);
-    case 256 * 4 + 1: return launch_gf<256, 1, false>(tm, a, st);
-    case 256 * 4 + 2: return launch_gf<256, 2, false>(tm, a, st);
-    case 192 * 4 + 0: return launch_gf<192, 0, false>(tm, a, st);
-    case 192 * 4 + 1: return launch_gf<192, 1, false>(tm, a, st);
-    case 192 * 4 + 2: return launch_gf<192, 2, false>(tm, a, st);
+    case 256 * 4 + 0: return rec ? launch_gf<256, 0, true, true>(tm, a, st) : launch_gf<256, 0, true>(tm, a, st);
+    case 256 * 4 + 1: return rec ? launch_gf<256, 1, true, true>(tm, a, st) : launch_gf<256, 1, true>(tm, a, st);
+    case 256 * 4 + 2: return rec ? launch_gf<256, 2, true, true>(tm, a, st) : launch_gf<256, 2, true>(tm, a, st);
+    case 192 * 4 + 0: return launch_gf<192, 0, true>(tm, a, st);
+    case 192 * 4 + 1: return launch_gf<192, 1, true>(tm, a, st);
+    case 192 * 4 + 2: return launch_gf<192, 2, true>(tm, a, st);
     case 128 * 4 + 0: return launch_gf<128, 0, false>(tm, a, st);
     case 128 * 4 + 1: return launch_gf<128, 1, false>(tm, a, st);
     case 128 * 4 + 2: return launch_gf<128, 2, false>(tm, a, st);

@@ -106,7 +106,7 @@ __device__ __forceinline__ void gp_teardown(uint8_t* bars, int* status) {
     for (int n = ab[AB_WARP + (warp & 3)]; n < upto; ++n) mbar_arrive_cluster_relaxed(fb + 8u * (n % STAGES));
   }
   if (warp == 0 && one) {
-    if (cta == 0) drain_pair_ring(full, STAGES, own, peer, upto, Cfg::OP_TX / 2, status);
+    if (cta == 0) drain_pair_ring(full, STAGES, own, peer, upto, [&](int) -> uint32_t { return Cfg::OP_TX / 2; }, status);
     drain_ring(sffull, STAGES, own, status);
   }
   if (warp == 1 && one) {                              // in both CTAs, where the leader's commits arrive

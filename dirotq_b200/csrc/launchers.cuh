@@ -162,7 +162,8 @@ struct GemmIntF16Args {
   int n_chunks;
   const uint8_t* xq;           // activation codes [M, n_chunks * 32]
   int64_t x_row_bytes;
-  // Calls on CTA pairs (gemm_int_f16_wants_records) read what the folding kernel made of the scales, the others the scales
+  // Siblings on CTA pairs (gemm_int_f16_takes_records) read what the folding kernel made of the scales, once for all of them; other
+  // calls the scales
   const uint2* a_const = nullptr;          // [n_chunks, ld_rec] records {s*2^24/rs, -(z*s)/rs}, fp16 pairs
   const float* rs = nullptr;               // [M] row powers of two
   int64_t ld_rec = 0;                      // f16_ld_act(M)
@@ -235,7 +236,7 @@ int launch_gemm_int(const GemmIntArgs& a, cudaStream_t st);
 int launch_gemm_nvfp4(const GemmFp4Args& a, cudaStream_t st);
 int launch_gemm_nvfp4_pair(const GemmFp4Args& a, int bn, cudaStream_t st);
 int launch_gemm_int_f16(const GemmIntF16Args& a, cudaStream_t st);
-bool gemm_int_f16_wants_records(const GemmIntF16Args& a, bool quantise_out);
+bool gemm_int_f16_takes_records(const GemmIntF16Args& a, bool quantise_out);
 int launch_expand_weight_panel(const uint8_t* wq, int n_chunks, int64_t N, const void* rec, void* panel, cudaStream_t st,
                                int half_chunks = 0);
 int launch_fold_act_and_expand(const __nv_bfloat16* s, const __nv_bfloat16* z, int n_chunks, int64_t M, int64_t ldm, void* rec,

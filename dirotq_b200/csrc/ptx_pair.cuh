@@ -55,17 +55,17 @@ __device__ __forceinline__ void mbar_complete_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 // Teardown of a pair's ring after a wait ran out, by the leader's producer thread once both CTAs have stopped.  A stage's
-// barrier (in the leader) expects one arrival with the bytes of both halves, `half` from each CTA; of the stages below
+// barrier (in the leader) expects one arrival with the bytes of both halves, `half_of(stage)` from each CTA; of the stages below
 // `upto` -- as far as any role of either CTA got -- the leader has armed `own` and the peer issued copies for `peer`.
 // What one CTA did and the other did not is made up for, so that every such phase completes exactly when the copies that
 // were issued have landed (the warps that also arrive on these barriers make up for theirs); then the last ring of them
 // is awaited.  No role is more than a ring behind another: a slot is reused only after all arrived for its last stage.
 // (`upto` must not count a stage that a role merely walked past: two stages on one barrier would arrive more often than the
 // phase at hand expects while bytes are missing, which is a fault.)
-template <typename F>
-__device__ __forceinline__ void drain_pair_ring(F bar_of, int slots, int own, int peer, int upto, uint32_t half, int* status) {
-  for (int q = own; q < upto; ++q) mbar_expect_tx(bar_of(q % slots), q < peer ? half : 0u);
-  for (int q = peer; q < own; ++q) mbar_complete_tx(bar_of(q % slots), half);
+template <typename F, typename H>
+__device__ __forceinline__ void drain_pair_ring(F bar_of, int slots, int own, int peer, int upto, H half_of, int* status) {
+  for (int q = own; q < upto; ++q) mbar_expect_tx(bar_of(q % slots), q < peer ? half_of(q) : 0u);
+  for (int q = peer; q < own; ++q) mbar_complete_tx(bar_of(q % slots), half_of(q));
   drain_ring(bar_of, slots, upto, status);
 }
 
@@ -163,6 +163,22 @@ __device__ __forceinline__ uint32_t umma_f16_ss_stage_pair(uint32_t d_tmem, uint
 }
 // A from the tensor memory of both CTAs (each holds its own 128 rows at the same columns, 8 per step), B through a shared-memory
 // descriptor (each CTA holds N/2 rows at the same offset)
+__device__ __forceinline__ void umma_f16_ts_x4_pair(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc_lo, uint32_t bdesc_hi,
+                                                    uint32_t idesc, uint32_t accum0) {
+  asm volatile(
+      "{\n\t.reg .pred p, t;\n\t.reg .b64 d0, d1, d2, d3;\n\t.reg .b32 l1, l2, l3, a1, a2, a3;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "setp.eq.b32 t, 0, 0;\n\t"
+      "add.u32 l1, %2, 2;\n\tadd.u32 l2, %2, 4;\n\tadd.u32 l3, %2, 6;\n\t"
+      "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
+      "mov.b64 d0, {%2, %3};\n\tmov.b64 d1, {l1, %3};\n\tmov.b64 d2, {l2, %3};\n\tmov.b64 d3, {l3, %3};\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], d0, %4, p;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a1], d1, %4, t;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a2], d2, %4, t;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [a3], d3, %4, t;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "r"(bdesc_lo), "r"(bdesc_hi), "r"(idesc), "r"(accum0)
+      : "memory");
+}
 __device__ __forceinline__ uint32_t umma_f16_ts_stage_pair(uint32_t d_tmem, uint32_t a_tmem, uint32_t bdesc_lo, uint32_t bdesc_hi,
                                                            uint32_t idesc, uint32_t accum0, uint32_t done, uint32_t next, uint32_t nph) {
   uint32_t r;

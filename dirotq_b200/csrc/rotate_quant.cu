@@ -828,7 +828,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       const int own = abort_flag[AB_ISSUED];
       if constexpr (PAIR) {
         const int peer = ld_cluster_s32(map_to_rank(abort_addr + 4u * AB_ISSUED, rank ^ 1));
-        if (rank == 0) drain_pair_ring(full_bar, RQ_STAGES, own, peer, max(own, peer), RQ_A_BYTES + bn_own * 128, a.status);
+        if (rank == 0) drain_pair_ring(full_bar, RQ_STAGES, own, peer, max(own, peer), [&](int) -> uint32_t { return RQ_A_BYTES + bn_own * 128; }, a.status);
       } else {
         drain_ring(full_bar, RQ_STAGES, own, a.status);
       }

@@ -324,7 +324,7 @@ int dirotq_linear_gemm(const dirotq_linear* lin, int64_t M, void* y, void* works
                        int32_t* status, void* stream);
 
 /* dirotq_linear_forward (x given) and dirotq_linear_gemm (x NULL) for layers that share activations in one workspace, as above.
- * The GEMM of a long call reads records that a folding kernel makes of the activation scales, in the workspace; *records (the
+ * In long calls these GEMMs read records that a folding kernel makes of the activation scales, in the workspace; *records (the
  * caller's, host memory, one per workspace) says whether it holds those of its codes, so that only the first of the layers
  * that needs them makes them.  Cleared where x is given; not to be changed otherwise. */
 int dirotq_linear_sibling(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace,
@@ -343,8 +343,8 @@ int dirotq_linear_sibling(const dirotq_linear* lin, const void* x, int64_t M, vo
  * quantised part and its 16-bit tail both multiples of 64 channels (the tail may be empty), no
  * rotation, no channel selection, width == lin->out_features, w_mult set.  Anything else: DIROTQ_E_UNSUPPORTED, nothing launched. */
 int dirotq_linear_uses_half_chunks(const dirotq_linear* lin);
-/* Whether a GEMM of `lin` on M rows launches the scale-folding kernel first (long launches of integer layers): alone, or as
- * the producer of dirotq_linear_forward_chain, whose quantising epilogue does not take every tile width. */
+/* Whether dirotq_linear_sibling makes records of the activation scales for `lin` on M rows (long launches of integer layers); the
+ * GEMMs of all other entries read the scales themselves, the chain's among them (always 0). */
 int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M);
 int dirotq_linear_chain_folds_scales(const dirotq_linear* lin, int64_t M);
 int dirotq_linear_chain_supported(const dirotq_linear* lin, const dirotq_linear* next);
