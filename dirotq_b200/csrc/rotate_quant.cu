@@ -31,10 +31,13 @@ constexpr int RQ_A_BYTES = 128 * 128;           // 128 rows x 64 bf16
 // One CTA per tile: the whole rotation tile (up to 256 rows x 64 bf16) per stage, four stages.  CTA pairs
 // (tcgen05 cta_group::2, 256 token rows per pair): each CTA fetches only HALF of the rotation tile -- the tensor core
 // reads the other half from the peer's shared memory -- so a stage is 32 KB instead of 48 and six fit.
-template <bool PAIR> struct RqStage {
-  static constexpr int STAGES = PAIR ? 6 : 4;
-  static constexpr int B_BYTES = (PAIR ? 128 : 256) * 128;
-  static constexpr int STAGE_BYTES = RQ_A_BYTES + B_BYTES;
+// UNITS: 64-wide pieces of K per stage.  A stage costs producer and issuer a barrier test of 110 cycles and more, which the UMMAs of
+// tiles of at most 128 columns do not hide: two units for those (us, one / two: bf16 4096 x 4608 -> 1152 34.8 / 31.6, rotation of 16384 x 1152 on
+// 128 columns 43.8 / 33.6, of 4096 x 1152 13.1 / 12.7; 256 rows, where latencies add up, 7.4 either way).
+template <bool PAIR, int UNITS> struct RqStage {
+  static constexpr int STAGES = UNITS == 2 ? (PAIR ? 4 : 3) : (PAIR ? 6 : 4);
+  static constexpr int B_BYTES = (PAIR ? 128 : 256) / UNITS * 128;
+  static constexpr int UNIT_BYTES = RQ_A_BYTES + B_BYTES, STAGE_BYTES = UNITS * UNIT_BYTES;
 };
 // Epilogue warps per TMEM lane quarter: they take the 64-column chunks (per-head layouts: the heads) of their rows in
 // turns.  The NVFP4 epilogue is the longest (seven threshold compares per value) and latency-bound, and the per-head
@@ -46,7 +49,7 @@ template <bool PAIR> struct RqStage {
 #define RQ_WPQ_PERHEAD 4
 #endif
 constexpr int RQ_TAIL_STAGED = 16;              // high channels per head that go through the staging patch, at most
-template <int EPI, bool PAIR = false> struct RqCfg {
+template <int EPI, bool PAIR = false, int UNITS = 1> struct RqCfg {
   static constexpr int WPQ = (EPI == 2 /* EPI_NVFP4_HIDDEN */) ? RQ_WPQ_NVFP4 : (EPI == 3 || EPI == 4 /* per-head */) ? RQ_WPQ_PERHEAD : 2;
   static constexpr int EPI_WARPS = 4 * WPQ;
   static constexpr int THREADS = (2 + EPI_WARPS) * 32;
@@ -54,7 +57,7 @@ template <int EPI, bool PAIR = false> struct RqCfg {
   // channels of a head of its 32 rows
   static constexpr int STG_WARP = EPI == 0 ? 2048 : EPI == 3 ? 32 * RQ_TAIL_STAGED * 2 : 0;
   static constexpr int STG_BYTES = EPI_WARPS * STG_WARP;
-  static constexpr int SMEM_BYTES = RqStage<PAIR>::STAGES * RqStage<PAIR>::STAGE_BYTES + STG_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int SMEM_BYTES = RqStage<PAIR, UNITS>::STAGES * RqStage<PAIR, UNITS>::STAGE_BYTES + STG_BYTES + 1024 /*align*/ + 256 /*barriers*/;
 };
 
 enum : int { EPI_ROT_ONLY = 0, EPI_INT_HIDDEN = 1, EPI_NVFP4_HIDDEN = 2, EPI_INT_PERHEAD = 3, EPI_NVFP4_PERHEAD = 4 };
@@ -659,11 +662,12 @@ __device__ __forceinline__ void epi_rot_only(const RotArgs& a, const CUtensorMap
 // rows and half of the rotation tile); completions of both CTAs' loads are counted on the leader's full barrier, the
 // leader commits to both CTAs' empty / accumulator-full barriers, epilogue warps of both arrive on the leader's
 // accumulator-empty barrier (the peer's arrivals carry no memory ordering: their payload is tensor memory).
-template <int EPI, int MODE, bool PAIR>
+template <int EPI, int MODE, bool PAIR, int UNITS>
 __global__ void __launch_bounds__(RqCfg<EPI>::THREADS, 1)
 rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_u,
                     const __grid_constant__ CUtensorMap tm_y, const RotArgs a) {
-  constexpr int RQ_STAGES = RqStage<PAIR>::STAGES, RQ_STAGE_BYTES = RqStage<PAIR>::STAGE_BYTES;
+  using Stage = RqStage<PAIR, UNITS>;
+  constexpr int RQ_STAGES = Stage::STAGES, RQ_STAGE_BYTES = Stage::STAGE_BYTES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* stg_area = smem + RQ_STAGES * RQ_STAGE_BYTES;                  // 1024-byte aligned
@@ -705,7 +709,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   const int total_tiles = (PAIR ? (a.m_tiles + 1) / 2 : a.m_tiles) * a.n_tiles;
   const int first = PAIR ? (int)cluster_id_x() : (int)blockIdx.x, step = PAIR ? (int)cluster_count_x() : (int)gridDim.x;
   const int bn_own = PAIR ? a.BN / 2 : a.BN;                 // rotation-tile rows this CTA fetches
-  const uint32_t smem_base = smem_u32(smem);
+  const uint32_t smem_base = smem_u32(smem), stage_tx = UNITS * (RQ_A_BYTES + bn_own * 128);   // a CTA's bytes per stage
 
   if (warp == 0) {
     int s = 0;
@@ -719,19 +723,22 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       const int row_u = nb * a.BN + (int)rank * (tile_width(a, nb) >> 1);   // of a pair, each CTA fetches half of the tile's rows
       int kb, ke;
       tile_k_range(a, nb, kb, ke);
-      for (int kc = kb; kc < ke; ++kc) {
+      for (int kc = kb; kc < ke; kc += UNITS) {
         if (!mbar_wait_warp(empty_bar(s), ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
         if (elect_one()) {
-          const uint32_t sa = smem_base + s * RQ_STAGE_BYTES;
-          if constexpr (PAIR) {
-            const uint32_t fb = map_to_rank(full_bar(s), 0);
-            if (rank == 0) mbar_expect_tx(full_bar(s), 2u * (RQ_A_BYTES + bn_own * 128));
-            tma_load_2d_pair(sa, &tm_x, fb, kc * 64, mb * 128);
-            tma_load_2d_pair(sa + RQ_A_BYTES, &tm_u, fb, kc * 64, row_u);
-          } else {
-            mbar_expect_tx(full_bar(s), RQ_A_BYTES + a.BN * 128);
-            tma_load_2d(sa, &tm_x, full_bar(s), kc * 64, mb * 128);
-            tma_load_2d(sa + RQ_A_BYTES, &tm_u, full_bar(s), kc * 64, row_u);
+          const uint32_t sa = smem_base + s * RQ_STAGE_BYTES, fb = PAIR ? map_to_rank(full_bar(s), 0) : full_bar(s);
+          if (rank == 0) mbar_expect_tx(full_bar(s), (PAIR ? 2u : 1u) * stage_tx);
+#pragma unroll
+          for (int u = 0; u < UNITS; ++u) {
+            const int x = (UNITS == 1 ? kc : min(kc + u, ke - 1)) * 64;    // past the last unit: the last one again, which no UMMA reads
+            const uint32_t su = sa + u * Stage::UNIT_BYTES;
+            if constexpr (PAIR) {
+              tma_load_2d_pair(su, &tm_x, fb, x, mb * 128);
+              tma_load_2d_pair(su + RQ_A_BYTES, &tm_u, fb, x, row_u);
+            } else {
+              tma_load_2d(su, &tm_x, fb, x, mb * 128);
+              tma_load_2d(su + RQ_A_BYTES, &tm_u, fb, x, row_u);
+            }
           }
         }
         __syncwarp();
@@ -756,19 +763,24 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
         if (!mbar_wait_warp(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * 256;
-        for (int kc = kb; kc < ke; ++kc) {
+        for (int kc = kb; kc < ke; kc += UNITS) {
           if (!ready && !mbar_wait_warp(full_bar(s), ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
           // descriptors from loop-invariant words; the stage's four UMMAs, their commit and a test of the next stage's barrier in
           // one block (what this warp does between UMMAs is time the tensor pipe idles)
-          const uint32_t a_lo = op_lo0 + (uint32_t)s * (RQ_STAGE_BYTES >> 4), done = empty_bar(s);
+          uint32_t a_lo = op_lo0 + (uint32_t)s * (RQ_STAGE_BYTES >> 4), acc = kc > kb ? 1u : 0u;
+          const uint32_t done = empty_bar(s);
           if (++s == RQ_STAGES) { s = 0; ph ^= 1; }
           uint32_t next = 0u;
           if (elect_one()) {
-            if constexpr (PAIR)
-              next = umma_f16_ss_stage_pair(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u, done, full_bar(s), ph);
-            else
-              next = umma_f16_ss_stage(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, kc > kb ? 1u : 0u, done, full_bar(s), ph);
+            if (UNITS == 2 && kc + 2 <= ke) {
+              if constexpr (PAIR) umma_f16_ss_x4_pair(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, acc);
+              else umma_f16_ss_x4(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, acc);
+              a_lo += Stage::UNIT_BYTES >> 4;
+              acc = 1u;
+            }
+            if constexpr (PAIR) next = umma_f16_ss_stage_pair(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, acc, done, full_bar(s), ph);
+            else next = umma_f16_ss_stage(d_tmem, a_lo, a_lo + (RQ_A_BYTES >> 4), op_hi, idesc, acc, done, full_bar(s), ph);
           }
           ready = __any_sync(0xffffffffu, next != 0u);
           ++stages;
@@ -828,7 +840,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       const int own = abort_flag[AB_ISSUED];
       if constexpr (PAIR) {
         const int peer = ld_cluster_s32(map_to_rank(abort_addr + 4u * AB_ISSUED, rank ^ 1));
-        if (rank == 0) drain_pair_ring(full_bar, RQ_STAGES, own, peer, max(own, peer), [&](int) -> uint32_t { return RQ_A_BYTES + bn_own * 128; }, a.status);
+        if (rank == 0) drain_pair_ring(full_bar, RQ_STAGES, own, peer, max(own, peer), [&](int) -> uint32_t { return stage_tx; }, a.status);
       } else {
         drain_ring(full_bar, RQ_STAGES, own, a.status);
       }
@@ -869,10 +881,10 @@ int num_sms() {
   return n;
 }
 
-template <int EPI, int MODE, bool PAIR>
+template <int EPI, int MODE, bool PAIR, int UNITS>
 static int launch_rq_impl(const CUtensorMap& tx, const CUtensorMap& tu, const CUtensorMap& ty, const RotArgs& a, cudaStream_t st) {
-  using Cfg = RqCfg<EPI, PAIR>;
-  auto k = rotate_quant_kernel<EPI, MODE, PAIR>;
+  using Cfg = RqCfg<EPI, PAIR, UNITS>;
+  auto k = rotate_quant_kernel<EPI, MODE, PAIR, UNITS>;
   static PerDeviceOnce attr_once;
   if (int rc = set_max_dynamic_smem(attr_once, k, Cfg::SMEM_BYTES)) return rc;
   if constexpr (!PAIR) {
@@ -925,17 +937,12 @@ static int launch_rq(const CUtensorMap& tx, const CUtensorMap& tu, const CUtenso
     if (!strcmp(e, "single")) pair = false;
     else if (!strcmp(e, "pair")) pair = (a.BN / 2) % 8 == 0;
   }
-  if (pair) return launch_rq_impl<EPI, MODE, true>(tx, tu_pair, ty, a, st);
-  return launch_rq_impl<EPI, MODE, false>(tx, tu, ty, a, st);
+  if constexpr (EPI == EPI_ROT_ONLY || EPI == EPI_INT_HIDDEN || EPI == EPI_NVFP4_HIDDEN)
+    if (a.BN <= 128 && a.band == 0)
+      return pair ? launch_rq_impl<EPI, MODE, true, 2>(tx, tu_pair, ty, a, st) : launch_rq_impl<EPI, MODE, false, 2>(tx, tu, ty, a, st);
+  return pair ? launch_rq_impl<EPI, MODE, true, 1>(tx, tu_pair, ty, a, st) : launch_rq_impl<EPI, MODE, false, 1>(tx, tu, ty, a, st);
 }
 
-// Picks the N tile.  Per-head layouts: a whole number of heads (and a multiple of 16 for the UMMA shape).  Hidden
-// layouts: a multiple of 64; the persistent grid runs ceil(tiles / SMs) rounds, and a round costs a part that grows with
-// the tile width (the UMMAs) plus a part that does not (the per-stage barrier protocol of the issuer, the same for every
-// width).  Measured at D = 1152, 32768 rows: 6.03 / 6.68 / 7.59 us per round for 128 / 192 / 256 columns, i.e. the fixed
-// part is worth about 370 columns; the choice minimises rounds x (width + 370) less what narrow last columns save -- padding
-// of D and a nearly empty last round both count (32768 rows of a 1152-wide layer take 256: 68 us against 74 with 192; a 4096-row
-// shard takes 128).
 // The last column of tiles is only as wide as D needs, rounded up to 64 (1152 columns were five tiles of 256, and are four and a
 // half): 32768 x 1152 63.9 -> 62.3 us, 32768 x 4608 -> 1152 in bf16 246 -> 242.  The shared-memory pipe, which the operands
 // pass twice, keeps the gain below the UMMAs saved.
@@ -943,22 +950,29 @@ static int last_width(int D, int bn) {
   const int w = ((D % bn) + 63) & ~63;
   return w == 0 || w > bn ? bn : w;
 }
-int pick_bn(const ActGeom& g, int64_t M) {
+// Picks the N tile.  Per-head layouts: a whole number of heads (and a multiple of 16 for the UMMA shape).  Hidden layouts and
+// plain GEMMs: the persistent grid runs whole rounds over 74 CTA pairs; a round takes 190 / 255 / 335 ns per 64-wide unit of K (128 / 192 /
+// 256 columns) and 0.25 / 0.9 / 0.4 us besides, a call 5.3 / 4.6 / 5.8 us, and a tile of the last column saves 0.44 of the columns it
+// lacks.  The smallest sum is taken; measured (us, 128 / 192 / 256): rotation of 4096 x 1152 12.7 / 14.3 / 16.8, 6000 x 1152 16.0 / 15.6 /
+// 18.0, 16384 x 1152 33.6 / 33.6 / 35.2, 32768 x 1152 66.4 / 61.9 / 61.4, 2048 x 2240 19.3 / 24.2 / 18.8, 4096 x 2240 32.8 / 33.6 / 30.7, 4608 x 3072
+// 59.0 / 55.7 / 56.9, 16384 x 3072 214 / 201 / 198; bf16 4096 x 4608 -> 1152 31.9 / 40.1 / 49.6, 32768 rows 254 / 237 / 241, 1024 x 12288 ->
+// 3072 77.8 / 56.1 / 70.0.
+int pick_bn(const ActGeom& g, int64_t M, int64_t K) {
   if (g.H > 0) {
     int best = 0;
     for (int k = 1; k * g.d <= 256; ++k)
       if ((k * g.d) % 16 == 0) best = k * g.d;
     return best;
   }
-  const int cand[3] = {256, 192, 128};
-  const int64_t m_tiles = (M + 127) / 128, sms = num_sms();
-  int best = 256;
-  int64_t best_cost = -1;
+  static const int width[3] = {128, 192, 256}, unit_ns[3] = {190, 255, 335}, tile_ns[3] = {250, 900, 400}, call_ns[3] = {5300, 4600, 5800};
+  const int64_t m_pairs = (M + 255) / 256, pairs = num_sms() / 2, units = (K + 63) / 64;
+  int best = 128;
+  int64_t best_ns = -1;
   for (int i = 0; i < 3; ++i) {
-    const int64_t tiles = m_tiles * ceil_div(g.D, cand[i]);
-    const int64_t n_tiles = ceil_div(g.D, cand[i]), rounds = (tiles + sms - 1) / sms;
-    const int64_t cost = rounds * (cand[i] + 370) - rounds / n_tiles * (cand[i] - last_width(g.D, cand[i]));
-    if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = cand[i]; }
+    const int64_t n_tiles = ceil_div(g.D, width[i]), rounds = (m_pairs * n_tiles + pairs - 1) / pairs;
+    const int64_t lacks = width[i] - last_width(g.D, width[i]);
+    const int64_t ns = rounds * (units * unit_ns[i] + tile_ns[i]) + call_ns[i] - rounds / n_tiles * units * unit_ns[i] * lacks * 44 / (100 * width[i]);
+    if (best_ns < 0 || ns < best_ns) { best_ns = ns; best = width[i]; }
   }
   return best;
 }
@@ -988,7 +1002,7 @@ int launch_rotate_quantize(const ActGeom& g, const void* x, const void* rot_t, i
   // a tile follows the heads its columns touch either way.
   ActGeom g_tile = g;
   if (rot_only) g_tile.H = 0;
-  a.BN = pick_bn(g_tile, M);
+  a.BN = pick_bn(g_tile, M, g.D);
   if (a.BN <= 0) return DIROTQ_E_UNSUPPORTED;
   a.n_tiles = ceil_div(g.D, a.BN);
   a.bn_last = last_width(g.D, a.BN);
@@ -1044,7 +1058,7 @@ int launch_gemm_bf16(const void* x, const void* w_t, int64_t M, int64_t N, int64
   a.M = M;
   a.K = (int)K;
   a.ldm = ld_rows(M);
-  a.BN = pick_bn(a.g, M);
+  a.BN = pick_bn(a.g, M, K);
   a.n_tiles = ceil_div((int)N, a.BN);
   a.bn_last = last_width((int)N, a.BN);
   a.m_tiles = (int)((M + 127) / 128);
