@@ -68,6 +68,8 @@ SIGNATURES = {
     "dirotq_dequant_weight_nvfp4": (C.c_int, [_I64, _I64, _P, _P, _F, _P, _P, _P]),
     "dirotq_linear_workspace_bytes": (_SZ, [C.POINTER(LinearC), _I64]),
     "dirotq_linear_forward": (C.c_int, [C.POINTER(LinearC), _P, _I64, _P, _P, _SZ, _P, _P]),
+    "dirotq_linear_fuses_hadamard": (C.c_int, [C.POINTER(LinearC), _I32, _I64]),
+    "dirotq_linear_forward_hadamard": (C.c_int, [C.POINTER(LinearC), _P, _I32, _P, _I64, _P, _P, _SZ, _P, _P]),
     "dirotq_linear_gemm": (C.c_int, [C.POINTER(LinearC), _I64, _P, _P, _SZ, _P, _P]),
     "dirotq_linear_sibling": (C.c_int, [C.POINTER(LinearC), _P, _I64, _P, _P, _SZ, C.POINTER(_I32), _P, _P]),
     "dirotq_expand_weight_panel_f16_layout": (C.c_int, [_I32, _I64, _P, _P, _P, _I32, _P]),

@@ -304,9 +304,16 @@ def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
              (f.group_size == 64 or f.mode in (ops.NVFP4_HW, ops.NVFP4_REF)))
     if (st.rot_t is None or two_step) and lay.tail_total > 0 and not follower and not rides:
         n += 1                              # the passthrough channels, where the quantise kernel does not copy them too
-    if st.hadamard_low_dim:
+    if st.hadamard_low_dim and not _fuses_hadamard(st, st.rows or 1 << 20):
         n += 1
     return n
+
+
+def _fuses_hadamard(st: LayerState, M: int) -> bool:
+    """Whether the transform and the quantiser of this Hadamard layer are one launch in a call of M rows."""
+    f = st.hadamard_flips
+    return (st.shared is None and st.chain_next is None and (f is None or f.numel() == st.hadamard_low_dim) and
+            bool(_lib.lib().dirotq_linear_fuses_hadamard(C.byref(st._c or st.c_struct()), st.hadamard_low_dim, M)))
 
 
 def _reads_records(st: LayerState) -> bool:
@@ -371,8 +378,9 @@ def _linear(st: LayerState, x: torch.Tensor, M: int, shape: tuple, out: Optional
                 return out
             return part if len(shape) == 2 else part.view(shape)
     y = out if out is not None else torch.empty(shape, dtype=torch.bfloat16, device=dev)
-    if st.hadamard_low_dim:
-        x = ops.hadamard_low(x.view(M, -1), st.hadamard_low_dim, st.hadamard_flips)
+    low = st.hadamard_low_dim
+    if low and not _fuses_hadamard(st, M):
+        x, low = ops.hadamard_low(x.view(M, -1), low, st.hadamard_flips), 0
     folded = st.folded
     if folded is not None and folded.panel is None and CACHE_WEIGHT_PANEL == "auto":
         if not st.panel_declined and _panel_budget_take(st, dev, 2 * st.out_features * st.layout.n_chunks * 64,
@@ -430,7 +438,11 @@ def _linear(st: LayerState, x: torch.Tensor, M: int, shape: tuple, out: Optional
         if h is None:
             grp.store(x, st.member_id, place, ws, records=records)
     else:
-        rc = lib.dirotq_linear_forward(lin, xp, M, yp, wsp, wsn, status, stream)
+        if low:
+            f = st.hadamard_flips
+            rc = lib.dirotq_linear_forward_hadamard(lin, xp, low, None if f is None else f.data_ptr(), M, yp, wsp, wsn, status, stream)
+        else:
+            rc = lib.dirotq_linear_forward(lin, xp, M, yp, wsp, wsn, status, stream)
         if rc:
             check(rc, "dirotq_linear_forward")
     if out is not None:

@@ -102,15 +102,9 @@ static int check_act_outputs(const ActGeom& g, void* codes, void* scales, void* 
   return DIROTQ_OK;
 }
 
-int dirotq_quantize_act(const dirotq_act_format* fmt, const void* x, int64_t x_pitch, const int64_t* perm_idx,
-                        int64_t M, void* codes, void* scales, void* zeros, void* tail, void* stream) {
-  ActGeom g;
-  int rc = make_geom(fmt, &g);
-  if (rc) return rc;
-  if (!x || M < 0 || x_pitch < g.D) return DIROTQ_E_ARG;
-  rc = check_act_outputs(g, codes, scales, zeros, tail);
-  if (rc) return rc;
-  QuantArgs a;
+static QuantArgs quant_args(const ActGeom& g, const void* x, int64_t x_pitch, const int64_t* perm_idx, int64_t M, void* codes,
+                            void* scales, void* zeros, void* tail) {
+  QuantArgs a{};
   a.g = g;
   a.x = static_cast<const __nv_bfloat16*>(x);
   a.x_pitch = x_pitch;
@@ -122,7 +116,18 @@ int dirotq_quantize_act(const dirotq_act_format* fmt, const void* x, int64_t x_p
   a.sf = static_cast<uint8_t*>(scales);
   a.zeros = static_cast<__nv_bfloat16*>(zeros);
   a.tail = static_cast<__nv_bfloat16*>(tail);
-  return launch_quantize(a, static_cast<cudaStream_t>(stream));
+  return a;
+}
+
+int dirotq_quantize_act(const dirotq_act_format* fmt, const void* x, int64_t x_pitch, const int64_t* perm_idx,
+                        int64_t M, void* codes, void* scales, void* zeros, void* tail, void* stream) {
+  ActGeom g;
+  int rc = make_geom(fmt, &g);
+  if (rc) return rc;
+  if (!x || M < 0 || x_pitch < g.D) return DIROTQ_E_ARG;
+  rc = check_act_outputs(g, codes, scales, zeros, tail);
+  if (rc) return rc;
+  return launch_quantize(quant_args(g, x, x_pitch, perm_idx, M, codes, scales, zeros, tail), static_cast<cudaStream_t>(stream));
 }
 
 int dirotq_rotate_quantize(const dirotq_act_format* fmt, const void* x, const void* rot_t, int64_t M, void* x_rot,
@@ -578,10 +583,10 @@ static bool produces_epilogue_codes(const dirotq_linear* lin, const ActGeom& g, 
 
 // stages: 1 = rotate / quantise into the workspace, 2 = GEMM from the workspace, 3 = both.
 // qo != null: the GEMM's epilogue quantises its output into these buffers as well (16-bit-conversion INT path only).
-// have: see gemm_w4a4_int_f16_impl.
+// have: see gemm_w4a4_int_f16_impl.  low_dim > 0: the activations are transformed on the way (hadamard_quant.cu).
 static int linear_stages(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace,
                          size_t workspace_bytes, int stages, int32_t* status, void* stream,
-                         const QuantOut* qo = nullptr, int32_t* have = nullptr) {
+                         const QuantOut* qo = nullptr, int32_t* have = nullptr, int low_dim = 0, const void* sign_flips = nullptr) {
   if (!lin || !workspace || ((stages & 1) && !x) || ((stages & 2) && !y && !qo)) return DIROTQ_E_ARG;
   ActGeom g;
   WsCarve w;
@@ -596,7 +601,10 @@ static int linear_stages(const dirotq_linear* lin, const void* x, int64_t M, voi
   void* zeros = is_asym(g.mode) ? ws + w.zeros : nullptr;
   void* tail = g.tail_total > 0 ? ws + w.tail : nullptr;
   if (stages & 1) {
-    if (rotates_then_quantises(lin, g)) {
+    if (low_dim > 0) {
+      rc = launch_hadamard_quant(quant_args(g, x, g.D, nullptr, M, codes, scales, zeros, tail), low_dim, sign_flips,
+                                 static_cast<cudaStream_t>(stream));
+    } else if (rotates_then_quantises(lin, g)) {
       void* x_rot = ws + w.xrot;
       rc = dirotq_rotate_quantize(&lin->fmt, x, lin->rot_t, M, x_rot, nullptr, nullptr, nullptr, nullptr, status, stream);
       if (!rc) rc = dirotq_quantize_act(&lin->fmt, x_rot, g.D, lin->perm_idx, M, codes, scales, zeros, tail, stream);
@@ -629,6 +637,18 @@ static int linear_stages(const dirotq_linear* lin, const void* x, int64_t M, voi
 int dirotq_linear_forward(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace,
                           size_t workspace_bytes, int32_t* status, void* stream) {
   return linear_stages(lin, x, M, y, workspace, workspace_bytes, 3, status, stream);
+}
+
+int dirotq_linear_fuses_hadamard(const dirotq_linear* lin, int32_t low_dim, int64_t M) {
+  ActGeom g;
+  return lin && !lin->rot_t && !lin->perm_idx && make_geom(&lin->fmt, &g) == DIROTQ_OK && hadamard_quant_covers(g, low_dim, M);
+}
+
+int dirotq_linear_forward_hadamard(const dirotq_linear* lin, const void* x, int32_t low_dim, const void* sign_flips, int64_t M,
+                                   void* y, void* workspace, size_t workspace_bytes, int32_t* status, void* stream) {
+  if (!dirotq_linear_fuses_hadamard(lin, low_dim, M)) return DIROTQ_E_UNSUPPORTED;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(sign_flips)) & 15) return DIROTQ_E_ALIGN;
+  return linear_stages(lin, x, M, y, workspace, workspace_bytes, 3, status, stream, nullptr, nullptr, low_dim, sign_flips);
 }
 
 int dirotq_linear_gemm(const dirotq_linear* lin, int64_t M, void* y, void* workspace, size_t workspace_bytes,

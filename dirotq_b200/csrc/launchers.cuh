@@ -254,6 +254,8 @@ int launch_quantize(const QuantArgs& a, cudaStream_t st);
 int launch_pack_int4(const PackIntArgs& a, cudaStream_t st);
 int launch_pack_nvfp4(const PackFp4Args& a, cudaStream_t st);
 int launch_rotate_quantize(const ActGeom& g, const void* x, const void* rot_t, int64_t M, RotArgs a, cudaStream_t st);
+bool hadamard_quant_covers(const ActGeom& g, int n, int64_t M);
+int launch_hadamard_quant(const QuantArgs& a, int n, const void* flips, cudaStream_t st);
 int launch_hadamard_low(const void* x, int64_t M, int D, int n, const void* flips, void* y, cudaStream_t st);
 int num_sms();
 int wait_limit_k();   // process-wide setting of dirotq_set_wait_limit_cycles, in units of 1024 cycles

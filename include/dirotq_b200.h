@@ -315,6 +315,15 @@ size_t dirotq_linear_workspace_bytes(const dirotq_linear* lin, int64_t M);
 int dirotq_linear_forward(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace,
                           size_t workspace_bytes, int32_t* status, void* stream);
 
+/* dirotq_hadamard_low over the first low_dim channels and dirotq_linear_forward of the result, with transform and quantiser in
+ * one launch: the same codes, the transformed tensor is not stored.  For layers whose quantised channels are the transformed
+ * ones (dirotq_linear_fuses_hadamard: no rotation or channel selection, low_dim 1024, 2048 or 4096 of a hidden layout with
+ * groups of 64, or NVFP4 with a power-of-two tensor scale; 4096 only for more rows than the GPU has multiprocessors);
+ * DIROTQ_E_UNSUPPORTED, before any launch, for all others.  x and sign_flips 16-byte aligned. */
+int dirotq_linear_fuses_hadamard(const dirotq_linear* lin, int32_t low_dim, int64_t M);
+int dirotq_linear_forward_hadamard(const dirotq_linear* lin, const void* x, int32_t low_dim, const void* sign_flips, int64_t M,
+                                   void* y, void* workspace, size_t workspace_bytes, int32_t* status, void* stream);
+
 /* Second half of dirotq_linear_forward alone: the GEMM of `lin` on the quantised activations that an
  * earlier dirotq_linear_forward left in `workspace` (same M, a layer with the same activation format
  * and rotation -- e.g. to_k and to_v after to_q, which the reference rotates with the same matrix,
