@@ -724,7 +724,7 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
       int kb, ke;
       tile_k_range(a, nb, kb, ke);
       for (int kc = kb; kc < ke; kc += UNITS) {
-        if (!mbar_wait_warp(empty_bar(s), ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
+        if (!mbar_wait_hot_warp(empty_bar(s), ph ^ 1, abort_flag, a.status, ERR_WAIT_EMPTY)) { ok = false; break; }
         if (elect_one()) {
           const uint32_t sa = smem_base + s * RQ_STAGE_BYTES, fb = PAIR ? map_to_rank(full_bar(s), 0) : full_bar(s);
           if (rank == 0) mbar_expect_tx(full_bar(s), (PAIR ? 2u : 1u) * stage_tx);
@@ -760,11 +760,11 @@ rotate_quant_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
         const uint32_t idesc = idesc_dense(ACC_F32, FMT_BF16, FMT_BF16, PAIR ? 256 : 128, (uint32_t)tile_width(a, nb));
         int kb, ke;
         tile_k_range(a, nb, kb, ke);
-        if (!mbar_wait_warp(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
+        if (!mbar_wait_hot_warp(acce_bar(buf), aph ^ 1, abort_flag, a.status, ERR_WAIT_ACC_EMPTY)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * 256;
         for (int kc = kb; kc < ke; kc += UNITS) {
-          if (!ready && !mbar_wait_warp(full_bar(s), ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
+          if (!ready && !mbar_wait_hot_warp(full_bar(s), ph, abort_flag, a.status, ERR_WAIT_FULL)) { ok = false; break; }
           tc_fence_after();
           // descriptors from loop-invariant words; the stage's four UMMAs, their commit and a test of the next stage's barrier in
           // one block (what this warp does between UMMAs is time the tensor pipe idles)
