@@ -228,7 +228,7 @@ __device__ __forceinline__ bool mbar_wait2_hot_warp(uint32_t b0, uint32_t p0, ui
 
 // One lane of a warp whose lanes are all here, the same one every time.  Issuer warps, and the producers of the rotation and the
 // FP4 GEMMs, run their loops with all lanes (waits by vote) and let the elected lane issue (in one lane remain the exact-integer
-// GEMM's issuer, the producers of both integer GEMMs and the FP4 pair GEMM's scale-factor waits): under elect.sync the compiler knows that one thread is active and keeps
+// GEMM's issuer and producers, the activation producer of the other integer GEMM and the FP4 pair GEMM's scale-factor waits): under elect.sync the compiler knows that one thread is active and keeps
 // descriptors and addresses in uniform registers.  The same loop run by `lane == 0` alone took 395 cycles per stage of four
 // UMMAs of 128 columns (nominal 256), this one 278 on CTA pairs and 304 on single CTAs; with 256 columns both are hidden behind
 // the UMMAs.  Rotation of 4096 x 1152 14.1 -> 11.9 us, of 1024 x 2240 14.1 -> 11.6; INT GEMM 4096 x 1152 x 1152 20.7 -> 19.4;

@@ -71,11 +71,6 @@ __device__ __forceinline__ float rint_bf16(float r) { return fabsf(r) < 4194304.
 // two's-complement nibble of an integer-valued float in [-8, 7] (or the byte of one in [0, 255])
 __device__ __forceinline__ uint32_t int_bits(float c) { return __float_as_uint(c + 12582912.f); }
 
-__device__ __forceinline__ uint32_t int_sym_nibble_fast(float x, float s, float rcp_s) {
-  float r = div_round_bf16(x, s, rcp_s);
-  r = fminf(fmaxf(r, -8.f), 7.f);          // clamp commutes with round-half-even for integer bounds
-  return int_bits(r) & 0xFu;               // the add rounds half-even, the low mantissa bits are the code
-}
 __device__ __forceinline__ uint32_t int_asym_code_fast(float x, float s, float rcp_s, float zero, float maxq) {
   float r = rint_bf16(div_round_bf16(x, s, rcp_s));
   float q = __bfloat162float(__float2bfloat16_rn(__fadd_rn(r, zero)));
@@ -125,21 +120,6 @@ __device__ __forceinline__ uint32_t int_sym_nib8_fast(const float* v, float s, f
     r = __hadd2(__hmin2(__hmax2(r, lo2), hi2), magic);
     const uint32_t b = *reinterpret_cast<const uint32_t*>(&r) & 0x000F000Fu;
     w |= ((b & 0xFu) | (b >> 12)) << (4 * j);
-  }
-  return w;
-}
-// The same from four words of packed bf16 pairs (as loaded): value 2 i in the low half of word i.
-__device__ __forceinline__ uint32_t int_sym_nib8_packed(const uint32_t* p, float rcp_s) {
-  const __nv_bfloat162 lo2 = __floats2bfloat162_rn(-8.f, -8.f), hi2 = __floats2bfloat162_rn(7.f, 7.f),
-                       magic = __floats2bfloat162_rn(192.f, 192.f);
-  uint32_t w = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float f0 = __uint_as_float(p[i] << 16), f1 = __uint_as_float(p[i] & 0xFFFF0000u);
-    __nv_bfloat162 r = __floats2bfloat162_rn(__fmul_rn(f0, rcp_s), __fmul_rn(f1, rcp_s));
-    r = __hadd2(__hmin2(__hmax2(r, lo2), hi2), magic);
-    const uint32_t b = *reinterpret_cast<const uint32_t*>(&r) & 0x000F000Fu;
-    w |= ((b & 0xFu) | (b >> 12)) << (8 * i);
   }
   return w;
 }

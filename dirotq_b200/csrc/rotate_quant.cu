@@ -40,7 +40,7 @@ template <bool PAIR, int UNITS> struct RqStage {
   static constexpr int UNIT_BYTES = RQ_A_BYTES + B_BYTES, STAGE_BYTES = UNITS * UNIT_BYTES;
 };
 // Epilogue warps per TMEM lane quarter: they take the 64-column chunks (per-head layouts: the heads) of their rows in
-// turns.  The NVFP4 epilogue is the longest (seven threshold compares per value) and latency-bound, and the per-head
+// turns.  The NVFP4 epilogue has four scales per chunk to make and is latency-bound, and the per-head
 // epilogues wait on several tensor-memory reads per head, so those get more warps.
 #ifndef RQ_WPQ_NVFP4
 #define RQ_WPQ_NVFP4 4
