@@ -833,17 +833,17 @@ def roofline_pass(step, x_dev, M, quant, dev, steps, exact_int=False):
                                          "(profiles/); the output of a launch is still in the 126 MB L2 when it ends"}}
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of the captured launch (16.3 MB: the 38 MB of output it wrote
-# were still in the 126 MB L2 when the launch ended) / its algorithmic bytes (52 MB); see profiles/
-NCU_TRAFFIC_RATIO = 0.31
+# dram__bytes_read.sum + dram__bytes_write.sum of the captured launch (14.6 MB: the 38 MB of output it wrote
+# were still in the 126 MB L2 when the launch ended) / its algorithmic bytes (50.2 MB); see profiles/
+NCU_TRAFFIC_RATIO = 0.29
 
 
 def gemm_algorithmic_bytes(M, N, lay, quant):
     """Bytes one W4A4 GEMM call must move: activation codes, scale data and tail, the weight's, bias, output."""
     if quant == "nvfp4":
         per_row = lay.code_row_bytes + lay.n_chunks * 4 + lay.tail_pitch * 2
-    else:   # long launches: codes + 8-byte records per chunk + bf16 scales read by the fold kernel + tail read, written, read again
-        per_row = lay.code_row_bytes + lay.n_chunks * (8 + 2 + 8) + lay.tail_pitch * 2 * 3
+    else:
+        per_row = lay.code_row_bytes + lay.n_chunks * 2 + lay.tail_pitch * 2
     w_row = lay.code_row_bytes + lay.n_chunks * 8 + lay.tail_pitch * 2 + 2
     return float(M * per_row + N * w_row + 2 * M * N)
 

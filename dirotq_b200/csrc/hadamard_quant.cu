@@ -11,8 +11,8 @@
 // writes their codes as full sectors.  The next row arrives by asynchronous copies meanwhile.  All buffers have their blocks
 // 16 bytes further apart than their length: every access below is free of bank conflicts.
 //
-// Bound by instruction issue and the shared-memory pipe together (n = 4096, 18432 rows: 51 % of issue slots, 63 % of the
-// pipe's wavefronts, 30 % of DRAM); 12 warps of 168 registers a multiprocessor, 16 of 128 for the shorter rows.  Transform and
+// Bound by instruction issue and the shared-memory pipe together (n = 4096, 18432 rows: 53 % of issue slots, 60 % of the
+// pipe's wavefronts, 31 % of DRAM); 12 warps of 168 registers a multiprocessor, 16 of 128 for the shorter rows.  Transform and
 // quantiser, separate launches -> this one, us, for 4-bit symmetric / asymmetric / 8-bit / NVFP4 codes:
 //   4096 rows, n = 1024 of 1152    10.4 ->  6.6   10.9 ->  7.1   11.6 ->  7.7   13.3 ->  6.9
 //              n = 2048 of 2240    18.1 -> 12.1   19.3 -> 13.2   20.0 -> 15.0   19.8 -> 12.9
