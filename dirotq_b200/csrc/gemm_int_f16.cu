@@ -454,7 +454,9 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
       // Only once what was read has arrived in registers: an arrival overtakes shared-memory loads that still wait in their queue, behind
       // stores of the quantising epilogue for instance, and the next copy would overwrite what they read.  Either instructions
       // that use it have been issued, or the arrival's own address depends on it (`read`, a word of every load, under a mask that
-      // is zero for reasons the compiler does not know).
+      // is zero for reasons the compiler does not know).  A record made here comes of two loads where there are zero points, the
+      // scale's (and 1 / rs) in its multiplier, the zero point's only in its addend.
+      auto words_of = [](uint2 k) { return ASYM && !REC ? k.x ^ k.y : k.x; };
       auto release_raw = [&](uint32_t read = 0u) {
         __syncwarp();
         if (lane == 0) mbar_arrive(rawe_bar(r.s) + (read & never));
@@ -513,11 +515,11 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
           };
           if constexpr (!LATE) {
             fetch1();
-            uint32_t read = k0.x ^ k1.x;
+            uint32_t read = words_of(k0) ^ words_of(k1);
 #pragma unroll
             for (int i = 0; i < PC; ++i) read ^= p0[i].x ^ p1[i].x;
             if constexpr (UNITS == 2) {
-              read ^= k2.x ^ k3.x;
+              read ^= words_of(k2) ^ words_of(k3);
 #pragma unroll
               for (int i = 0; i < PC; ++i) read ^= p2[i].x ^ p3[i].x;
             }
@@ -568,7 +570,7 @@ gemm_int_f16_kernel(const __grid_constant__ GfMaps tm, const GemmIntF16Args a) {
         };
         if constexpr (!LATE) {
           fetch1();
-          uint32_t read = k0.x ^ k1.x;
+          uint32_t read = words_of(k0) ^ words_of(k1);
 #pragma unroll
           for (int i = 0; i < PC; ++i) read ^= two ? p0[i].x ^ p1[i].x : p0[i].x;
           release_raw(read);

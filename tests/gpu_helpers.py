@@ -1,4 +1,8 @@
-"""Decoders from the device buffer layouts (include/dirotq_b200.h) to plain tensors, for parity tests."""
+"""Decoders from the device buffer layouts (include/dirotq_b200.h) to plain tensors, for parity tests; layers by other routes of the
+library than the backend's; launches of a call."""
+import ctypes as C
+import os
+
 import torch
 
 from oracle import dirotq_oracle as O
@@ -121,6 +125,27 @@ def dense_reference_weight(w, ld) -> torch.Tensor:
         H, d, hl = ld.heads, ld.head_dim, ld.tail
         return torch.cat([low.reshape(N, H, d - hl), tail.reshape(N, H, hl)], dim=2).reshape(N, H * d)
     return torch.cat([low, tail], dim=1)
+
+
+def forward_on_records(st, x2d):
+    """An integer layer (backend.LayerState) as the first of a group that shares activations: its GEMM, 256 columns wide whatever the
+    size, reads what the folding kernel made of the activation scales."""
+    from dirotq_b200 import _lib
+    lib, lin, M = _lib.lib(), C.byref(st.c_struct()), x2d.shape[0]
+    ws = torch.zeros(lib.dirotq_linear_workspace_bytes(lin, M), dtype=torch.uint8, device=x2d.device)
+    y = torch.empty(M, st.out_features, dtype=torch.bfloat16, device=x2d.device)
+    records, before = C.c_int32(0), os.environ.get("DIROTQ_GF_BN")
+    os.environ["DIROTQ_GF_BN"] = "256"
+    try:
+        rc = lib.dirotq_linear_sibling(lin, x2d.data_ptr(), M, y.data_ptr(), ws.data_ptr(), ws.numel(), C.byref(records),
+                                       ops.status_word(x2d.device).data_ptr(), ops.stream_ptr())
+    finally:
+        if before is None:
+            del os.environ["DIROTQ_GF_BN"]
+        else:
+            os.environ["DIROTQ_GF_BN"] = before
+    assert rc == 0 and records.value == 1
+    return y
 
 
 def kernels_of(fn):
