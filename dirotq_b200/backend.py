@@ -281,8 +281,8 @@ class LayerState:
 def kernel_launches(st: Optional[LayerState], w4a16=None) -> int:
     """Library kernels one forward of a wrapped linear launches.  A W4A16 layer (no LayerState): weight
     dequantisation + GEMM.  W4A4: rotate/quantise + GEMM; the tensor-rate integer GEMM adds one preparation launch where
-    the layer keeps no resident panel (the weight-panel pre-pass) or the call is long (scale folding; asked for the rows
-    of the last call, counted before any call); a sibling that reuses the activations of the layer before it runs only its
+    the layer keeps no resident panel (the weight-panel pre-pass) or shares its activations in a long call (scale folding;
+    asked for the rows of the last call, counted before any call); a sibling that reuses the activations of the layer before it runs only its
     own GEMM (and preparation; scales that an earlier sibling has folded are not folded again)."""
     if st is None:
         return 1 if (w4a16 is not None and w4a16.dense is not None) else 2    # resident dequantised weight: GEMM only

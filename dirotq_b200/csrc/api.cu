@@ -416,7 +416,7 @@ static int gemm_w4a4_int_f16_impl(int32_t a_mode, int64_t M, int64_t N, int32_t 
     a.q_mode = qo->mode;
     a.q_clip = qo->clip;
   }
-  const bool records = have && gemm_int_f16_takes_records(a, qo != nullptr);
+  const bool records = have && gemm_int_f16_takes_records(M, N);
   if (records && *have) {
     if (!w_panel) {
       int rc = launch_expand_weight_panel(static_cast<const uint8_t*>(w_codes), n_chunks, N, w_mult, ws + c.panel, st, hc);
@@ -656,8 +656,8 @@ int dirotq_linear_gemm(const dirotq_linear* lin, int64_t M, void* y, void* works
   return linear_stages(lin, nullptr, M, y, workspace, workspace_bytes, 2, status, stream);
 }
 
-// Long launches fold their activation scales by a kernel, 14 MB at 32768 x 1152: one for all siblings of a tensor, whichever
-// of them first needs it, and not one each.
+// The GEMMs of long sibling calls read folded activation scales, 14 MB at 32768 x 1152, that a kernel makes once for all siblings
+// of a tensor, for whichever of them first needs them; no other entry makes any.
 int dirotq_linear_sibling(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace, size_t workspace_bytes,
                           int32_t* records, int32_t* status, void* stream) {
   if (!records) return DIROTQ_E_ARG;
@@ -691,10 +691,7 @@ int dirotq_linear_uses_half_chunks(const dirotq_linear* lin) {
 int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M) {
   ActGeom g;
   if (!lin || M <= 0 || make_geom(&lin->fmt, &g) || !uses_f16_gemm(lin, g)) return 0;
-  GemmIntF16Args a;
-  a.M = M;
-  a.N = lin->out_features;
-  return gemm_int_f16_takes_records(a, false) ? 1 : 0;
+  return gemm_int_f16_takes_records(M, lin->out_features) ? 1 : 0;
 }
 int dirotq_linear_chain_folds_scales(const dirotq_linear*, int64_t) { return 0; }
 

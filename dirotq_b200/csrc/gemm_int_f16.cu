@@ -1343,10 +1343,10 @@ static int pick_raster_f16(int BN, int64_t N, int64_t k_total) {
 // folding kernel + GEMM / GEMM alone, 256 columns: 32768 x 1152 x 3456 199.5 / 197.4, 16384 x 2240 x 2240 120.0 / 113.9, 4608 x 3072 x
 // 3072 63.1 / 59.4, x 12288 232.5 / 230.4; before the converters read a raw stage at once the long launches were 2-4 % slower alone).
 // For long launches (more than four rounds of 148 tiles) of three siblings the two come out even, and a group keeps its records.
-bool gemm_int_f16_takes_records(const GemmIntF16Args& a, bool quantise_out) {
-  if (const char* e = getenv("DIROTQ_GF_BN"))
-    return pick_bn_f16(a.M, a.N, 1, quantise_out) == 256 && !(getenv("DIROTQ_GF_PAIR") && atoi(getenv("DIROTQ_GF_PAIR")) == 0);
-  return a.N > 128 && ((a.M + 127) / 128) * ((a.N + 255) / 256) > 4 * (int64_t)num_sms();
+// DIROTQ_GF_BN overrides: 256 takes records, narrower tiles do not.
+bool gemm_int_f16_takes_records(int64_t M, int64_t N) {
+  if (getenv("DIROTQ_GF_BN")) return pick_bn_f16(M, N, 1, false) == 256;
+  return N > 128 && ((M + 127) / 128) * ((N + 255) / 256) > 4 * (int64_t)num_sms();
 }
 
 int launch_gemm_int_f16(const GemmIntF16Args& a_in, cudaStream_t st) {

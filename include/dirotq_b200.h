@@ -210,8 +210,9 @@ int dirotq_gemm_w4a4_int(int32_t a_mode, int64_t M, int64_t N, int32_t n_chunks,
  * dirotq_gemm_w4a4_int_f16: a_mode DIROTQ_INT4_SYM, DIROTQ_INT4_ASYM or DIROTQ_INT8_ASYM; w_panel NULL: the panel
  *   is rebuilt from w_codes / w_mult in the workspace on every call (w_codes / w_mult may be NULL when w_panel
  *   is given); workspace of dirotq_gemm_w4a4_int_f16_workspace_bytes(M, N_panel, n_chunks, tail_pitch) bytes,
- *   256-byte aligned (activation multipliers and the scaled copy of the tail, which long launches have made by a kernel of
- *   their own, and, for N_panel = N > 0, the panel; N_panel = 0 for callers that pass their own).
+ *   256-byte aligned: for N_panel = N > 0 the panel (N_panel = 0 for callers that pass their own), and room for the records
+ *   and the scaled copy of the tail that dirotq_linear_sibling's long calls make -- this entry keeps nothing there but a copy of
+ *   x_scales / x_zeros that are not 16-byte aligned.
  */
 size_t dirotq_fold_weight_records_bytes(int32_t n_chunks, int64_t N);
 int dirotq_fold_weight_scales_f16(int32_t n_chunks, int64_t N, const float* w_scales, const void* w_tail,

@@ -7,6 +7,7 @@ import torch
 
 from oracle import dirotq_oracle as O
 from dirotq_b200 import ops
+from dirotq_b200._lib import LinearC
 
 
 def decode_act(buf: ops.ActBuffers):
@@ -130,15 +131,29 @@ def dense_reference_weight(w, ld) -> torch.Tensor:
 def forward_on_records(st, x2d):
     """An integer layer (backend.LayerState) as the first of a group that shares activations: its GEMM, 256 columns wide whatever the
     size, reads what the folding kernel made of the activation scales."""
+    return _sibling(st.c_struct(), x2d.shape[0], x2d, None)
+
+
+def gemm_on_records(act: ops.ActBuffers, pk, folded, bias):
+    """ops.gemm_w4a4_int_f16 by that route, on activations that are there already."""
+    p = lambda t: C.c_void_p(0 if t is None else t.data_ptr())
+    lin = LinearC(act.fmt.c(), pk.N, p(None), p(None), p(pk.codes), p(pk.scales), p(pk.wsum), p(None), p(bias), 1.0, p(folded.mult),
+                  p(folded.colscale), p(folded.tail), 0, p(folded.panel))
+    return _sibling(lin, act.M, None, torch.cat([t.view(torch.uint8) for t in (act.codes, act.scales, act.zeros, act.tail) if t is not None]))
+
+
+def _sibling(lin, M, x2d, held):
     from dirotq_b200 import _lib
-    lib, lin, M = _lib.lib(), C.byref(st.c_struct()), x2d.shape[0]
-    ws = torch.zeros(lib.dirotq_linear_workspace_bytes(lin, M), dtype=torch.uint8, device=x2d.device)
-    y = torch.empty(M, st.out_features, dtype=torch.bfloat16, device=x2d.device)
+    lib, N = _lib.lib(), lin.out_features
+    ws = torch.zeros(lib.dirotq_linear_workspace_bytes(C.byref(lin), M), dtype=torch.uint8, device="cuda")
+    if held is not None:                    # codes, scales, zero points and 16-bit channels side by side
+        ws[:held.numel()] = held
+    y = torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
     records, before = C.c_int32(0), os.environ.get("DIROTQ_GF_BN")
     os.environ["DIROTQ_GF_BN"] = "256"
     try:
-        rc = lib.dirotq_linear_sibling(lin, x2d.data_ptr(), M, y.data_ptr(), ws.data_ptr(), ws.numel(), C.byref(records),
-                                       ops.status_word(x2d.device).data_ptr(), ops.stream_ptr())
+        rc = lib.dirotq_linear_sibling(C.byref(lin), None if x2d is None else x2d.data_ptr(), M, y.data_ptr(), ws.data_ptr(), ws.numel(),
+                                       C.byref(records), ops.status_word("cuda").data_ptr(), ops.stream_ptr())
     finally:
         if before is None:
             del os.environ["DIROTQ_GF_BN"]
@@ -149,8 +164,12 @@ def forward_on_records(st, x2d):
 
 
 def kernels_of(fn):
-    """Kernel launches of fn(), counted in a captured graph; what fn builds lazily exists by then."""
-    from cuda.bindings import runtime as rt
+    return len(kernel_names(fn))
+
+
+def kernel_names(fn):
+    """Mangled names of the kernels that fn() launches, as a captured graph lists them; what fn builds lazily exists by then."""
+    from cuda.bindings import driver as cu, runtime as rt
     from dirotq_b200 import backend
     with backend.WorkspaceScope(), torch.no_grad():
         side = torch.cuda.Stream()
@@ -166,5 +185,12 @@ def kernels_of(fn):
     assert err == rt.cudaError_t.cudaSuccess
     err, nodes, n = rt.cudaGraphGetNodes(raw, n)
     assert err == rt.cudaError_t.cudaSuccess
-    kinds = [rt.cudaGraphNodeGetType(node)[1] for node in nodes[:n]]
-    return sum(k == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel for k in kinds)
+    names = []
+    for node in nodes[:n]:
+        if rt.cudaGraphNodeGetType(node)[1] == rt.cudaGraphNodeType.cudaGraphNodeTypeKernel:
+            err, p = cu.cuGraphKernelNodeGetParams(cu.CUgraphNode(int(node)))
+            assert err == cu.CUresult.CUDA_SUCCESS
+            err, name = cu.cuFuncGetName(p.func) if int(p.func) else cu.cuKernelGetName(p.kern)
+            assert err == cu.CUresult.CUDA_SUCCESS
+            names.append(name.decode())
+    return names

@@ -242,11 +242,14 @@ def test_int_f16_gemm_edge_shapes(mode, M, N, D, tail):
 @pytest.mark.parametrize("mode,M,N,D,tail", [("sym", 2401, 2056, 64, 0), ("int8", 2401, 2056, 192, 8),
                                              ("sym", 15204, 1032, 128, 8), ("asym", 15240, 1032, 64, 0),
                                              ("int8", 15233, 1032, 192, 72), ("sym", 15359, 1280, 576, 64)])
-def test_int_f16_gemm_wide_tiles(mode, M, N, D, tail):
-    """256-wide tiles on one CTA (2401 rows) and on CTA pairs (over four rounds of tiles): a last pair whose second half lies
-    past the end (15204 = 118 * 128 + 100), holds one row (15233) or all but one; a last column tile of 8 columns; K from one
-    stage to more stages than the operand ring holds."""
+@pytest.mark.parametrize("bn", [None, "256"])
+def test_int_f16_gemm_wide_tiles(monkeypatch, bn, mode, M, N, D, tail):
+    """Several rounds of tiles, by the dispatch's own choice (128-wide for 2401 rows, 192-wide CTA pairs for the others) and 256-wide:
+    a last pair whose second half lies past the end (2401, and 15204 = 118 * 128 + 100 has 100 of its rows), holds one row (15233)
+    or all but one; a last column tile of 8 columns; K from one stage to more stages than the operand ring holds."""
     from dirotq_b200 import ops
+    if bn:
+        monkeypatch.setenv("DIROTQ_GF_BN", bn)
     m = {"sym": ops.INT4_SYM, "asym": ops.INT4_ASYM, "int8": ops.INT8_ASYM}[mode]
     fmt = ops.ActFormat(m, D, tail_len=tail)
     x, act, dec, qw, sw, pk, w_tail, bias = _setup_int(ops, M, N, fmt, 37)
@@ -261,14 +264,12 @@ def test_int_f16_gemm_wide_tiles(mode, M, N, D, tail):
     assert rel_l2(y[-(M % 128 or 128):], y_ref[-(M % 128 or 128):]) < 4e-3 and rel_l2(y[:, -8:], y_ref[:, -8:]) < 4e-3
 
 
-@pytest.mark.parametrize("pair", ["0", "1"])
 @pytest.mark.parametrize("mode,M,N,D,tail", [("sym", 1, 8, 64, 0), ("asym", 128, 136, 1152, 64), ("int8", 129, 264, 192, 72),
                                              ("sym", 257, 264, 640, 8), ("int8", 257, 8, 1152, 0), ("asym", 1, 264, 192, 128)])
-def test_int_f16_gemm_forced_wide_tiles(monkeypatch, pair, mode, M, N, D, tail):
-    """The 256-wide kernels on one CTA and on CTA pairs where the launcher would not pick them, whatever its thresholds: one
-    row, one column block of 8, one operand stage, a pair whose second half is empty or holds a row, more stages than slots."""
+def test_int_f16_gemm_forced_wide_tiles(monkeypatch, mode, M, N, D, tail):
+    """The 256-wide kernels where the launcher would not pick them, whatever its thresholds: one row, one column block of 8, one
+    operand stage, a pair whose second half is empty or holds a row, more stages than slots."""
     monkeypatch.setenv("DIROTQ_GF_BN", "256")
-    monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
     test_int_f16_gemm_edge_shapes(mode, M, N, D, tail)
 
 
@@ -284,19 +285,17 @@ def test_int_f16_gemm_192_wide_tiles(monkeypatch, mode, M, N, D, tail):
 @pytest.mark.parametrize("mode", ["sym", "asym", "int8"])
 @pytest.mark.parametrize("M,N,D,tail", [(3000, 1152, 192, 8), (1001, 3456, 640, 64)])
 def test_int_f16_gemm_unforced_192_wide_tiles(mode, M, N, D, tail):
-    """Sizes for which 192-wide tiles need as many rounds as 256-wide ones, and fewer than 128-wide ones."""
+    """Sizes for which 192-wide pair tiles need one round and 128-wide ones two."""
     test_int_f16_gemm_edge_shapes(mode, M, N, D, tail)
 
 
-@pytest.mark.parametrize("pair", ["0", "1"])
 @pytest.mark.parametrize("quant,a_sym,H", [("int4", True, 5), ("int4", False, 70), ("int8", False, 7)])
-def test_int_f16_gemm_forced_wide_tiles_with_half_chunks(monkeypatch, pair, quant, a_sym, H):
+def test_int_f16_gemm_forced_wide_tiles_with_half_chunks(monkeypatch, quant, a_sym, H):
     """The same with two half-filled chunks per operand stage (short per-head groups, odd and even head counts)."""
     from dirotq_b200 import backend
     from dirotq_b200.wrapper import ActQuantWrapper
     import test_gpu_models
     monkeypatch.setenv("DIROTQ_GF_BN", "256")
-    monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
     monkeypatch.setattr(ActQuantWrapper, "forward", backend._fused_forward_b200)
     test_gpu_models.test_short_per_head_groups_share_operand_stages(quant, a_sym, H, 300, monkeypatch)
 

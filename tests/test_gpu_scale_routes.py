@@ -1,8 +1,9 @@
-"""The two ways a row's scales reach the 16-bit-conversion GEMM -- records of the folding kernel (CTA pairs), or the scales
-themselves (single CTAs) -- give the same bits, from any scales and from any address; and the rotation kernel's packed
+"""The two ways a row's scales reach the 16-bit-conversion GEMM -- the scales themselves, or records of the folding kernel (long
+calls of siblings, 256-wide tiles) -- give the same bits, from any scales and from any address; and the rotation kernel's packed
 quantiser agrees with the oracle where a group lies far from zero or is clipped; 16-bit channels copied in the quantiser's
 launch or behind it."""
 import dataclasses
+import re
 
 import pytest
 import torch
@@ -17,6 +18,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("mode", ["sym", "asym", "int8"])
 def test_both_scale_routes_give_the_same_bits(mode, M, D, tail, monkeypatch):
     from dirotq_b200 import ops
+    from gpu_helpers import gemm_on_records, kernel_names
     from test_gpu_gemm import _setup_int
     m = {"sym": ops.INT4_SYM, "asym": ops.INT4_ASYM, "int8": ops.INT8_ASYM}[mode]
     x, act, dec, qw, sw, pk, w_tail, bias = _setup_int(ops, M, 264, ops.ActFormat(m, D, tail_len=tail), 71)
@@ -30,16 +32,23 @@ def test_both_scale_routes_give_the_same_bits(mode, M, D, tail, monkeypatch):
         s[:, M // 2] = 0
     wt = ops.pad_tail_weight(w_tail, lay.tail_pitch, 264, "cuda")
     folded = ops.fold_weight_scales_f16(pk, wt, lay.tail_total)
-    run = lambda a: ops.gemm_w4a4_int_f16(a, pk, folded, bias.cuda())
-    out = {}
-    for bn, pair in (("256", "1"), ("128", "0"), ("192", "0"), ("256", "0")):
+    bias = bias.cuda()
+    run = lambda a: ops.gemm_w4a4_int_f16(a, pk, folded, bias)
+    on_records = lambda: gemm_on_records(act, pk, folded, bias)
+    want = on_records()
+    assert torch.isfinite(want.float()).all()
+    for bn in ("128", "192", "256"):
         monkeypatch.setenv("DIROTQ_GF_BN", bn)
-        monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
-        out[bn, pair] = run(act)
+        assert torch.equal(run(act), want), bn
     ops.check_status()
-    assert torch.isfinite(out["256", "1"].float()).all()
-    for k, y in out.items():
-        assert torch.equal(y, out["256", "1"]), k
+    # what each route launches beside the GEMM: the folding kernel (with the panel's pre-pass, where there is no resident panel), or
+    # none
+    pre = lambda fn: [re.search("fold_expand|fold_scales|expand_weight_panel|$", n)[0] for n in kernel_names(fn)
+                      if "2dq" in n and "gemm_int_f16" not in n]
+    assert pre(on_records) == ["fold_expand"] and pre(lambda: run(act)) == ["expand_weight_panel"]
+    folded.panel = ops.expand_weight_panel_f16(pk, folded)
+    assert torch.equal(on_records(), want)
+    assert pre(on_records) == ["fold_scales"] and pre(lambda: run(act)) == []
 
     def shifted(t):                                   # the same values at an address that is no multiple of 16
         if t is None:
@@ -48,10 +57,9 @@ def test_both_scale_routes_give_the_same_bits(mode, M, D, tail, monkeypatch):
         return buf.copy_(t)
     moved = dataclasses.replace(act, scales=shifted(act.scales), zeros=shifted(act.zeros))
     assert moved.scales.data_ptr() % 16
-    for bn, pair in (("128", "0"), ("256", "1")):
+    for bn in ("128", "256"):
         monkeypatch.setenv("DIROTQ_GF_BN", bn)
-        monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
-        assert torch.equal(run(moved), out["256", "1"])
+        assert torch.equal(run(moved), want)
     ops.check_status()
 
 
@@ -61,8 +69,9 @@ def test_both_scale_routes_give_the_same_bits(mode, M, D, tail, monkeypatch):
 @pytest.mark.parametrize("mode", ["sym", "asym", "int8"])
 def test_row_powers_of_many_tiles_per_cta(mode, D, tail, monkeypatch):
     from dirotq_b200 import ops
+    from gpu_helpers import gemm_on_records
     from test_gpu_gemm import _setup_int
-    M, N = 34300, 1032                               # 268 x 5 tiles of 256 columns on 148 SMs
+    M, N = 34300, 1032                               # 134 x 5 tiles of 256 columns on 74 pairs of SMs
     m = {"sym": ops.INT4_SYM, "asym": ops.INT4_ASYM, "int8": ops.INT8_ASYM}[mode]
     x, act, dec, qw, sw, pk, w_tail, bias = _setup_int(ops, M, N, ops.ActFormat(m, D, tail_len=tail), 75)
     lay = act.layout
@@ -71,18 +80,36 @@ def test_row_powers_of_many_tiles_per_cta(mode, D, tail, monkeypatch):
     s *= torch.exp2(((rows // 3 * 7) % 49 - 24).float()).to(torch.bfloat16)     # a wrong tile's or row's power shows
     folded = ops.fold_weight_scales_f16(pk, ops.pad_tail_weight(w_tail, lay.tail_pitch, N, "cuda"), lay.tail_total)
     bias = bias.cuda()
-    out = {}
-    for bn, pair in (("256", "1"), ("128", "0"), ("192", "0"), ("256", "0")):
+    want = gemm_on_records(act, pk, folded, bias)
+    for bn in ("128", "192", "256"):
         monkeypatch.setenv("DIROTQ_GF_BN", bn)
-        monkeypatch.setenv("DIROTQ_GF_PAIR", pair)
-        out[bn, pair] = ops.gemm_w4a4_int_f16(act, pk, folded, bias)
+        assert torch.equal(ops.gemm_w4a4_int_f16(act, pk, folded, bias), want), bn
     ops.check_status()
-    for k, y in out.items():
-        assert torch.equal(y, out["256", "1"]), k
 
 
-def test_unforced_call_of_five_single_cta_rounds(monkeypatch):
-    """15360 x 1152 x 1152: 192-wide tiles on single CTAs, five rounds, by the dispatch's own choice."""
+@pytest.mark.parametrize("quant,H", [("int4", 5), ("int4", 70), ("int8", 7)])
+@pytest.mark.parametrize("a_sym", [True, False])
+@pytest.mark.parametrize("M", [1, 300])
+def test_both_scale_routes_with_half_chunks(quant, a_sym, H, M, monkeypatch):
+    """Two half-filled chunks per operand stage, odd and even head counts: one to eighteen raw stages."""
+    from dirotq_b200 import backend, dit, ops
+    from dirotq_b200.synth import synth_activations
+    from gpu_helpers import forward_on_records
+    ld = dit.LayerDef("attn1.to_out.0", H * 32, 264, kind="perhead", tail=4, heads=H, head_dim=32)
+    w = dit.make_wrapped_linear(ld, quant, 77, "cuda", a_sym=a_sym)
+    backend.preconvert_rotations_to_device(torch.nn.ModuleDict({"l": w}), "cuda")
+    st, x = w._b200_state, synth_activations(M, H * 32, torch.Generator().manual_seed(H)).cuda()
+    x *= torch.exp2((torch.arange(M, device="cuda") % 49 - 24).float()).to(torch.bfloat16)[:, None]
+    want = forward_on_records(st, x)
+    assert torch.isfinite(want.float()).all()
+    for bn in ("128", "192", "256"):
+        monkeypatch.setenv("DIROTQ_GF_BN", bn)
+        assert torch.equal(backend.linear_forward(st, x), want), bn
+    ops.check_status()
+
+
+def test_unforced_call_of_five_rounds_of_192_wide_pairs(monkeypatch):
+    """15360 x 1152 x 1152: 192-wide tiles on CTA pairs, five rounds, by the dispatch's own choice."""
     from dirotq_b200 import ops
     from test_gpu_gemm import _setup_int
     x, act, dec, qw, sw, pk, w_tail, bias = _setup_int(ops, 15360, 1152, ops.ActFormat(ops.INT4_ASYM, 1152, tail_len=64), 76)
@@ -90,7 +117,6 @@ def test_unforced_call_of_five_single_cta_rounds(monkeypatch):
     folded = ops.fold_weight_scales_f16(pk, ops.pad_tail_weight(w_tail, lay.tail_pitch, 1152, "cuda"), lay.tail_total)
     y = ops.gemm_w4a4_int_f16(act, pk, folded, bias.cuda())
     monkeypatch.setenv("DIROTQ_GF_BN", "256")
-    monkeypatch.setenv("DIROTQ_GF_PAIR", "1")
     assert torch.equal(y, ops.gemm_w4a4_int_f16(act, pk, folded, bias.cuda()))
     ops.check_status()
 

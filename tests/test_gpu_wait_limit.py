@@ -8,7 +8,7 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _int_gemm(mode, M, N, D, tail, exact=False):
+def _int_gemm(mode, M, N, D, tail, exact=False, records=False):
     from dirotq_b200 import ops
     from test_gpu_gemm import _setup_int
     m = {"sym": ops.INT4_SYM, "asym": ops.INT4_ASYM, "int8": ops.INT8_ASYM}[mode]
@@ -18,6 +18,9 @@ def _int_gemm(mode, M, N, D, tail, exact=False):
     if exact:
         return lambda: ops.gemm_w4a4_int(act, pk, wt, b)
     folded = ops.fold_weight_scales_f16(pk, wt, lay.tail_total)
+    if records:
+        from gpu_helpers import gemm_on_records
+        return lambda: gemm_on_records(act, pk, folded, b)
     return lambda: ops.gemm_w4a4_int_f16(act, pk, folded, b)
 
 
@@ -53,9 +56,10 @@ _KERNELS = {
     "int exact": ({}, lambda: _int_gemm("asym", 300, 264, 4608, 64, exact=True)),
     "int 128": ({"DIROTQ_GF_BN": "128"}, lambda: _int_gemm("sym", 300, 264, 12288, 320)),
     "int 192": ({"DIROTQ_GF_BN": "192"}, lambda: _int_gemm("int8", 300, 264, 12288, 320)),
-    "int 256": ({"DIROTQ_GF_BN": "256", "DIROTQ_GF_PAIR": "0"}, lambda: _int_gemm("asym", 300, 264, 12288, 320)),
-    "int pair": ({"DIROTQ_GF_BN": "256", "DIROTQ_GF_PAIR": "1"}, lambda: _int_gemm("sym", 300, 264, 12288, 320)),
-    "int pair, many tiles": ({"DIROTQ_GF_BN": "256", "DIROTQ_GF_PAIR": "1"}, lambda: _int_gemm("int8", 5000, 2056, 3072, 384)),
+    "int 256": ({"DIROTQ_GF_BN": "256"}, lambda: _int_gemm("asym", 300, 264, 12288, 320)),
+    "int 256, many tiles": ({"DIROTQ_GF_BN": "256"}, lambda: _int_gemm("int8", 5000, 2056, 3072, 384)),
+    "int records": ({}, lambda: _int_gemm("sym", 300, 264, 12288, 320, records=True)),
+    "int records, many tiles": ({}, lambda: _int_gemm("int8", 5000, 2056, 3072, 384, records=True)),
     "nvfp4 single": ({"DIROTQ_NVFP4_TILE": "single"}, lambda: _nvfp4_gemm(300, 264, 12288, 320)),
     "nvfp4 pair 128": ({"DIROTQ_NVFP4_TILE": "pair128"}, lambda: _nvfp4_gemm(300, 264, 12288, 320)),
     "nvfp4 pair 256": ({"DIROTQ_NVFP4_TILE": "pair256"}, lambda: _nvfp4_gemm(5000, 2056, 12288, 64)),
