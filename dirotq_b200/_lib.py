@@ -75,7 +75,6 @@ SIGNATURES = {
     "dirotq_expand_weight_panel_f16_layout": (C.c_int, [_I32, _I64, _P, _P, _P, _I32, _P]),
     "dirotq_linear_uses_half_chunks": (C.c_int, [C.POINTER(LinearC)]),
     "dirotq_linear_folds_scales": (C.c_int, [C.POINTER(LinearC), _I64]),
-    "dirotq_linear_chain_folds_scales": (C.c_int, [C.POINTER(LinearC), _I64]),
     "dirotq_layernorm_modulate": (C.c_int, [_P, _I64, _I32, _I64, _P, _P, _I64, _F, _P, _P]),
     "dirotq_gated_residual": (C.c_int, [_P, _P, _P, _P, _I64, _I64, _I32, _I64, _P, _P]),
     "dirotq_qkv_norm_rope": (C.c_int, [_P, _P, _P, _I64, _I64, _I64, _I32, _I32, _P, _P, _P, _P, _I64, _I64, _F, _P, _P, _P, _P]),
@@ -88,7 +87,7 @@ SIGNATURES = {
     "dirotq_linear_forward_static": (C.c_int, [C.POINTER(LinearC), _P, _I64, _P, _P, _P]),
 }
 
-ABI_VERSION = 6
+ABI_VERSION = 7
 _lib = None
 
 

@@ -693,7 +693,6 @@ int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M) {
   if (!lin || M <= 0 || make_geom(&lin->fmt, &g) || !uses_f16_gemm(lin, g)) return 0;
   return gemm_int_f16_takes_records(M, lin->out_features) ? 1 : 0;
 }
-int dirotq_linear_chain_folds_scales(const dirotq_linear*, int64_t) { return 0; }
 
 int dirotq_linear_chain_supported(const dirotq_linear* lin, const dirotq_linear* next) {
   if (!lin || !next) return 0;

@@ -21,7 +21,7 @@
 extern "C" {
 #endif
 
-#define DIROTQ_ABI_VERSION 6
+#define DIROTQ_ABI_VERSION 7
 
 /* ---- activation quantiser modes (ActQuantizer.configure, utils/quant_utils.py:182-199) ---- */
 enum {
@@ -354,9 +354,8 @@ int dirotq_linear_sibling(const dirotq_linear* lin, const void* x, int64_t M, vo
  * rotation, no channel selection, width == lin->out_features, w_mult set.  Anything else: DIROTQ_E_UNSUPPORTED, nothing launched. */
 int dirotq_linear_uses_half_chunks(const dirotq_linear* lin);
 /* Whether dirotq_linear_sibling makes records of the activation scales for `lin` on M rows (long launches of integer layers); the
- * GEMMs of all other entries read the scales themselves, the chain's among them (always 0). */
+ * GEMMs of all other entries read the scales themselves. */
 int dirotq_linear_folds_scales(const dirotq_linear* lin, int64_t M);
-int dirotq_linear_chain_folds_scales(const dirotq_linear* lin, int64_t M);
 int dirotq_linear_chain_supported(const dirotq_linear* lin, const dirotq_linear* next);
 int dirotq_linear_forward_chain(const dirotq_linear* lin, const void* x, int64_t M, void* y, void* workspace,
                                 size_t workspace_bytes, const dirotq_linear* next, void* next_workspace,
