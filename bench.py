@@ -833,7 +833,7 @@ def roofline_pass(step, x_dev, M, quant, dev, steps, exact_int=False):
                                          "(profiles/); the output of a launch is still in the 126 MB L2 when it ends"}}
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of the captured launch (14.6 MB: the 38 MB of output it wrote
+# dram__bytes_read.sum + dram__bytes_write.sum of the captured launch (14.5 MB: the 38 MB of output it wrote
 # were still in the 126 MB L2 when the launch ended) / its algorithmic bytes (50.2 MB); see profiles/
 NCU_TRAFFIC_RATIO = 0.29
 
