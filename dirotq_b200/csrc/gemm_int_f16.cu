@@ -1037,7 +1037,7 @@ template <> __device__ __forceinline__ float scale_to_float<__nv_bfloat16>(__nv_
 
 // Block = ROWS rows x 256 / ROWS chunk phases (thread tid: row tid % ROWS, chunks c = tid / ROWS (mod 256 / ROWS)).
 // What this kernel takes is latency: two dependent passes over a few hundred bytes per thread.  So a thread's scales and zero
-// points are loaded at once, ahead of the maximum, and kept; and short calls get 16-row blocks (see fold_small_blocks).
+// points are loaded at once, ahead of the maximum, and kept; and calls of few rows get 16-row blocks (see fold_small_blocks).
 template <typename ST, int ROWS>
 __device__ __forceinline__ void fold_scales_block(int block, const ST* __restrict__ s, const __nv_bfloat16* __restrict__ z,
                                                   int n_chunks, int64_t rows, int64_t ld_in, uint2* __restrict__ rec,
@@ -1216,10 +1216,11 @@ int launch_expand_weight_panel(const uint8_t* wq, int n_chunks, int64_t N, const
 int64_t f16_ld_act(int64_t M) { return round_up64(M, 128); }
 int64_t f16_ld_weight(int64_t N) { return round_up64(N, 768); }
 
-// Rows per block of the folding kernels: 64 keeps whole sectors of scales in a warp; with fewer than two such blocks per SM
-// the chip is mostly idle, and 16 rows (a 32-byte sector of scales) spread the work over four times as many: the four linears
-// of a 2240-wide block at 1024 rows (320 16-bit channels, 16 blocks of 64 rows) 186 -> 165 us, of a 1152-wide block at 4096
-// rows 287 -> 281, 3072-wide blocks at 4608 rows 4285 -> 4225; at 32768 rows 64 rows are 0.5 % ahead.
+// Rows per block of the folding kernels: 64 keeps whole sectors of scales in a warp, 16 (a 32-byte sector of scales) spread a call
+// of fewer than two 64-row blocks per SM over four times as many.  Wide 16-bit tails, which are most of the bytes, want the latter,
+// narrow ones the former (us, folding + GEMM of a long sibling call, 16 / 64 rows: 16384 x 2240 x 2240, 320 16-bit channels, 125.3 / 129.0, 8192 x
+// 3072 x 3072, 384 of them, 120.1 / 126.4, 18432 rows 236.9 / 239.3; 16384 x 1152 x 1152, 64 of them, 50.3 / 48.6, 18000 rows 51.2 / 49.5, 32768 rows
+// 86.5 / 81.4); the line, by rows alone, costs the narrow ones below it 1.7 us.
 static bool fold_small_blocks(int64_t ld_rec) { return ld_rec / 64 < 2 * (int64_t)num_sms(); }
 
 int launch_fold_act_scales(const __nv_bfloat16* s, const __nv_bfloat16* z, int n_chunks, int64_t M, int64_t ldm,

@@ -290,13 +290,13 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, uint
       ::"r"(dst), "l"(tmap), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
-// TMA store smem -> global (box clipped at the tensor's edges); completion is tracked per thread in bulk groups
 // 32 bytes (a whole sector) in one store; p 32-byte aligned
 __device__ __forceinline__ void st_global_32(void* p, uint4 a, uint4 b) {
   asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y),
                "r"(b.z), "r"(b.w)
                : "memory");
 }
+// TMA store smem -> global (box clipped at the tensor's edges); completion is tracked per thread in bulk groups
 __device__ __forceinline__ void tma_store_2d(const void* tmap, uint32_t src, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
                ::"l"(tmap), "r"(src), "r"(x), "r"(y)
